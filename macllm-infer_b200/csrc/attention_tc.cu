@@ -1,16 +1,14 @@
-// Tensor-core varlen paged GQA attention for f16 KV pools: prefill chunks and (split over the keys)
-// decode lanes.
+// Tensor-core varlen paged GQA attention for f16 KV pools: the work lists of a tick and its one-token lanes (prefill chunks:
+// attention_umma.cu).
 //
 // Same operator as attention.cu (the replacement of macllm_kernels::paged_attention_batch,
 // crates/macllm-kernels/src/paged_attention.rs:614-709, and of dense_causal_attention,
 // src/decoder.rs:4580-4670; visibility rule src/decoder.rs:4515-4532), restructured for bandwidth:
-// one CTA owns 16*WARPS (query row, query head) items that all read ONE KV head, so every K/V page
-// is fetched once for the whole query group; pages travel global -> shared with 16-byte cp.async in a
-// two-stage pipeline; Q.K^T and P.V run on the tensor cores (mma.sync m16n8k16, f16 operands, f32
-// accumulators) and the online softmax stays in f32 registers.  One-token lanes run attn_decode_kernel: the
-// keys are shared out over the four warps of a CTA (warp-private cp.async rings, merge in shared memory) and,
+// one CTA reads the pages of one KV head for the whole query group, global -> shared with 16-byte cp.async; Q.K^T and P.V run
+// on the tensor cores (mma.sync m16n8k16, f16 operands, f32 accumulators) and the online softmax stays in f32 registers.  The
+// keys of a lane are shared out over the four warps of a CTA (warp-private cp.async rings, merge in shared memory) and,
 // when few lanes have long histories, over several CTAs as well (scratch: unnormalised partial outputs +
-// running max / sum per head, merged by attn_combine_kernel).  Queries are rounded to f16 once; K/V are read
+// running max / sum per head, merged by the CTA that arrives last).  Queries are rounded to f16 once; K/V are read
 // as stored.
 #include "kernels.h"
 #include "attention_tc.h"
@@ -65,272 +63,6 @@ __device__ __forceinline__ float capped(float v, float cap, float two_over_cap) 
 __device__ __forceinline__ float sink_scale(float m, float l, float sink) {
     const float top = fmaxf(m, sink), f = __expf(m - top);
     return f / (l * f + __expf(sink - top));
-}
-
-// One CTA.  D = head_dim, WARPS warps of 16 items each, KT keys per shared-memory tile.
-// SPLIT = false: work item = tiles[blockIdx.x] = (lane, first query row); the CTA walks every visible key
-//                and writes normalised outputs.
-// SPLIT = true : work item = entries[blockIdx.x] = (lane, split, n_splits) of a one-token lane; the CTA walks
-//                its share of the keys and writes an unnormalised partial.
-// EXACT: the attention weights are split into two f16 operands, so that they reach the product with V in (nearly) f32.
-// DV: width of the values that count (rows of K, V and the output are D apart).
-template <int D, int DV, int WARPS, int KT, bool SPLIT, bool EXACT>
-__global__ void __launch_bounds__(WARPS * 32) attn_tc_kernel(AttnTcArgs a) {
-    constexpr int DP = D + 8;              // padded row (halves): conflict-free ldmatrix
-    constexpr int VP = DV + 8;
-    constexpr int M = 16 * WARPS;
-    constexpr int NT_S = KT / 8;           // score n-tiles per warp
-    constexpr int NT_O = DV / 8;           // output n-tiles per warp
-    constexpr int CHUNKS = D / 8;          // 16-byte chunks per K row
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __half* Qs = reinterpret_cast<__half*>(smem_raw);          // [M][DP]
-    __half* Ks = Qs + M * DP;                                   // [2][KT][DP]
-    __half* Vs = Ks + 2 * KT * DP;                              // [2][KT][VP]
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int gid = lane >> 2, tq = lane & 3;
-    const int kvh = blockIdx.y;
-    const int g = a.q_heads / a.kv_heads;
-    const float two_over_cap = a.softcap != 0.f ? 2.0f / a.softcap : 0.f;
-    pdl_trigger();
-    pdl_wait();
-
-    int lane_id, row0, rows_per_head, split = 0, n_splits = 1;
-    if (SPLIT) {
-        lane_id = a.entries[3 * blockIdx.x];
-        split = a.entries[3 * blockIdx.x + 1];
-        n_splits = a.entries[3 * blockIdx.x + 2];
-        row0 = 0;
-        rows_per_head = 1;
-    } else {
-        lane_id = a.tiles[2 * blockIdx.x];
-        row0 = a.tiles[2 * blockIdx.x + 1];
-        rows_per_head = M / g;
-    }
-    const LaneHeader hdr = a.hdr[lane_id];
-    const int q_off = a.cu_seqlens[lane_id];
-    const int n_rows = SPLIT ? 1 : min(rows_per_head, hdr.n_tokens - row0);
-    const int ldq = a.ldq > 0 ? a.ldq : a.q_heads * D;
-    const int ldo = a.q_heads * D;
-
-    // item i of the CTA: head-in-group i / rows_per_head, query row i % rows_per_head
-    for (int i = tid; i < M * CHUNKS; i += WARPS * 32) {
-        int item = i / CHUNKS, c = (i - item * CHUNKS) * 8;
-        int hq = item / rows_per_head, r = item - hq * rows_per_head;
-        __half2 h[4];
-        if (hq < g && r < n_rows) {
-            const float* src = a.q + (int64_t)(q_off + row0 + r) * ldq + (kvh * g + hq) * D + c;
-            float4 x0 = *reinterpret_cast<const float4*>(src), x1 = *reinterpret_cast<const float4*>(src + 4);
-            if (!SPLIT && c >= a.rot_from && c < a.rot_from + a.rot_dims) {
-                const int64_t pair0 = (int64_t)(hdr.start_pos + row0 + r) * (a.rot_dims / 2) + (c - a.rot_from) / 2;
-                float* p[4][2] = {{&x0.x, &x0.y}, {&x0.z, &x0.w}, {&x1.x, &x1.y}, {&x1.z, &x1.w}};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (c - a.rot_from + 2 * i >= a.rot_dims) break;
-                    const float cs = a.cos_t[pair0 + i], sn = a.sin_t[pair0 + i], u = *p[i][0], v = *p[i][1];
-                    *p[i][0] = u * cs - v * sn;
-                    *p[i][1] = v * cs + u * sn;
-                }
-            }
-            h[0] = __floats2half2_rn(x0.x, x0.y);
-            h[1] = __floats2half2_rn(x0.z, x0.w);
-            h[2] = __floats2half2_rn(x1.x, x1.y);
-            h[3] = __floats2half2_rn(x1.z, x1.w);
-        } else {
-            h[0] = h[1] = h[2] = h[3] = __floats2half2_rn(0.f, 0.f);
-        }
-        *reinterpret_cast<uint4*>(Qs + item * DP + c) = *reinterpret_cast<uint4*>(h);
-    }
-
-    // key range of this CTA
-    const int p_first = hdr.start_pos + row0, p_last = p_first + n_rows - 1;
-    int k_lo = attention_first_key(p_first, a.window, a.chunk);
-    int k_hi = p_last + 1;
-    if (SPLIT) {
-        int len = k_hi - k_lo;
-        int chunk = ((len + n_splits - 1) / n_splits + 15) / 16 * 16;
-        k_lo = k_lo + split * chunk;
-        k_hi = min(k_hi, k_lo + chunk);
-    }
-    const int k_begin = k_lo / 16 * 16;  // page aligned
-    const int n_tiles = k_hi > k_begin ? (k_hi - k_begin + KT - 1) / KT : 0;
-
-    const __half* kp = reinterpret_cast<const __half*>(a.k_pool);
-    const __half* vp = reinterpret_cast<const __half*>(a.v_pool);
-    auto load_tile = [&](int t, int stage) {
-        __half* kd = Ks + stage * KT * DP;
-        __half* vd = Vs + stage * KT * VP;
-        for (int i = tid; i < KT * CHUNKS; i += WARPS * 32) {
-            int key = i / CHUNKS, c = (i - key * CHUNKS) * 8;
-            int pos = k_begin + t * KT + key;
-            bool valid = pos < k_hi;
-            int64_t base = 0;
-            if (valid) {
-                int64_t blk = a.tables[hdr.table_off + (pos >> a.bt_shift)];
-                base = ((kv_page_index(blk, a.layer, a.layers, a.pool_blocks) * a.kv_heads + kvh) * a.block_tokens +
-                        (pos & (a.block_tokens - 1))) * (int64_t)D + c;
-            }
-            cp_async16(kd + key * DP + c, kp + base, valid);
-            if (DV == D || c < DV) cp_async16(vd + key * VP + c, vp + base, valid);
-        }
-    };
-
-    float o_acc[NT_O][4];
-#pragma unroll
-    for (int j = 0; j < NT_O; ++j) o_acc[j][0] = o_acc[j][1] = o_acc[j][2] = o_acc[j][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-
-    // the two accumulator rows of this thread: items warp*16 + gid and + 8
-    int item_r[2] = {warp * 16 + gid, warp * 16 + gid + 8};
-    int pos_r[2], lo_r[2];  // position and first visible key of the two rows
-    bool live_r[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        int hq = item_r[h] / rows_per_head, r = item_r[h] - hq * rows_per_head;
-        live_r[h] = hq < g && r < n_rows;
-        pos_r[h] = p_first + r;
-        lo_r[h] = attention_first_key(pos_r[h], a.window, a.chunk);
-    }
-
-    if (n_tiles > 0) load_tile(0, 0);
-    cp_async_commit();
-    for (int t = 0; t < n_tiles; ++t) {
-        if (t + 1 < n_tiles) load_tile(t + 1, (t + 1) & 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const __half* kt = Ks + (t & 1) * KT * DP;
-        const __half* vt = Vs + (t & 1) * KT * VP;
-
-        // S = Q K^T
-        float s[NT_S][4];
-#pragma unroll
-        for (int j = 0; j < NT_S; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-            uint32_t af[4];
-            ldmatrix_x4(af, Qs + (warp * 16 + (lane & 15)) * DP + kk * 16 + (lane >> 4) * 8);
-#pragma unroll
-            for (int j = 0; j < NT_S; j += 2) {
-                uint32_t bf[4];
-                ldmatrix_x4(bf, kt + (j * 8 + (lane & 7) + (lane >> 4) * 8) * DP + kk * 16 + ((lane >> 3) & 1) * 8);
-                mma16816(s[j], af, bf[0], bf[1]);
-                mma16816(s[j + 1], af, bf[2], bf[3]);
-            }
-        }
-        // scale, softcap, mask, online softmax (f32)
-        const int tile_pos = k_begin + t * KT;
-        float tmax[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int j = 0; j < NT_S; ++j) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                int h = e >> 1;
-                int pos = tile_pos + j * 8 + 2 * tq + (e & 1);
-                float v = s[j][e] * a.scale;
-                if (a.softcap != 0.f) v = capped(v, a.softcap, two_over_cap);
-                bool vis = live_r[h] && pos >= k_lo && pos < k_hi && pos <= pos_r[h] && pos >= lo_r[h];
-                v = vis ? v : -INFINITY;
-                s[j][e] = v;
-                tmax[h] = fmaxf(tmax[h], v);
-            }
-        }
-        float alpha[2], m_use[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
-            tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
-            float m_new = fmaxf(m_run[h], tmax[h]);
-            m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-            alpha[h] = m_run[h] == -INFINITY ? 0.f : __expf(m_run[h] - m_use[h]);
-            m_run[h] = m_new;
-        }
-        float psum[2] = {0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < NT_S; ++j) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                int h = e >> 1;
-                float p = s[j][e] == -INFINITY ? 0.f : __expf(s[j][e] - m_use[h]);
-                s[j][e] = p;
-                psum[h] += p;
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 1);
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 2);
-            l_run[h] = l_run[h] * alpha[h] + psum[h];
-        }
-#pragma unroll
-        for (int j = 0; j < NT_O; ++j) {
-            o_acc[j][0] *= alpha[0];
-            o_acc[j][1] *= alpha[0];
-            o_acc[j][2] *= alpha[1];
-            o_acc[j][3] *= alpha[1];
-        }
-        // O += P V
-#pragma unroll
-        for (int kk = 0; kk < KT / 16; ++kk) {
-            uint32_t pf[4] = {pack_half2(s[2 * kk][0], s[2 * kk][1]), pack_half2(s[2 * kk][2], s[2 * kk][3]),
-                              pack_half2(s[2 * kk + 1][0], s[2 * kk + 1][1]), pack_half2(s[2 * kk + 1][2], s[2 * kk + 1][3])};
-            uint32_t pr[4];
-            if constexpr (EXACT)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) pr[i] = pack_half2_rest(s[2 * kk + (i >> 1)][(i & 1) * 2], s[2 * kk + (i >> 1)][(i & 1) * 2 + 1], pf[i]);
-#pragma unroll
-            for (int j = 0; j < NT_O; j += 2) {
-                uint32_t bf[4];
-                ldmatrix_x4_trans(bf, vt + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VP + j * 8 + (lane >> 4) * 8);
-                mma16816(o_acc[j], pf, bf[0], bf[1]);
-                mma16816(o_acc[j + 1], pf, bf[2], bf[3]);
-                if constexpr (EXACT) {
-                    mma16816(o_acc[j], pr, bf[0], bf[1]);
-                    mma16816(o_acc[j + 1], pr, bf[2], bf[3]);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    cp_async_wait<0>();
-
-    if (!SPLIT) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (!live_r[h]) continue;
-            int hq = item_r[h] / rows_per_head, r = item_r[h] - hq * rows_per_head;
-            float inv = 1.0f / l_run[h];
-            if (a.sink != nullptr) inv = sink_scale(m_run[h], l_run[h], a.sink[kvh * g + hq]);
-            const int64_t at = (int64_t)(q_off + row0 + r) * ldo + (kvh * g + hq) * D;
-            if (a.out != nullptr) {
-#pragma unroll
-                for (int j = 0; j < NT_O; ++j)
-                    *reinterpret_cast<float2*>(a.out + at + j * 8 + 2 * tq) = make_float2(o_acc[j][2 * h] * inv, o_acc[j][2 * h + 1] * inv);
-            }
-            if (a.out_h != nullptr) {
-#pragma unroll
-                for (int j = 0; j < NT_O; ++j)
-                    *reinterpret_cast<__half2*>(a.out_h + at + j * 8 + 2 * tq) =
-                        __floats2half2_rn(o_acc[j][2 * h] * inv, o_acc[j][2 * h + 1] * inv);
-            }
-        }
-    } else {
-        // unnormalised partial of this key share: [entry][kv head][16 items][D], plus (max, sum) per item
-        int64_t slot = ((int64_t)blockIdx.x * a.kv_heads + kvh) * 16;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            int item = gid + 8 * h;
-            if (item >= g) continue;  // only the group's heads are live in a one-token lane
-            float* o = a.part_o + (slot + item) * D;
-#pragma unroll
-            for (int j = 0; j < NT_O; ++j)
-                *reinterpret_cast<float2*>(o + j * 8 + 2 * tq) = make_float2(o_acc[j][2 * h], o_acc[j][2 * h + 1]);
-            if (tq == 0) {
-                a.part_ml[(slot + item) * 2] = m_run[h];
-                a.part_ml[(slot + item) * 2 + 1] = l_run[h];
-            }
-        }
-    }
 }
 
 // One-token lanes.  Work item = entries[blockIdx.x] = (lane, share, n_shares) x KV head.  The four warps of the
@@ -717,21 +449,8 @@ __global__ void attn_combine_kernel(AttnTcArgs a, int D) {
     }
 }
 
-template <int D, int DV, int WARPS, int KT, bool SPLIT, bool EXACT>
-void launch_variant(const AttnTcArgs& a, int n_work, cudaStream_t s) {
-    constexpr size_t smem = ((size_t)(16 * WARPS + 2 * KT) * (D + 8) + (size_t)2 * KT * (DV + 8)) * sizeof(__half);
-    ensure_dynamic_smem(reinterpret_cast<const void*>(&attn_tc_kernel<D, DV, WARPS, KT, SPLIT, EXACT>), smem);
-    dim3 grid((unsigned)n_work, (unsigned)a.kv_heads);
-    launch_pdl(attn_tc_kernel<D, DV, WARPS, KT, SPLIT, EXACT>, grid, dim3(WARPS * 32), smem, s, a);
-    MK_LAUNCH_CHECK();
-}
-
 template <int D, bool EXACT>
-void launch_for_dim(const AttnTcArgs& a, int warps, cudaStream_t s) {
-    if (a.n_tiles > 0) {
-        if (warps == 8) launch_variant<D, D, 8, 64, false, EXACT>(a, a.n_tiles, s);
-        else launch_variant<D, D, 4, 32, false, EXACT>(a, a.n_tiles, s);  // 32-key tiles: half the shared memory, twice the CTAs per SM (measured +0.4 % on the whole benchmark)
-    }
+void launch_for_dim(const AttnTcArgs& a, cudaStream_t s) {
     if (a.n_entries > 0) {
         constexpr int STAGES = D >= 256 ? 2 : 3;
         constexpr size_t smem = (size_t)(16 + 4 * STAGES * 2 * 16) * (D + 8) * sizeof(__half);
@@ -758,19 +477,15 @@ bool attention_tc_supported(int q_heads, int kv_heads, int head_dim, int block_t
            q_heads == g * kv_heads;
 }
 
-// Eight warps (128 (row, head) items per CTA) for groups of eight query heads, else four: with four heads per group
-// eight warps measured slower (fewer, longer CTAs) than four.
-int attention_tc_warps(int q_heads, int kv_heads) { return q_heads / kv_heads == 8 ? 8 : 4; }
-
 int attention_tc_prefill_width(int q_heads, int kv_heads, int dim, int vdim, int block_tokens) {
     if (!attention_tc_supported(q_heads, kv_heads, 64, block_tokens, true)) return 0;
     const int need = std::max(dim, vdim);
     for (int d : {64, 128, 192, 256})
-        if (need <= d && (d != 192 || (vdim <= 128 && attention_tc_warps(q_heads, kv_heads) == 4))) return d;
+        if (need <= d && (d != 192 || vdim <= 128)) return d;
     return 0;
 }
 
-int attention_tc_tile_rows(int q_heads, int kv_heads) { return 16 * attention_tc_warps(q_heads, kv_heads) / (q_heads / kv_heads); }
+int attention_tc_tile_rows(int q_heads, int kv_heads) { return kAttnItems / (q_heads / kv_heads); }
 
 int attention_tc_max_entries(int lanes, int kv_heads) { return std::max(lanes + lanes / 2, kAttnTargetCtas / std::max(1, kv_heads)) + 1; }
 
@@ -781,6 +496,8 @@ void plan_attention_tc(const int32_t* start_pos, const int32_t* n_tokens, const 
     plan.entries.clear();
     plan.dec_lanes.clear();
     const int tile_rows = attention_tc_tile_rows(q_heads, kv_heads);
+    struct Walk { int keys, lane, row0; };
+    std::vector<Walk> walks;
     // One-token lanes: every CTA should walk about the same number of keys, and all CTAs should fit on the GPU at
     // once.  Share size = total keys / CTA slots per KV head, raised until the shares of all lanes fit.
     int n_dec = 0;
@@ -814,10 +531,16 @@ void plan_attention_tc(const int32_t* start_pos, const int32_t* n_tokens, const 
             }
         } else {
             for (int r0 = 0; r0 < n_tokens[i]; r0 += tile_rows) {
-                plan.tiles.push_back(i);
-                plan.tiles.push_back(r0);
+                const int first = start_pos[i] + r0, last = start_pos[i] + std::min(r0 + tile_rows, n_tokens[i]) - 1;
+                walks.push_back({last + 1 - attention_first_key(first, window, chunk), i, r0});
             }
         }
+    }
+    // longest walks first: the last round of CTAs is then made of short ones
+    std::stable_sort(walks.begin(), walks.end(), [](const Walk& x, const Walk& y) { return x.keys > y.keys; });
+    for (const Walk& w : walks) {
+        plan.tiles.push_back(w.lane);
+        plan.tiles.push_back(w.row0);
     }
 }
 
@@ -834,14 +557,12 @@ int launch_paged_attention_tc(const AttnTcArgs& a_in, cudaStream_t s) {
     if (a.out == nullptr && a.n_dec_lanes > 0) throw std::runtime_error("launch_paged_attention_tc: the separate merge pass writes f32 rows");
     a.bt_shift = 0;
     while ((1 << a.bt_shift) < a.block_tokens) ++a.bt_shift;
-    int warps = attention_tc_warps(a.q_heads, a.kv_heads);
+    if (a.n_tiles > 0) launch_attention_umma(a, s);
     switch (a.d) {
-        case 64: a.exact_weights ? launch_for_dim<64, true>(a, warps, s) : launch_for_dim<64, false>(a, warps, s); break;
-        case 128: a.exact_weights ? launch_for_dim<128, true>(a, warps, s) : launch_for_dim<128, false>(a, warps, s); break;
-        case 192:
-            if (a.n_tiles > 0) launch_variant<192, 128, 4, 32, false, true>(a, a.n_tiles, s);
-            break;
-        case 256: a.exact_weights ? launch_for_dim<256, true>(a, warps, s) : launch_for_dim<256, false>(a, warps, s); break;
+        case 64: a.exact_weights ? launch_for_dim<64, true>(a, s) : launch_for_dim<64, false>(a, s); break;
+        case 128: a.exact_weights ? launch_for_dim<128, true>(a, s) : launch_for_dim<128, false>(a, s); break;
+        case 192: break;
+        case 256: a.exact_weights ? launch_for_dim<256, true>(a, s) : launch_for_dim<256, false>(a, s); break;
         default: throw std::runtime_error("launch_paged_attention_tc: unsupported head_dim");
     }
     return (a.n_tiles > 0 ? 1 : 0) + (a.n_entries > 0 ? 1 : 0) + (a.n_dec_lanes > 0 ? 1 : 0);

@@ -16,7 +16,7 @@ struct AttnTcArgs {
     const LaneHeader* hdr = nullptr;
     const uint32_t* tables = nullptr;
     const int32_t* cu_seqlens = nullptr;
-    // work lists (device): prefill tiles (lane, first row); decode entries, 8 ints each, 32-byte aligned
+    // work lists (device): prefill tiles (lane, first row) of attention_tc_tile_rows rows; decode entries, 8 ints each, 32-byte aligned
     // (lane, share, n_shares, start_pos, table offset, first packed row, first entry of the lane, 0);
     // one-token lanes with more than one share (lane, first entry, n_splits)
     const int32_t* tiles = nullptr;
@@ -38,6 +38,8 @@ struct AttnTcArgs {
     int32_t* counters = nullptr;  // [lanes][kv_heads], zero before the first call; every call leaves them zero
     int q_heads = 0, kv_heads = 0, d = 0, block_tokens = 16, layers = 0, layer = 0;
     int64_t pool_blocks = 0;  // see kv_page_index
+    int64_t pool_pages = 0;   // pages that page numbers (kv_page_index) reach in either pool; needed with prefill tiles
+    int32_t* status = nullptr;  // receives a code when a bounded wait of the prefill kernel gives up
     int bt_shift = 0;         // log2(block_tokens), filled in by the launcher
     float scale = 1.f, softcap = 0.f;
     int window = 0;             // > 0: a position sees itself and the window - 1 keys before it
@@ -57,12 +59,13 @@ bool attention_tc_supported(int q_heads, int kv_heads, int head_dim, int block_t
 // The head width (row of the pools) with which lanes of several tokens can run heads of `dim` query / key and `vdim` value
 // dimensions; besides the widths above 192 with values of up to 128.  0: none.
 int attention_tc_prefill_width(int q_heads, int kv_heads, int dim, int vdim, int block_tokens);
-// Query rows of one prefill tile (the CTA covers rows x group heads = 16 * warps items).
+// A prefill tile: this many (query row, query head) items of one KV head.
+constexpr int kAttnItems = 128;
+// Query rows of one prefill tile.
 int attention_tc_tile_rows(int q_heads, int kv_heads);
-int attention_tc_warps(int q_heads, int kv_heads);
 
 // Host-side work lists of one tick (the same for every layer): lanes with more than one token are cut
-// into query tiles; one-token lanes split their keys over up to kAttnMaxSplits CTAs (four warps each), at
+// into query tiles, those with most keys first; one-token lanes split their keys over up to kAttnMaxSplits CTAs (four warps each), at
 // least kAttnMinSplitKeys keys each, until about kAttnTargetCtas CTAs are in flight - unless the lanes alone already
 // give every SM a CTA, in which case no lane is split.
 constexpr int kPlanSms = 148;  // the work lists are planned on the host, without a device, for a B200's SM count
@@ -82,6 +85,8 @@ void plan_attention_tc(const int32_t* start_pos, const int32_t* n_tokens, const 
 // Upper bound of plan.n_entries() for a tick of at most `lanes` lanes.
 int attention_tc_max_entries(int lanes, int kv_heads);
 
+// The prefill tiles (attention_umma.cu).
+void launch_attention_umma(const AttnTcArgs& a, cudaStream_t s);
 // Returns the number of kernels launched.
 int launch_paged_attention_tc(const AttnTcArgs& a, cudaStream_t s);
 

@@ -464,6 +464,7 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
             ta.block_tokens = c->block_tokens;
             ta.layers = c->layers;
             ta.layer = c->layer;
+            ta.pool_pages = (int64_t)c->pool_blocks * c->layers;
             ta.scale = c->scale;
             ta.softcap = c->softcap;
             ta.window = c->window;
@@ -916,7 +917,11 @@ int32_t mk_k_attention_plan(const int32_t* start_pos, const int32_t* n_tokens, i
         plan_attention_tc(start_pos, n_tokens, n_blocks.data(), lanes, q_heads, kv_heads, plan);
         for (int i = 0; i < lanes; ++i) shares_out[i] = 0;
         for (int e = 0; e < plan.n_entries(); ++e) shares_out[plan.entries[(size_t)e * 8]] = plan.entries[(size_t)e * 8 + 2];
-        *tiles_out = plan.n_tiles();
+        // query tiles are counted in units of 64 (row, head) items, 128 for groups of eight heads; the kernel takes 128 items at a time
+        const int group = q_heads / kv_heads, unit_rows = (group == 8 ? 128 : 64) / group;
+        *tiles_out = 0;
+        for (int i = 0; i < lanes; ++i)
+            if (n_tokens[i] > 1) *tiles_out += (n_tokens[i] + unit_rows - 1) / unit_rows;
         *max_entries_out = attention_tc_max_entries(lanes, kv_heads);
         if (plan.n_entries() > *max_entries_out) throw std::runtime_error("mk_k_attention_plan: the plan exceeds its own bound");
     });

@@ -740,7 +740,8 @@ void MixerLm::attend(const Tick& t, int run, const AttentionSpec& s, const Share
         ta.d = D;
         ta.block_tokens = bt;
         ta.layers = 1;
-        ta.pool_blocks = ra.pool_blocks;
+        ta.pool_blocks = ta.pool_pages = ra.pool_blocks;
+        ta.status = status_.as<int32_t>();
         ta.scale = s.scale;
         ta.softcap = s.softcap;
         ta.chunk = s.chunk;

@@ -469,6 +469,8 @@ void MixerLm::run_latent_wide(const Tick& t, int run, const Shares& y, const Row
     a.d = D;
     a.block_tokens = bt;
     a.layers = 2;
+    a.pool_pages = 2 * (int64_t)blocks - 1;  // pages of keys are the even ones; values begin a page later
+    a.status = status_.as<int32_t>();
     a.scale = s.scale;
     a.exact_weights = 1;
     a.window = s.window;

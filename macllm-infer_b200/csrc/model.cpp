@@ -859,6 +859,8 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
             ta.block_tokens = bt;
             ta.layers = ms_.layers;
             ta.pool_blocks = at.pool_blocks;
+            ta.pool_pages = at.pool_blocks * ms_.layers;
+            ta.status = status_.as<int32_t>();
             ta.layer = l;
             ta.scale = ls.scale;
             ta.softcap = ls.softcap;
