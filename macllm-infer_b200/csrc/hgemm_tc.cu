@@ -8,10 +8,10 @@
 // y[t][n] = sum_k xh[t][k] * wh[n][k] with f32 accumulation in tensor memory.
 //
 // One persistent CTA per SM, 320 threads in three roles:
-//   warp 0   - one lane issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a 128 x 64 weight
-//              box and a BN x 64 activation box per stage into a ring of shared-memory stages;
+//   warp 0   - one lane issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of 128 x 64 weight
+//              and BN x 64 activation boxes into a ring of shared-memory stages;
 //   warp 1   - one lane issues the MMAs (tcgen05.mma kind::f16, M = 128 weight rows, N = BN tokens,
-//              four K = 16 steps per stage), commits each stage back to the loader, and commits the tile
+//              four K = 16 steps per block of 64), commits each stage back to the loader, and commits the tile
 //              to the epilogue; two accumulators in tensor memory alternate so the next tile's main
 //              loop runs under the previous tile's epilogue;
 //   warps 2-9 - read the accumulator (tcgen05.ld, one lane per weight row, two warps per lane quadrant that take
@@ -19,6 +19,9 @@
 //              token per store instruction).  A tile's main loop is as long as K, its epilogue is not: with short K
 //              it is the epilogue's instructions that count, hence eight warps and whole 32-column groups without
 //              a test per column.
+// Wide calls run in pairs of CTAs (cta_group::2): one 256 x 256 tile, each CTA with its own weight rows and accumulators and half of the
+// activation rows, so that a block of K takes 32 KB into an SM instead of 48 (an SM takes in about 64 bytes per clock, which
+// one CTA's 256-token tile would need all of).  No load is a multicast.
 // Every mbarrier wait is bounded; a wait that gives up records a status word and the role leaves its
 // loop, the other roles run into their own limits, and tensor memory is always released.
 #include "hgemm_tc.h"
@@ -90,6 +93,44 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// The same over the two CTAs of a cluster: A's 256 rows and B's N rows lie half in each, the leader issues for both, and a commit
+// arrives at the barrier's place in both.
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+                 : "memory");
+}
+// A box into this CTA's own shared memory whose bytes count on the leader's barrier.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, int x, int y, uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(leader_bar)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t leader_address(const void* p) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+    return a;
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t leader_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -234,11 +275,17 @@ __device__ __forceinline__ int group_row0(const HgParams& p, int m_tile) {
     return g * p.T;
 }
 
-template <int BN, int STAGES>
+// A stage holds KB blocks of K, all weight boxes in front of the activation boxes.  The issuer's loop takes some 0.2 us for a stage
+// besides its MMAs: with tiles of up to 128 tokens that is more than the MMAs of one block take, hence two blocks a stage (2048 x
+// 11008 at 2048 tokens: 0.30 -> 0.27 us per block), while tiles of 256 do better with twice the stages (0.35 against 0.36 us).
+constexpr int hg_stage_blocks(int bn) { return bn <= 128 ? 2 : 1; }
+template <int BN, int STAGES, bool PAIR>
 struct HgSmem {
-    static constexpr int A_BYTES = HG_BM * HG_BK * 2;   // 16 KiB
-    static constexpr int B_BYTES = BN * HG_BK * 2;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int A_BYTES = HG_BM * HG_BK * 2;   // 16 KiB: a block's weights
+    static constexpr int B_ROWS = PAIR ? BN / 2 : BN;   // activation rows that this CTA loads
+    static constexpr int B_BYTES = B_ROWS * HG_BK * 2;
+    static constexpr int KB = hg_stage_blocks(BN);
+    static constexpr int STAGE_BYTES = KB * (A_BYTES + B_BYTES);
     static constexpr size_t TOTAL = (size_t)STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
@@ -261,12 +308,14 @@ __device__ __forceinline__ float hg_gelu_tanh(float x) {
 }
 
 // GATED: scattered results are multiplied by a gate (MatmulScatter::gate).
-template <int BN, int STAGES, bool GATED>
+// PAIR: two CTAs of a cluster make one 256 x BN tile; each holds half of the weight rows and their accumulators, and half of the
+// activation rows.
+template <int BN, int STAGES, bool GATED, bool PAIR>
 __global__ void __launch_bounds__(HG_THREADS, 1)
 hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1,
                 const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ HgParams p) {
-    using L = HgSmem<BN, STAGES>;
-    constexpr int LD_COLS = BN >= 32 ? 32 : BN;
+    using L = HgSmem<BN, STAGES, PAIR>;
+    constexpr int LD_COLS = BN >= 32 ? 32 : BN, HG_KB = L::KB;
     extern __shared__ uint8_t hg_smem_raw[];
     __shared__ int32_t first_item[HG_MAX_EXPERTS + 1];  // grouped by expert: items of the experts before
     __shared__ int32_t first_row[HG_MAX_EXPERTS + 1];
@@ -279,8 +328,10 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     __shared__ uint32_t tmem_base_slot;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = PAIR ? (int)cluster_rank() : 0;
+    const int first = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, stride = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
     const int k_blocks = p.K / HG_BK;
-    const int mn_tiles = p.row_tiles * p.n_tiles;
+    const int mn_tiles = (PAIR ? (p.row_tiles + 1) / 2 : p.row_tiles) * p.n_tiles;
     int total_items = mn_tiles * p.splits;
     constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
 
@@ -291,18 +342,22 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], HG_EPI_THREADS);
+            mbar_init(&acc_empty[i], (PAIR ? 2 : 1) * HG_EPI_THREADS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();  // the peer's barriers are there
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_slot;
     // Everything above is private to the CTA.  The weights do not depend on the predecessor kernel either, so
@@ -348,18 +403,18 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     // a few row tiles across every token tile: each weight box comes from HBM once and the activations stay in L2
     auto decode = [&](int item, HgTile& t, int& kb0, int& kb1) {
         if (p.experts > 0) {
-            int e = 0, first = 0, row = 0, n = p.part[1].T;
+            int e = 0, item0 = 0, row = 0, n = p.part[1].T;
             t.part = item < first_item[0] ? 1 : 0;
             if (t.part == 0) {
                 // the last expert whose items begin at or before this one; experts without rows have none
                 for (int step = HG_MAX_EXPERTS; step > 0; step >>= 1)
                     if (e + step < p.experts && first_item[e + step] <= item) e += step;
-                first = first_item[e];
+                item0 = first_item[e];
                 row = first_row[e];
                 n = first_row[e + 1] - row;
             }
             const HgPart& part = p.part[t.part];
-            const int mn = item - first, n_tiles = (n + BN - 1) / BN, m_tile = mn / n_tiles, each = even_tile(n, BN);
+            const int mn = item - item0, n_tiles = (n + BN - 1) / BN, m_tile = mn / n_tiles, each = even_tile(n, BN);
             t.w_row = (e * part.row_tiles + m_tile) * HG_BM;
             t.row0 = m_tile * HG_BM;
             t.x_row = t.tok0 = row + mn % n_tiles * each;
@@ -370,10 +425,10 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             return;
         }
         t.part = 0;
-        const int mn = item % mn_tiles, split = item / mn_tiles, m_tile = mn / p.n_tiles;
+        const int mn = item % mn_tiles, split = item / mn_tiles, m_tile = mn / p.n_tiles * (PAIR ? 2 : 1) + rank;
         t.w_row = t.row0 = m_tile * HG_BM;
         t.tok0 = mn % p.n_tiles * BN;
-        t.x_row = group_row0(p, m_tile) + t.tok0;
+        t.x_row = group_row0(p, m_tile) + t.tok0 + rank * L::B_ROWS;
         t.tok_end = p.T;
         t.rows = p.rows;
         kb0 = split * p.kb_per_split;
@@ -385,18 +440,25 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true, waited = p.experts > 0;
-            int held_x[STAGES], held_y[STAGES];  // activation boxes of the stages filled before the wait
-            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+            int held_kb[STAGES], held_n[STAGES], held_y[STAGES];  // activation boxes of the stages filled before the wait
+            auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int st) {
+                if constexpr (PAIR) tma_load_2d_pair(dst, map, x, y, leader_address(&full[st]));
+                else tma_load_2d(dst, map, x, y, &full[st]);
+            };
+            auto load_x = [&](int st, int kb, int n, int y) {
+                for (int k = 0; k < n; ++k) load(tiles + (size_t)st * L::STAGE_BYTES + HG_KB * L::A_BYTES + k * L::B_BYTES, &tm_x, (kb + k) * HG_BK, y, st);
+            };
+            for (int item = first; item < total_items && ok; item += stride) {
                 HgTile tile;
                 int kb0, kb1;
                 decode(item, tile, kb0, kb1);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                for (int kb = kb0; kb < kb1; kb += HG_KB, ++it) {
                     const uint32_t st = it % STAGES, ph = (it / STAGES) & 1;
+                    const int n = min(HG_KB, kb1 - kb);
                     if (it == STAGES && !waited) {  // the ring is full of weights: now the activations
                         pdl_wait();
                         waited = true;
-                        for (int h = 0; h < STAGES; ++h)
-                            tma_load_2d(tiles + (size_t)h * L::STAGE_BYTES + L::A_BYTES, &tm_x, held_x[h], held_y[h], &full[h]);
+                        for (int h = 0; h < STAGES; ++h) load_x(h, held_kb[h], held_n[h], held_y[h]);
                     }
                     if (!mbar_wait(&empty[st], ph ^ 1, HG_SPIN_LIMIT)) {
                         atomicExch(p.status, 11);
@@ -404,39 +466,45 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         break;
                     }
                     uint8_t* a_dst = tiles + (size_t)st * L::STAGE_BYTES;
-                    uint8_t* b_dst = a_dst + L::A_BYTES;
+                    uint8_t* b_dst = a_dst + HG_KB * L::A_BYTES;
                     if (p.experts > 0) {
                         // as many activation boxes as the tile has rows for
                         const int boxes = (max(tile.tok_end - tile.tok0, 1) + p.box_rows - 1) / p.box_rows;
-                        mbar_expect_tx(&full[st], (uint32_t)(L::A_BYTES + boxes * p.box_rows * HG_BK * 2));
-                        tma_load_2d(a_dst, tile.part == 0 ? &tm_w : &tm_w1, kb * HG_BK, tile.w_row, &full[st]);
-                        for (int b = 0; b < boxes; ++b)
-                            tma_load_2d(b_dst + b * p.box_rows * HG_BK * 2, tile.part == 0 ? &tm_x : &tm_x1, kb * HG_BK, tile.x_row + b * p.box_rows, &full[st]);
+                        mbar_expect_tx(&full[st], (uint32_t)(n * (L::A_BYTES + boxes * p.box_rows * HG_BK * 2)));
+                        for (int k = 0; k < n; ++k) {
+                            tma_load_2d(a_dst + k * L::A_BYTES, tile.part == 0 ? &tm_w : &tm_w1, (kb + k) * HG_BK, tile.w_row, &full[st]);
+                            for (int b = 0; b < boxes; ++b)
+                                tma_load_2d(b_dst + k * L::B_BYTES + b * p.box_rows * HG_BK * 2, tile.part == 0 ? &tm_x : &tm_x1, (kb + k) * HG_BK, tile.x_row + b * p.box_rows, &full[st]);
+                        }
                         continue;
                     }
-                    mbar_expect_tx(&full[st], (uint32_t)L::STAGE_BYTES);
-                    tma_load_2d(a_dst, &tm_w, kb * HG_BK, tile.w_row, &full[st]);
+                    if (rank == 0) mbar_expect_tx(&full[st], (uint32_t)((PAIR ? 2 : 1) * n * (L::A_BYTES + L::B_BYTES)));
+                    for (int k = 0; k < n; ++k) load(a_dst + k * L::A_BYTES, &tm_w, (kb + k) * HG_BK, tile.w_row, (int)st);
                     if (waited) {
-                        tma_load_2d(b_dst, &tm_x, kb * HG_BK, tile.x_row, &full[st]);
+                        load_x((int)st, kb, n, tile.x_row);
                     } else {
-                        held_x[st] = kb * HG_BK;
+                        held_kb[st] = kb;
+                        held_n[st] = n;
                         held_y[st] = tile.x_row;
                     }
                 }
             }
             if (!waited) {  // fewer stages of work than the ring holds
                 pdl_wait();
-                for (uint32_t h = 0; h < it && h < (uint32_t)STAGES; ++h)
-                    tma_load_2d(tiles + (size_t)h * L::STAGE_BYTES + L::A_BYTES, &tm_x, held_x[h], held_y[h], &full[h]);
+                for (uint32_t h = 0; h < it && h < (uint32_t)STAGES; ++h) load_x((int)h, held_kb[h], held_n[h], held_y[h]);
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_wide = (1u << 4) | (p.bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(HG_BM >> 4) << 24);
+        // ---- MMA issuer (the leader's, for both CTAs of a pair)
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc_wide = (1u << 4) | (p.bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)((PAIR ? 2 : 1) * HG_BM >> 4) << 24);
+            auto commit = [&](uint64_t* bar) {
+                if constexpr (PAIR) umma_commit_pair(bar);
+                else umma_commit(bar);
+            };
             uint32_t it = 0, tile_it = 0;
             bool ok = true;
-            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++tile_it) {
+            for (int item = first; item < total_items && ok; item += stride, ++tile_it) {
                 HgTile tile;
                 int kb0, kb1;
                 decode(item, tile, kb0, kb1);
@@ -450,7 +518,7 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 // grouped: no wider than the tile's rows, in steps of 16
                 const uint32_t wide = p.experts > 0 ? (uint32_t)((tile.tok_end - tile.tok0 + 15) & ~15) : (uint32_t)BN;
                 const uint32_t idesc = idesc_wide | ((wide >> 3) << 17);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                for (int kb = kb0; kb < kb1; kb += HG_KB, ++it) {
                     const uint32_t st = it % STAGES, ph = (it / STAGES) & 1;
                     if (!mbar_wait(&full[st], ph, HG_SPIN_LIMIT)) {
                         atomicExch(p.status, 13);
@@ -459,16 +527,19 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a_addr = smem_u32(tiles + (size_t)st * L::STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + L::A_BYTES;
-                    const uint64_t adesc = make_sw128_desc(a_addr), bdesc = make_sw128_desc(b_addr);
+                    const uint64_t adesc = make_sw128_desc(a_addr), bdesc = make_sw128_desc(a_addr + HG_KB * L::A_BYTES);
+                    const int steps = min(HG_KB, kb1 - kb) * (HG_BK / 16);
 #pragma unroll
-                    for (int k = 0; k < HG_BK / 16; ++k) {
+                    for (int k = 0; k < HG_KB * HG_BK / 16; ++k) {
+                        if (k >= HG_BK / 16 && k >= steps) break;
                         // 16 halves = 32 bytes further along K inside the swizzled row: +2 in 16-byte units
-                        umma_f16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        const uint64_t ad = adesc + (uint64_t)((k >> 2) * (L::A_BYTES / 16) + 2 * (k & 3)), bd = bdesc + (uint64_t)((k >> 2) * (L::B_BYTES / 16) + 2 * (k & 3));
+                        if constexpr (PAIR) umma_f16_pair(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        else umma_f16(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    umma_commit(&empty[st]);
+                    commit(&empty[st]);
                 }
-                if (ok) umma_commit(&acc_full[acc]);
+                if (ok) commit(&acc_full[acc]);
             }
         }
     } else {
@@ -478,7 +549,7 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         const bool plain = p.out_scale == 1.0f && p.softcap == 0.f;
         if (GATED || p.part[0].act_post != nullptr) pdl_wait();   // the factors of the rows, or the gates, come from a predecessor
         uint32_t tile_it = 0;
-        for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++tile_it) {
+        for (int item = first; item < total_items; item += stride, ++tile_it) {
             HgTile tile;
             int kb0, kb1;
             decode(item, tile, kb0, kb1);
@@ -604,15 +675,18 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(&acc_empty[acc]);
+            if constexpr (PAIR) mbar_arrive_leader(leader_address(&acc_empty[acc]));
+            else mbar_arrive(&acc_empty[acc]);
         }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();  // the peer is done with this CTA's barriers and shared memory
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -648,19 +722,20 @@ void encode_half_matrix(CUtensorMap* out, const void* base, int64_t n_rows, int6
     if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool PAIR>
 void launch_hg(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tx1, const HgParams& p, int grid, cudaStream_t s) {
-    constexpr size_t smem = HgSmem<BN, STAGES>::TOTAL;
-    auto* kernel = p.scattered != 0 && p.scatter.gate != nullptr ? hgemm_tc_kernel<BN, STAGES, true> : hgemm_tc_kernel<BN, STAGES, false>;
+    constexpr size_t smem = HgSmem<BN, STAGES, PAIR>::TOTAL;
+    auto* kernel = p.scattered != 0 && p.scatter.gate != nullptr ? hgemm_tc_kernel<BN, STAGES, true, PAIR> : hgemm_tc_kernel<BN, STAGES, false, PAIR>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    launch_pdl(kernel, dim3(grid), dim3(HG_THREADS), smem, s, tw, tx, tw1, tx1, p);
+    if (PAIR) launch_pdl_cluster(kernel, 2, dim3(grid), dim3(HG_THREADS), smem, s, tw, tx, tw1, tx1, p);
+    else launch_pdl(kernel, dim3(grid), dim3(HG_THREADS), smem, s, tw, tx, tw1, tx1, p);
     MK_LAUNCH_CHECK();
 }
 
 void launch_hg_width(int bn, const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tx1, const HgParams& p, int grid, cudaStream_t s) {
-    if (bn == 256) launch_hg<256, 4>(tw, tx, tw1, tx1, p, grid, s);
-    else if (bn == 128) launch_hg<128, 6>(tw, tx, tw1, tx1, p, grid, s);
-    else launch_hg<64, 8>(tw, tx, tw1, tx1, p, grid, s);
+    if (bn == 256) launch_hg<256, 4, false>(tw, tx, tw1, tx1, p, grid, s);
+    else if (bn == 128) launch_hg<128, 3, false>(tw, tx, tw1, tx1, p, grid, s);
+    else launch_hg<64, 4, false>(tw, tx, tw1, tx1, p, grid, s);
 }
 
 }  // namespace
@@ -806,6 +881,30 @@ HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits) {
     return pl;
 }
 
+// Wide calls can go in 256 x 256 tiles of two CTAs instead.  Measured on a B200 with K = 2048 and 11008, microseconds: a pair's tile takes
+// 0.36 per block of K and 1.2 besides, a CTA's 128 x 128 tile 0.27 and 0.8, its 128 x 256 tile 0.41 and 1.2; K shares cost their partial
+// sums twice at about 5 TB/s.  Fewest rounds of CTAs times tile time wins (22016 x 2048 at 2048 tokens: 152 -> 127 us, 8192 x 2048: 89 -> 58).
+bool hgemm_tc_pairs(int64_t rows, int64_t cols, int T, int max_splits, const HgemmPlan& single, HgemmPlan& pairs) {
+    if (T <= 128 || rows <= HG_BM) return false;
+    const int64_t kb = cols / HG_BK, row_tiles = (rows + HG_BM - 1) / HG_BM, n_tiles = (T + 255) / 256, tiles = (row_tiles + 1) / 2 * n_tiles;
+    auto shares_us = [&](int s) { return s > 1 ? 8.0 * s * T * (double)rows / 5e6 : 0.0; };
+    auto rounds = [](int64_t items, int64_t at_once) { return (double)((items + at_once - 1) / at_once); };
+    double best = rounds((int64_t)single.row_tiles * single.n_tiles * single.splits, 148) *
+                      ((single.bn == 256 ? 0.41 : 0.27) * single.kb_per_split + (single.bn == 256 ? 1.2 : 0.8)) + shares_us(single.splits);
+    bool better = false;
+    for (int s = 1; s <= std::max(1, std::min(max_splits, 16)); ++s) {
+        const int64_t per = (kb + s - 1) / s;
+        if (s > 1 && (per < 4 || (size_t)s * T * rows * 4 > ((size_t)16 << 20))) break;
+        if ((kb + per - 1) / per != s) continue;
+        const double us = rounds(tiles * s, 74) * (0.36 * (double)per + 1.2) + shares_us(s);
+        if (us >= best) continue;
+        best = us;
+        better = true;
+        pairs = HgemmPlan{256, (int)row_tiles, (int)n_tiles, s, (int)per, s > 1 ? (size_t)s * T * rows : 0};
+    }
+    return better;
+}
+
 namespace {
 int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int ldy, float out_scale, float softcap,
                      const HgemmScratch& ws, cudaStream_t s, int max_splits, const GatedAct* act, __half* yh, int ldyh,
@@ -887,6 +986,15 @@ void launch_hgemm_tc_experts(const ExpertRows& experts, const ExpertRows* every,
 }
 
 namespace {
+// No pair of row tiles belongs to two stacked projections with inputs of their own.
+bool whole_pairs(const HalfWeight& W) {
+    if (W.n_groups == 1) return true;
+    if (W.group_tiles > 0) return W.group_tiles % 2 == 0;
+    for (int g = 0; g < W.n_groups; ++g)
+        if (W.group_end[g] % 2 != 0) return false;
+    return true;
+}
+
 int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int ldy, float out_scale, float softcap,
                      const HgemmScratch& ws, cudaStream_t s, int max_splits, const GatedAct* act, __half* yh, int ldyh,
                      const MatmulScatter* scatter) {
@@ -894,13 +1002,15 @@ int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int
     if (!W.ready) throw std::runtime_error("launch_hgemm_tc: the f16 image of the matrix was not built");
     if (xh == nullptr) throw std::runtime_error("launch_hgemm_tc: f16 activations missing");
     if (out_scale != 1.0f || softcap != 0.f || ws.partial == nullptr) max_splits = 1;
-    HgemmPlan pl = hgemm_tc_plan(W.rows, W.cols, T, max_splits);
+    HgemmPlan pl = hgemm_tc_plan(W.rows, W.cols, T, max_splits), pairs;
+    const bool pair = whole_pairs(W) && hgemm_tc_pairs(W.rows, W.cols, T, max_splits, pl, pairs);
+    if (pair) pl = pairs;
     if (pl.splits > 1 && pl.partial_floats > ws.partial_floats) {
         pl.splits = 1;
         pl.kb_per_split = (int)(W.cols / HG_BK);
     }
     alignas(64) CUtensorMap tx;
-    encode_half_matrix(&tx, xh, (int64_t)T * W.n_groups, W.cols, pl.bn, W.bf16);
+    encode_half_matrix(&tx, xh, (int64_t)T * W.n_groups, W.cols, pair ? pl.bn / 2 : pl.bn, W.bf16);
     HgParams p{};
     p.T = T;
     p.K = (int)W.cols;
@@ -929,8 +1039,13 @@ int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int
     p.group_tiles = W.group_tiles;
     p.scattered = scatter != nullptr ? 1 : 0;
     if (scatter != nullptr) p.scatter = *scatter;
-    const int grid = std::min(device_sm_count(), p.row_tiles * p.n_tiles * p.splits);
     const CUtensorMap& tw = *reinterpret_cast<const CUtensorMap*>(W.tmap);
+    if (pair) {
+        const int grid = 2 * std::min(device_sm_count() / 2, (p.row_tiles + 1) / 2 * p.n_tiles * p.splits);
+        launch_hg<256, 6, true>(tw, tx, tw, tx, p, grid, s);
+        return pl.splits;
+    }
+    const int grid = std::min(device_sm_count(), p.row_tiles * p.n_tiles * p.splits);
     launch_hg_width(pl.bn, tw, tx, tw, tx, p, grid, s);
     return pl.splits;
 }

@@ -36,7 +36,7 @@ void build_bf16_weight(const float* values, int64_t rows, int64_t cols, HalfWeig
 // The same with `groups` stacked projections of rows / groups rows each (a multiple of 128), every one with an input of its own.
 void build_bf16_weight_groups(const float* values, int64_t rows, int64_t cols, int groups, HalfWeight& out, cudaStream_t s);
 
-// How a call is cut into work items (see hgemm_tc.cu); partial_floats is the scratch a split call needs.
+// How a call is cut into work items of one CTA each (see hgemm_tc.cu; wide calls may run in tiles of two CTAs instead); partial_floats is the scratch a split call needs.
 struct HgemmPlan {
     int bn = 0, row_tiles = 0, n_tiles = 0, splits = 1, kb_per_split = 0;
     size_t partial_floats = 0;
