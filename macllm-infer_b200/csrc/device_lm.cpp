@@ -29,7 +29,7 @@ void DeviceLm::open_device() {
     MK_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     MK_CUDA(cudaEventCreate(&ev_start_));
     MK_CUDA(cudaEventCreate(&ev_stop_));
-    status_.alloc(4);
+    status_.alloc((size_t)(2 + cfg_.max_batch_lanes) * 4);
     status_.zero(stream_);
 }
 
@@ -43,14 +43,11 @@ void DeviceLm::alloc_tick(size_t extra_stage_bytes) {
     tile_lane_.alloc((size_t)(T + B) * 4);
     tile_row_.alloc((size_t)(T + B) * 4);
     ntiles_.alloc(4);
-    err_.alloc(4);
-    err_.zero(stream_);
     logits_.alloc((size_t)B * spec_.vocab * 4);
-    tokens_.alloc((size_t)B * 4);
     argmax_scratch_.alloc(argmax_scratch_bytes(B));
     argmax_scratch_.zero(stream_);
     const size_t bytes = (size_t)B * sizeof(LaneHeader) + (size_t)(pool_->max_blocks() + B) * 4 + (size_t)T * 8 + 128 +
-                         (size_t)B * sizeof(LaneSampling) + extra_stage_bytes;
+                         (size_t)B * (sizeof(LaneSampling) + sizeof(CowCopy)) + 16 + extra_stage_bytes;
     stage_host_.ensure(bytes);
     stage_dev_.alloc(bytes);
     out_host_.ensure((size_t)B * spec_.vocab * 4 + (size_t)B * 4 + 16);
@@ -116,6 +113,14 @@ DeviceLm::Tick DeviceLm::stage_tick(const std::vector<LmLane>& lanes, KvReservat
         }
         t.off_sampling = stage_bytes(t, sp.data(), sp.size() * sizeof(LaneSampling));
     }
+    // copy-on-write page copies of shared partial tails, one per lane at most
+    if (!r.cow_copies().empty()) {
+        std::vector<CowCopy> cows;
+        for (const KvCowCopy& c : r.cow_copies())
+            if (c.rows > 0) cows.push_back(CowCopy{c.src_slot, c.dst_slot, c.rows});
+        t.n_cows = (int)cows.size();
+        t.off_cows = stage_bytes(t, cows.data(), cows.size() * sizeof(CowCopy));
+    }
     // room for the results
     if (flags & FWD_WANT_LOGITS) {
         logits_.ensure((size_t)t.R * spec_.vocab * 4);
@@ -137,6 +142,7 @@ void DeviceLm::upload_tick(Tick& t, int q_tile, int prof_class) {
     MK_CUDA(cudaEventRecord(ev_start_, stream_));
     MK_CUDA(cudaMemcpyAsync(stage_dev_.ptr(), t.hp, t.bytes, cudaMemcpyHostToDevice, stream_));
     h2d_bytes_ += (int64_t)t.bytes;
+    if (t.n_cows > 0) copy_shared_pages(t);
     int tiles = 0;
     for (int i = 0; i < t.B; ++i) tiles += (t.hdr[i].n_tokens + q_tile - 1) / q_tile;
     BatchDesc& bd = t.bd;
@@ -153,7 +159,7 @@ void DeviceLm::upload_tick(Tick& t, int q_tile, int prof_class) {
     bd.tile_lane = tile_lane_.as<int32_t>();
     bd.tile_row0 = tile_row_.as<int32_t>();
     bd.n_tiles = ntiles_.as<int32_t>();
-    bd.error_flag = err_.as<int32_t>();
+    bd.error_flag = error_word();
     prof_begin(prof_class, 0, 0);
     launch_build_batch(bd, pool_->block_tokens(), q_tile, stream_);
     prof_end();
@@ -167,10 +173,10 @@ void DeviceLm::finish_tick(const Tick& t, int prof_class) {
     if (t.flags & FWD_WANT_TOKENS) {
         prof_begin(prof_class, 4.0 * B * spec_.vocab, 0);
         if (t.off_sampling != 0)
-            launch_sample(logits_.as<float>(), B, spec_.vocab, reinterpret_cast<const LaneSampling*>(t.dp + t.off_sampling), tokens_.as<uint32_t>(),
+            launch_sample(logits_.as<float>(), B, spec_.vocab, reinterpret_cast<const LaneSampling*>(t.dp + t.off_sampling), token_words(),
                           status_.as<int32_t>(), stream_);
         else
-            launch_argmax(logits_.as<float>(), B, spec_.vocab, tokens_.as<uint32_t>(), argmax_scratch_.ptr(), stream_);
+            launch_argmax(logits_.as<float>(), B, spec_.vocab, token_words(), argmax_scratch_.ptr(), stream_);
         prof_end();
         ++launches_;
     }
@@ -178,9 +184,8 @@ void DeviceLm::finish_tick(const Tick& t, int prof_class) {
     uint8_t* oh = out_host_.as<uint8_t>();
     const size_t tok_off = (size_t)((t.flags & FWD_WANT_LOGITS) ? t.R : 0) * spec_.vocab * 4;
     if (tok_off) MK_CUDA(cudaMemcpyAsync(oh, logits_.ptr(), tok_off, cudaMemcpyDeviceToHost, stream_));
-    if (t.flags & FWD_WANT_TOKENS) MK_CUDA(cudaMemcpyAsync(oh + tok_off, tokens_.ptr(), (size_t)B * 4, cudaMemcpyDeviceToHost, stream_));
-    MK_CUDA(cudaMemcpyAsync(oh + tok_off + (size_t)B * 4, err_.ptr(), 4, cudaMemcpyDeviceToHost, stream_));
-    MK_CUDA(cudaMemcpyAsync(oh + tok_off + (size_t)B * 4 + 4, status_.ptr(), 4, cudaMemcpyDeviceToHost, stream_));
+    // the status word, the descriptor's error word and the tokens in one copy
+    MK_CUDA(cudaMemcpyAsync(oh + tok_off, status_.ptr(), 8 + ((t.flags & FWD_WANT_TOKENS) ? (size_t)B * 4 : 0), cudaMemcpyDeviceToHost, stream_));
     d2h_bytes_ += 8 + (int64_t)tok_off + ((t.flags & FWD_WANT_TOKENS) ? (int64_t)B * 4 : 0);
     MK_CUDA(cudaEventRecord(ev_stop_, stream_));
     timed_ = true;
@@ -201,12 +206,12 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     const uint8_t* oh = out_host_.as<uint8_t>();
     const size_t tok_off = (size_t)((out_flags_ & FWD_WANT_LOGITS) ? out_rows_ : 0) * spec_.vocab * 4;
     int32_t flags[2];
-    memcpy(flags, oh + tok_off + (size_t)out_lanes_ * 4, 8);
-    if (flags[0] != 0) throw std::runtime_error("batch descriptor index out of range on the device (flag " + std::to_string(flags[0]) + ")");
-    if (flags[1] != 0) {
+    memcpy(flags, oh + tok_off, 8);
+    if (flags[1] != 0) throw std::runtime_error("batch descriptor index out of range on the device (flag " + std::to_string(flags[1]) + ")");
+    if (flags[0] != 0) {
         // the status word is sticky on the device: clear it so that the next forward starts clean
         cudaMemsetAsync(status_.ptr(), 0, 4, stream_);
-        throw std::runtime_error(status_message(flags[1]));
+        throw std::runtime_error(status_message(flags[0]));
     }
     if (logits) {
         if (!(out_flags_ & FWD_WANT_LOGITS)) throw std::runtime_error("logits were not requested for this forward");
@@ -214,7 +219,7 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     }
     if (tokens) {
         if (!(out_flags_ & FWD_WANT_TOKENS)) throw std::runtime_error("tokens were not requested for this forward");
-        memcpy(tokens, oh + tok_off, (size_t)out_lanes_ * 4);
+        memcpy(tokens, oh + tok_off + 8, (size_t)out_lanes_ * 4);
     }
 }
 

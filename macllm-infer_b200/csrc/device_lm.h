@@ -36,7 +36,9 @@ protected:
         uint8_t* dp = nullptr;    // its device copy
         size_t bytes = 0;         // staged so far
         const LaneHeader* hdr = nullptr;  // host copy
-        size_t off_tables = 0, off_ids = 0, off_rows = 0, off_sampling = 0;
+        size_t off_tables = 0, off_ids = 0, off_rows = 0, off_sampling = 0, off_cows = 0;
+        int n_cows = 0;           // copy-on-write page copies
+        const CowCopy* cows() const { return reinterpret_cast<const CowCopy*>(dp + off_cows); }  // device, after upload_tick
         BatchDesc bd;
         const uint32_t* ids = nullptr;          // device, after upload_tick
         const int32_t* out_rows = nullptr;      // device: packed index of every row projected to logits [R]
@@ -46,6 +48,9 @@ protected:
     size_t stage_bytes(Tick& t, const void* src, size_t bytes);
     // Starts the tick's clock, copies the staging buffer and expands the batch descriptor.
     void upload_tick(Tick& t, int q_tile, int prof_class);
+    // Copy-on-write page copies of shared partial tails (cache.rs:3042-3089): ahead of the descriptor's launch, which waits for them like for any
+    // ordinary predecessor, so that kernels which read history before they wait for theirs find it complete.
+    virtual void copy_shared_pages(const Tick& t) = 0;
     // Selects tokens from logits_ (FWD_WANT_TOKENS) and sends the results to pinned memory.
     void finish_tick(const Tick& t, int prof_class);
     void fetch_output(float* logits, uint32_t* tokens) override;
@@ -60,9 +65,12 @@ protected:
     cudaStream_t stream_ = nullptr;
     int64_t launches_ = 0, h2d_bytes_ = 0, d2h_bytes_ = 0;
     bool profiling_ = false;
-    DevBuf cu_, pos_, tok_lane_, slots_, last_, tile_lane_, tile_row_, ntiles_, err_;
-    DevBuf logits_, tokens_;
-    DevBuf status_;  // one word: non-zero when a bounded wait or a device-side check gave up
+    DevBuf cu_, pos_, tok_lane_, slots_, last_, tile_lane_, tile_row_, ntiles_;
+    DevBuf logits_;
+    // first word: non-zero when a bounded wait or a device-side check gave up; then the batch descriptor's error word and a token per lane
+    DevBuf status_;
+    int32_t* error_word() const { return status_.as<int32_t>() + 1; }
+    uint32_t* token_words() const { return status_.as<uint32_t>() + 2; }
 
 private:
     void prof_resolve();

@@ -20,6 +20,7 @@ __device__ __forceinline__ void q4k_scale_min(const uint8_t* s, int j, int& sc, 
 }
 
 __global__ void embed_kernel(QWeight W, const uint32_t* ids, float scale, float* out) {
+    pdl_trigger();
     int t = blockIdx.x;
     int64_t row = ids[t];
     int cols = (int)W.cols;
@@ -62,13 +63,15 @@ __global__ void embed_kernel(QWeight W, const uint32_t* ids, float scale, float*
         }
         o[k] = scale == 1.0f ? v : __fmul_rn(v, scale);
     }
+    pdl_wait();  // the ids were staged before the predecessor began, which writes nothing that is read here; who waits for this kernel waits for both
 }
 
 }  // namespace
 
 void launch_embed(const QWeight& W, const uint32_t* ids, int T, float scale, float* out, cudaStream_t s) {
     if (T <= 0) return;
-    embed_kernel<<<T, 256, 0, s>>>(W, ids, scale, out);
+    // few rows: more threads share a row, whose latency then counts
+    launch_pdl(embed_kernel, dim3((unsigned)T), dim3(T <= 148 ? 1024 : 256), 0, s, W, ids, scale, out);
     MK_LAUNCH_CHECK();
 }
 

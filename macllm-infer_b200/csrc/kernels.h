@@ -115,9 +115,14 @@ void launch_rope_kv(const RopeKvArgs& a, cudaStream_t s);
 // The same for projections with biases whose query and key norms run over all heads at once (q_out required).
 void launch_rope_kv_rows(const RopeKvArgs& a, cudaStream_t s);
 
-// Copy `rows` token rows of every layer and head from block src to block dst (copy-on-write).
-void launch_cow_copy(void* k_pool, void* v_pool, int kv_f16, int64_t src_block, int64_t dst_block, int rows,
-                     int layers, int64_t pool_blocks, int kv_heads, int block_tokens, int d, cudaStream_t s);
+// Copy the first `rows` token rows of every layer and head from block src to block dst (copy-on-write); `copies` is on the device, and
+// no copy's source is another one's destination.
+struct CowCopy {
+    uint32_t src, dst;
+    int32_t rows;
+};
+void launch_cow_copies(void* k_pool, void* v_pool, int kv_f16, const CowCopy* copies, int n_copies, int layers, int64_t pool_blocks, int kv_heads, int block_tokens, int d,
+                       cudaStream_t s);
 
 // ---- attention ---------------------------------------------------------------------------------
 struct AttnArgs {

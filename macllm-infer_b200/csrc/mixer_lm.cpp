@@ -876,6 +876,18 @@ void MixerLm::run_parallel(const Tick& t, int run, Pending& pend, const std::vec
     pend.coef = 0.5f;
 }
 
+void MixerLm::copy_shared_pages(const Tick& t) {
+    for (size_t i = 0; i < rs_.size(); ++i) {
+        RunState& st = rs_[i];
+        const int l = runs_[i].layer;
+        if (st.k_pool.size() == 0) continue;
+        const bool latent = st.v_pool.size() == 0;  // one pool: both arguments name it
+        launch_cow_copies(st.k_pool.ptr(), latent ? st.k_pool.ptr() : st.v_pool.ptr(), cfg_.kv_f16 ? 1 : 0, t.cows(), t.n_cows, 1, pool_->max_blocks(),
+                          latent ? 1 : ms_.layers[(size_t)l].attn.kv_heads, cfg_.block_tokens, lw_[(size_t)l].row_width, stream_);
+        ++launches_;
+    }
+}
+
 void MixerLm::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint32_t flags) {
     Tick t = stage_tick(lanes, r, flags);
     const int B = t.B, T = t.T, R = t.R, C = ms_.width;
@@ -921,17 +933,6 @@ void MixerLm::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, ui
     state_lanes_.lane = reinterpret_cast<const StateLane*>(t.dp + off_halves);
     state_lanes_.lanes = B;
     for (LaneSet* s : {&delta_one_, &delta_rows_, &delta_chunks_}) s->lanes.lane = reinterpret_cast<const StateLane*>(t.dp + s->off);
-    // copy-on-write page copies of shared partial tails
-    for (const KvCowCopy& c : r.cow_copies())
-        for (size_t i = 0; i < rs_.size(); ++i) {
-            RunState& st = rs_[i];
-            const int l = runs_[i].layer;
-            if (st.k_pool.size() == 0) continue;
-            const bool latent = st.v_pool.size() == 0;  // one pool: both arguments name it
-            launch_cow_copy(st.k_pool.ptr(), latent ? st.k_pool.ptr() : st.v_pool.ptr(), cfg_.kv_f16 ? 1 : 0, c.src_slot, c.dst_slot, c.rows, 1,
-                            pool_->max_blocks(), latent ? 1 : ms_.layers[(size_t)l].attn.kv_heads, cfg_.block_tokens, lw_[(size_t)l].row_width, stream_);
-            ++launches_;
-        }
     cur_ = 0;
     if (moe_.counts > 0) {  // whatever a forward that failed half-way left of its counts
         MK_CUDA(cudaMemsetAsync(moe_.count, 0, (size_t)moe_.counts * 2 * 4, stream_));

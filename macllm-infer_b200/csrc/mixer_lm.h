@@ -29,6 +29,7 @@ public:
 
 protected:
     void run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint32_t flags) override;
+    void copy_shared_pages(const Tick& t) override;
     void copy_state(int from, int to) override;
 
 private:

@@ -616,6 +616,12 @@ int Model::matmul_stream(const QStreamWeight& W, const ActQ& x, int T, float* y,
 
 static int act_kind_of(const QWeight& w) { return w.type == QT_Q8_0 ? ACT_Q80 : ACT_Q8K; }
 
+void Model::copy_shared_pages(const Tick& t) {
+    launch_cow_copies(k_pool_.ptr(), v_pool_.ptr(), cfg_.kv_f16 ? 1 : 0, t.cows(), t.n_cows, ms_.layers, pool_->max_blocks(), ms_.kv_heads, pool_->block_tokens(),
+                      ms_.head_dim, stream_);
+    ++launches_;
+}
+
 void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint32_t flags) {
     Tick tick = stage_tick(lanes, r, flags);
     const int B = tick.B, T = tick.T, R = tick.R;
@@ -650,13 +656,6 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
     const uint8_t* dp = tick.dp;
     const BatchDesc& bd = tick.bd;
     const uint32_t* ids_dev = tick.ids;
-
-    // ---- copy-on-write page copies of shared partial tails (cache.rs:3042-3089)
-    for (const KvCowCopy& c : r.cow_copies()) {
-        launch_cow_copy(k_pool_.ptr(), v_pool_.ptr(), cfg_.kv_f16 ? 1 : 0, c.src_slot, c.dst_slot, c.rows, ms_.layers, pool_->max_blocks(), ms_.kv_heads, bt,
-                        d, stream_);
-        ++launches_;
-    }
 
     // ---- embedding (src/decoder.rs:3194-3197)
     prof_begin(KC_EMBED, 4.0 * T * H, 0);

@@ -62,6 +62,7 @@ public:
 
 protected:
     void run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint32_t flags) override;
+    void copy_shared_pages(const Tick& t) override;
     std::string status_message(int32_t status) const override;
 
 private:
