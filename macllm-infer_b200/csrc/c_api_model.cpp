@@ -2,6 +2,7 @@
 // prefix-cache handles.
 #include "../../include/macllm_b200.h"
 #include "c_api_util.h"
+#include "device_util.h"
 #include "engine.h"
 #include "mixer_spec.h"
 #include "model_registry.h"
@@ -545,7 +546,7 @@ int32_t mk_engine_logits(mk_engine* e, int32_t request_id, float* out, int32_t* 
     return guarded([&] {
         const EngineResult& r = e->e->result(request_id);
         // rows are vocab wide; the caller sizes the buffer from the token count
-        if (out != nullptr) memcpy(out, r.logits.data(), r.logits.size() * 4);
+        if (out != nullptr) copy_wide(out, r.logits.data(), r.logits.size() * 4);
         *n_rows = r.logit_rows;
     });
 }

@@ -215,7 +215,7 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     }
     if (logits) {
         if (!(out_flags_ & FWD_WANT_LOGITS)) throw std::runtime_error("logits were not requested for this forward");
-        memcpy(logits, oh, tok_off);
+        copy_wide(logits, oh, tok_off);
     }
     if (tokens) {
         if (!(out_flags_ & FWD_WANT_TOKENS)) throw std::runtime_error("tokens were not requested for this forward");

@@ -54,6 +54,7 @@ protected:
     // Selects tokens from logits_ (FWD_WANT_TOKENS) and sends the results to pinned memory.
     void finish_tick(const Tick& t, int prof_class);
     void fetch_output(float* logits, uint32_t* tokens) override;
+    const float* output_rows() const override { return (out_flags_ & FWD_WANT_LOGITS) ? out_host_.as<float>() : nullptr; }
     void device_synchronize() override;
     // Message of a non-zero status word left by a kernel.
     virtual std::string status_message(int32_t status) const;

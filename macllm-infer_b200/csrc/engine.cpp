@@ -311,6 +311,15 @@ static inline uint64_t next_u64(uint64_t& state) {
 // One uniform draw in [0, 1) per sampled token, the same stream whether the token is picked on the host or on the device.
 static inline float next_uniform(uint64_t& state) { return (float)(next_u64(state) >> 40) * (1.0f / 16777216.0f); }
 
+namespace {
+// Appends a row of logits to each result, which has room for it.
+void record_rows(const std::vector<std::pair<EngineResult*, const float*>>& rows, int vocab) {
+    const int n = (int)rows.size();
+#pragma omp parallel for schedule(static) num_threads(std::min(8, n)) if ((size_t)n * (size_t)vocab >= (size_t)1 << 18)
+    for (int i = 0; i < n; ++i) rows[(size_t)i].first->logits.insert(rows[(size_t)i].first->logits.end(), rows[(size_t)i].second, rows[(size_t)i].second + vocab);
+}
+}  // namespace
+
 uint32_t Engine::sample(Sequence& s, float* row) {  // Sampler::sample_with_generated, sampling.rs:95-169
     const int vocab = model_.spec().vocab;
     const EngineRequest& rq = s.req;
@@ -511,8 +520,8 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
         std::vector<LmLane> lanes;
         std::vector<TickLaneTrace> tick;
         // tokens are picked on the device unless some lane needs what only the host sampler has: penalties (they read
-        // the request's history), an unbounded or very wide top-k, or recorded logits
-        bool device_greedy = !cfg_.host_sampling && !cfg_.record_logits;
+        // the request's history), an unbounded or very wide top-k, or draws beside recorded logits
+        bool device_greedy = !cfg_.host_sampling;
         for (int i = 0; i < visits; ++i) {
             const Visit& v = actions[(size_t)i];
             if (v.kind != Visit::Forward) continue;
@@ -522,6 +531,7 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
             const ForwardKind phase = !v.was_prefill ? ForwardKind::Decode : (v.ready_to_sample ? ForwardKind::FirstToken : ForwardKind::SuffixPrefill);
             tick.push_back(TickLaneTrace{s.id, v.start_pos, v.n_tokens, (int32_t)phase});
             const EngineRequest& rq = s.req;
+            if (v.ready_to_sample && cfg_.record_logits && rq.temperature > 0.f) device_greedy = false;
             if (v.ready_to_sample && (std::fabs(rq.repetition_penalty - 1.f) >= 1.1920929e-07f || rq.presence_penalty != 0.f ||
                                       rq.frequency_penalty != 0.f || !model_.device_sampling_covers(rq.temperature, rq.top_k)))
                 device_greedy = false;
@@ -544,7 +554,7 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
                 }
             }
         }
-        uint32_t flags = device_greedy ? FWD_WANT_TOKENS : FWD_WANT_LOGITS;
+        uint32_t flags = (device_greedy ? FWD_WANT_TOKENS : FWD_WANT_LOGITS) | (cfg_.record_logits ? FWD_WANT_LOGITS : 0);
         forward_needs_drain_ = true;  // engine.rs:2294
         model_.forward_batch_reserved(lanes, std::move(reservation), flags);
         // validate every lane's cache length BEFORE sampling (engine.rs:2258-2265)
@@ -554,13 +564,17 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
         // complete_mixed_forward (engine.rs:2378-2409): the completion barrier
         const int vocab = model_.spec().vocab;
         forward_needs_drain_ = false;  // the read-back is the barrier; a failure inside it is not drained again (engine.rs:2388-2391)
-        if (device_greedy) {
-            tokens_host_.resize((size_t)lane_count);
+        const float* rows = nullptr;  // logits; the host sampler's own copy, or where the model left them
+        tokens_host_.resize((size_t)lane_count);
+        if (device_greedy && (!cfg_.record_logits || model_.output_rows() != nullptr)) {
             model_.read_output(nullptr, tokens_host_.data());
+            rows = cfg_.record_logits ? model_.output_rows() : nullptr;
         } else {
             logits_host_.resize((size_t)lane_count * vocab);
-            model_.read_output(logits_host_.data(), nullptr);
+            model_.read_output(logits_host_.data(), device_greedy ? tokens_host_.data() : nullptr);
+            rows = logits_host_.data();
         }
+        std::vector<std::pair<EngineResult*, const float*>> recorded;  // rows to keep, copied together behind the loop over the lanes
         const double tick_ms = model_.last_forward_ms();   // read once: the device time of this packed forward
         stats_.device_ms += tick_ms;
         {   // collect_pending_benchmark_forwards + record_packed_forward (engine.rs:2306-2375,2394-2405,601-619)
@@ -629,16 +643,21 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
                 continue;
             }
             uint32_t token;
+            if (cfg_.record_logits) {
+                EngineResult& r = results_[s.id];
+                const size_t size = r.logits.size() + (size_t)vocab;
+                if (r.logits.capacity() < size) r.logits.reserve(std::max(size + (size_t)vocab * (size_t)std::min(31, s.req.max_new_tokens - s.generated - 1), 2 * r.logits.capacity()));
+                recorded.emplace_back(&r, rows + (size_t)row * vocab);
+                ++r.logit_rows;
+            }
             if (device_greedy) {
                 token = tokens_host_[(size_t)row];
             } else {
-                float* lrow = logits_host_.data() + (size_t)row * vocab;
-                if (cfg_.record_logits) {
-                    EngineResult& r = results_[s.id];
-                    r.logits.insert(r.logits.end(), lrow, lrow + vocab);
-                    ++r.logit_rows;
+                if (cfg_.record_logits) {  // as they came: penalties change the row
+                    record_rows(recorded, vocab);
+                    recorded.clear();
                 }
-                token = sample(s, lrow);
+                token = sample(s, logits_host_.data() + (size_t)row * vocab);
             }
             ++row;
             EngineResult& res = results_[s.id];
@@ -663,6 +682,7 @@ int Engine::drive_once(double now_ms) {  // engine.rs:1938-1964
             s.phase = Phase::Decode;
             s.decode_token = token;
         }
+        record_rows(recorded, vocab);
     } else {
         reservation.reset();
         forward_needs_drain_ = false;

@@ -91,6 +91,8 @@ public:
     // CausalLm::read_output_to_cpu: completion barrier; retired pages become free.  `logits` takes one row per row asked
     // for (see LmLane::logit_rows), lanes in order.
     void read_output(float* logits, uint32_t* tokens);
+    // The rows that read_output would copy, where the model keeps them until its next forward (null: it does not).
+    virtual const float* output_rows() const { return nullptr; }
     // CausalLm::synchronize
     void synchronize();
 

@@ -32,6 +32,11 @@ class Request:
     event_send_timeout_ms: float = 0.0  # how long a full channel is tolerated before the request is given up
 
 
+# mk_lane, as a record of an array
+_LANE = np.dtype([("session", np.uint64), ("input_ids", np.uint64), ("n_tokens", np.int32), ("start_pos", np.int32)])
+assert _LANE.itemsize == C.sizeof(capi.Lane)
+
+
 class Session:
     def __init__(self, model: "Model", _handle=None):
         self.model = model
@@ -215,17 +220,17 @@ class Model:
         return d.as_dict()
 
     def _lanes(self, lanes):
-        """lanes: list of (session, token ids, start_pos).  Returns (ctypes array, keep-alive list)."""
-        arr = (capi.Lane * len(lanes))()
-        keep = []
-        for i, (session, ids, start_pos) in enumerate(lanes):
-            t = np.ascontiguousarray(ids, dtype=np.uint32)
-            keep.append(t)
-            arr[i].session = session._h
-            arr[i].input_ids = t.ctypes.data_as(C.POINTER(C.c_uint32))
-            arr[i].n_tokens = len(t)
-            arr[i].start_pos = start_pos
-        return arr, keep
+        """lanes: list of (session, token ids, start_pos).  Returns (pointer to the lane records, what keeps them alive)."""
+        ids = [np.ascontiguousarray(t, dtype=np.uint32) for _, t, _ in lanes]
+        counts = [len(t) for t in ids]
+        # one buffer of ids and one of records, filled column by column: 64 lanes through ctypes fields took 0.3 ms
+        flat = np.concatenate([t if t.ndim == 1 else t.reshape(-1)[:len(t)] for t in ids]) if ids else np.empty(0, np.uint32)
+        arr = np.empty(len(lanes), _LANE)
+        arr["session"] = [s._h.value or 0 if s._h else 0 for s, _, _ in lanes]
+        arr["n_tokens"] = counts
+        arr["input_ids"] = flat.ctypes.data + 4 * (np.cumsum(counts, dtype=np.int64) - counts).astype(np.uint64) if counts else 0
+        arr["start_pos"] = [p for _, _, p in lanes]
+        return C.cast(arr.ctypes.data, C.POINTER(capi.Lane)), (arr, flat)
 
     def forward_batch(self, lanes, want_logits=True, want_tokens=True, rows=None):
         """reserve_batch_kv + forward_batch_tokens_reserved + read_output_to_cpu for one packed ragged
