@@ -72,8 +72,12 @@ __device__ __forceinline__ float sink_scale(float m, float l, float sink) {
 // partial, and the CTA that arrives last at the lane's counter merges the shares.
 // LOW8: at most eight query heads per KV head, so rows 8-15 of the A operand are zero and everything that concerns
 // them (half of the softmax and of the accumulator rescaling) is skipped.
-template <int D, int STAGES, bool LOW8, bool EXACT>
-__global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
+// History does not wait for the predecessor: every key but the newest was written before this tick's first kernel, so the first tiles are
+// requested ahead of pdl_wait.  THREADS: while the CTAs have an SM each, four more warps help with what is not a walk - a CTA has up to ten
+// head vectors to prepare, whose shares come from the L2 one after the other (4 lanes of 300 keys, 32 heads of 64 over 4: 17 -> 11 us a launch, one
+// lane of 200, 16 heads of 128 over 4: 13 -> 9); with two CTAs on an SM the registers are worth more (64 lanes: 27 us, 37 with the help).
+template <int D, int STAGES, bool LOW8, bool EXACT, int THREADS>
+__global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
     constexpr int NH = LOW8 ? 1 : 2;  // accumulator row halves that can hold live rows
     constexpr int DP = D + 8;
     constexpr int KT = 16;
@@ -91,7 +95,6 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
     const int g = a.q_heads / a.kv_heads;
     const float two_over_cap = a.softcap != 0.f ? 2.0f / a.softcap : 0.f;
     pdl_trigger();
-    pdl_wait();
     // one 32-byte record per work item, so that nothing but the block table and the queries is a dependent load
     const int4 e0 = reinterpret_cast<const int4*>(a.entries)[2 * blockIdx.x];
     const int4 e1 = reinterpret_cast<const int4*>(a.entries)[2 * blockIdx.x + 1];
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
     // Rows straight from the projection's output (see AttnTcArgs::fused_rope): one warp per head, the head vector staged
     // in f32; the group's query heads, and in the CTA that walks the lane's newest keys also the new K and V rows, which
     // reach the pool before any tile is requested (block-wide barrier below).
-    __shared__ __align__(16) float head_stage[4][D];
+    __shared__ __align__(16) float head_stage[THREADS / 32][D];
     auto prepare_head = [&](int kind, int item) {  // kind 0: query head `item` of the group; 1 / 2: the new K / V row
         float* xs = head_stage[warp];
         rope_head_prepare(a.rk, kind, kind == 0 ? kvh * g + item : kvh, q_off, start_pos, xs, lane);
@@ -116,33 +119,6 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
         }
         __syncwarp();
     };
-    if (a.fused_rope) {
-        for (int i = tid; i < (16 - g) * CHUNKS; i += 128) {
-            int item = g + i / CHUNKS, c = (i % CHUNKS) * 8;
-            *reinterpret_cast<uint4*>(Qs + item * DP + c) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        const int n_heads = g + (split == n_splits - 1 ? 2 : 0);
-        for (int h = warp; h < n_heads; h += 4) prepare_head(h < g ? 0 : (h == g ? 1 : 2), h);
-        __syncthreads();  // the new K / V rows are visible to every tile load of this CTA
-    } else {
-    // the group's query heads -> rows 0..g-1 of the A operand, the rest zero
-    for (int i = tid; i < 16 * CHUNKS; i += 128) {
-        int item = i / CHUNKS, c = (i - item * CHUNKS) * 8;
-        __half2 h[4];
-        if (item < g) {
-            const float* src = a.q + (int64_t)q_off * ldq + (kvh * g + item) * D + c;
-            float4 x0 = *reinterpret_cast<const float4*>(src), x1 = *reinterpret_cast<const float4*>(src + 4);
-            h[0] = __floats2half2_rn(x0.x, x0.y);
-            h[1] = __floats2half2_rn(x0.z, x0.w);
-            h[2] = __floats2half2_rn(x1.x, x1.y);
-            h[3] = __floats2half2_rn(x1.z, x1.w);
-        } else {
-            h[0] = h[1] = h[2] = h[3] = __floats2half2_rn(0.f, 0.f);
-        }
-        *reinterpret_cast<uint4*>(Qs + item * DP + c) = *reinterpret_cast<uint4*>(h);
-    }
-    }
-
     const int p = start_pos;  // the query's position
     int k_lo = attention_first_key(p, a.window, a.chunk);
     int k_hi = p + 1;
@@ -154,11 +130,11 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
     }
     const int k_begin = k_lo / 16 * 16;
     const int n_tiles = k_hi > k_begin ? (k_hi - k_begin + KT - 1) / KT : 0;
-    const int my_tiles = n_tiles > warp ? (n_tiles - warp + 3) / 4 : 0;  // tiles warp, warp + 4, ...
+    const int my_tiles = warp < 4 && n_tiles > warp ? (n_tiles - warp + 3) / 4 : 0;  // tiles warp, warp + 4, ...
 
     const __half* kp = reinterpret_cast<const __half*>(a.k_pool);
     const __half* vp = reinterpret_cast<const __half*>(a.v_pool);
-    __half* ring = rings + warp * RING_HALVES;
+    __half* ring = rings + (warp & 3) * RING_HALVES;
     uint32_t tile_blk = 0;
     auto load_tile = [&](int i) {  // the warp's i-th tile into stage i % STAGES (called with i = 0, 1, 2, ... in order)
         __half* kd = ring + (i % STAGES) * 2 * KT * DP;
@@ -185,18 +161,44 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
         }
     };
 
+    // tiles that may travel before the predecessor is done: all but the one with the newest key
+    const int old_tiles = my_tiles - (my_tiles > 0 && k_begin + (warp + 4 * (my_tiles - 1)) * KT + KT > p ? 1 : 0);
+    const int early = min(old_tiles, STAGES - 1);
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i)
+        if (i < early) {
+            load_tile(i);
+            cp_async_commit();
+        }
+    // rows of the A operand without a query head
+    for (int i = tid; i < (16 - g) * CHUNKS; i += THREADS) *reinterpret_cast<uint4*>(Qs + (g + i / CHUNKS) * DP + (i % CHUNKS) * 8) = make_uint4(0u, 0u, 0u, 0u);
+    pdl_wait();
+    if (a.fused_rope) {
+        const int n_heads = g + (split == n_splits - 1 ? 2 : 0);
+        for (int h = warp; h < n_heads; h += THREADS / 32) prepare_head(h < g ? 0 : (h == g ? 1 : 2), h);
+    } else {
+        // the group's query heads -> rows 0..g-1 of the A operand
+        for (int i = tid; i < g * CHUNKS; i += THREADS) {
+            const int item = i / CHUNKS, c = (i - item * CHUNKS) * 8;
+            const float* src = a.q + (int64_t)q_off * ldq + (kvh * g + item) * D + c;
+            const float4 x0 = *reinterpret_cast<const float4*>(src), x1 = *reinterpret_cast<const float4*>(src + 4);
+            const __half2 h[4] = {__floats2half2_rn(x0.x, x0.y), __floats2half2_rn(x0.z, x0.w), __floats2half2_rn(x1.x, x1.y), __floats2half2_rn(x1.z, x1.w)};
+            *reinterpret_cast<uint4*>(Qs + item * DP + c) = *reinterpret_cast<const uint4*>(h);
+        }
+    }
+    __syncthreads();  // the queries, and the new K / V rows for every tile load that follows
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i)
+        if (i >= early) {
+            if (i < my_tiles) load_tile(i);
+            cp_async_commit();
+        }
+
     float o_acc[NT_O][4];
 #pragma unroll
     for (int j = 0; j < NT_O; ++j) o_acc[j][0] = o_acc[j][1] = o_acc[j][2] = o_acc[j][3] = 0.f;
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     const bool live_r[2] = {gid < g, gid + 8 < g};
-
-#pragma unroll
-    for (int i = 0; i < STAGES - 1; ++i) {
-        if (i < my_tiles) load_tile(i);
-        cp_async_commit();
-    }
-    __syncthreads();  // Qs complete
     constexpr bool Q_IN_REGS = D <= 128;
     uint32_t qf[Q_IN_REGS ? D / 16 : 1][4];
     if (Q_IN_REGS) {
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         int item = gid + 8 * h;
-        if (item >= g) continue;
+        if (item >= g || warp >= 4) continue;
 #pragma unroll
         for (int j = 0; j < NT_O; ++j)
             *reinterpret_cast<float2*>(w_o + item * D + j * 8 + 2 * tq) = make_float2(o_acc[j][2 * h], o_acc[j][2 * h + 1]);
@@ -328,21 +330,21 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
         const int col0 = kvh * g * D;
         const bool fuse_quant = a.qout.qs != nullptr;  // uniform
         if (!fuse_quant) {
-            for (int idx = tid; idx < g * D; idx += 128) {
+            for (int idx = tid; idx < g * D; idx += THREADS) {
                 float v = value_of(idx);
                 if (a.out != nullptr) a.out[row * a.q_heads * D + col0 + idx] = v;
                 if (a.out_h != nullptr) a.out_h[row * a.q_heads * D + col0 + idx] = __float2half_rn(v);
             }
             return;
         }
-        for (int idx = tid; idx < g * D; idx += 128) {
+        for (int idx = tid; idx < g * D; idx += THREADS) {
             float v = value_of(idx);
             stage[idx] = v;
             if (a.out != nullptr) a.out[row * a.q_heads * D + col0 + idx] = v;
         }
         __syncthreads();
         // one warp per 256-wide group, eight consecutive values per lane (g * D is a multiple of 256 here)
-        for (int grp = warp; grp < g * D / 256; grp += 4) {
+        for (int grp = warp; grp < g * D / 256; grp += THREADS / 32) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = stage[grp * 256 + lane * 8 + i];
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnTcArgs a) {
             return a.sink != nullptr ? o * sink_scale(m, l, a.sink[kvh * g + idx / D]) : o / l;
         });
     } else {
-        for (int idx = tid; idx < g * D; idx += 128) {
+        for (int idx = tid; idx < g * D; idx += THREADS) {
             int item = idx / D, c = idx - item * D;
             float m, l;
             float o = merged_local(idx, m, l);
@@ -454,11 +456,12 @@ void launch_for_dim(const AttnTcArgs& a, cudaStream_t s) {
     if (a.n_entries > 0) {
         constexpr int STAGES = D >= 256 ? 2 : 3;
         constexpr size_t smem = (size_t)(16 + 4 * STAGES * 2 * 16) * (D + 8) * sizeof(__half);
-        ensure_dynamic_smem(reinterpret_cast<const void*>(&attn_decode_kernel<D, STAGES, true, EXACT>), smem);
-        ensure_dynamic_smem(reinterpret_cast<const void*>(&attn_decode_kernel<D, STAGES, false, EXACT>), smem);
         dim3 grid((unsigned)a.n_entries, (unsigned)a.kv_heads);
-        if (a.q_heads / a.kv_heads <= 8) launch_pdl(attn_decode_kernel<D, STAGES, true, EXACT>, grid, dim3(128), smem, s, a);
-        else launch_pdl(attn_decode_kernel<D, STAGES, false, EXACT>, grid, dim3(128), smem, s, a);
+        const bool low8 = a.q_heads / a.kv_heads <= 8, alone = a.n_entries * a.kv_heads <= kPlanSms;
+        auto* kernel = alone ? (low8 ? attn_decode_kernel<D, STAGES, true, EXACT, 256> : attn_decode_kernel<D, STAGES, false, EXACT, 256>)
+                             : (low8 ? attn_decode_kernel<D, STAGES, true, EXACT, 128> : attn_decode_kernel<D, STAGES, false, EXACT, 128>);
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+        launch_pdl(kernel, grid, dim3(alone ? 256 : 128), smem, s, a);
         MK_LAUNCH_CHECK();
     }
     if (a.n_dec_lanes > 0) {  // lanes whose keys were shared out over several CTAs
