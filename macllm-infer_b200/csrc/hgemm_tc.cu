@@ -307,6 +307,27 @@ __device__ __forceinline__ float hg_gelu_tanh(float x) {
     return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * x * (1.0f + 0.044715f * x * x)));
 }
 
+// 32 columns of a gated tile: lanes 2i / 2i+1 hold gate / up of one feature; the even lane finishes the even token columns, the odd lane the odd
+// ones, after one exchange per pair of columns.  n columns count; act gets the lane's column.
+template <typename Act>
+__device__ __forceinline__ void gated_columns(const uint32_t (&r)[32], int n, bool live, int feature, int tok0, const HgPart& part, int bf16, Act act) {
+    const bool odd = (threadIdx.x & 1) != 0;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        if (i >= n) break;  // uniform
+        const float mine = __uint_as_float(odd ? r[i] : r[i + 1]);  // what the partner needs
+        const float theirs = __shfl_xor_sync(0xffffffffu, mine, 1);
+        const float g = odd ? theirs : __uint_as_float(r[i]), u = odd ? __uint_as_float(r[i + 1]) : theirs;
+        const int column = i + (odd ? 1 : 0);
+        const float a = act(g, u, column);
+        if (live && column < n) {
+            const int64_t at = (int64_t)(tok0 + column) * part.ldyh + feature;
+            if (bf16) reinterpret_cast<__nv_bfloat16*>(part.yh)[at] = __float2bfloat16_rn(a);
+            else part.yh[at] = __float2half_rn(a);
+        }
+    }
+}
+
 // GATED: scattered results are multiplied by a gate (MatmulScatter::gate).
 // PAIR: two CTAs of a cluster make one 256 x BN tile; each holds half of the weight rows and their accumulators, and half of the
 // activation rows.
@@ -590,34 +611,17 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + (uint32_t)cb, r);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (p.gated != 0) {
-                    // lanes 2i / 2i+1 hold gate / up of one feature: the even lane finishes the even token columns,
-                    // the odd lane the odd ones, after one exchange per pair of columns
-                    const bool odd = (lane & 1) != 0;
-                    const int feature = row >> 1;
+                    const int n = min(32, tile.tok_end - tok0 - cb);
                     const bool weighed = part.act_pre != nullptr || part.act_post != nullptr;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        float mine = __uint_as_float(odd ? r[i] : r[i + 1]);       // what the partner needs
-                        float theirs = __shfl_xor_sync(0xffffffffu, mine, 1);
-                        float g = odd ? theirs : __uint_as_float(r[i]);
-                        float u = odd ? __uint_as_float(r[i + 1]) : theirs;
-                        int tok = tok0 + cb + i + (odd ? 1 : 0);
-                        float w_in = 1.0f, w_out = 1.0f;
-                        if (weighed) {  // uniform
-                            w_in = __shfl_sync(0xffffffffu, pre, i + (odd ? 1 : 0));
-                            w_out = __shfl_sync(0xffffffffu, post, i + (odd ? 1 : 0));
-                        }
-                        if (row < tile.rows && tok < tile.tok_end) {
-                            float a;
-                            if (p.gated == 1 + GatedAct::Clamped) {
-                                a = hg_clamped(w_in * g, w_in * u, part.act_limit) * w_out;
-                            } else {
-                                a = (p.gated == 1 + GatedAct::Silu ? hg_silu(g) : hg_gelu_tanh(g)) * u;
-                            }
-                            if (p.bf16) reinterpret_cast<__nv_bfloat16*>(part.yh)[(int64_t)tok * part.ldyh + feature] = __float2bfloat16_rn(a);
-                            else part.yh[(int64_t)tok * part.ldyh + feature] = __float2half_rn(a);
-                        }
-                    }
+                    if (p.gated == 1 + GatedAct::Silu) gated_columns(r, n, row < tile.rows, row >> 1, tok0 + cb, part, p.bf16, [](float g, float u, int) { return hg_silu(g) * u; });
+                    else if (p.gated != 1 + GatedAct::Clamped)
+                        gated_columns(r, n, row < tile.rows, row >> 1, tok0 + cb, part, p.bf16, [](float g, float u, int) { return hg_gelu_tanh(g) * u; });
+                    else if (!weighed) gated_columns(r, n, row < tile.rows, row >> 1, tok0 + cb, part, p.bf16, [&](float g, float u, int) { return hg_clamped(g, u, part.act_limit); });
+                    else
+                        gated_columns(r, n, row < tile.rows, row >> 1, tok0 + cb, part, p.bf16, [&](float g, float u, int column) {
+                            const float w_in = __shfl_sync(0xffffffffu, pre, column), w_out = __shfl_sync(0xffffffffu, post, column);
+                            return hg_clamped(w_in * g, w_in * u, part.act_limit) * w_out;
+                        });
                 } else if (p.scattered != 0 && p.scatter.rest != nullptr && row >= p.scatter.rest_from) {
                     float* out = p.scatter.rest + (int64_t)(tok0 + cb) * p.scatter.ld_rest + row - p.scatter.rest_from;
                     if (row < tile.rows) {
@@ -662,15 +666,23 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     float* out = dst + (int64_t)(tok0 + cb) * ld + row;
 #pragma unroll
                     for (int i = 0; i < 32; ++i, out += ld) *out = __uint_as_float(r[i]);
+                } else if (row < tile.rows && (plain || p.splits > 1)) {
+                    // the last columns of a tile, or all there are on narrow ticks: eight at a time, nothing but stores (with scale and
+                    // cap in between, 32 times over, a launch waited 3.4 us for its instructions alone)
+                    float* out = dst + (int64_t)(tok0 + cb) * ld + row;
+                    const int n = tile.tok_end - tok0 - cb;
+#pragma unroll
+                    for (int i0 = 0; i0 < 32; i0 += 8) {
+                        if (i0 >= n) break;
+#pragma unroll
+                        for (int i = i0; i < i0 + 8; ++i, out += ld)
+                            if (i < n) *out = __uint_as_float(r[i]);
+                    }
                 } else if (row < tile.rows) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         int tok = tok0 + cb + i;
-                        if (tok < tile.tok_end) {
-                            float v = __uint_as_float(r[i]);
-                            if (p.splits == 1) v = finish_value(v, p);
-                            dst[(int64_t)tok * ld + row] = v;
-                        }
+                        if (tok < tile.tok_end) dst[(int64_t)tok * ld + row] = finish_value(__uint_as_float(r[i]), p);
                     }
                 }
             }
@@ -883,7 +895,7 @@ HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits) {
 
 // Wide calls can go in 256 x 256 tiles of two CTAs instead.  Measured on a B200 with K = 2048 and 11008, microseconds: a pair's tile takes
 // 0.36 per block of K and 1.2 besides, a CTA's 128 x 128 tile 0.27 and 0.8, its 128 x 256 tile 0.41 and 1.2; K shares cost their partial
-// sums twice at about 5 TB/s.  Fewest rounds of CTAs times tile time wins (22016 x 2048 at 2048 tokens: 152 -> 127 us, 8192 x 2048: 89 -> 58).
+// sums twice at about 5 TB/s.  Fewest rounds of CTAs times tile time wins (L2 flushed, 22016 x 2048 at 2048 tokens: 152 -> 138 us, 8192 x 2048: 89 -> 62).
 bool hgemm_tc_pairs(int64_t rows, int64_t cols, int T, int max_splits, const HgemmPlan& single, HgemmPlan& pairs) {
     if (T <= 128 || rows <= HG_BM) return false;
     const int64_t kb = cols / HG_BK, row_tiles = (rows + HG_BM - 1) / HG_BM, n_tiles = (T + 255) / 256, tiles = (row_tiles + 1) / 2 * n_tiles;
