@@ -192,7 +192,8 @@ __global__ void add_inplace_kernel(float* h, const float* a, float scale, int64_
 
 
 // One CTA per row, NG groups of 256 per warp held in registers (dim <= 8 warps * NG * 256).
-template <int NG>
+// SHARED: the branch output comes in shares; the registers that several of them take on their way are spared otherwise.
+template <int NG, bool SHARED>
 __global__ void __launch_bounds__(NQ_THREADS) add_norm_quant_fast_kernel(NormQuantArgs a) {
     __shared__ float red[32];
     pdl_trigger();
@@ -230,12 +231,18 @@ __global__ void __launch_bounds__(NQ_THREADS) add_norm_quant_fast_kernel(NormQua
         for (int g = 0; g < NG; ++g) {
             if (live[g]) {
                 load8(av + (warp + g * 8) * 256 + lane * 8, y[g]);
-#pragma unroll 4
-                for (int sp = 1; sp < a.a_splits; ++sp) {
-                    float part[8];
-                    load8(av + (int64_t)sp * a.a_split_stride + (warp + g * 8) * 256 + lane * 8, part);
+                // shares a row at a time, several on their way together: on narrow ticks a row's CTA waits for little else
+                constexpr int AHEAD = NG == 1 ? 6 : 4;
+                for (int sp = 1; SHARED && sp < a.a_splits; sp += AHEAD) {
+                    float part[AHEAD][8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) y[g][i] += part[i];
+                    for (int j = 0; j < AHEAD; ++j)
+                        if (sp + j < a.a_splits) load8(av + (int64_t)(sp + j) * a.a_split_stride + (warp + g * 8) * 256 + lane * 8, part[j]);
+#pragma unroll
+                    for (int j = 0; j < AHEAD; ++j)
+                        if (sp + j < a.a_splits)
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) y[g][i] += part[j][i];
                 }
             } else {
 #pragma unroll
@@ -342,9 +349,11 @@ void launch_add_norm_quant(const NormQuantArgs& a, cudaStream_t s) {
     }
     if (vec_ok && a.dim <= 8 * 4 * 256) {
         int ng = (a.dim / 256 + 7) / 8;
-        if (ng == 1) launch_pdl(add_norm_quant_fast_kernel<1>, dim3(a.rows), dim3(NQ_THREADS), 0, s, a);
-        else if (ng == 2) launch_pdl(add_norm_quant_fast_kernel<2>, dim3(a.rows), dim3(NQ_THREADS), 0, s, a);
-        else launch_pdl(add_norm_quant_fast_kernel<4>, dim3(a.rows), dim3(NQ_THREADS), 0, s, a);
+        const bool shared = a.a != nullptr && a.a_splits > 1;
+        auto* kernel = ng == 1 ? (shared ? add_norm_quant_fast_kernel<1, true> : add_norm_quant_fast_kernel<1, false>)
+                     : ng == 2 ? (shared ? add_norm_quant_fast_kernel<2, true> : add_norm_quant_fast_kernel<2, false>)
+                               : (shared ? add_norm_quant_fast_kernel<4, true> : add_norm_quant_fast_kernel<4, false>);
+        launch_pdl(kernel, dim3(a.rows), dim3(NQ_THREADS), 0, s, a);
         MK_LAUNCH_CHECK();
         return;
     }
