@@ -8,7 +8,10 @@
 // Memory plan: one warp owns one output row and streams that row's blocks with 128-bit (Q4_K,
 // Q8_0) or 64-bit (Q6_K planes) loads, eight lanes per 256-weight block, so a warp consumes whole
 // 128-byte lines; activations (T*K bytes) are re-read from L1/L2.  Each weight byte leaves HBM once
-// per call when T <= ROWS_PER_PASS; larger T re-walks the row from cache in passes.
+// per call when T <= NT; larger T re-walks the row from cache in passes.  A warp takes R output rows that follow one
+// another: their weights travel together, and an activation that was fetched meets all of them (with one row per warp and
+// eight sums whatever T, 32000 x 2048 in Q6_K took 26 us at one activation row,
+// this 15).
 #include "kernels.h"
 
 namespace mk {
@@ -16,7 +19,7 @@ namespace mk {
 namespace {
 
 constexpr int GEMV_WARPS = 4;
-constexpr int NT = 8;  // activation rows per pass
+constexpr int NT_MAX = 8;  // most activation rows of a pass
 
 // Optional expert grouping: blockIdx.y selects the expert, whose output rows are [offsets[e], offsets[e+1]).
 struct Group {
@@ -39,13 +42,13 @@ __device__ __forceinline__ void q4k_scale_min(const uint8_t* s, int j, int& sc, 
     }
 }
 
-template <int ROWS>
-__device__ __forceinline__ void finish_rows(float (&acc)[NT], int n, int t0, int T, float* y, int ldy, float out_scale,
+template <int NT>
+__device__ __forceinline__ void finish_rows(float (&acc)[NT], int n, int out, int t0, int T, float* y, int ldy, float out_scale,
                                             float softcap) {
 #pragma unroll
-    for (int t = 0; t < ROWS; ++t) {
+    for (int t = 0; t < NT; ++t) {
         float v = warp_sum(acc[t]);
-        if ((threadIdx.x & 31) == 0 && t0 + t < T) {
+        if ((threadIdx.x & 31) == 0 && t0 + t < T && n < out) {
             v *= out_scale;
             if (softcap != 0.f) v = tanhf(v * (1.0f / softcap)) * softcap;
             y[(int64_t)(t0 + t) * ldy + n] = v;
@@ -54,67 +57,93 @@ __device__ __forceinline__ void finish_rows(float (&acc)[NT], int n, int t0, int
 }
 
 // ---------------------------------------------------------------- Q4_K
+template <int NT, int R>
 __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q4k_kernel(const uint8_t* __restrict__ W, int nb, int out,
                                                                     const int8_t* __restrict__ xq,
                                                                     const float* __restrict__ xd,
                                                                     const int16_t* __restrict__ xbs, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
-    int n = blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5);
-    if (n >= out) return;
+    pdl_trigger();
+    bool waited = grp.offsets != nullptr;  // the weights do not wait for the predecessor, row ranges and activations do
+    if (waited) pdl_wait();
+    const int n0 = (blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5)) * R;
+    if (n0 >= out) {
+        if (!waited) pdl_wait();
+        return;
+    }
     int lane = threadIdx.x & 31;
     int part = lane & 7;       // 16-byte slice of the 128 nibble bytes
     int j = part >> 1;         // 64-weight chunk
     int h = part & 1;          // half of the chunk's 32 bytes
     const int K = nb * 256;
-    const uint8_t* wrow = W + ((int64_t)blockIdx.y * out + n) * nb * 144;
+    const uint8_t* w_row[R];  // a row behind the last one reads the last one and is not stored
+#pragma unroll
+    for (int r = 0; r < R; ++r) w_row[r] = W + ((int64_t)blockIdx.y * out + min(n0 + r, out - 1)) * nb * 144;
     int t_first;
     group_range(grp, T, t_first, T);
 
     for (int t0 = t_first; t0 < T; t0 += NT) {
-        float acc[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = 0.f;
+        float acc[R][NT] = {};
         int rows = min(NT, T - t0);
         for (int ib = lane >> 3; ib < nb; ib += 4) {
-            const uint8_t* blk = wrow + (int64_t)ib * 144;
-            uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 16 * part);
-            uint32_t dm = *reinterpret_cast<const uint32_t*>(blk);
-            float d = __half2float(__ushort_as_half((unsigned short)(dm & 0xFFFF)));
-            float dmin = __half2float(__ushort_as_half((unsigned short)(dm >> 16)));
-            int sc_lo, m_lo, sc_hi, m_hi;
-            q4k_scale_min(blk + 4, 2 * j, sc_lo, m_lo);
-            q4k_scale_min(blk + 4, 2 * j + 1, sc_hi, m_hi);
-            uint32_t ql[4] = {q.x & 0x0F0F0F0Fu, q.y & 0x0F0F0F0Fu, q.z & 0x0F0F0F0Fu, q.w & 0x0F0F0F0Fu};
-            uint32_t qh[4] = {(q.x >> 4) & 0x0F0F0F0Fu, (q.y >> 4) & 0x0F0F0F0Fu, (q.z >> 4) & 0x0F0F0F0Fu,
-                              (q.w >> 4) & 0x0F0F0F0Fu};
+            uint32_t ql[R][4], qh[R][4];
+            float d[R], dmin[R];
+            int sc_lo[R], m_lo[R], sc_hi[R], m_hi[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint8_t* blk = w_row[r] + (int64_t)ib * 144;
+                uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 16 * part);
+                uint32_t dm = *reinterpret_cast<const uint32_t*>(blk);
+                d[r] = __half2float(__ushort_as_half((unsigned short)(dm & 0xFFFF)));
+                dmin[r] = __half2float(__ushort_as_half((unsigned short)(dm >> 16)));
+                q4k_scale_min(blk + 4, 2 * j, sc_lo[r], m_lo[r]);
+                q4k_scale_min(blk + 4, 2 * j + 1, sc_hi[r], m_hi[r]);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    ql[r][i] = w[i] & 0x0F0F0F0Fu;
+                    qh[r][i] = (w[i] >> 4) & 0x0F0F0F0Fu;
+                }
+            }
+            if (!waited) {
+                pdl_wait();
+                waited = true;
+            }
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 if (t < rows) {
                     const int64_t xrow = src_of(grp, t0 + t);
                     const int8_t* xr = xq + xrow * K + ib * 256 + 64 * j + 16 * h;
-                    int4 xl = *reinterpret_cast<const int4*>(xr);
-                    int4 xh = *reinterpret_cast<const int4*>(xr + 32);
-                    int s_lo = __dp4a((int)ql[0], xl.x, 0);
-                    s_lo = __dp4a((int)ql[1], xl.y, s_lo);
-                    s_lo = __dp4a((int)ql[2], xl.z, s_lo);
-                    s_lo = __dp4a((int)ql[3], xl.w, s_lo);
-                    int s_hi = __dp4a((int)qh[0], xh.x, 0);
-                    s_hi = __dp4a((int)qh[1], xh.y, s_hi);
-                    s_hi = __dp4a((int)qh[2], xh.z, s_hi);
-                    s_hi = __dp4a((int)qh[3], xh.w, s_hi);
+                    const int4 xl = *reinterpret_cast<const int4*>(xr), xh = *reinterpret_cast<const int4*>(xr + 32);
                     const int16_t* bs = xbs + xrow * (K / 16) + ib * 16 + 4 * j + h;
-                    int isum = sc_lo * s_lo + sc_hi * s_hi;
-                    int msum = m_lo * (int)bs[0] + m_hi * (int)bs[2];
-                    acc[t] += xd[xrow * nb + ib] * (d * (float)isum - dmin * (float)msum);
+                    const int b0 = (int)bs[0], b2 = (int)bs[2];
+                    const float dx = xd[xrow * nb + ib];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        int s_lo = __dp4a((int)ql[r][0], xl.x, 0);
+                        s_lo = __dp4a((int)ql[r][1], xl.y, s_lo);
+                        s_lo = __dp4a((int)ql[r][2], xl.z, s_lo);
+                        s_lo = __dp4a((int)ql[r][3], xl.w, s_lo);
+                        int s_hi = __dp4a((int)qh[r][0], xh.x, 0);
+                        s_hi = __dp4a((int)qh[r][1], xh.y, s_hi);
+                        s_hi = __dp4a((int)qh[r][2], xh.z, s_hi);
+                        s_hi = __dp4a((int)qh[r][3], xh.w, s_hi);
+                        int isum = sc_lo[r] * s_lo + sc_hi[r] * s_hi;
+                        int msum = m_lo[r] * b0 + m_hi[r] * b2;
+                        acc[r][t] += dx * (d[r] * (float)isum - dmin[r] * (float)msum);
+                    }
                 }
             }
         }
-        finish_rows<NT>(acc, n, t0, T, y, ldy, out_scale, softcap);
+#pragma unroll
+        for (int r = 0; r < R; ++r) finish_rows<NT>(acc[r], n0 + r, out, t0, T, y, ldy, out_scale, softcap);
     }
+    if (!waited) pdl_wait();  // a lane without blocks
 }
 
 // ---------------------------------------------------------------- Q6_K (planar layout)
+template <int NT, int R>
 __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q6k_kernel(const uint8_t* __restrict__ ql_p,
                                                                     const uint8_t* __restrict__ qh_p,
                                                                     const int8_t* __restrict__ sc_p,
@@ -123,107 +152,144 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q6k_kernel(const uint8_
                                                                     const float* __restrict__ xd, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
-    int n = blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5);
-    if (n >= out) return;
+    pdl_trigger();
+    bool waited = grp.offsets != nullptr;  // the weights do not wait for the predecessor, row ranges and activations do
+    if (waited) pdl_wait();
+    const int n0 = (blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5)) * R;
+    if (n0 >= out) {
+        if (!waited) pdl_wait();
+        return;
+    }
     int lane = threadIdx.x & 31;
     int part = lane & 7;
     int half = part >> 2;          // 128-weight half of the block
     int l0 = (part & 3) * 8;       // eight consecutive positions inside the half
     const int K = nb * 256;
-    int64_t row_blk = ((int64_t)blockIdx.y * out + n) * nb;
+    int64_t row_blk[R];  // a row behind the last one reads the last one and is not stored
+#pragma unroll
+    for (int r = 0; r < R; ++r) row_blk[r] = ((int64_t)blockIdx.y * out + min(n0 + r, out - 1)) * nb;
     int t_first;
     group_range(grp, T, t_first, T);
 
     for (int t0 = t_first; t0 < T; t0 += NT) {
-        float acc[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = 0.f;
+        float acc[R][NT] = {};
         int rows = min(NT, T - t0);
         for (int ib = lane >> 3; ib < nb; ib += 4) {
-            int64_t b = row_blk + ib;
-            uint2 qa = *reinterpret_cast<const uint2*>(ql_p + b * 128 + half * 64 + l0);
-            uint2 qb = *reinterpret_cast<const uint2*>(ql_p + b * 128 + half * 64 + 32 + l0);
-            uint2 qhh = *reinterpret_cast<const uint2*>(qh_p + b * 64 + half * 32 + l0);
-            const int8_t* sc = sc_p + b * 16 + half * 8 + (l0 >> 4);
-            int s0 = sc[0], s1 = sc[2], s2 = sc[4], s3 = sc[6];
-            float d = __half2float(d_p[b]);
-            // four groups of eight 6-bit values, re-centred to [-32, 31]
-            uint32_t g[4][2];
-            g[0][0] = __vsub4((qa.x & 0x0F0F0F0Fu) | (((qhh.x >> 0) & 0x03030303u) << 4), 0x20202020u);
-            g[0][1] = __vsub4((qa.y & 0x0F0F0F0Fu) | (((qhh.y >> 0) & 0x03030303u) << 4), 0x20202020u);
-            g[1][0] = __vsub4((qb.x & 0x0F0F0F0Fu) | (((qhh.x >> 2) & 0x03030303u) << 4), 0x20202020u);
-            g[1][1] = __vsub4((qb.y & 0x0F0F0F0Fu) | (((qhh.y >> 2) & 0x03030303u) << 4), 0x20202020u);
-            g[2][0] = __vsub4(((qa.x >> 4) & 0x0F0F0F0Fu) | (((qhh.x >> 4) & 0x03030303u) << 4), 0x20202020u);
-            g[2][1] = __vsub4(((qa.y >> 4) & 0x0F0F0F0Fu) | (((qhh.y >> 4) & 0x03030303u) << 4), 0x20202020u);
-            g[3][0] = __vsub4(((qb.x >> 4) & 0x0F0F0F0Fu) | (((qhh.x >> 6) & 0x03030303u) << 4), 0x20202020u);
-            g[3][1] = __vsub4(((qb.y >> 4) & 0x0F0F0F0Fu) | (((qhh.y >> 6) & 0x03030303u) << 4), 0x20202020u);
+            uint32_t g[R][4][2];  // four groups of eight 6-bit values, re-centred to [-32, 31]
+            int sc[R][4];
+            float d[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int64_t b = row_blk[r] + ib;
+                const uint2 qa = *reinterpret_cast<const uint2*>(ql_p + b * 128 + half * 64 + l0);
+                const uint2 qb = *reinterpret_cast<const uint2*>(ql_p + b * 128 + half * 64 + 32 + l0);
+                const uint2 qhh = *reinterpret_cast<const uint2*>(qh_p + b * 64 + half * 32 + l0);
+                const int8_t* scale = sc_p + b * 16 + half * 8 + (l0 >> 4);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sc[r][i] = scale[2 * i];
+                d[r] = __half2float(d_p[b]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint2 lo = (i & 1) ? qb : qa;
+                    const int sh = (i >> 1) * 4;
+                    g[r][i][0] = __vsub4(((lo.x >> sh) & 0x0F0F0F0Fu) | (((qhh.x >> (2 * i)) & 0x03030303u) << 4), 0x20202020u);
+                    g[r][i][1] = __vsub4(((lo.y >> sh) & 0x0F0F0F0Fu) | (((qhh.y >> (2 * i)) & 0x03030303u) << 4), 0x20202020u);
+                }
+            }
+            if (!waited) {
+                pdl_wait();
+                waited = true;
+            }
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 if (t < rows) {
                     const int64_t xrow = src_of(grp, t0 + t);
                     const int8_t* xr = xq + xrow * K + ib * 256 + half * 128 + l0;
-                    int2 x0 = *reinterpret_cast<const int2*>(xr);
-                    int2 x1 = *reinterpret_cast<const int2*>(xr + 32);
-                    int2 x2 = *reinterpret_cast<const int2*>(xr + 64);
-                    int2 x3 = *reinterpret_cast<const int2*>(xr + 96);
-                    int i0 = __dp4a((int)g[0][1], x0.y, __dp4a((int)g[0][0], x0.x, 0));
-                    int i1 = __dp4a((int)g[1][1], x1.y, __dp4a((int)g[1][0], x1.x, 0));
-                    int i2 = __dp4a((int)g[2][1], x2.y, __dp4a((int)g[2][0], x2.x, 0));
-                    int i3 = __dp4a((int)g[3][1], x3.y, __dp4a((int)g[3][0], x3.x, 0));
-                    int isum = s0 * i0 + s1 * i1 + s2 * i2 + s3 * i3;
-                    acc[t] += xd[xrow * nb + ib] * (d * (float)isum);
+                    int2 x[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const int2*>(xr + 32 * i);
+                    const float dx = xd[xrow * nb + ib];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        int isum = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) isum += sc[r][i] * __dp4a((int)g[r][i][1], x[i].y, __dp4a((int)g[r][i][0], x[i].x, 0));
+                        acc[r][t] += dx * (d[r] * (float)isum);
+                    }
                 }
             }
         }
-        finish_rows<NT>(acc, n, t0, T, y, ldy, out_scale, softcap);
+#pragma unroll
+        for (int r = 0; r < R; ++r) finish_rows<NT>(acc[r], n0 + r, out, t0, T, y, ldy, out_scale, softcap);
     }
+    if (!waited) pdl_wait();  // a lane without blocks
 }
 
 // ---------------------------------------------------------------- Q8_0 (planar layout)
+template <int NT, int R>
 __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q80_kernel(const int8_t* __restrict__ qs_p,
                                                                     const __half* __restrict__ d_p, int K, int out,
                                                                     const int8_t* __restrict__ xq,
                                                                     const float* __restrict__ xd, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
-    int n = blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5);
-    if (n >= out) return;
+    pdl_trigger();
+    bool waited = grp.offsets != nullptr;  // the weights do not wait for the predecessor, row ranges and activations do
+    if (waited) pdl_wait();
+    const int n0 = (blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5)) * R;
+    if (n0 >= out) {
+        if (!waited) pdl_wait();
+        return;
+    }
     int lane = threadIdx.x & 31;
     int nb = K / 32;
-    const int8_t* wq = qs_p + ((int64_t)blockIdx.y * out + n) * K;
-    const __half* wd = d_p + ((int64_t)blockIdx.y * out + n) * nb;
+    int64_t w_row[R];  // a row behind the last one reads the last one and is not stored
+#pragma unroll
+    for (int r = 0; r < R; ++r) w_row[r] = (int64_t)blockIdx.y * out + min(n0 + r, out - 1);
     int t_first;
     group_range(grp, T, t_first, T);
     for (int t0 = t_first; t0 < T; t0 += NT) {
-        float acc[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = 0.f;
+        float acc[R][NT] = {};
         int rows = min(NT, T - t0);
         for (int b = lane; b < nb; b += 32) {
-            int4 w0 = *reinterpret_cast<const int4*>(wq + b * 32);
-            int4 w1 = *reinterpret_cast<const int4*>(wq + b * 32 + 16);
-            float d = __half2float(wd[b]);
+            int4 w0[R], w1[R];
+            float d[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                w0[r] = *reinterpret_cast<const int4*>(qs_p + w_row[r] * K + b * 32);
+                w1[r] = *reinterpret_cast<const int4*>(qs_p + w_row[r] * K + b * 32 + 16);
+                d[r] = __half2float(d_p[w_row[r] * nb + b]);
+            }
+            if (!waited) {
+                pdl_wait();
+                waited = true;
+            }
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 if (t < rows) {
                     const int64_t xrow = src_of(grp, t0 + t);
                     const int8_t* xr = xq + xrow * K + b * 32;
-                    int4 x0 = *reinterpret_cast<const int4*>(xr);
-                    int4 x1 = *reinterpret_cast<const int4*>(xr + 16);
-                    int s = __dp4a(w0.x, x0.x, 0);
-                    s = __dp4a(w0.y, x0.y, s);
-                    s = __dp4a(w0.z, x0.z, s);
-                    s = __dp4a(w0.w, x0.w, s);
-                    s = __dp4a(w1.x, x1.x, s);
-                    s = __dp4a(w1.y, x1.y, s);
-                    s = __dp4a(w1.z, x1.z, s);
-                    s = __dp4a(w1.w, x1.w, s);
-                    acc[t] += (float)s * (d * xd[xrow * nb + b]);
+                    const int4 x0 = *reinterpret_cast<const int4*>(xr), x1 = *reinterpret_cast<const int4*>(xr + 16);
+                    const float dx = xd[xrow * nb + b];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        int s = __dp4a(w0[r].x, x0.x, 0);
+                        s = __dp4a(w0[r].y, x0.y, s);
+                        s = __dp4a(w0[r].z, x0.z, s);
+                        s = __dp4a(w0[r].w, x0.w, s);
+                        s = __dp4a(w1[r].x, x1.x, s);
+                        s = __dp4a(w1[r].y, x1.y, s);
+                        s = __dp4a(w1[r].z, x1.z, s);
+                        s = __dp4a(w1[r].w, x1.w, s);
+                        acc[r][t] += (float)s * (d[r] * dx);
+                    }
                 }
             }
         }
-        finish_rows<NT>(acc, n, t0, T, y, ldy, out_scale, softcap);
+#pragma unroll
+        for (int r = 0; r < R; ++r) finish_rows<NT>(acc[r], n0 + r, out, t0, T, y, ldy, out_scale, softcap);
     }
+    if (!waited) pdl_wait();  // a lane without blocks
 }
 
 // ---------------------------------------------------------------- F32 (router)
@@ -235,6 +301,8 @@ constexpr int F32_GEMV_ROWS = 8;
 __global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_kernel(const float* __restrict__ W, int out, int in,
                                                                    const float* __restrict__ x, int T,
                                                                    float* __restrict__ y) {
+    pdl_trigger();
+    pdl_wait();
     int n = blockIdx.x * GEMV_WARPS + (threadIdx.x >> 5);
     if (n >= out) return;
     int lane = threadIdx.x & 31;
@@ -267,29 +335,78 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_kernel(const float* 
     }
 }
 
+// The same sums for many rows: a warp takes F32_GEMV_ROWS rows and F32_WIDE_OUT outputs, so that a value of x or W that was fetched meets
+// eight others instead of one.  Bound by the L1's load rate and the FMA pipe alike (128 outputs x 2048 for 1420 rows: 90 -> 50 us).
+constexpr int F32_WIDE_OUT = 8;
+__global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_wide_kernel(const float* __restrict__ W, int out, int in, const float* __restrict__ x, int T,
+                                                                        float* __restrict__ y) {
+    pdl_trigger();
+    pdl_wait();
+    const int n0 = (blockIdx.x * GEMV_WARPS + (int)(threadIdx.x >> 5)) * F32_WIDE_OUT, t0 = (int)blockIdx.y * F32_GEMV_ROWS, lane = threadIdx.x & 31;
+    if (n0 >= out) return;
+    // rows and outputs behind the end repeat the last one and are not stored
+    const float *xr[F32_GEMV_ROWS], *wr[F32_WIDE_OUT];
+#pragma unroll
+    for (int r = 0; r < F32_GEMV_ROWS; ++r) xr[r] = x + (int64_t)min(t0 + r, T - 1) * in;
+#pragma unroll
+    for (int j = 0; j < F32_WIDE_OUT; ++j) wr[j] = W + (int64_t)min(n0 + j, out - 1) * in;
+    float acc[F32_GEMV_ROWS][F32_WIDE_OUT] = {};
+#pragma unroll 2
+    for (int k = lane; k < in; k += 32) {
+        float xv[F32_GEMV_ROWS], wv[F32_WIDE_OUT];
+#pragma unroll
+        for (int r = 0; r < F32_GEMV_ROWS; ++r) xv[r] = xr[r][k];
+#pragma unroll
+        for (int j = 0; j < F32_WIDE_OUT; ++j) wv[j] = wr[j][k];
+#pragma unroll
+        for (int r = 0; r < F32_GEMV_ROWS; ++r)
+#pragma unroll
+            for (int j = 0; j < F32_WIDE_OUT; ++j) acc[r][j] += xv[r] * wv[j];
+    }
+#pragma unroll
+    for (int r = 0; r < F32_GEMV_ROWS; ++r) {
+        float mine = 0.f;
+#pragma unroll
+        for (int j = 0; j < F32_WIDE_OUT; ++j) {
+            const float v = warp_sum(acc[r][j]);
+            if (lane == j) mine = v;
+        }
+        if (lane < F32_WIDE_OUT && n0 + lane < out && t0 + r < T) y[(int64_t)(t0 + r) * out + n0 + lane] = mine;
+    }
+}
+
 }  // namespace
 
-static void launch_qgemv_impl(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap,
-                              int experts, Group grp, cudaStream_t s) {
-    dim3 grid((unsigned)((W.rows + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)experts);
+template <int NT, int R>
+static void launch_qgemv_rows(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap, int experts, Group grp, cudaStream_t s) {
+    dim3 grid((unsigned)((W.rows + GEMV_WARPS * R - 1) / (GEMV_WARPS * R)), (unsigned)experts);
     switch (W.type) {
         case QT_Q4_K:
-            qgemv_q4k_kernel<<<grid, GEMV_WARPS * 32, 0, s>>>((const uint8_t*)W.p0, (int)(W.cols / 256), (int)W.rows, x.qs,
-                                                              x.d, x.bsums, T, y, ldy, out_scale, softcap, grp);
+            launch_pdl(qgemv_q4k_kernel<NT, R>, grid, dim3(GEMV_WARPS * 32), 0, s, (const uint8_t*)W.p0, (int)(W.cols / 256), (int)W.rows, x.qs, x.d, x.bsums, T, y, ldy, out_scale, softcap, grp);
             break;
         case QT_Q6_K:
-            qgemv_q6k_kernel<<<grid, GEMV_WARPS * 32, 0, s>>>((const uint8_t*)W.p0, (const uint8_t*)W.p1,
-                                                              (const int8_t*)W.p2, (const __half*)W.p3,
-                                                              (int)(W.cols / 256), (int)W.rows, x.qs, x.d, T, y, ldy,
-                                                              out_scale, softcap, grp);
+            launch_pdl(qgemv_q6k_kernel<NT, R>, grid, dim3(GEMV_WARPS * 32), 0, s, (const uint8_t*)W.p0, (const uint8_t*)W.p1, (const int8_t*)W.p2, (const __half*)W.p3,
+                                                                      (int)(W.cols / 256), (int)W.rows, x.qs, x.d, T, y, ldy, out_scale, softcap, grp);
             break;
         case QT_Q8_0:
-            qgemv_q80_kernel<<<grid, GEMV_WARPS * 32, 0, s>>>((const int8_t*)W.p0, (const __half*)W.p1, (int)W.cols,
-                                                              (int)W.rows, x.qs, x.d, T, y, ldy, out_scale, softcap, grp);
+            launch_pdl(qgemv_q80_kernel<NT, R>, grid, dim3(GEMV_WARPS * 32), 0, s, (const int8_t*)W.p0, (const __half*)W.p1, (int)W.cols, (int)W.rows, x.qs, x.d, T, y, ldy, out_scale, softcap,
+                                                                      grp);
             break;
         default:
             throw std::runtime_error("launch_qgemv: unsupported weight type");
     }
+}
+
+static void launch_qgemv_impl(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap,
+                              int experts, Group grp, cudaStream_t s) {
+    // several output rows per warp only while there are warps for every scheduler all the same
+    const bool many = W.rows * experts >= 148 * 4 * 8 * 4;
+    if (grp.offsets != nullptr || (!many && T > 4)) launch_qgemv_rows<NT_MAX, 1>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
+    else if (!many && T == 1) launch_qgemv_rows<1, 1>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
+    else if (!many) launch_qgemv_rows<4, 1>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
+    else if (T == 1) launch_qgemv_rows<1, 4>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
+    else if (T <= 4) launch_qgemv_rows<4, 2>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
+    else launch_qgemv_rows<NT_MAX, 2>(W, x, T, y, ldy, out_scale, softcap, experts, grp, s);
     MK_LAUNCH_CHECK();
 }
 
@@ -310,8 +427,15 @@ void launch_qgemv_grouped(const QWeight& W, int experts, const int32_t* offsets,
 
 void launch_f32_gemv(const float* W, int out, int in, const float* x, int T, float* y, cudaStream_t s) {
     if (T <= 0) return;
-    dim3 grid((unsigned)((out + GEMV_WARPS - 1) / GEMV_WARPS), (unsigned)((T + F32_GEMV_ROWS - 1) / F32_GEMV_ROWS));
-    f32_gemv_kernel<<<grid, GEMV_WARPS * 32, 0, s>>>(W, out, in, x, T, y);
+    const unsigned runs = (unsigned)((T + F32_GEMV_ROWS - 1) / F32_GEMV_ROWS);
+    // the wide form once its warps (an eighth as many) still give every SM's schedulers one
+    if ((int64_t)runs * out / F32_WIDE_OUT >= 148 * 4) {
+        launch_pdl(f32_gemv_wide_kernel, dim3((unsigned)((out + GEMV_WARPS * F32_WIDE_OUT - 1) / (GEMV_WARPS * F32_WIDE_OUT)), runs), dim3(GEMV_WARPS * 32), 0, s, W, out, in, x, T, y);
+        MK_LAUNCH_CHECK();
+        return;
+    }
+    dim3 grid((unsigned)((out + GEMV_WARPS - 1) / GEMV_WARPS), runs);
+    launch_pdl(f32_gemv_kernel, grid, dim3(GEMV_WARPS * 32), 0, s, W, out, in, x, T, y);
     MK_LAUNCH_CHECK();
 }
 
