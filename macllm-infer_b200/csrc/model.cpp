@@ -279,9 +279,10 @@ void Model::ep_init(const uint8_t* id) {
 // MACLLM_B200_MOE_CHUNK=16|32|64 pins it.
 static int moe_chunk_rows(int T, int k, int experts) {
     static const int pinned = [] { const char* e = std::getenv("MACLLM_B200_MOE_CHUNK"); return e ? atoi(e) : 0; }();
-    if (pinned == 16 || pinned == 32 || pinned == 64) return pinned;
+    if (pinned == 16 || pinned == 32 || pinned == 64 || pinned == 128) return pinned;
     const double avg = (double)T * k / std::max(experts, 1);
-    return avg <= 6.0 ? 16 : (avg <= 14.0 ? 32 : 64);
+    // above 64 rows by two deviations of the routed counts, one pass over the expert's weights instead of two
+    return avg <= 6.0 ? 16 : (avg <= 14.0 ? 32 : (avg <= 48.0 ? 64 : 128));
 }
 
 // One MoE layer's experts under data-parallel expert parallelism: this rank's routed rows (grouped by expert, f16) go to

@@ -31,7 +31,8 @@
 // Expert-grouped form (sparse-MoE layers): the matrix is a bank of experts, the activation rows are grouped by expert,
 // and the row ranges live on the device (they come from the routing kernels of the same forward).  Warp 0 first builds
 // this CTA's share of the job list - (expert, chunk of up to BN of its rows, group of row tiles) - from the ranges, with
-// no host round trip; a job then runs like a whole group of the plain form.
+// no host round trip; a job then runs like a whole group of the plain form.  Chunks are up to 128 rows wide (two accumulators): every
+// chunk converts the expert's weights again, and the converters set the pace.
 // Q4_K arithmetic: sc * q (an integer below 1024) is formed exactly, then w = fma(sc * q, d, -f16(dmin * m)): the f16
 // weight carries the rounding of the product and that of dmin * m.  Q6_K: w = (q - 32) * f16(d * sc).
 // Every mbarrier wait is bounded; a wait that gives up records a status word and the role leaves its loop.
@@ -50,10 +51,12 @@ constexpr int QS_CONV_WARPS = 16;
 constexpr int QS_EPI_WARPS = 8;
 constexpr int QS_THREADS = (3 + QS_CONV_WARPS + QS_EPI_WARPS) * 32;  // 864
 constexpr int QS_MAX_STAGES = 8;
-constexpr int QS_X_STAGES = 3;    // activation blocks in flight (L2 latency)
+constexpr int qs_x_stages(int bn) { return bn <= 64 ? 3 : 2; }    // activation blocks in flight (L2 latency)
 constexpr int QS_Q4K_UNIT = QS_BM * 144;                         // 18432
 constexpr int QS_Q6K_UNIT = QS_BM * (128 + 64 + 16) + 256;       // 26880: ql, qh, scales planes + d (f16, padded)
-constexpr int QS_ACC = 4;                                        // accumulators in tensor memory
+constexpr int QS_ACC = 4;                                        // most accumulators in tensor memory
+constexpr int qs_accumulators(int bn) { return bn <= 64 ? QS_ACC : 2; }
+constexpr int QS_SMEM_LIMIT = 212 * 1024;                        // rings of the widest form, beside 8 KB of job table
 constexpr uint32_t QS_SPIN_LIMIT = 1u << 22;
 constexpr uint32_t QS_TMEM_COLS = 512;
 constexpr uint32_t QS_A_COL0 = 256;                              // two A buffers of 128 columns
@@ -279,6 +282,7 @@ struct QsParams {
 template <int BN>
 struct QsSmem {
     static constexpr int X_BYTES = 4 * BN * 128;   // four 64-column boxes
+    static constexpr int X_STAGES = qs_x_stages(BN), ACC = qs_accumulators(BN);
 };
 
 __device__ __forceinline__ float act_fn(float g, int act) {
@@ -310,6 +314,7 @@ template <int BN, bool PROF, bool GROUPED>
 __global__ void __launch_bounds__(QS_THREADS, 1)
 qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
     using L = QsSmem<BN>;
+    constexpr int QS_X_STAGES = L::X_STAGES;
     long long prof_acc[4] = {0, 0, 0, 0};
     const long long prof_t0 = PROF ? clock64() : 0;
     __shared__ uint32_t tlog[PROF ? 5 : 1][PROF ? 400 : 1];
@@ -327,7 +332,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
     uint64_t* a_full = x_empty + QS_X_STAGES;               // [2]   converters -> MMA
     uint64_t* a_empty = a_full + 2;                         // [2]   MMA -> converters
     uint64_t* acc_full = a_empty + 2;                       // [4]   MMA -> epilogue
-    uint64_t* acc_empty = acc_full + QS_ACC;                // [4]   epilogue -> MMA
+    uint64_t* acc_empty = acc_full + QS_ACC;                // [4]   epilogue -> MMA (wide form: two of each)
     uint64_t* tmem_ready = acc_empty + QS_ACC;              // [1]   allocating warp -> everyone
     __shared__ uint32_t tmem_base_slot;
 
@@ -399,7 +404,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
         i1 = (int)((int64_t)(c + 1) * p.items / C);
     }
     const int g0 = i0 / nb, b0 = i0 - g0 * nb;       // the only division of the item walk: (g, b) advance by counting
-    const int acc_shift = R == 1 ? 2 : (R == 2 ? 1 : 0);  // QS_ACC / R accumulator sets
+    const int acc_sets = L::ACC / R, acc_shift = acc_sets == 4 ? 2 : (acc_sets == 2 ? 1 : 0);
     const int n_stages = p.n_stages;
     // row tile r of group g: its index inside its matrix, whether it exists, and the index of its first unit
     const int tiles_limit = GROUPED ? p.tiles_pe : p.row_tiles;
@@ -415,7 +420,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
         else if (lane >= 24 && lane < 26) mbar_init(&a_full[lane - 24], QS_CONV_WARPS / 2);
         else if (lane >= 26 && lane < 28) mbar_init(&a_empty[lane - 26], 1);
         else if (lane == 28) mbar_init(tmem_ready, 1);
-        if (lane < QS_ACC) {
+        if (lane < L::ACC) {
             mbar_init(&acc_full[lane], 1);
             mbar_init(&acc_empty[lane], QS_EPI_WARPS);
         }
@@ -492,7 +497,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
             const bool first = it == i0 || b == 0, last = it + 1 == i1 || b + 1 == nb;
             if (!QS_WAIT(0, &x_full[xs], xph)) { if (lane == 0) atomicExch(p.status, 24); break; }
             QS_LOG(1, 1);
-            const int set = piece & ((QS_ACC >> (2 - acc_shift)) - 1), set_use = piece >> acc_shift;
+            const int set = piece & (acc_sets - 1), set_use = piece >> acc_shift;
             const uint64_t b_stage = b_desc0 + (uint64_t)((xs * L::X_BYTES) >> 4);
             for (int r = 0; r < R; ++r) {
                 if (tile_of(g, r) >= tiles_limit) break;
@@ -608,7 +613,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
         // share a tile's token columns (first half / second half)
         const int quad = warp & 3, chalf = (warp - 3 - QS_CONV_WARPS) >> 2;
         const int row_in_tile = quad * 32 + lane;
-        constexpr int CH = BN >= 64 ? 32 : (BN >= 32 ? 16 : 8);  // token columns per warp and tile
+        constexpr int CH = BN >= 64 ? 32 : (BN >= 32 ? 16 : 8);  // token columns a warp takes of a tile at a time
         int g = g0, b = b0, piece = 0;
         uint32_t tmem_base = 0;
         auto cta_of_item = [&](int i) {
@@ -625,7 +630,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
                     if (!mbar_wait(tmem_ready, 0, QS_SPIN_LIMIT)) { if (lane == 0) atomicExch(p.status, 29); break; }
                     tmem_base = *reinterpret_cast<volatile uint32_t*>(&tmem_base_slot);
                 }
-                const int set = piece & ((QS_ACC >> (2 - acc_shift)) - 1), set_use = piece >> acc_shift;
+                const int set = piece & (acc_sets - 1), set_use = piece >> acc_shift;
                 // split results: this piece's slot of the scratch
                 int my_slot = 0;
                 if (p.mode == 0 && p.slots > 1) my_slot = c - cta_of_item(g * nb);
@@ -644,8 +649,8 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
                     if (warp == 3 + QS_CONV_WARPS) QS_LOG(4, 1);
                     const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)slot * BN;
                     const int row = tile * QS_BM + row_in_tile;
-                    {
-                        const int c0 = chalf * CH;
+#pragma unroll 1
+                    for (int c0 = chalf * (BN / 2); c0 < (chalf + 1) * (BN / 2); c0 += CH) {
                         uint32_t v[CH];
                         if constexpr (CH == 32) tmem_ld32(t_acc + c0, v);
                         else if constexpr (CH == 16) tmem_ld16(t_acc + c0, v);
@@ -764,16 +769,22 @@ __global__ void retile_q6k_kernel(const uint8_t* ql, const uint8_t* qh, const ui
 
 template <int BN>
 size_t qs_smem_bytes(int n_stages, int stage_bytes) {
-    return (size_t)QS_X_STAGES * QsSmem<BN>::X_BYTES + (size_t)n_stages * stage_bytes + 64 * sizeof(uint64_t) + 1024;
+    return (size_t)QsSmem<BN>::X_STAGES * QsSmem<BN>::X_BYTES + (size_t)n_stages * stage_bytes + 64 * sizeof(uint64_t) + 1024;
+}
+
+template <int BN>
+void launch_qs_grouped(const CUtensorMap& tx, const QsParams& p, int ctas, cudaStream_t s) {
+    const size_t smem = qs_smem_bytes<BN>(p.n_stages, p.stage_bytes);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(&qstream_tc_kernel<BN, false, true>), smem);
+    launch_pdl(qstream_tc_kernel<BN, false, true>, dim3(ctas), dim3(QS_THREADS), smem, s, tx, p);
+    MK_LAUNCH_CHECK();
 }
 
 template <int BN>
 void launch_qs(const CUtensorMap& tx, const QsParams& p, int ctas, cudaStream_t s) {
+    if (p.grouped) return launch_qs_grouped<BN>(tx, p, ctas, s);
     const size_t smem = qs_smem_bytes<BN>(p.n_stages, p.stage_bytes);
-    if (p.grouped) {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(&qstream_tc_kernel<BN, false, true>), smem);
-        launch_pdl(qstream_tc_kernel<BN, false, true>, dim3(ctas), dim3(QS_THREADS), smem, s, tx, p);
-    } else if (p.prof != nullptr) {
+    if (p.prof != nullptr) {
         ensure_dynamic_smem(reinterpret_cast<const void*>(&qstream_tc_kernel<BN, true, false>), smem);
         launch_pdl(qstream_tc_kernel<BN, true, false>, dim3(ctas), dim3(QS_THREADS), smem, s, tx, p);
     } else {
@@ -916,7 +927,7 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
     p.fmt_a = W.fmt;
     p.fmt_b = W2 ? W2->fmt : W.fmt;
     p.stage_bytes = (p.fmt_a || p.fmt_b) ? QS_Q6K_UNIT : QS_Q4K_UNIT;
-    const size_t x_bytes = (size_t)QS_X_STAGES * 4 * pl.bn * 128;
+    const size_t x_bytes = (size_t)qs_x_stages(pl.bn) * 4 * pl.bn * 128;
     p.n_stages = (int)std::min<size_t>(QS_MAX_STAGES, ((size_t)200 * 1024 - x_bytes) / (size_t)p.stage_bytes);
     p.mode = gated ? 1 : 0;
     p.act = gated ? gated_act : 0;
@@ -948,9 +959,9 @@ int launch_qstream_tc_grouped(const QStreamWeight& W, int experts, const int32_t
     if (gated && (!W.gated || yh == nullptr)) throw std::runtime_error("launch_qstream_tc_grouped: the gated form needs an interleaved gate|up bank and an f16 output");
     const int nb = (int)(W.cols / 256);
     const int tiles_pe = (int)(W.rows / experts / QS_BM);
-    const int bound = std::max(1, std::min(max_rows_per_expert, kQStreamMaxRows));
-    const int bn = bound <= 16 ? 16 : (bound <= 32 ? 32 : 64);
-    const int R = tiles_pe % 2 == 0 ? 2 : 1;
+    const int bn = max_rows_per_expert <= 16 ? 16 : (max_rows_per_expert <= 32 ? 32 : (max_rows_per_expert <= 64 ? 64 : 128));
+    // two accumulators of 128 columns: a row tile at a time, so that its epilogue runs under the next one's products
+    const int R = tiles_pe % 2 == 0 && bn <= 64 ? 2 : 1;
     const int sms = device_sm_count();
     // a bound on the jobs any CTA is handed: every expert may add one partly filled chunk
     const int64_t max_jobs = ((int64_t)rows_total / bn + experts) * (tiles_pe / R);
@@ -970,8 +981,8 @@ int launch_qstream_tc_grouped(const QStreamWeight& W, int experts, const int32_t
     p.tiles_a = W.row_tiles;
     p.fmt_a = p.fmt_b = W.fmt;
     p.stage_bytes = W.fmt ? QS_Q6K_UNIT : QS_Q4K_UNIT;
-    const size_t x_bytes = (size_t)QS_X_STAGES * 4 * bn * 128;
-    p.n_stages = (int)std::min<size_t>(QS_MAX_STAGES, ((size_t)200 * 1024 - x_bytes) / (size_t)p.stage_bytes);
+    const size_t x_bytes = (size_t)qs_x_stages(bn) * 4 * bn * 128;
+    p.n_stages = (int)std::min<size_t>(QS_MAX_STAGES, ((size_t)(bn <= 64 ? 200 * 1024 : QS_SMEM_LIMIT) - x_bytes) / (size_t)p.stage_bytes);
     p.grouped = 1;
     p.experts = experts;
     p.tiles_pe = tiles_pe;
@@ -988,7 +999,8 @@ int launch_qstream_tc_grouped(const QStreamWeight& W, int experts, const int32_t
     p.prof = nullptr;
     if (bn == 16) launch_qs<16>(tx, p, sms, s);
     else if (bn == 32) launch_qs<32>(tx, p, sms, s);
-    else launch_qs<64>(tx, p, sms, s);
+    else if (bn == 64) launch_qs<64>(tx, p, sms, s);
+    else launch_qs_grouped<128>(tx, p, sms, s);
     return 1;
 }
 

@@ -52,7 +52,7 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
 // Expert-grouped form: W is a bank of `experts` matrices stacked by rows (each a whole number of 128-row tiles);
 // activation rows [offsets[e], offsets[e + 1]) of xh [rows_total][cols] (grouped by expert, device array of experts + 1
 // row numbers) are multiplied by expert e's matrix: y[r][n] for those rows r and n < rows per expert, or, gated,
-// yh[r][f].  max_rows_per_expert picks the chunk width (16, 32 or 64 rows): an expert's rows are processed a chunk at a
+// yh[r][f].  max_rows_per_expert picks the chunk width (16, 32, 64 or 128 rows): an expert's rows are processed a chunk at a
 // time, each chunk one pass over the expert's matrix, so any width is correct for any row count.  The kernel reads the
 // row ranges on the device: no host round trip.  rows_known = false: rows_total is only the extent of xh (the true row
 // count lives on the device); the host then cannot bound the jobs per CTA, and a launch that overflows the kernel's job

@@ -287,30 +287,36 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float* log
 // src/decoder.rs:474-483).  Here such a row records kMoeRouteStatus | row in *status, which fails the forward at its
 // completion barrier, and the offending values compete as the lowest finite number, so that the k choices written
 // are always k distinct experts in range and nothing downstream indexes out of bounds.
+// PER_LANE: candidates a lane can hold, in registers (with the length known only at run time they were in local memory: 31 -> 7 us for
+// 1420 rows of 128 experts).  A pick stays with the lane of its number until all are made, 32 picks at a time.
+template <int PER_LANE>
 __global__ void __launch_bounds__(128) moe_route_kernel(const float* logits, int T, int experts, int k,
                                                         int32_t* sel_experts, float* sel_weights, int32_t* status) {
+    pdl_trigger();
+    pdl_wait();
     int t = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (t >= T) return;
     int lane = threadIdx.x & 31;
     const float* row = logits + (int64_t)t * experts;
-    constexpr int MAX_PER_LANE = 32;
-    float v[MAX_PER_LANE];
-    int cnt = 0;
+    float v[PER_LANE];
     bool bad = false;
-    for (int e = lane; e < experts && cnt < MAX_PER_LANE; e += 32, ++cnt) {
-        float x = row[e];
+#pragma unroll
+    for (int c = 0; c < PER_LANE; ++c) {
+        const int e = lane + 32 * c;
+        float x = e < experts ? row[e] : 0.f;
         if (!isfinite(x)) { bad = true; x = -3.402823466e38f; }
-        v[cnt] = x;
+        v[c] = x;
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0 && status != nullptr) atomicCAS(status, 0, kMoeRouteStatus | (t & 0xFFFF));
     unsigned taken = 0;  // bit c set when this lane's c-th candidate was selected
-    float mx = -INFINITY;
+    float mx = -INFINITY, my_pick = 0.f;
     for (int i = 0; i < k; ++i) {
         float bv = -INFINITY;
         int be = INT_MAX;
-        for (int c = 0; c < cnt; ++c) {
-            if (taken >> c & 1u) continue;
+#pragma unroll
+        for (int c = 0; c < PER_LANE; ++c) {
             int e = lane + 32 * c;
+            if ((taken >> c & 1u) || e >= experts) continue;
             if (v[c] > bv || (v[c] == bv && e < be)) { bv = v[c]; be = e; }
         }
 #pragma unroll
@@ -321,10 +327,22 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* logits, int
         }
         if ((be & 31) == lane) taken |= 1u << (be >> 5);
         if (i == 0) mx = bv;  // the first pick is the maximum of the selected set
-        if (lane == 0) { sel_experts[(int64_t)t * k + i] = be; sel_weights[(int64_t)t * k + i] = bv; }
+        if (lane == 0) sel_experts[(int64_t)t * k + i] = be;
+        if (k <= 32) {
+            if (lane == i) my_pick = bv;
+        } else if (lane == 0) {
+            sel_weights[(int64_t)t * k + i] = bv;
+        }
+    }
+    // softmax over the selected logits: exp(l - max) / sum in selection order
+    if (k <= 32) {
+        const float e = expf(my_pick - mx);
+        float den = 0.f;
+        for (int i = 0; i < k; ++i) den += __shfl_sync(0xffffffffu, e, i);
+        if (lane < k) sel_weights[(int64_t)t * k + lane] = e / den;
+        return;
     }
     __syncwarp();
-    // softmax over the selected logits: exp(l - max) / sum in selection order
     if (lane == 0) {
         float den = 0.f;
         for (int i = 0; i < k; ++i) den += expf(sel_weights[(int64_t)t * k + i] - mx);
@@ -361,7 +379,8 @@ void launch_moe_route(const float* logits, int T, int experts, int k, int32_t* s
     if (T <= 0) return;
     if (experts > 1024) throw std::runtime_error("launch_moe_route: more than 1024 experts");
     if (k <= 0 || k > experts) throw std::runtime_error("experts per token " + std::to_string(k) + " must be in 1..=" + std::to_string(experts));  // src/decoder.rs:456-458
-    moe_route_kernel<<<(T + 3) / 4, 128, 0, s>>>(logits, T, experts, k, sel_experts, sel_weights, status);
+    auto* kernel = experts <= 64 ? moe_route_kernel<2> : (experts <= 128 ? moe_route_kernel<4> : (experts <= 256 ? moe_route_kernel<8> : moe_route_kernel<32>));
+    launch_pdl(kernel, dim3((unsigned)((T + 3) / 4)), dim3(128), 0, s, logits, T, experts, k, sel_experts, sel_weights, status);
     MK_LAUNCH_CHECK();
 }
 
