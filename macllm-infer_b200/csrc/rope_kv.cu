@@ -5,7 +5,7 @@
 // the first rotary_dim dims) and PagedKvBatchReservation::write_layer
 // (crates/macllm-kv/src/cache.rs:2543-2643): K is stored after the rotation, V unmodified, both at
 // KV-head cardinality, token at slot block*block_tokens + row.
-// One warp per (token, head); the head vector is staged in shared memory so any head_dim works.
+// One warp per (token, head), the head vector staged in shared memory so any head_dim works; the usual widths a few heads per warp in registers.
 #include "kernels.h"
 #include "rope_head.cuh"
 #include <algorithm>
@@ -50,6 +50,106 @@ __global__ void __launch_bounds__(RK_WARPS * 32) rope_kv_kernel(RopeKvArgs a) {
         int64_t base = ((kv_page_index(blk, a.layer, a.layers, a.pool_blocks) * a.kv_heads + hh) * a.block_tokens + row) * (int64_t)d;
         KV* pool = reinterpret_cast<KV*>(kind == 1 ? a.k_pool : a.v_pool);
         for (int i = lane; i < d; i += 32) pool[base + i] = to_kv<KV>(x[i]);
+    }
+}
+
+// Heads of 32 J dimensions that turn whole (or not at all), from whole projections: a warp takes U heads of a token, lane l the dimensions
+// l + 32 j.  Both halves of a half-split pair are then the lane's own, the angles serve all U heads, and nothing passes through shared memory.
+// The sums run as in rope_head.cuh, so both give the same bits.  Bound by HBM; with a warp per head, each waiting for its own load,
+// position, slot and angles in turn, 1420 rows of 40 heads took 34 us, this 19.
+template <typename KV, int J, int U>
+__global__ void __launch_bounds__(RK_WARPS * 32) rope_kv_whole_kernel(RopeKvArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, heads_total = a.q_heads + 2 * a.kv_heads, runs = (heads_total + U - 1) / U;
+    const int64_t item = (int64_t)blockIdx.x * RK_WARPS + (threadIdx.x >> 5);
+    const int t = (int)(item / runs), h0 = (int)(item - (int64_t)t * runs) * U;
+    if (t >= a.T) return;
+    constexpr int D = 32 * J;
+    float x[U][J];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int h = min(h0 + u, heads_total - 1), k = h - a.q_heads, v = k - a.kv_heads;
+        const float* src = k < 0 ? a.q + (int64_t)t * a.ldq + h * D : (v < 0 ? a.k + (int64_t)t * a.ldk + k * D : a.v + (int64_t)t * a.ldv + v * D);
+#pragma unroll
+        for (int j = 0; j < J; ++j) x[u][j] = src[lane + 32 * j];
+    }
+    const bool turns = a.cos_t != nullptr;
+    float c[J], s[J];  // half-split: the first J / 2 count
+    if (turns) {
+        const int64_t at = (int64_t)a.positions[t] * (D / 2);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            if (!a.interleaved && j >= J / 2) break;
+            const int i = a.interleaved ? (lane >> 1) + 16 * j : lane + 32 * j;
+            c[j] = a.cos_t[at + i];
+            s[j] = a.sin_t[at + i];
+        }
+    }
+    const int64_t slot = a.slots[t], blk = slot / a.block_tokens, row = slot - blk * a.block_tokens;
+    const int64_t page = kv_page_index(blk, a.layer, a.layers, a.pool_blocks) * a.kv_heads;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int h = h0 + u, k = h - a.q_heads, v = k - a.kv_heads;
+        if (h >= heads_total) break;
+        const float* bias = k < 0 ? a.q_bias : (v < 0 ? a.k_bias : a.v_bias);
+        if (bias != nullptr) {
+            bias += (k < 0 ? h : (v < 0 ? k : v)) * D;
+#pragma unroll
+            for (int j = 0; j < J; ++j) x[u][j] += bias[lane + 32 * j];
+        }
+        const float* nw = k < 0 ? a.q_norm_w : (v < 0 ? a.k_norm_w : nullptr);
+        if (nw != nullptr) {
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < J; ++j) ss += x[u][j] * x[u][j];
+            ss = warp_sum(ss);
+            const float m = sqrtf(ss / (float)D + a.norm_eps);
+#pragma unroll
+            for (int j = 0; j < J; ++j) x[u][j] = x[u][j] / m * nw[lane + 32 * j];
+        }
+        if (v < 0 && turns) {
+            if (a.interleaved) {
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    const float other = __shfl_xor_sync(0xffffffffu, x[u][j], 1);
+                    x[u][j] = (lane & 1) ? __fadd_rn(__fmul_rn(other, s[j]), __fmul_rn(x[u][j], c[j])) : __fsub_rn(__fmul_rn(x[u][j], c[j]), __fmul_rn(other, s[j]));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < J / 2; ++j) {
+                    const float x1 = x[u][j], x2 = x[u][j + J / 2];
+                    x[u][j] = __fsub_rn(__fmul_rn(x1, c[j]), __fmul_rn(x2, s[j]));
+                    x[u][j + J / 2] = __fadd_rn(__fmul_rn(x1, s[j]), __fmul_rn(x2, c[j]));
+                }
+            }
+        }
+        if (k < 0) {
+            float* dst = a.q_out != nullptr ? a.q_out + (int64_t)t * a.ldq_out + h * D : a.q + (int64_t)t * a.ldq + h * D;
+#pragma unroll
+            for (int j = 0; j < J; ++j) dst[lane + 32 * j] = x[u][j];
+        } else {
+            KV* pool = reinterpret_cast<KV*>(v < 0 ? a.k_pool : a.v_pool) + ((page + (v < 0 ? k : v)) * a.block_tokens + row) * D;
+#pragma unroll
+            for (int j = 0; j < J; ++j) pool[lane + 32 * j] = to_kv<KV>(x[u][j]);
+        }
+    }
+}
+
+template <typename KV>
+bool launch_rope_whole(const RopeKvArgs& a, cudaStream_t s) {
+    const int row = rope_row_width(a);
+    if (a.qk_splits > 1 || a.v_splits > 1 || row != a.d || (a.dv > 0 && a.dv != a.d) || (a.cos_t != nullptr && a.rotary_dim != a.d)) return false;
+    constexpr int U = 4;
+    auto launch = [&](auto* kernel, int per) {
+        const int64_t warps = (int64_t)a.T * ((a.q_heads + 2 * a.kv_heads + per - 1) / per);
+        launch_pdl(kernel, dim3((unsigned)((warps + RK_WARPS - 1) / RK_WARPS)), dim3(RK_WARPS * 32), 0, s, a);
+    };
+    switch (a.d) {
+        case 64: launch(rope_kv_whole_kernel<KV, 2, U>, U); return true;
+        case 128: launch(rope_kv_whole_kernel<KV, 4, U>, U); return true;
+        case 256: launch(rope_kv_whole_kernel<KV, 8, U / 2>, U / 2); return true;
+        default: return false;
     }
 }
 
@@ -173,6 +273,10 @@ void launch_rope_kv(const RopeKvArgs& a, cudaStream_t s) {
     if (a.d_row > 0 && (a.d_row < a.d || a.d_row < a.dv || a.q_out == nullptr))
         throw std::runtime_error("launch_rope_kv: padded heads need a separate query output at least as wide as the heads");
     int heads_total = a.q_heads + 2 * a.kv_heads;
+    if (a.kv_f16 ? launch_rope_whole<__half>(a, s) : launch_rope_whole<float>(a, s)) {
+        MK_LAUNCH_CHECK();
+        return;
+    }
     dim3 grid((unsigned)a.T, (unsigned)((heads_total + RK_WARPS - 1) / RK_WARPS));
     if (a.kv_f16)
         launch_pdl(rope_kv_kernel<__half>, grid, dim3(RK_WARPS * 32), 0, s, a);
