@@ -759,6 +759,9 @@ int32_t mk_k_penalties(float* logits, int32_t vocab, const uint32_t* history, in
  * kernel (greedy rows, or 1 <= top_k <= 1024).  Both use the same arithmetic and return the same tokens. */
 int32_t mk_k_sample(const float* logits, int32_t B, int32_t vocab, const mk_lane_sampling* settings, int32_t where, uint32_t* out);
 
+/* The router's product in f32: y[T][experts] = x[T][cols] . w[experts][cols]^T (host memory).  A row's results do not depend on T. */
+int32_t mk_k_router_logits(const float* w, int32_t experts, int32_t cols, const float* x, int32_t T, float* y);
+
 /* selected_softmax_routes (src/decoder.rs:448-554): sel_experts / sel_weights are [T][k], best first. */
 int32_t mk_k_moe_route(const float* logits, int32_t T, int32_t experts, int32_t k, int32_t* sel_experts, float* sel_weights);
 

@@ -267,6 +267,7 @@ SIGNATURES = {
     "mk_rotary_frequencies": (_i32, [_i32, C.c_double, P, P]),
     "mk_rotary_frequencies_yarn": (_i32, [_i32, C.c_double, C.c_double, C.c_double, C.c_double, C.c_double, P, P]),
     "mk_state_slots_query": (_i32, [P, C.POINTER(_i32), C.POINTER(_i32)]),
+    "mk_k_router_logits": (_i32, [P, _i32, _i32, P, _i32, P]),
     "mk_k_moe_route": (_i32, [P, _i32, _i32, _i32, P, P]),
 }
 

@@ -866,6 +866,20 @@ int32_t mk_k_sample(const float* logits, int32_t B, int32_t vocab, const mk_lane
     });
 }
 
+int32_t mk_k_router_logits(const float* w, int32_t experts, int32_t cols, const float* x, int32_t T, float* y) {
+    return guarded([&] {
+        require_device();
+        if (T <= 0 || experts <= 0 || cols <= 0) throw std::runtime_error("mk_k_router_logits: bad arguments");
+        DevBuf dw((size_t)experts * cols * 4), dx((size_t)T * cols * 4), dy((size_t)T * experts * 4);
+        dw.upload(w, (size_t)experts * cols * 4);
+        dx.upload(x, (size_t)T * cols * 4);
+        launch_f32_gemv(dw.as<float>(), experts, cols, dx.as<float>(), T, dy.as<float>(), nullptr);
+        MK_CUDA(cudaDeviceSynchronize());
+        dy.download(y, (size_t)T * experts * 4);
+        MK_CUDA(cudaDeviceSynchronize());
+    });
+}
+
 int32_t mk_k_moe_route(const float* logits, int32_t T, int32_t experts, int32_t k, int32_t* sel_experts, float* sel_weights) {
     return guarded([&] {
         require_device();

@@ -21,6 +21,9 @@ __device__ __forceinline__ void mc_cp_async16(void* dst, const void* src, bool v
     const int bytes = valid ? 16 : 0;  // 0: the 16 bytes become zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mc_smem(dst)), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void mc_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // x and y as bfloat16 numbers, and what that left of them.
 __device__ __forceinline__ void mc_split(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);

@@ -13,6 +13,8 @@
 // eight sums whatever T, 32000 x 2048 in Q6_K took 26 us at one activation row,
 // this 15).
 #include "kernels.h"
+#include "mma_bf16.cuh"
+#include <algorithm>
 
 namespace mk {
 
@@ -335,44 +337,83 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_kernel(const float* 
     }
 }
 
-// The same sums for many rows: a warp takes F32_GEMV_ROWS rows and F32_WIDE_OUT outputs, so that a value of x or W that was fetched meets
-// eight others instead of one.  Bound by the L1's load rate and the FMA pipe alike (128 outputs x 2048 for 1420 rows: 90 -> 50 us).
-constexpr int F32_WIDE_OUT = 8;
-__global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_wide_kernel(const float* __restrict__ W, int out, int in, const float* __restrict__ x, int T,
-                                                                        float* __restrict__ y) {
+// The same sums for many rows.  A CTA of 4 x 4 warps takes F32_TILE_OUT outputs and 4 R rows, a warp eight of the outputs with R of the rows: a
+// value of x meets eight others and one of W meets R.  Both pass through shared memory, F32_TILE_K columns at a time and F32_TILE_STAGES - 1
+// of these on their way, because what bounds the plain loads is that a warp can't have enough of them under way beside 64 sums; the tile
+// is nearly square because the L2 then bounds the copies (1420 rows x 128 outputs x 2048: 64 us with eight rows and outputs per warp
+// straight from the L1, 34 with tiles of 128 x 10, this 28; the multiply-adds take 11).
+// A lane's columns and their order are those of the kernel above, columns behind the end are zeros: the same bits.
+constexpr int F32_TILE_OUT = 32, F32_TILE_K = 64, F32_TILE_STAGES = 4, F32_TILE_WARPS = 16, F32_WARP_OUT = 8;
+template <int R>
+__global__ void __launch_bounds__(F32_TILE_WARPS * 32) f32_gemv_tile_kernel(const float* __restrict__ W, int out, int in, const float* __restrict__ x, int T,
+                                                                            float* __restrict__ y) {
+    extern __shared__ __align__(16) float f32_tile[];
+    constexpr int ROWS = 4 * R, STAGE = (F32_TILE_OUT + ROWS) * F32_TILE_K, VECS = F32_TILE_K / 4;
     pdl_trigger();
-    pdl_wait();
-    const int n0 = (blockIdx.x * GEMV_WARPS + (int)(threadIdx.x >> 5)) * F32_WIDE_OUT, t0 = (int)blockIdx.y * F32_GEMV_ROWS, lane = threadIdx.x & 31;
-    if (n0 >= out) return;
+    const int n0 = (int)blockIdx.x * F32_TILE_OUT, t0 = (int)blockIdx.y * ROWS, lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
+    const int wn = (warp & 3) * F32_WARP_OUT, wt = (warp >> 2) * R;   // this warp's first output and row of the tile
+    const int chunks = (in + F32_TILE_K - 1) / F32_TILE_K;
     // rows and outputs behind the end repeat the last one and are not stored
-    const float *xr[F32_GEMV_ROWS], *wr[F32_WIDE_OUT];
-#pragma unroll
-    for (int r = 0; r < F32_GEMV_ROWS; ++r) xr[r] = x + (int64_t)min(t0 + r, T - 1) * in;
-#pragma unroll
-    for (int j = 0; j < F32_WIDE_OUT; ++j) wr[j] = W + (int64_t)min(n0 + j, out - 1) * in;
-    float acc[F32_GEMV_ROWS][F32_WIDE_OUT] = {};
-#pragma unroll 2
-    for (int k = lane; k < in; k += 32) {
-        float xv[F32_GEMV_ROWS], wv[F32_WIDE_OUT];
-#pragma unroll
-        for (int r = 0; r < F32_GEMV_ROWS; ++r) xv[r] = xr[r][k];
-#pragma unroll
-        for (int j = 0; j < F32_WIDE_OUT; ++j) wv[j] = wr[j][k];
-#pragma unroll
-        for (int r = 0; r < F32_GEMV_ROWS; ++r)
-#pragma unroll
-            for (int j = 0; j < F32_WIDE_OUT; ++j) acc[r][j] += xv[r] * wv[j];
-    }
-#pragma unroll
-    for (int r = 0; r < F32_GEMV_ROWS; ++r) {
-        float mine = 0.f;
-#pragma unroll
-        for (int j = 0; j < F32_WIDE_OUT; ++j) {
-            const float v = warp_sum(acc[r][j]);
-            if (lane == j) mine = v;
+    auto fetch = [&](int c, bool weights) {
+        float* to = f32_tile + (c % F32_TILE_STAGES) * STAGE + (weights ? 0 : F32_TILE_OUT * F32_TILE_K);
+        for (int i = threadIdx.x; i < (weights ? F32_TILE_OUT : ROWS) * VECS; i += F32_TILE_WARPS * 32) {
+            const int row = i / VECS, k = c * F32_TILE_K + (i % VECS) * 4;
+            const float* from = weights ? W + (int64_t)min(n0 + row, out - 1) * in : x + (int64_t)min(t0 + row, T - 1) * in;
+            mc_cp_async16(to + i * 4, from + (k < in ? k : 0), k < in);
         }
-        if (lane < F32_WIDE_OUT && n0 + lane < out && t0 + r < T) y[(int64_t)(t0 + r) * out + n0 + lane] = mine;
+    };
+    for (int c = 0; c < F32_TILE_STAGES - 1 && c < chunks; ++c) fetch(c, true);   // the weights don't depend on the predecessor
+    pdl_wait();
+    for (int c = 0; c < F32_TILE_STAGES - 1; ++c) {
+        if (c < chunks) fetch(c, false);
+        mc_cp_commit();
     }
+    float acc[R][F32_WARP_OUT] = {};
+    for (int c = 0; c < chunks; ++c) {
+        mc_cp_wait<F32_TILE_STAGES - 2>();
+        __syncthreads();   // chunk c is here for everyone, and everyone is done with the one whose place the next takes
+        if (c + F32_TILE_STAGES - 1 < chunks) { fetch(c + F32_TILE_STAGES - 1, true); fetch(c + F32_TILE_STAGES - 1, false); }
+        mc_cp_commit();
+        const float* ws = f32_tile + (c % F32_TILE_STAGES) * STAGE + wn * F32_TILE_K + lane;
+        const float* xs = f32_tile + (c % F32_TILE_STAGES) * STAGE + (F32_TILE_OUT + wt) * F32_TILE_K + lane;
+#pragma unroll
+        for (int k = 0; k < F32_TILE_K; k += 32) {
+            float wv[F32_WARP_OUT];
+#pragma unroll
+            for (int j = 0; j < F32_WARP_OUT; ++j) wv[j] = ws[j * F32_TILE_K + k];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float xv = xs[r * F32_TILE_K + k];
+#pragma unroll
+                for (int j = 0; j < F32_WARP_OUT; ++j) acc[r][j] += xv * wv[j];
+            }
+        }
+    }
+    mc_cp_wait<0>();
+    // The warp's tree for eight outputs at once: each of its first three steps hands half of the sums to the other lane of the pair, the pairs
+    // and with them the bits are those of eight trees.
+    const int hi = lane >> 4, mid = (lane >> 3) & 1, lo = (lane >> 2) & 1;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        float a4[4], a2[2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a4[j] = (hi ? acc[r][j + 4] : acc[r][j]) + __shfl_xor_sync(0xffffffffu, hi ? acc[r][j] : acc[r][j + 4], 16);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) a2[j] = (mid ? a4[j + 2] : a4[j]) + __shfl_xor_sync(0xffffffffu, mid ? a4[j] : a4[j + 2], 8);
+        float v = (lo ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, lo ? a2[0] : a2[1], 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        const int n = n0 + wn + 4 * hi + 2 * mid + lo, t = t0 + wt + r;
+        if ((lane & 3) == 0 && n < out && t < T) y[(int64_t)t * out + n] = v;
+    }
+}
+
+template <int R>
+void launch_f32_tile(const float* W, int out, int in, const float* x, int T, float* y, cudaStream_t s) {
+    const size_t smem = (size_t)F32_TILE_STAGES * (F32_TILE_OUT + 4 * R) * F32_TILE_K * sizeof(float);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(&f32_gemv_tile_kernel<R>), smem);
+    launch_pdl(f32_gemv_tile_kernel<R>, dim3((unsigned)((out + F32_TILE_OUT - 1) / F32_TILE_OUT), (unsigned)((T + 4 * R - 1) / (4 * R))), dim3(F32_TILE_WARPS * 32),
+               smem, s, W, out, in, x, T, y);
 }
 
 }  // namespace
@@ -428,9 +469,15 @@ void launch_qgemv_grouped(const QWeight& W, int experts, const int32_t* offsets,
 void launch_f32_gemv(const float* W, int out, int in, const float* x, int T, float* y, cudaStream_t s) {
     if (T <= 0) return;
     const unsigned runs = (unsigned)((T + F32_GEMV_ROWS - 1) / F32_GEMV_ROWS);
-    // the wide form once its warps (an eighth as many) still give every SM's schedulers one
-    if ((int64_t)runs * out / F32_WIDE_OUT >= 148 * 4) {
-        launch_pdl(f32_gemv_wide_kernel, dim3((unsigned)((out + GEMV_WARPS * F32_WIDE_OUT - 1) / (GEMV_WARPS * F32_WIDE_OUT)), runs), dim3(GEMV_WARPS * 32), 0, s, W, out, in, x, T, y);
+    // Tiles once an eighth of this kernel's warps would still give every SM's schedulers one; they take as few rows as keep the CTAs to one per SM,
+    // 48 at most (the sums' registers).
+    if ((int64_t)runs * out / 8 >= 148 * 4 && in % 4 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
+        const int64_t columns = (out + F32_TILE_OUT - 1) / F32_TILE_OUT, rows = (T + std::max<int64_t>(148 / columns, 1) - 1) / std::max<int64_t>(148 / columns, 1);
+        if (rows <= 16) launch_f32_tile<4>(W, out, in, x, T, y, s);
+        else if (rows <= 24) launch_f32_tile<6>(W, out, in, x, T, y, s);
+        else if (rows <= 32) launch_f32_tile<8>(W, out, in, x, T, y, s);
+        else if (rows <= 40) launch_f32_tile<10>(W, out, in, x, T, y, s);
+        else launch_f32_tile<12>(W, out, in, x, T, y, s);
         MK_LAUNCH_CHECK();
         return;
     }

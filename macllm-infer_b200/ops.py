@@ -206,6 +206,14 @@ def argmax(logits) -> np.ndarray:
     return out
 
 
+def router_logits(w, x) -> np.ndarray:
+    """x . w^T in f32: the router's product."""
+    w, x = _f32(w), _f32(x)
+    y = np.empty((x.shape[0], w.shape[0]), dtype=np.float32)
+    capi.check(capi.lib().mk_k_router_logits(_p(w), w.shape[0], w.shape[1], _p(x), x.shape[0], _p(y)))
+    return y
+
+
 def moe_route(logits, k: int):
     logits = _f32(logits)
     T, E = logits.shape
