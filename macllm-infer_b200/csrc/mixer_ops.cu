@@ -78,9 +78,9 @@ __device__ __forceinline__ Pack<VEC> branch_pack(const RowUpdateArgs& a, int b, 
 }
 
 // The updated row into `dst` (shared memory): x + coef * (branches + bias).  Normed branches are staged in `dst` / `other` first.
-template <int VEC>
+template <int VEC, int THREADS>
 __device__ __forceinline__ void updated_row(const RowUpdateArgs& a, int64_t row, float* dst, float* other, float* red) {
-    const int step = RU_THREADS * VEC;
+    const int step = THREADS * VEC;
     float inv[2] = {1.f, 1.f};
     const bool normed = a.n_add > 0 && a.add_w[0] != nullptr;
     if (normed) {
@@ -129,9 +129,9 @@ __device__ __forceinline__ void updated_row(const RowUpdateArgs& a, int64_t row,
 struct RowStats {
     float mean = 0.f, root = 1.f;
 };
-template <int VEC>
+template <int VEC, int THREADS = RU_THREADS>
 __device__ __forceinline__ RowStats row_stats(const float* x, int width, float eps, float* red, bool centred = true) {
-    const int step = RU_THREADS * VEC;
+    const int step = THREADS * VEC;
     float s = 0.f;
     RowStats r;
     if (centred) {
@@ -168,8 +168,9 @@ __device__ __forceinline__ Pack<VEC> norm_pack(const RowUpdateArgs& a, const Row
 }
 
 // Shared memory: the row, its neighbour (n_mix > 0), and a staging row for a second normed branch.
-template <int VEC>
-__global__ void __launch_bounds__(RU_THREADS) row_update_kernel(RowUpdateArgs a) {
+// THREADS: twice as many where the rows leave SMs idle - a row's latency counts then, and with 2048 columns every thread has one pack.
+template <int VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS) row_update_kernel(RowUpdateArgs a) {
     extern __shared__ __align__(16) float ru_smem[];
     __shared__ float red[32];
     float* cur = ru_smem;
@@ -179,8 +180,8 @@ __global__ void __launch_bounds__(RU_THREADS) row_update_kernel(RowUpdateArgs a)
     pdl_wait();
     const int64_t r = blockIdx.x;
     const int64_t row = a.row_index ? a.row_index[r] : r;
-    const int step = RU_THREADS * VEC;
-    updated_row<VEC>(a, row, cur, other, red);
+    const int step = THREADS * VEC;
+    updated_row<VEC, THREADS>(a, row, cur, other, red);
     if (a.x_out != nullptr)
         for (int c = threadIdx.x * VEC; c < a.width; c += step) store_pack<VEC>(a.x_out + row * a.width + c, load_pack<VEC>(cur + c));
     if (a.raw.any()) {
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(RU_THREADS) row_update_kernel(RowUpdateArgs a)
     // a thread has written the columns of `cur` that it reads itself; block_sum's barriers are all the sums need
     RowStats st, st_prev;
     const bool stats = a.norm != NormKind::DynTanh, centred = a.norm == NormKind::Layer;
-    if (stats) st = row_stats<VEC>(cur, a.width, a.norm_eps, red, centred);
+    if (stats) st = row_stats<VEC, THREADS>(cur, a.width, a.norm_eps, red, centred);
     if (a.n_mix == 0) {
         for (int c = threadIdx.x * VEC; c < a.width; c += step) put_pack<VEC>(a.normed, r, c, norm_pack<VEC>(a, st, load_pack<VEC>(cur + c), c));
         zero_tail(a.normed, r, a.width);
@@ -202,8 +203,8 @@ __global__ void __launch_bounds__(RU_THREADS) row_update_kernel(RowUpdateArgs a)
     const int first = sl.first, last = sl.first + sl.n - 1;
     const bool inside = row > first;
     if (inside) {
-        updated_row<VEC>(a, row - 1, prv, other, red);
-        if (stats) st_prev = row_stats<VEC>(prv, a.width, a.norm_eps, red, centred);
+        updated_row<VEC, THREADS>(a, row - 1, prv, other, red);
+        if (stats) st_prev = row_stats<VEC, THREADS>(prv, a.width, a.norm_eps, red, centred);
     }
     for (int c = threadIdx.x * VEC; c < a.width; c += step) {
         const Pack<VEC> h = norm_pack<VEC>(a, st, load_pack<VEC>(cur + c), c);
@@ -967,13 +968,10 @@ void launch_row_update(const RowUpdateArgs& a, cudaStream_t s) {
     }
     const size_t smem = (size_t)a.width * 4 * (1 + (a.n_mix > 0 ? 1 : 0) + (a.n_add == 2 ? 1 : 0));
     if (smem > (size_t)200 * 1024) throw std::runtime_error("launch_row_update: the model is too wide");
-    if (vec) {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(&row_update_kernel<4>), smem);
-        launch_pdl(row_update_kernel<4>, dim3((unsigned)a.rows), dim3(RU_THREADS), smem, s, a);
-    } else {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(&row_update_kernel<1>), smem);
-        launch_pdl(row_update_kernel<1>, dim3((unsigned)a.rows), dim3(RU_THREADS), smem, s, a);
-    }
+    const bool few = a.rows <= 148;
+    auto* kernel = vec ? (few ? row_update_kernel<4, 2 * RU_THREADS> : row_update_kernel<4, RU_THREADS>) : (few ? row_update_kernel<1, 2 * RU_THREADS> : row_update_kernel<1, RU_THREADS>);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    launch_pdl(kernel, dim3((unsigned)a.rows), dim3(few ? 2 * RU_THREADS : RU_THREADS), smem, s, a);
     MK_LAUNCH_CHECK();
 }
 
