@@ -166,50 +166,54 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 }
 
 // ---- Q4_K ------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t scale_byte(uint32_t y, uint32_t z, uint32_t w, int i) {
-    uint32_t word = (i >> 2) == 0 ? y : ((i >> 2) == 1 ? z : w);
-    return (word >> ((i & 3) * 8)) & 0xFFu;
-}
-__device__ __forceinline__ void q4k_scale_min_reg(uint32_t y, uint32_t z, uint32_t w, int j, int& sc, int& mn) {
-    if (j < 4) {
-        sc = scale_byte(y, z, w, j) & 63;
-        mn = scale_byte(y, z, w, j + 4) & 63;
-    } else {
-        uint32_t a = scale_byte(y, z, w, j + 4);
-        sc = (a & 0xF) | ((scale_byte(y, z, w, j - 4) >> 6) << 4);
-        mn = (a >> 4) | ((scale_byte(y, z, w, j) >> 6) << 4);
+// Half a row's 256-wide block: groups 4h .. 4h + 3 of 32 weights, whose scales and minima come out of `hdr` (d, dmin, the twelve scale bytes)
+// four at a time.  `blk` is the row's 144-byte block; groups 2J and 2J + 1 share the 32 bytes at 16 + 32 J, low nibbles / high nibbles.
+// Four nibbles become (1024 + q) or, where they are, (1024 + 16 q) as f16 by byte permutation; a fma with the scale (a sixteenth of it) and -1024
+// (-64) of it gives sc * q exactly (below 1024); then fma(sc * q, d, -dmin * m): the dequantised weight, rounded once.  The scales too stay
+// in f16, where whole numbers below 64 and one product's rounding are what they are in f32.
+// The converters' integer instructions bound a narrow matmul: a group at a time, with its scales by way of f32 and its bytes
+// read twice, a block took half as many of them again (75776 x 2048 at one row: 35.3 us, this 34.1; at 64 rows 38.9 and 37.1).
+struct Q4Half {
+    uint32_t sc4, m4;
+    __half2 d, nd;
+    __device__ __forceinline__ Q4Half(const uint4& hdr, int h) {
+        if (h == 0) {
+            sc4 = hdr.y & 0x3F3F3F3Fu;
+            m4 = hdr.z & 0x3F3F3F3Fu;
+        } else {
+            sc4 = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+            m4 = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+        }
+        const uint32_t dd = __byte_perm(hdr.x, 0, 0x1010), nn = __byte_perm(hdr.x, 0, 0x3232) ^ 0x80008000u;
+        d = *reinterpret_cast<const __half2*>(&dd);
+        nd = *reinterpret_cast<const __half2*>(&nn);
     }
-}
-// Four nibbles in the low halves of four bytes -> (1024 + q) as f16 by byte permutation; fma(1024 + q, sc, -1024 sc)
-// = sc * q exactly (below 1024); then fma(sc * q, d, -dmin * m): the dequantised weight, rounded once.
-__device__ __forceinline__ void nibbles_to_weights(uint32_t bytes, __half2 sc, __half2 nbias, __half2 d, __half2 nmin, uint32_t& o01,
-                                                   uint32_t& o23) {
-    uint32_t p01 = __byte_perm(bytes, 0x64646464u, 0x4140);
-    uint32_t p23 = __byte_perm(bytes, 0x64646464u, 0x4342);
-    __half2 h01 = __hfma2(__hfma2(*reinterpret_cast<__half2*>(&p01), sc, nbias), d, nmin);
-    __half2 h23 = __hfma2(__hfma2(*reinterpret_cast<__half2*>(&p23), sc, nbias), d, nmin);
-    o01 = *reinterpret_cast<uint32_t*>(&h01);
-    o23 = *reinterpret_cast<uint32_t*>(&h23);
-}
-// Group G (32 weights, columns [32 G, 32 G + 32)) of a 256-wide block -> 32 f16 weights, two per register.  `blk` is
-// the row's 144-byte block, `hdr` its first 16 bytes (d, dmin, the twelve scale bytes).  Groups 2J and 2J + 1 share the
-// 32 bytes at 16 + 32 J: low nibbles / high nibbles.  G is a template argument so that the scale bytes are picked apart
-// with constant shifts.
-template <int G>
-__device__ __forceinline__ void convert_q4k_group(const uint8_t* blk, const uint4& hdr, uint32_t (&out)[16]) {
-    constexpr int J = G >> 1, SH = (G & 1) * 4;
-    const uint4 q0 = *reinterpret_cast<const uint4*>(blk + 16 + 32 * J);
-    const uint4 q1 = *reinterpret_cast<const uint4*>(blk + 16 + 32 * J + 16);
-    int sc, m;
-    q4k_scale_min_reg(hdr.y, hdr.z, hdr.w, G, sc, m);
-    const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-    const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)(hdr.x & 0xFFFF)));
-    const __half2 s2 = __float2half2_rn((float)sc);
-    const __half2 nb = __float2half2_rn(-1024.f * (float)sc);
-    const __half2 nm = __float2half2_rn(-dmin * (float)m);
-    const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    // byte i of four as an f16 pair
+    static __device__ __forceinline__ __half2 pair(uint32_t four, int i) {
+        const uint32_t p = __byte_perm(four, 0x64646464u, 0x4040 + 0x0101 * i);
+        return __hadd2(*reinterpret_cast<const __half2*>(&p), __float2half2_rn(-1024.f));
+    }
+    // group g (0 .. 3 of this half) out of its eight words
+    template <int g>
+    __device__ __forceinline__ void convert(const uint32_t (&words)[8], uint32_t (&out)[16]) const {
+        constexpr bool HIGH = (g & 1) != 0;
+        const __half2 sc = pair(sc4, g), nm = __hmul2(nd, pair(m4, g));
+        const __half2 s = HIGH ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc, nb = __hmul2(sc, __float2half2_rn(HIGH ? -64.f : -1024.f));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) nibbles_to_weights((words[i] >> SH) & 0x0F0F0F0Fu, s2, nb, d2, nm, out[2 * i], out[2 * i + 1]);
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t bytes = words[i] & (HIGH ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+            const uint32_t p01 = __byte_perm(bytes, 0x64646464u, 0x4140), p23 = __byte_perm(bytes, 0x64646464u, 0x4342);
+            const __half2 h01 = __hfma2(__hfma2(*reinterpret_cast<const __half2*>(&p01), s, nb), d, nm);
+            const __half2 h23 = __hfma2(__hfma2(*reinterpret_cast<const __half2*>(&p23), s, nb), d, nm);
+            out[2 * i] = *reinterpret_cast<const uint32_t*>(&h01);
+            out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h23);
+        }
+    }
+};
+__device__ __forceinline__ void load_words(const uint8_t* p, uint32_t (&words)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4*>(p), b = *reinterpret_cast<const uint4*>(p + 16);
+    words[0] = a.x; words[1] = a.y; words[2] = a.z; words[3] = a.w;
+    words[4] = b.x; words[5] = b.y; words[6] = b.z; words[7] = b.w;
 }
 
 // ---- Q6_K ------------------------------------------------------------------------------------------------------
@@ -217,9 +221,8 @@ __device__ __forceinline__ void convert_q4k_group(const uint8_t* blk, const uint
 // chunks of a row of the ql and qh planes are stored at chunk ^ (row & 7) / chunk ^ (row & 3) so that the 32 rows a
 // warp reads at once fall into different banks.
 constexpr int Q6_QL = 0, Q6_QH = QS_BM * 128, Q6_SC = Q6_QH + QS_BM * 64, Q6_D = Q6_SC + QS_BM * 16;
-// Four 6-bit values (low nibbles in `lo4`, the two high bits in bits 0-1 of each byte of `hi2`) -> (q - 32) * s.
-__device__ __forceinline__ void q6_to_weights(uint32_t lo4, uint32_t hi2, __half2 s, uint32_t& o01, uint32_t& o23) {
-    const uint32_t q = lo4 | (hi2 << 4);
+// Four 6-bit values, a byte each, -> (q - 32) * s.
+__device__ __forceinline__ void q6_to_weights(uint32_t q, __half2 s, uint32_t& o01, uint32_t& o23) {
     uint32_t p01 = __byte_perm(q, 0x64646464u, 0x4140);
     uint32_t p23 = __byte_perm(q, 0x64646464u, 0x4342);
     const __half2 bias = __float2half2_rn(-1056.f);  // 1024 + q - 1056 = q - 32, exact
@@ -228,8 +231,7 @@ __device__ __forceinline__ void q6_to_weights(uint32_t lo4, uint32_t hi2, __half
     o01 = *reinterpret_cast<uint32_t*>(&h01);
     o23 = *reinterpret_cast<uint32_t*>(&h23);
 }
-// Group G (32 weights, columns [32 G, 32 G + 32)) of the block: half n = G / 4 of the block, quarter qq = G % 4 of that
-// half: weight l of the group comes from ql[64 n + 32 (qq & 1) + l] (low nibbles for qq < 2, high nibbles otherwise) with
+// Quarter qq (32 weights) of half n of the block: weight l of the group comes from ql[64 n + 32 (qq & 1) + l] (low nibbles for qq < 2, high nibbles otherwise) with
 // its two high bits in qh[32 n + l] at bit 2 qq; scales sc[8 n + 2 qq] for l < 16 and sc[8 n + 2 qq + 1] for l >= 16.
 __device__ __forceinline__ void convert_q6k_group(const uint8_t* raw, int row, int G, uint32_t (&out)[16]) {
     const int n = G >> 2, qq = G & 3;
@@ -246,7 +248,8 @@ __device__ __forceinline__ void convert_q6k_group(const uint8_t* raw, int row, i
         const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, hw[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            q6_to_weights((aw[i] >> sh_lo) & 0x0F0F0F0Fu, (hw[i] >> sh_hi) & 0x03030303u, c == 0 ? s0 : s1, out[8 * c + 2 * i], out[8 * c + 2 * i + 1]);
+            q6_to_weights(((aw[i] >> sh_lo) & 0x0F0F0F0Fu) | ((sh_hi <= 4 ? hw[i] << (4 - sh_hi) : hw[i] >> (sh_hi - 4)) & 0x30303030u), c == 0 ? s0 : s1,
+                          out[8 * c + 2 * i], out[8 * c + 2 * i + 1]);
     }
 }
 
@@ -573,18 +576,14 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
                         for (int q = 0; q < 4; ++q) tmem_st16(t_dst + 16 * q, w);
                     } else if (!q6) {
                         const uint8_t* blk = raw + row * 144;
-                        const uint4 hdr = *reinterpret_cast<const uint4*>(blk);
-                        if (h == 0) {
-                            convert_q4k_group<0>(blk, hdr, w); tmem_st16(t_dst, w);
-                            convert_q4k_group<1>(blk, hdr, w); tmem_st16(t_dst + 16, w);
-                            convert_q4k_group<2>(blk, hdr, w); tmem_st16(t_dst + 32, w);
-                            convert_q4k_group<3>(blk, hdr, w); tmem_st16(t_dst + 48, w);
-                        } else {
-                            convert_q4k_group<4>(blk, hdr, w); tmem_st16(t_dst, w);
-                            convert_q4k_group<5>(blk, hdr, w); tmem_st16(t_dst + 16, w);
-                            convert_q4k_group<6>(blk, hdr, w); tmem_st16(t_dst + 32, w);
-                            convert_q4k_group<7>(blk, hdr, w); tmem_st16(t_dst + 48, w);
-                        }
+                        uint32_t q0[8], q1[8], w2[16];
+                        const Q4Half half(*reinterpret_cast<const uint4*>(blk), h);
+                        load_words(blk + 16 + 64 * h, q0);
+                        half.convert<0>(q0, w); tmem_st16(t_dst, w);
+                        half.convert<1>(q0, w2); tmem_st16(t_dst + 16, w2);
+                        load_words(blk + 48 + 64 * h, q1);
+                        half.convert<2>(q1, w); tmem_st16(t_dst + 32, w);
+                        half.convert<3>(q1, w2); tmem_st16(t_dst + 48, w2);
                     } else {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
