@@ -75,3 +75,29 @@ def test_expert_chunks_above_64_rows(env, orc, counts, gated):
             off_by *= 2 * np.abs(want).max() + np.abs(u).max() + 1   # both factors' errors, and the f16 result's
             want = orc.act_mul(want, u, 0)
         assert np.abs(got[r] - want).max() < off_by
+
+
+@pytest.mark.parametrize("kv_dtype", [np.float32, np.float16])
+@pytest.mark.parametrize("q_heads,kv_heads,d,rotary", [(1, 1, 64, 64), (8, 1, 64, 64), (4, 1, 128, 128), (1, 1, 256, 256), (2, 2, 256, 0), (4, 1, 128, 64), (2, 2, 96, 96)])
+def test_rotation_of_whole_heads(env, orc, kv_dtype, q_heads, kv_heads, d, rotary):
+    """Head counts that leave a warp's last run of heads short; part-turned and odd-sized heads take the other kernel."""
+    ops, _ = env
+    bt, layers, layer, lens, starts = 16, 2, 1, [19, 5], [0, 40]
+    rng = np.random.default_rng(d + q_heads)
+    tables, T = [[4, 0], [2, 5, 1]], sum(lens)
+    pools = [rng.standard_normal((6, layers, kv_heads, bt, d)).astype(np.float32).astype(kv_dtype) for _ in range(2)]
+    q, k, v = (rng.standard_normal((T, n * d)).astype(np.float32) for n in (q_heads, kv_heads, kv_heads))
+    cos, sin = orc.rope_tables(10000.0, rotary, 64) if rotary else (None, None)
+    qn, kn = ((1 + 0.1 * rng.standard_normal(d)).astype(np.float32) for _ in range(2)) if q_heads != 2 else (None, None)
+    kp, vp = (p.copy() for p in pools)
+    res = ops.attention_step(q, k, v, kp, vp, tables, starts, lens, q_heads=q_heads, kv_heads=kv_heads, head_dim=d, block_tokens=bt, layers=layers, layer=layer,
+                             scale=d ** -0.5, cos_table=cos, sin_table=sin, rotary_dim=rotary, q_norm_w=qn, k_norm_w=kn, norm_eps=1e-6)
+    want_q, want_k = (x if w is None else orc.rmsnorm(x.reshape(-1, d), w, 1e-6).reshape(x.shape) for x, w in ((q, qn), (k, kn)))
+    if rotary:
+        want_q = orc.rope_apply(want_q, q_heads, d, rotary, res["positions"], cos, sin)
+        want_k = orc.rope_apply(want_k, kv_heads, d, rotary, res["positions"], cos, sin)
+    okp, ovp = (p.copy() for p in pools)
+    orc.kv_scatter(want_k, v, okp, ovp, res["slots"], kv_heads, d, bt, layers, layer)
+    # values below 8: a sum of squares in another order, a division and two products: a few 2^-24 of them (in f16 one rounding more)
+    assert np.abs(res["q_rot"] - want_q).max() < 4e-6
+    assert np.abs(kp.astype(np.float32) - okp.astype(np.float32)).max() < (4e-6 if kv_dtype == np.float32 else 2.0 ** -8) and np.array_equal(vp, ovp)
