@@ -74,7 +74,8 @@ __host__ __device__ __forceinline__ int64_t kv_page_index(int64_t blk, int layer
 // Programmatic dependent launch: a kernel launched through launch_pdl may start (be scheduled, run its
 // prologue) while the previous kernel of the stream is still running; pdl_wait() blocks until that kernel has
 // completed and its writes are visible, so it must precede the first access to anything the predecessor wrote
-// or still reads.  pdl_trigger() lets the next kernel of the stream begin its own launch early.  Both are no-ops
+// or still reads.  Such data never comes in through a `const T* __restrict__` parameter: that promises that nobody writes it while the kernel
+// runs, and lets the compiler load it ahead of the wait.  pdl_trigger() lets the next kernel of the stream begin its own launch early.  Both are no-ops
 // for kernels launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -881,9 +881,9 @@ __global__ void __launch_bounds__(LP_THREADS) latent_rows_kernel(LatentPrepArgs 
 constexpr int FM_TILE = 64, FM_K = 16;
 
 // 64 x 64 outputs per CTA, 4 x 4 per thread.
-__global__ void __launch_bounds__(256) f32_matmul_kernel(const float* __restrict__ w, int64_t rows, int cols, const float* __restrict__ x, int T, float* y,
+__global__ void __launch_bounds__(256) f32_matmul_kernel(const float* __restrict__ w, int64_t rows, int cols, const float* x, int T, float* y,
                                                          int ldy, float scale, float softcap, int n_groups, int group_tiles, int4 end_lo, int4 end_hi,
-                                                         MatmulScatter to, const int32_t* __restrict__ offsets, int64_t matrix_rows) {
+                                                         MatmulScatter to, const int32_t* offsets, int64_t matrix_rows) {
     __shared__ float ws[FM_K][FM_TILE + 4], xs[FM_K][FM_TILE + 4];
     pdl_trigger();
     pdl_wait();

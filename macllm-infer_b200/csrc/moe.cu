@@ -19,7 +19,7 @@ constexpr int MAX_EXPERTS = 1024;
 // the pairs and counts them by expert in a row of its own, a scan over the warps' rows gives every (warp, expert) its first position, and the
 // warp hands them out as it walks its run again (a warp per expert that walked all pairs took 45 us for 11 360 of them, this 19).
 constexpr int GROUP_WARPS = 32;
-__global__ void __launch_bounds__(GROUP_WARPS * 32) moe_group_kernel(const int32_t* __restrict__ sel, int pairs, int k, int experts, int32_t* offsets,
+__global__ void __launch_bounds__(GROUP_WARPS * 32) moe_group_kernel(const int32_t* sel, int pairs, int k, int experts, int32_t* offsets,
                                                                      int32_t* pos_of_pair, int32_t* token_of_pos) {
     extern __shared__ int32_t rows[];  // [GROUP_WARPS][experts]
     __shared__ int32_t start[MAX_EXPERTS];
@@ -83,9 +83,8 @@ __global__ void __launch_bounds__(GROUP_WARPS * 32) moe_group_kernel(const int32
 
 // Only choices whose expert lies in [e_lo, e_hi) contribute (the whole range on one GPU, a rank's share under
 // expert parallelism).
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ expert_out, const int32_t* __restrict__ sel,
-                                                          const float* __restrict__ w, const int32_t* __restrict__ pos_of_pair, int k,
-                                                          int hidden, int e_lo, int e_hi, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* expert_out, const int32_t* sel, const float* w, const int32_t* pos_of_pair, int k, int hidden,
+                                                          int e_lo, int e_hi, float* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x;

@@ -5,6 +5,9 @@
 // HBM (block sizes src/gguf.rs:386-408), activations arrive as 8-bit blocks, and every block dot
 // product is an exact integer sum (dp4a) scaled in f32 - the arithmetic of the reference's CPU path.
 //
+// Only the weights are promised to the compiler as constant (const __restrict__): a load of such memory may move in front of pdl_wait(), and
+// what a predecessor produces must not.
+//
 // Memory plan: one warp owns one output row and streams that row's blocks with 128-bit (Q4_K,
 // Q8_0) or 64-bit (Q6_K planes) loads, eight lanes per 256-weight block, so a warp consumes whole
 // 128-byte lines; activations (T*K bytes) are re-read from L1/L2.  Each weight byte leaves HBM once
@@ -61,9 +64,9 @@ __device__ __forceinline__ void finish_rows(float (&acc)[NT], int n, int out, in
 // ---------------------------------------------------------------- Q4_K
 template <int NT, int R>
 __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q4k_kernel(const uint8_t* __restrict__ W, int nb, int out,
-                                                                    const int8_t* __restrict__ xq,
-                                                                    const float* __restrict__ xd,
-                                                                    const int16_t* __restrict__ xbs, int T,
+                                                                    const int8_t* xq,
+                                                                    const float* xd,
+                                                                    const int16_t* xbs, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
     pdl_trigger();
@@ -150,8 +153,8 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q6k_kernel(const uint8_
                                                                     const uint8_t* __restrict__ qh_p,
                                                                     const int8_t* __restrict__ sc_p,
                                                                     const __half* __restrict__ d_p, int nb, int out,
-                                                                    const int8_t* __restrict__ xq,
-                                                                    const float* __restrict__ xd, int T,
+                                                                    const int8_t* xq,
+                                                                    const float* xd, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
     pdl_trigger();
@@ -231,8 +234,8 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q6k_kernel(const uint8_
 template <int NT, int R>
 __global__ void __launch_bounds__(GEMV_WARPS * 32) qgemv_q80_kernel(const int8_t* __restrict__ qs_p,
                                                                     const __half* __restrict__ d_p, int K, int out,
-                                                                    const int8_t* __restrict__ xq,
-                                                                    const float* __restrict__ xd, int T,
+                                                                    const int8_t* xq,
+                                                                    const float* xd, int T,
                                                                     float* __restrict__ y, int ldy, float out_scale,
                                                                     float softcap, Group grp) {
     pdl_trigger();
@@ -301,7 +304,7 @@ constexpr int F32_GEMV_ROWS = 8;
 // loads in flight per step instead of one chain.  The sum of one (row, output) pair is always formed the same way -
 // lane-strided partial sums in ascending k, then the warp tree - whatever the grid or the number of rows.
 __global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_kernel(const float* __restrict__ W, int out, int in,
-                                                                   const float* __restrict__ x, int T,
+                                                                   const float* x, int T,
                                                                    float* __restrict__ y) {
     pdl_trigger();
     pdl_wait();
@@ -345,7 +348,7 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) f32_gemv_kernel(const float* 
 // A lane's columns and their order are those of the kernel above, columns behind the end are zeros: the same bits.
 constexpr int F32_TILE_OUT = 32, F32_TILE_K = 64, F32_TILE_STAGES = 4, F32_TILE_WARPS = 16, F32_WARP_OUT = 8;
 template <int R>
-__global__ void __launch_bounds__(F32_TILE_WARPS * 32) f32_gemv_tile_kernel(const float* __restrict__ W, int out, int in, const float* __restrict__ x, int T,
+__global__ void __launch_bounds__(F32_TILE_WARPS * 32) f32_gemv_tile_kernel(const float* __restrict__ W, int out, int in, const float* x, int T,
                                                                             float* __restrict__ y) {
     extern __shared__ __align__(16) float f32_tile[];
     constexpr int ROWS = 4 * R, STAGE = (F32_TILE_OUT + ROWS) * F32_TILE_K, VECS = F32_TILE_K / 4;
