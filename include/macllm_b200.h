@@ -695,6 +695,11 @@ int32_t mk_k_grouped_qmatmul(int32_t type, const void* w, const void* up_w, int3
  * of partial sums, row tiles per group, groups}.  Needs no GPU. */
 int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t* out8);
 
+/* Host-only: how mk_k_grouped_qmatmul cuts a call on MK_PATH_STREAM.  rows_per_expert: rows of an expert's matrix (gate and up together when
+ * gated), a multiple of 128; rows_total: routed rows; max_rows_per_expert: the most any expert is expected to have.  out = {rows of a chunk, row
+ * tiles of a job, most jobs a CTA can be handed, jobs a CTA's table holds}; a call whose third number is above its fourth is refused. */
+int32_t mk_k_grouped_matmul_plan(int32_t experts, int64_t rows_per_expert, int32_t rows_total, int32_t max_rows_per_expert, int64_t* out4);
+
 /* Host-only: how one tick's attention work is cut (the plan the model builds before every forward).  Lanes with more
  * than one token become query tiles; one-token lanes become one CTA per KV head, or several key shares when that pays.
  * shares_out[i] = key shares of lane i (0 for lanes with more than one token); *tiles_out = query tiles;

@@ -920,6 +920,16 @@ int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, in
     });
 }
 
+int32_t mk_k_grouped_matmul_plan(int32_t experts, int64_t rows_per_expert, int32_t rows_total, int32_t max_rows_per_expert, int64_t* out4) {
+    return guarded([&] {
+        if (experts <= 0 || rows_per_expert <= 0 || rows_per_expert % 128 != 0 || rows_total <= 0 || out4 == nullptr)
+            throw std::runtime_error("mk_k_grouped_matmul_plan: arguments out of range");
+        const QStreamGroupedPlan p = qstream_grouped_plan(experts, (int)(rows_per_expert / 128), rows_total, max_rows_per_expert, true, kPlanSms);
+        const int64_t v[4] = {p.bn, p.R, p.jobs, kQStreamMaxJobs};
+        memcpy(out4, v, sizeof v);
+    });
+}
+
 int32_t mk_k_attention_plan(const int32_t* start_pos, const int32_t* n_tokens, int32_t lanes, int32_t q_heads, int32_t kv_heads,
                             int32_t block_tokens, int32_t* shares_out, int32_t* tiles_out, int32_t* max_entries_out) {
     return guarded([&] {

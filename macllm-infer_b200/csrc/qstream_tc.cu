@@ -60,7 +60,7 @@ constexpr int QS_SMEM_LIMIT = 212 * 1024;                        // rings of the
 constexpr uint32_t QS_SPIN_LIMIT = 1u << 22;
 constexpr uint32_t QS_TMEM_COLS = 512;
 constexpr uint32_t QS_A_COL0 = 256;                              // two A buffers of 128 columns
-constexpr int QS_MAX_JOBS = 320;                                 // jobs one CTA can be handed in the expert-grouped form
+constexpr int QS_MAX_JOBS = kQStreamMaxJobs;                     // jobs one CTA can be handed in the expert-grouped form
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -946,6 +946,21 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
     return pl.slots;
 }
 
+QStreamGroupedPlan qstream_grouped_plan(int experts, int tiles_per_expert, int rows_total, int max_rows_per_expert, bool rows_known, int sms) {
+    QStreamGroupedPlan pl;
+    auto cut = [&](int bn) {
+        pl.bn = bn;
+        // two accumulators of 128 columns: a row tile at a time, so that its epilogue runs under the next one's products
+        pl.R = tiles_per_expert % 2 == 0 && bn <= 64 ? 2 : 1;
+        // every expert may add one partly filled chunk
+        pl.jobs = (((int64_t)rows_total / bn + experts) * (tiles_per_expert / pl.R) + sms - 1) / sms + 1;
+    };
+    cut(max_rows_per_expert <= 16 ? 16 : (max_rows_per_expert <= 32 ? 32 : (max_rows_per_expert <= 64 ? 64 : 128)));
+    // with many experts of many row tiles it is the partly filled chunks that count, and half as many tiles a job make twice the jobs
+    if (pl.bn == 128 && rows_known && pl.jobs > kQStreamMaxJobs) cut(64);
+    return pl;
+}
+
 // Expert-grouped form (SparseMoeFeedForward::forward, src/decoder.rs:394-441: every expert multiplies the rows routed to it).
 int launch_qstream_tc_grouped(const QStreamWeight& W, int experts, const int32_t* offsets_dev, const __half* xh, int rows_total,
                               int max_rows_per_expert, float* y, int ldy, int32_t* status, cudaStream_t s, int gated_act, __half* yh, int ldyh, bool rows_known) {
@@ -958,13 +973,10 @@ int launch_qstream_tc_grouped(const QStreamWeight& W, int experts, const int32_t
     if (gated && (!W.gated || yh == nullptr)) throw std::runtime_error("launch_qstream_tc_grouped: the gated form needs an interleaved gate|up bank and an f16 output");
     const int nb = (int)(W.cols / 256);
     const int tiles_pe = (int)(W.rows / experts / QS_BM);
-    const int bn = max_rows_per_expert <= 16 ? 16 : (max_rows_per_expert <= 32 ? 32 : (max_rows_per_expert <= 64 ? 64 : 128));
-    // two accumulators of 128 columns: a row tile at a time, so that its epilogue runs under the next one's products
-    const int R = tiles_pe % 2 == 0 && bn <= 64 ? 2 : 1;
     const int sms = device_sm_count();
-    // a bound on the jobs any CTA is handed: every expert may add one partly filled chunk
-    const int64_t max_jobs = ((int64_t)rows_total / bn + experts) * (tiles_pe / R);
-    if (rows_known && (max_jobs + sms - 1) / sms + 1 > QS_MAX_JOBS) throw std::runtime_error("launch_qstream_tc_grouped: more jobs per CTA than the kernel's table holds");
+    const QStreamGroupedPlan pl = qstream_grouped_plan(experts, tiles_pe, rows_total, max_rows_per_expert, rows_known, sms);
+    const int bn = pl.bn, R = pl.R;
+    if (rows_known && pl.jobs > QS_MAX_JOBS) throw std::runtime_error("launch_qstream_tc_grouped: more jobs per CTA than the kernel's table holds");
     alignas(64) CUtensorMap tx;
     encode_tma_2d(&tx, false, xh, (uint64_t)W.cols, (uint64_t)rows_total, (uint64_t)W.cols * 2, 64, (uint32_t)bn, true);
     QsParams p{};

@@ -49,10 +49,19 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
                       int32_t* status, cudaStream_t s, int max_splits, const QStreamWeight* W2 = nullptr, int gated_act = -1,
                       __half* yh = nullptr, int ldyh = 0);
 
+// How the expert-grouped form cuts a call: chunk width, row tiles of a job, and the most jobs that a CTA can be handed (its table holds
+// kQStreamMaxJobs).  max_rows_per_expert picks the width, 16, 32, 64 or 128 rows.
+constexpr int kQStreamMaxJobs = 320;
+struct QStreamGroupedPlan {
+    int bn = 0, R = 1;
+    int64_t jobs = 0;
+};
+QStreamGroupedPlan qstream_grouped_plan(int experts, int tiles_per_expert, int rows_total, int max_rows_per_expert, bool rows_known, int sms);
+
 // Expert-grouped form: W is a bank of `experts` matrices stacked by rows (each a whole number of 128-row tiles);
 // activation rows [offsets[e], offsets[e + 1]) of xh [rows_total][cols] (grouped by expert, device array of experts + 1
 // row numbers) are multiplied by expert e's matrix: y[r][n] for those rows r and n < rows per expert, or, gated,
-// yh[r][f].  max_rows_per_expert picks the chunk width (16, 32, 64 or 128 rows): an expert's rows are processed a chunk at a
+// yh[r][f].  max_rows_per_expert picks the chunk width (qstream_grouped_plan): an expert's rows are processed a chunk at a
 // time, each chunk one pass over the expert's matrix, so any width is correct for any row count.  The kernel reads the
 // row ranges on the device: no host round trip.  rows_known = false: rows_total is only the extent of xh (the true row
 // count lives on the device); the host then cannot bound the jobs per CTA, and a launch that overflows the kernel's job

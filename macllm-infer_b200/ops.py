@@ -277,6 +277,13 @@ def matmul_plan(path: int, rows: int, cols: int, T: int, max_splits: int = 16) -
     return dict(zip(names, map(int, out)))
 
 
+def grouped_matmul_plan(experts: int, rows_per_expert: int, rows_total: int, max_rows_per_expert: int) -> dict:
+    """Host-only: how the expert-grouped streamed matmul cuts a call."""
+    out = np.zeros(4, dtype=np.int64)
+    capi.check(capi.lib().mk_k_grouped_matmul_plan(experts, rows_per_expert, rows_total, max_rows_per_expert, _p(out)))
+    return dict(zip(("rows", "tiles", "jobs", "table"), map(int, out)))
+
+
 def attention_plan(start_pos, n_tokens, q_heads: int, kv_heads: int, block_tokens: int = 16):
     """Host-only: (key shares per lane, query tiles, entry bound) of one tick's attention plan."""
     sp = np.ascontiguousarray(start_pos, dtype=np.int32)

@@ -71,6 +71,25 @@ def test_streamed_matmul_plans_of_the_benchmark_shapes(env):
     assert head["slots"] == 1 and head["ctas"] == 148                                          # 32 MB per slot: never cut
 
 
+@pytest.mark.parametrize("experts,rows,total,most", [(256, 18432, 16384, 65), (512, 9216, 8192, 4000), (128, 36864, 8192, 65), (128, 6144, 11360, 89),
+                                                     (8, 28672, 4096, 2000), (1024, 128, 65536, 65), (16, 128, 40, 17), (3, 384, 64, 64), (5, 256, 16, 9)])
+def test_grouped_plans_take_what_64_row_chunks_take(env, experts, rows, total, most):
+    """Chunks of 128 rows halve the chunks of full experts but not the one that every expert adds, and a job has half the row tiles: where that
+    would not fit the table of a CTA's jobs, chunks are 64 rows."""
+    ops, _ = env
+    p, tiles = ops.grouped_matmul_plan(experts, rows, total, most), rows // 128
+
+    def jobs(width, r):
+        return -(-((total // width + experts) * (tiles // r)) // SMS) + 1
+
+    assert p["jobs"] == jobs(p["rows"], p["tiles"]) <= p["table"] == 320
+    if most > 64:
+        assert p["rows"] == (128 if jobs(128, 1) <= p["table"] else 64)
+    else:
+        assert p["rows"] // 2 < max(most, 9) <= p["rows"]
+    assert p["tiles"] == (2 if tiles % 2 == 0 and p["rows"] <= 64 else 1)
+
+
 def test_plans_refuse_what_the_kernels_do_not_cover(env):
     ops, capi = env
     with pytest.raises(capi.MkError):
