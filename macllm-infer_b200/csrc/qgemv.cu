@@ -473,9 +473,12 @@ void launch_f32_gemv(const float* W, int out, int in, const float* x, int T, flo
     if (T <= 0) return;
     const unsigned runs = (unsigned)((T + F32_GEMV_ROWS - 1) / F32_GEMV_ROWS);
     // Tiles once an eighth of this kernel's warps would still give every SM's schedulers one; they take as few rows as keep the CTAs to one per SM,
-    // 48 at most (the sums' registers).
-    if ((int64_t)runs * out / 8 >= 148 * 4 && in % 4 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
-        const int64_t columns = (out + F32_TILE_OUT - 1) / F32_TILE_OUT, rows = (T + std::max<int64_t>(148 / columns, 1) - 1) / std::max<int64_t>(148 / columns, 1);
+    // 48 at most (the sums' registers).  A tile computes 32 outputs whatever there are: with 17 or more it is the faster one (24 us against 36 at
+    // 4096 rows x 2048 columns), in its first round from 12 on (25 against 33); with 8 it takes 30 us instead of 19 (4800 rows), and behind
+    // the first round 16 take 63 instead of 55 (8192 rows).
+    const int64_t columns = (out + F32_TILE_OUT - 1) / F32_TILE_OUT, places = std::max<int64_t>(148 / columns, 1), rows = (T + places - 1) / places;
+    const bool full = out > F32_TILE_OUT / 2 || (out >= 12 && rows <= 48);
+    if (full && (int64_t)runs * out / 8 >= 148 * 4 && in % 4 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
         if (rows <= 16) launch_f32_tile<4>(W, out, in, x, T, y, s);
         else if (rows <= 24) launch_f32_tile<6>(W, out, in, x, T, y, s);
         else if (rows <= 32) launch_f32_tile<8>(W, out, in, x, T, y, s);

@@ -37,7 +37,7 @@ def test_router_choices_at_every_register_size(env, orc, experts, k):
 
 
 @pytest.mark.parametrize("T,experts,cols", [(297, 128, 2048), (600, 128, 2052), (1010, 130, 100), (1184, 128, 64), (1420, 128, 2048), (2001, 129, 516),
-                                            (300, 128, 2050), (1, 4096, 64)])
+                                            (300, 128, 2050), (1, 4096, 64), (4800, 8, 64), (4736, 12, 64), (7105, 16, 64), (7104, 16, 64), (2700, 17, 64)])
 def test_router_product_of_many_rows(env, T, experts, cols):
     ops, _ = env
     rng = np.random.default_rng(T)
