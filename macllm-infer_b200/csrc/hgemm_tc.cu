@@ -456,6 +456,8 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         kb1 = min(k_blocks, kb0 + p.kb_per_split);
     };
 
+    uint32_t loaded = 0;   // the loader's stages
+    bool gave_up = false;
     if (warp == 0) {
         // ---- loader
         if (lane == 0) {
@@ -514,6 +516,8 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 pdl_wait();
                 for (uint32_t h = 0; h < it && h < (uint32_t)STAGES; ++h) load_x((int)h, held_kb[h], held_n[h], held_y[h]);
             }
+            loaded = it;
+            gave_up = !ok;
         }
     } else if (warp == 1) {
         // ---- MMA issuer (the leader's, for both CTAs of a pair)
@@ -694,6 +698,20 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (warp == 0) {
+        // The commits that hand back the last stages are waited for by nobody else, and in a pair they come from the other CTA: none may find
+        // this one gone.  Where a wait gave up, copies in flight land first.
+        loaded = __shfl_sync(0xffffffffu, loaded, 0);
+        gave_up = __shfl_sync(0xffffffffu, (int)gave_up, 0) != 0;
+        if (lane < STAGES && (uint32_t)lane < loaded) {
+            const uint32_t ph = ((loaded - 1 - lane) / STAGES) & 1;
+            if (gave_up || !mbar_wait(&empty[lane], ph, HG_SPIN_LIMIT)) {
+                atomicExch(p.status, 11);
+                if (rank == 0) mbar_wait(&full[lane], ph, HG_SPIN_LIMIT);
+            }
+        }
+        __syncwarp();
+    }
     if constexpr (PAIR) cluster_sync();  // the peer is done with this CTA's barriers and shared memory
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
