@@ -25,7 +25,7 @@ __device__ __forceinline__ __half to_kv<__half>(float v) { return __float2half_r
 
 template <typename KV>
 __global__ void __launch_bounds__(RK_WARPS * 32) rope_kv_kernel(RopeKvArgs a) {
-    __shared__ float buf[RK_WARPS][RK_MAX_D];
+    __shared__ __align__(16) float buf[RK_WARPS][RK_MAX_D];  // rows are filled in pieces of up to 16 bytes
     pdl_trigger();
     pdl_wait();
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
