@@ -39,7 +39,7 @@ struct AttnTcArgs {
     int q_heads = 0, kv_heads = 0, d = 0, block_tokens = 16, layers = 0, layer = 0;
     int64_t pool_blocks = 0;  // see kv_page_index
     int64_t pool_pages = 0;   // pages that page numbers (kv_page_index) reach in either pool; needed with prefill tiles
-    int32_t* status = nullptr;  // receives a code when a bounded wait of the prefill kernel gives up
+    int32_t* status = nullptr;  // receives a code when a bounded wait of the prefill kernel gives up (its output is then incomplete); needed with prefill tiles
     int bt_shift = 0;         // log2(block_tokens), filled in by the launcher
     float scale = 1.f, softcap = 0.f;
     int window = 0;             // > 0: a position sees itself and the window - 1 keys before it

@@ -144,7 +144,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             if (vof < pages) tma_load_2d(smem_u32(vs) + st * L::V_BYTES + vpanel * AU_PANEL + vof * (AU_PAGE * 128), &tm_v, vpanel * 64, row_of(vblk, vof), &v_full[st]);
         }
         if (!ok) {
-            if (lane == 0 && a.status != nullptr) atomicExch(a.status, 31);
+            if (lane == 0) atomicExch(a.status, 31);
             for (int u = max(0, t - ST); u <= t && u < n_tiles; ++u) {  // copies in flight land before the CTA ends
                 bar_wait(&k_full[u % ST], u / ST & 1);
                 if (u < t) bar_wait(&v_full[u % ST], u / ST & 1);
@@ -188,7 +188,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 commit(&v_empty[st]);
                 commit(o_done);
             }
-            if (!ok && a.status != nullptr) atomicExch(a.status, 32);
+            if (!ok) atomicExch(a.status, 32);
         }
     } else {
         // ---- one item per thread
@@ -337,7 +337,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     }
                 }
             }
-        } else if (lane == 0 && a.status != nullptr) {
+        } else if (lane == 0) {
             atomicExch(a.status, 33);
         }
     }
@@ -365,6 +365,7 @@ void launch_variant(const AttnTcArgs& a, cudaStream_t s) {
 }  // namespace
 
 void launch_attention_umma(const AttnTcArgs& a, cudaStream_t s) {
+    if (a.status == nullptr) throw std::runtime_error("launch_attention_umma: a wait that gives up has nowhere to say so");
     if (a.pool_pages <= 0) throw std::runtime_error("launch_attention_umma: the pools' size is missing");
     switch (a.d) {
         case 64: a.exact_weights ? launch_variant<64, 64, true>(a, s) : launch_variant<64, 64, false>(a, s); break;

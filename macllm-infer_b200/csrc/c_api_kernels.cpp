@@ -424,7 +424,8 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
         const bool tc_ok = attention_tc_supported(c->q_heads, c->kv_heads, d, c->block_tokens, c->kv_f16 != 0);
         if (c->kernel == 2 && !tc_ok) throw std::runtime_error("mk_k_attention_step: the tensor-core kernel does not cover this shape");
         if (c->kernel < 0 || c->kernel > 2) throw std::runtime_error("mk_k_attention_step: unknown kernel selector");
-        DevBuf work, part_o, part_ml;
+        DevBuf work, part_o, part_ml, status(4);
+        status.zero(nullptr);
         if (tc_ok && c->kernel != 1) {
             AttnTcPlan plan;
             // the kernels address block tables through LaneHeader::table_off; the plan assumes tables packed in lane order
@@ -465,6 +466,7 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
             ta.layers = c->layers;
             ta.layer = c->layer;
             ta.pool_pages = (int64_t)c->pool_blocks * c->layers;
+            ta.status = status.as<int32_t>();
             ta.scale = c->scale;
             ta.softcap = c->softcap;
             ta.window = c->window;
@@ -474,8 +476,9 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
         }
         MK_CUDA(cudaDeviceSynchronize());
 
-        int32_t flag = 0;
+        int32_t flag = 0, gave_up = 0;
         err.download(&flag, 4);
+        status.download(&gave_up, 4);
         dout.download(c->out, qn);
         if (c->q_rot_out) dq.download(c->q_rot_out, qn);
         if (c->slots_out) slots.download(c->slots_out, (size_t)T * 8);
@@ -486,6 +489,7 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
         vpool.download(c->v_pool, pool_elems * esz);
         MK_CUDA(cudaDeviceSynchronize());
         if (flag != 0) throw std::runtime_error("mk_k_attention_step: batch descriptor index out of range (flag " + std::to_string(flag) + ")");
+        if (gave_up != 0) throw std::runtime_error("mk_k_attention_step: a bounded wait of the prefill kernel gave up (code " + std::to_string(gave_up) + ")");
     });
 }
 

@@ -197,7 +197,7 @@ void DeviceLm::finish_tick(const Tick& t, int prof_class) {
 std::string DeviceLm::status_message(int32_t status) const {
     if ((status & 0xFFFF0000) == kSampleEmptyStatus)
         return "sampling distribution is empty (lane " + std::to_string(status & 0xFFFF) + ")";  // src/sampling.rs:352-355
-    return "a bounded wait inside a kernel gave up (tensor-core matmul pipeline or expert exchange; status " + std::to_string(status) + ")";
+    return "a bounded wait inside a kernel gave up (tensor-core pipeline of a matmul or of attention, or expert exchange; status " + std::to_string(status) + ")";
 }
 
 void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
