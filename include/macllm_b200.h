@@ -706,6 +706,10 @@ int32_t mk_k_grouped_matmul_plan(int32_t experts, int64_t rows_per_expert, int32
  * *max_entries_out = the bound buffers are sized for.  Needs no GPU. */
 int32_t mk_k_attention_plan(const int32_t* start_pos, const int32_t* n_tokens, int32_t lanes, int32_t q_heads, int32_t kv_heads,
                             int32_t block_tokens, int32_t* shares_out, int32_t* tiles_out, int32_t* max_entries_out);
+/* Host-only: the query tiles of that plan in the order of their launch, those that walk most keys first.  window / chunk: the layer's visibility
+ * rules (0: none).  pairs [capacity][2] (or NULL: only count) receives (lane, first query row within the lane); *n_out = tiles. */
+int32_t mk_k_attention_tiles(const int32_t* start_pos, const int32_t* n_tokens, int32_t lanes, int32_t q_heads, int32_t kv_heads, int32_t window, int32_t chunk,
+                             int32_t* pairs, int32_t capacity, int32_t* n_out);
 
 /* argmax of src/sampling.rs:425-433 for each row of logits [B][vocab]. */
 /* ------------------------------------------------------------------------------------------------

@@ -945,13 +945,24 @@ int32_t mk_k_attention_plan(const int32_t* start_pos, const int32_t* n_tokens, i
         plan_attention_tc(start_pos, n_tokens, n_blocks.data(), lanes, q_heads, kv_heads, plan);
         for (int i = 0; i < lanes; ++i) shares_out[i] = 0;
         for (int e = 0; e < plan.n_entries(); ++e) shares_out[plan.entries[(size_t)e * 8]] = plan.entries[(size_t)e * 8 + 2];
-        // query tiles are counted in units of 64 (row, head) items, 128 for groups of eight heads; the kernel takes 128 items at a time
-        const int group = q_heads / kv_heads, unit_rows = (group == 8 ? 128 : 64) / group;
-        *tiles_out = 0;
-        for (int i = 0; i < lanes; ++i)
-            if (n_tokens[i] > 1) *tiles_out += (n_tokens[i] + unit_rows - 1) / unit_rows;
+        *tiles_out = plan.n_tiles();
         *max_entries_out = attention_tc_max_entries(lanes, kv_heads);
         if (plan.n_entries() > *max_entries_out) throw std::runtime_error("mk_k_attention_plan: the plan exceeds its own bound");
+    });
+}
+
+int32_t mk_k_attention_tiles(const int32_t* start_pos, const int32_t* n_tokens, int32_t lanes, int32_t q_heads, int32_t kv_heads, int32_t window, int32_t chunk,
+                             int32_t* pairs, int32_t capacity, int32_t* n_out) {
+    return guarded([&] {
+        if (lanes <= 0 || q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || q_heads / kv_heads > kAttnItems || window < 0 || chunk < 0 || n_out == nullptr)
+            throw std::runtime_error("mk_k_attention_tiles: arguments out of range");
+        std::vector<int32_t> n_blocks((size_t)lanes, 1);
+        AttnTcPlan plan;
+        plan_attention_tc(start_pos, n_tokens, n_blocks.data(), lanes, q_heads, kv_heads, plan, chunk, window);
+        *n_out = plan.n_tiles();
+        if (pairs == nullptr) return;
+        if (capacity < plan.n_tiles()) throw std::runtime_error("mk_k_attention_tiles: more tiles than the buffer holds");
+        memcpy(pairs, plan.tiles.data(), plan.tiles.size() * 4);
     });
 }
 

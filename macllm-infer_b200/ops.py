@@ -295,6 +295,18 @@ def attention_plan(start_pos, n_tokens, q_heads: int, kv_heads: int, block_token
     return shares, int(tiles.value), int(bound.value)
 
 
+def attention_tiles(start_pos, n_tokens, q_heads: int, kv_heads: int, window: int = 0, chunk: int = 0) -> np.ndarray:
+    """Host-only: the query tiles of one tick's attention plan in launch order, [tiles][2] of (lane, first row)."""
+    sp = np.ascontiguousarray(start_pos, dtype=np.int32)
+    nt = np.ascontiguousarray(n_tokens, dtype=np.int32)
+    n = C.c_int32(0)
+    args = (_p(sp), _p(nt), len(sp), q_heads, kv_heads, window, chunk)
+    capi.check(capi.lib().mk_k_attention_tiles(*args, None, 0, C.byref(n)))
+    pairs = np.zeros((n.value, 2), dtype=np.int32)
+    capi.check(capi.lib().mk_k_attention_tiles(*args, _p(pairs), n.value, C.byref(n)))
+    return pairs
+
+
 def moe_combine_exchange(expert_out, sel, weights, e_lo: int, e_hi: int, ranks: int, rank: int, peer_rows=None, wait_ms: int = 50,
                          epochs: int = 1):
     """One rank's launch(es) of the fused expert-parallel combine + exchange kernel with every rank's exchange block on

@@ -44,7 +44,26 @@ def test_one_long_history_among_many_short_ones_is_cut(ops):
 def test_prefill_lanes_become_query_tiles(ops):
     shares, tiles, _ = ops.attention_plan([0, 100, 40], [512, 1, 33], 16, 4)
     assert shares.tolist() == [0, 1, 0]
-    assert tiles == 512 // 16 + (33 + 15) // 16   # 16 query rows x 4 heads per tile of four warps
+    assert tiles == 512 // 32 + 2   # 32 query rows x 4 heads per tile of 128 items; 33 rows take two
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(8, 8), (8, 4), (16, 4), (32, 4)])
+@pytest.mark.parametrize("window,chunk", [(0, 0), (64, 0), (0, 128)])
+def test_query_tiles_cover_every_row_once_and_the_longest_walks_come_first(ops, q_heads, kv_heads, window, chunk):
+    start, n = [0, 100, 40, 7, 3000, 0, 513], [512, 1, 33, 128, 129, 2, 700]
+    tiles = ops.attention_tiles(start, n, q_heads, kv_heads, window, chunk)
+    _, count, _ = ops.attention_plan(start, n, q_heads, kv_heads)
+    per = 128 * kv_heads // q_heads
+    assert len(tiles) == count == sum(-(-k // per) for k in n if k > 1)
+    seen = [np.zeros(k, int) for k in n]
+    walks = []
+    for lane, row in tiles:
+        last = min(row + per, n[lane]) - 1
+        seen[lane][row:last + 1] += 1
+        first_key = max(start[lane] + row - window + 1 if window else 0, (start[lane] + row) // chunk * chunk if chunk else 0, 0)
+        walks.append(start[lane] + last + 1 - first_key)
+    assert all((s == (k > 1)).all() for s, k in zip(seen, n))
+    assert walks == sorted(walks, reverse=True)
 
 
 def test_bad_arguments_are_refused(ops):
