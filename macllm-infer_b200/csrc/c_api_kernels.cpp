@@ -905,13 +905,23 @@ int32_t mk_k_moe_route(const float* logits, int32_t T, int32_t experts, int32_t 
     });
 }
 
+int32_t mk_k_half_matmul_plan(int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t scratch_floats, int32_t may_pair, int64_t* out8) {
+    return guarded([&] {
+        if (rows <= 0 || cols <= 0 || T <= 0 || out8 == nullptr) throw std::runtime_error("mk_k_half_matmul_plan: arguments out of range");
+        if (cols % 64 != 0) throw std::runtime_error("mk_k_half_matmul_plan: the f16-image GEMM needs columns in multiples of 64");
+        const HgemmPlan p = hgemm_tc_plan(rows, cols, T, max_splits, scratch_floats < 0 ? SIZE_MAX : (size_t)scratch_floats, may_pair != 0);
+        const int64_t v[8] = {p.bn, p.row_tiles, p.n_tiles, p.splits, p.kb_per_split, (int64_t)p.partial_floats, p.pairs ? 1 : 0, 0};
+        memcpy(out8, v, sizeof v);
+    });
+}
+
 int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t* out8) {
     return guarded([&] {
         if (rows <= 0 || cols <= 0 || T <= 0 || out8 == nullptr) throw std::runtime_error("mk_k_matmul_plan: arguments out of range");
         if (path == MK_PATH_HALF) {
             if (cols % 64 != 0) throw std::runtime_error("mk_k_matmul_plan: the f16-image GEMM needs columns in multiples of 64");
             HgemmPlan p = hgemm_tc_plan(rows, cols, T, max_splits);
-            const int64_t v[8] = {p.bn, p.row_tiles, p.n_tiles, p.splits, p.kb_per_split, (int64_t)p.partial_floats, 0, 0};
+            const int64_t v[8] = {p.bn, p.row_tiles, p.n_tiles, p.splits, p.kb_per_split, (int64_t)p.partial_floats, p.pairs ? 1 : 0, 0};
             memcpy(out8, v, sizeof v);
         } else if (path == MK_PATH_STREAM) {
             if (cols % 256 != 0 || T > kQStreamMaxRows) throw std::runtime_error("mk_k_matmul_plan: the streamed matmul covers 256-wide blocks and at most 64 rows");

@@ -877,7 +877,9 @@ void build_half_weight(const QWeight& W, HalfWeight& out, cudaStream_t s) {
     build_half_weight_stacked(&one, 1, out, s);
 }
 
-HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits) {
+namespace {
+// Tiles of one CTA.
+HgemmPlan single_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t scratch_floats) {
     HgemmPlan pl;
     pl.bn = T <= 64 ? 64 : 128;
     if (T > 128) {
@@ -905,6 +907,7 @@ HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits) {
         long cost = waves * (per + 3) + (s > 1 ? 1 : 0);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
+    if (best > 1 && (size_t)best * T * rows > scratch_floats) best = 1;
     pl.splits = best;
     pl.kb_per_split = (kb + best - 1) / best;
     pl.partial_floats = best > 1 ? (size_t)best * T * rows : 0;
@@ -914,7 +917,7 @@ HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits) {
 // Wide calls can go in 256 x 256 tiles of two CTAs instead.  Measured on a B200 with K = 2048 and 11008, microseconds: a pair's tile takes
 // 0.36 per block of K and 1.2 besides, a CTA's 128 x 128 tile 0.27 and 0.8, its 128 x 256 tile 0.41 and 1.2; K shares cost their partial
 // sums twice at about 5 TB/s.  Fewest rounds of CTAs times tile time wins (L2 flushed, 22016 x 2048 at 2048 tokens: 152 -> 138 us, 8192 x 2048: 89 -> 62).
-bool hgemm_tc_pairs(int64_t rows, int64_t cols, int T, int max_splits, const HgemmPlan& single, HgemmPlan& pairs) {
+bool pair_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t scratch_floats, const HgemmPlan& single, HgemmPlan& pairs) {
     if (T <= 128 || rows <= HG_BM) return false;
     const int64_t kb = cols / HG_BK, row_tiles = (rows + HG_BM - 1) / HG_BM, n_tiles = (T + 255) / 256, tiles = (row_tiles + 1) / 2 * n_tiles;
     auto shares_us = [&](int s) { return s > 1 ? 8.0 * s * T * (double)rows / 5e6 : 0.0; };
@@ -924,15 +927,22 @@ bool hgemm_tc_pairs(int64_t rows, int64_t cols, int T, int max_splits, const Hge
     bool better = false;
     for (int s = 1; s <= std::max(1, std::min(max_splits, 16)); ++s) {
         const int64_t per = (kb + s - 1) / s;
-        if (s > 1 && (per < 4 || (size_t)s * T * rows * 4 > ((size_t)16 << 20))) break;
+        if (s > 1 && (per < 4 || (size_t)s * T * rows * 4 > ((size_t)16 << 20) || (size_t)s * T * rows > scratch_floats)) break;
         if ((kb + per - 1) / per != s) continue;
         const double us = rounds(tiles * s, 74) * (0.36 * (double)per + 1.2) + shares_us(s);
         if (us >= best) continue;
         best = us;
         better = true;
-        pairs = HgemmPlan{256, (int)row_tiles, (int)n_tiles, s, (int)per, s > 1 ? (size_t)s * T * rows : 0};
+        pairs = HgemmPlan{256, (int)row_tiles, (int)n_tiles, s, (int)per, s > 1 ? (size_t)s * T * rows : 0, true};
     }
     return better;
+}
+}  // namespace
+
+HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t scratch_floats, bool may_pair) {
+    const HgemmPlan single = single_plan(rows, cols, T, max_splits, scratch_floats);
+    HgemmPlan pairs;
+    return may_pair && pair_plan(rows, cols, T, max_splits, scratch_floats, single, pairs) ? pairs : single;
 }
 
 namespace {
@@ -1032,15 +1042,9 @@ int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int
     if (!W.ready) throw std::runtime_error("launch_hgemm_tc: the f16 image of the matrix was not built");
     if (xh == nullptr) throw std::runtime_error("launch_hgemm_tc: f16 activations missing");
     if (out_scale != 1.0f || softcap != 0.f || ws.partial == nullptr) max_splits = 1;
-    HgemmPlan pl = hgemm_tc_plan(W.rows, W.cols, T, max_splits), pairs;
-    const bool pair = whole_pairs(W) && hgemm_tc_pairs(W.rows, W.cols, T, max_splits, pl, pairs);
-    if (pair) pl = pairs;
-    if (pl.splits > 1 && pl.partial_floats > ws.partial_floats) {
-        pl.splits = 1;
-        pl.kb_per_split = (int)(W.cols / HG_BK);
-    }
+    const HgemmPlan pl = hgemm_tc_plan(W.rows, W.cols, T, max_splits, ws.partial != nullptr ? ws.partial_floats : 0, whole_pairs(W));
     alignas(64) CUtensorMap tx;
-    encode_half_matrix(&tx, xh, (int64_t)T * W.n_groups, W.cols, pair ? pl.bn / 2 : pl.bn, W.bf16);
+    encode_half_matrix(&tx, xh, (int64_t)T * W.n_groups, W.cols, pl.pairs ? pl.bn / 2 : pl.bn, W.bf16);
     HgParams p{};
     p.T = T;
     p.K = (int)W.cols;
@@ -1070,7 +1074,7 @@ int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int
     p.scattered = scatter != nullptr ? 1 : 0;
     if (scatter != nullptr) p.scatter = *scatter;
     const CUtensorMap& tw = *reinterpret_cast<const CUtensorMap*>(W.tmap);
-    if (pair) {
+    if (pl.pairs) {
         const int grid = 2 * std::min(device_sm_count() / 2, (p.row_tiles + 1) / 2 * p.n_tiles * p.splits);
         launch_hg<256, 6, true>(tw, tx, tw, tx, p, grid, s);
         return pl.splits;

@@ -36,12 +36,15 @@ void build_bf16_weight(const float* values, int64_t rows, int64_t cols, HalfWeig
 // The same with `groups` stacked projections of rows / groups rows each (a multiple of 128), every one with an input of its own.
 void build_bf16_weight_groups(const float* values, int64_t rows, int64_t cols, int groups, HalfWeight& out, cudaStream_t s);
 
-// How a call is cut into work items of one CTA each (see hgemm_tc.cu; wide calls may run in tiles of two CTAs instead); partial_floats is the scratch a split call needs.
+// How a call is cut into work items (see hgemm_tc.cu).  pairs: tiles of two CTAs, 256 rows x 256 tokens (row_tiles counts 128-row tiles all the
+// same).  partial_floats is the scratch that the call's K shares take, never more than scratch_floats.
 struct HgemmPlan {
     int bn = 0, row_tiles = 0, n_tiles = 0, splits = 1, kb_per_split = 0;
     size_t partial_floats = 0;
+    bool pairs = false;
 };
-HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits);
+// may_pair: no two row tiles of a pair belong to stacked projections with inputs of their own.
+HgemmPlan hgemm_tc_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t scratch_floats = SIZE_MAX, bool may_pair = true);
 
 // Device scratch of the GEMM: split-K partial sums and the status word that receives a non-zero code when
 // a bounded wait gave up.

@@ -268,13 +268,22 @@ def sample(logits: np.ndarray, settings, where: int) -> np.ndarray:
     return out
 
 
+_HALF_PLAN = ("bn", "row_tiles", "n_tiles", "splits", "kb_per_split", "partial_floats", "pairs")
+
+
 def matmul_plan(path: int, rows: int, cols: int, T: int, max_splits: int = 16) -> dict:
     """Host-only: how a launch of the f16-image GEMM (PATH_HALF) or the streamed matmul (PATH_STREAM) is cut."""
     out = np.zeros(8, dtype=np.int64)
     capi.check(capi.lib().mk_k_matmul_plan(path, rows, cols, T, max_splits, _p(out)))
-    names = ("bn", "row_tiles", "n_tiles", "splits", "kb_per_split", "partial_floats") if path == capi.PATH_HALF else \
-        ("bn", "row_tiles", "items", "ctas", "slots", "partial_floats", "tiles_per_group", "groups")
+    names = _HALF_PLAN if path == capi.PATH_HALF else ("bn", "row_tiles", "items", "ctas", "slots", "partial_floats", "tiles_per_group", "groups")
     return dict(zip(names, map(int, out)))
+
+
+def half_matmul_plan(rows: int, cols: int, T: int, max_splits: int = 16, scratch_floats: int = -1, may_pair: bool = True) -> dict:
+    """Host-only: the same for the f16-image GEMM with that much scratch (negative: any)."""
+    out = np.zeros(8, dtype=np.int64)
+    capi.check(capi.lib().mk_k_half_matmul_plan(rows, cols, T, max_splits, scratch_floats, 1 if may_pair else 0, _p(out)))
+    return dict(zip(_HALF_PLAN, map(int, out)))
 
 
 def grouped_matmul_plan(experts: int, rows_per_expert: int, rows_total: int, max_rows_per_expert: int) -> dict:

@@ -22,7 +22,9 @@ def test_f16_gemm_plans_of_the_benchmark_shapes(env):
     assert (down["row_tiles"], down["splits"], down["kb_per_split"]) == (16, 9, 20)
     gate_up = ops.matmul_plan(capi.PATH_HALF, 22016, 2048, 2048)
     assert (gate_up["bn"], gate_up["n_tiles"], gate_up["splits"]) == (256, 8, 1)  # wide ticks never share K
-    assert ops.matmul_plan(capi.PATH_HALF, 3072, 2048, 2048)["bn"] == 128         # 2.6 rounds of 128 beat 1.3 rounds of 256
+    qkv = ops.matmul_plan(capi.PATH_HALF, 3072, 2048, 2048)
+    assert (qkv["bn"], qkv["pairs"], qkv["splits"]) == (256, 1, 1)               # 96 tiles of two CTAs on 74 places beat three rounds of 128 x 128
+    assert ops.half_matmul_plan(3072, 2048, 2048, may_pair=False)["bn"] == 128    # 2.6 rounds of 128 beat 1.3 rounds of 256
     head = ops.matmul_plan(capi.PATH_HALF, 128256, 2048, 64)
     assert head["splits"] == 1                                                    # enough row tiles already
 
@@ -41,6 +43,21 @@ def test_f16_gemm_plan_invariants(env, rows, cols, T):
     else:
         assert p["partial_floats"] == 0
     assert ops.matmul_plan(capi.PATH_HALF, rows, cols, T, max_splits=1)["splits"] == 1
+    assert p["pairs"] in (0, 1) and (p["pairs"] == 0 or (T > 128 and p["bn"] == 256))
+    assert ops.half_matmul_plan(rows, cols, T) == p and ops.half_matmul_plan(rows, cols, T, may_pair=False)["pairs"] == 0
+    # shares never take more than the scratch there is; with room for one less, a plan of fewer shares
+    for floats in (0, p["partial_floats"] - 1, p["partial_floats"]):
+        less = ops.half_matmul_plan(rows, cols, T, scratch_floats=max(floats, 0))
+        assert less["partial_floats"] <= max(floats, 0) and less["kb_per_split"] * less["splits"] >= kb
+        assert less == p if floats == p["partial_floats"] else floats < 0 or less["splits"] < p["splits"] or p["splits"] == 1
+
+
+@pytest.mark.parametrize("rows,cols,T", [(22016, 2048, 2048), (2048, 11008, 2048), (8192, 2048, 2048), (9812, 256, 129), (1100, 256, 2049), (1100, 11008, 400)])
+def test_wide_calls_run_in_pairs_and_say_so(env, rows, cols, T):
+    """The shapes of the pair kernel's own tests, an odd number of row tiles among them, and those the rule was measured at."""
+    ops, capi = env
+    p = ops.matmul_plan(capi.PATH_HALF, rows, cols, T)
+    assert p["pairs"] == 1 and p["bn"] == 256 and p["n_tiles"] == -(-T // 256) and p["row_tiles"] == -(-rows // 128)
 
 
 @pytest.mark.parametrize("rows,cols", [(2560, 2048), (2048, 2048), (22016, 2048), (2048, 11008), (1000, 11008), (128, 256), (128256, 2048)])
