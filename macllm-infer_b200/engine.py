@@ -229,7 +229,7 @@ class Model:
         arr["session"] = [s._h.value or 0 if s._h else 0 for s, _, _ in lanes]
         arr["n_tokens"] = counts
         arr["input_ids"] = flat.ctypes.data + 4 * (np.cumsum(counts, dtype=np.int64) - counts).astype(np.uint64) if counts else 0
-        arr["start_pos"] = [p for _, _, p in lanes]
+        arr["start_pos"] = (C.c_int32 * len(lanes))(*[p for _, _, p in lanes])   # ctypes takes whole numbers only
         return C.cast(arr.ctypes.data, C.POINTER(capi.Lane)), (arr, flat)
 
     def forward_batch(self, lanes, want_logits=True, want_tokens=True, rows=None):

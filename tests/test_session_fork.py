@@ -16,6 +16,15 @@ def eng(mk):
     return importlib.import_module("macllm_infer_b200.engine")
 
 
+@pytest.mark.parametrize("start", [0.0, 1.5, "0", None, [0]])
+def test_a_start_position_is_a_whole_number(eng, start):
+    model = eng.Model.fake(vocab=32, kv_capacity_tokens=1024)
+    session = model.new_session()
+    with pytest.raises(TypeError):
+        model.forward_batch([(session, [1, 2, 3], start)])
+    model.forward_batch([(session, [1, 2, 3], 0)])   # nothing was reserved or run by the refused call
+
+
 def oracle_fork(om, s, n):
     return dict(table=s["table"].fork_prefix(n), len=n)
 
