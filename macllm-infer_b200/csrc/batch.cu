@@ -89,6 +89,8 @@ __global__ void __launch_bounds__(1024) build_batch_kernel(BatchDesc b, int bloc
 }  // namespace
 
 void launch_build_batch(const BatchDesc& b, int block_tokens, int q_tile, cudaStream_t s) {
+    // An ordinary launch: it begins when everything before it is done, uploads, page copies and the last tick among it, and kernels of this tick that
+    // touch memory ahead of their pdl_wait() rely on that (see launch_pdl).
     build_batch_kernel<<<1, 1024, 0, s>>>(b, block_tokens, q_tile);
     MK_LAUNCH_CHECK();
 }

@@ -63,7 +63,9 @@ __global__ void embed_kernel(QWeight W, const uint32_t* ids, float scale, float*
         }
         o[k] = scale == 1.0f ? v : __fmul_rn(v, scale);
     }
-    pdl_wait();  // the ids were staged before the predecessor began, which writes nothing that is read here; who waits for this kernel waits for both
+    // Ids were staged, and the rows' last readers done, before the predecessor began: that is the batch descriptor, an ordinary launch, which touches
+    // neither.  Who waits for this kernel waits for both.
+    pdl_wait();
 }
 
 }  // namespace

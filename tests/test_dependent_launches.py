@@ -56,6 +56,17 @@ def test_only_weights_are_declared_constant_in_kernels_that_wait():
     assert seen > 30
 
 
+def test_the_batch_descriptor_is_an_ordinary_launch_behind_the_page_copies():
+    """Kernels that touch memory ahead of their wait rely on a launch that begins when everything before the tick, and the page copies, are done."""
+    assert "build_batch_kernel<<<" in (CSRC / "batch.cu").read_text()
+    rope = (CSRC / "rope_kv.cu").read_text()
+    assert "cow_copy_kernel<uint4><<<" in rope and "cow_copy_kernel<uint16_t><<<" in rope
+    assert not any(re.search(r"launch_pdl\w*\(\s*(build_batch|cow_copy)_kernel", p.read_text()) for p in CSRC.glob("*.cu"))
+    upload = (CSRC / "device_lm.cpp").read_text()
+    upload = upload[upload.index("void DeviceLm::upload_tick"):]
+    assert 0 < upload.index("cudaMemcpyAsync(stage_dev_") < upload.index("copy_shared_pages(t)") < upload.index("launch_build_batch(")
+
+
 TICKS = """
 import hashlib, importlib, sys
 import numpy as np
