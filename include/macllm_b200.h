@@ -680,6 +680,20 @@ typedef struct mk_attn_case {
 } mk_attn_case;
 int32_t mk_k_attention_step(const mk_attn_case* c);
 
+/* Attention alone, over pools that hold every key already, in the forms that lanes of several tokens of mixer-built decoders take besides:
+ * from `c`, everything but k, v, the norms, q_rot_out and the index outputs (lanes of at least two tokens, f16 pools, tensor-core kernel);
+ * rotary_dim / rope_capacity / cos_table / sin_table turn dimensions rot_from .. rot_from + rotary_dim - 1 of the queries in adjacent
+ * pairs while they are read (rot_from a multiple of 8).  head_dim 192 takes value_dim 128 and exact weights. */
+typedef struct mk_attn_forms {
+    int32_t value_dim;            /* leading values of a row that count; 0: head_dim.  The rest of an output row stays as it is */
+    int32_t exact_weights;        /* attention weights as the sum of two f16 numbers instead of one */
+    int32_t chunk;                /* > 0: a position sees its own chunk's keys only */
+    int32_t rot_from;
+    const float* sink;            /* [q_heads]: one more term exp(sink) in the denominator; NULL: none */
+    uint16_t* out_half;           /* optional: the output rows as f16 */
+} mk_attn_forms;
+int32_t mk_k_attention_prefill(const mk_attn_case* c, const mk_attn_forms* f);
+
 /* The expert matmuls of SparseMoeFeedForward::forward (src/decoder.rs:394-441): w is a bank of `experts` matrices
  * [rows_pe][cols] of GGUF blocks of `type`, back to back; x [P][cols] holds the routed rows grouped by expert, rows
  * [offsets[e], offsets[e + 1]) going to expert e (offsets: experts + 1 ints); y [P][rows_pe].  path MK_PATH_GEMV: the

@@ -147,6 +147,11 @@ class AttnCase(C.Structure):
                 ("kernel", C.c_int32)]
 
 
+class AttnForms(C.Structure):
+    _fields_ = [("value_dim", C.c_int32), ("exact_weights", C.c_int32), ("chunk", C.c_int32), ("rot_from", C.c_int32), ("sink", C.c_void_p),
+                ("out_half", C.c_void_p)]
+
+
 # Every symbol include/macllm_b200.h declares, with its ctypes signature (restype is int32 unless noted).
 P = C.c_void_p
 _i32, _i64, _u32, _u64, _f32 = C.c_int32, C.c_int64, C.c_uint32, C.c_uint64, C.c_float
@@ -251,6 +256,7 @@ SIGNATURES = {
     "mk_k_attention_tiles": (_i32, [P, P, _i32, _i32, _i32, _i32, _i32, P, _i32, P]),
     "mk_k_attention_plan": (_i32, [P, P, _i32, _i32, _i32, _i32, P, P, P]),
     "mk_k_gated_ffn": (_i32, [_i32, P, P, _i64, _i64, P, _i32, _i32, P, _i32, P]),
+    "mk_k_attention_prefill": (_i32, [C.POINTER(AttnCase), C.POINTER(AttnForms)]),
     "mk_k_attention_step": (_i32, [C.POINTER(AttnCase)]),
     "mk_k_argmax": (_i32, [P, _i32, _i32, P]),
     "mk_k_gated_delta_decay": (_i32, [P, P, P, _i32, _i32, P]),

@@ -493,6 +493,96 @@ int32_t mk_k_attention_step(const mk_attn_case* c) {
     });
 }
 
+int32_t mk_k_attention_prefill(const mk_attn_case* c, const mk_attn_forms* f) {
+    return guarded([&] {
+        require_device();
+        const int lanes = c->lanes, d = c->head_dim, bt = c->block_tokens, heads = c->q_heads;
+        const bool turns = c->rotary_dim > 0 && c->cos_table != nullptr;
+        if (lanes <= 0 || c->kv_f16 != 1 || heads <= 0 || c->kv_heads <= 0 || heads % c->kv_heads != 0 || c->layer < 0 || c->layer >= c->layers || c->pool_blocks <= 0)
+            throw std::runtime_error("mk_k_attention_prefill: arguments out of range");
+        if (turns && (f->rot_from < 0 || f->rot_from + c->rotary_dim > d || c->rotary_dim % 2 != 0)) throw std::runtime_error("mk_k_attention_prefill: dimensions to turn out of range");
+        if (f->value_dim < 0 || f->value_dim > d) throw std::runtime_error("mk_k_attention_prefill: value width out of range");
+        std::vector<LaneHeader> hdr((size_t)lanes);
+        std::vector<int32_t> cu((size_t)lanes + 1, 0);
+        int blocks = 0;
+        for (int l = 0; l < lanes; ++l) {
+            const int end = c->start_pos[l] + c->lane_len[l];
+            if (c->lane_len[l] < 2 || c->start_pos[l] < 0 || c->table_off[l] != blocks || (int64_t)c->table_len[l] * bt < end)
+                throw std::runtime_error("mk_k_attention_prefill: lanes of at least two tokens, whose block tables are packed in lane order and cover them");
+            if (turns && end > c->rope_capacity) throw std::runtime_error("mk_k_attention_prefill: positions beyond the rotation's tables");
+            hdr[(size_t)l].start_pos = c->start_pos[l];
+            hdr[(size_t)l].n_tokens = c->lane_len[l];
+            hdr[(size_t)l].table_off = c->table_off[l];
+            hdr[(size_t)l].n_blocks = c->table_len[l];
+            blocks += c->table_len[l];
+            cu[(size_t)l + 1] = cu[(size_t)l] + c->lane_len[l];
+        }
+        if (cu[(size_t)lanes] != c->total_tokens) throw std::runtime_error("mk_k_attention_prefill: lanes do not add up to the tokens");
+        for (int i = 0; i < blocks; ++i)
+            if (c->tables[i] >= (uint32_t)c->pool_blocks) throw std::runtime_error("mk_k_attention_prefill: block id out of range");
+        const size_t pool = (size_t)c->pool_blocks * c->layers * c->kv_heads * bt * d * 2, n = (size_t)c->total_tokens * heads * d;
+        DevBuf kp(pool), vp(pool), dq(n * 4), out(n * 4), out_h(n * 2), dhdr(hdr.size() * sizeof(LaneHeader)), tab((size_t)blocks * 4), dcu(cu.size() * 4), work, dcos, dsin, dsink, status(4);
+        kp.upload(c->k_pool, pool);
+        vp.upload(c->v_pool, pool);
+        dq.upload(c->q, n * 4);
+        out.upload(c->out, n * 4);
+        if (f->out_half != nullptr) out_h.upload(f->out_half, n * 2);
+        dhdr.upload(hdr.data(), hdr.size() * sizeof(LaneHeader));
+        tab.upload(c->tables, (size_t)blocks * 4);
+        dcu.upload(cu.data(), cu.size() * 4);
+        status.zero(nullptr);
+        AttnTcPlan plan;
+        plan_attention_tc(c->start_pos, c->lane_len, c->table_len, lanes, heads, c->kv_heads, plan, f->chunk, c->window);
+        work.upload(plan.tiles.data(), plan.tiles.size() * 4);
+        AttnTcArgs a;
+        a.q = dq.as<float>();
+        a.out = out.as<float>();
+        a.out_h = f->out_half != nullptr ? out_h.as<__half>() : nullptr;
+        a.k_pool = kp.ptr();
+        a.v_pool = vp.ptr();
+        a.hdr = dhdr.as<LaneHeader>();
+        a.tables = tab.as<uint32_t>();
+        a.cu_seqlens = dcu.as<int32_t>();
+        a.tiles = work.as<int32_t>();
+        a.n_tiles = plan.n_tiles();
+        a.q_heads = heads;
+        a.kv_heads = c->kv_heads;
+        a.d = d;
+        a.dv = f->value_dim;
+        a.block_tokens = bt;
+        a.layers = c->layers;
+        a.layer = c->layer;
+        a.pool_pages = (int64_t)c->pool_blocks * c->layers;
+        a.status = status.as<int32_t>();
+        a.scale = c->scale;
+        a.softcap = c->softcap;
+        a.window = c->window;
+        a.chunk = f->chunk;
+        a.exact_weights = f->exact_weights;
+        if (f->sink != nullptr) {
+            dsink.upload(f->sink, (size_t)heads * 4);
+            a.sink = dsink.as<float>();
+        }
+        if (turns) {
+            const size_t table = (size_t)c->rope_capacity * (c->rotary_dim / 2) * 4;
+            dcos.upload(c->cos_table, table);
+            dsin.upload(c->sin_table, table);
+            a.cos_t = dcos.as<float>();
+            a.sin_t = dsin.as<float>();
+            a.rot_from = f->rot_from;
+            a.rot_dims = c->rotary_dim;
+        }
+        launch_paged_attention_tc(a, nullptr);
+        MK_CUDA(cudaDeviceSynchronize());
+        int32_t gave_up = 0;
+        status.download(&gave_up, 4);
+        out.download(c->out, n * 4);
+        if (f->out_half != nullptr) out_h.download(f->out_half, n * 2);
+        MK_CUDA(cudaDeviceSynchronize());
+        if (gave_up != 0) throw std::runtime_error("mk_k_attention_prefill: a bounded wait gave up (code " + std::to_string(gave_up) + ")");
+    });
+}
+
 namespace {
 
 // cu_seqlens as the launchers want it: on the device, rising from 0 to the number of rows

@@ -384,3 +384,30 @@ def attention_step(q, k, v, k_pool, v_pool, tables, start_pos, lane_len, *, q_he
         setattr(c, name, None if arr is None else arr.ctypes.data)
     capi.check(capi.lib().mk_k_attention_step(C.byref(c)))
     return dict(out=out, q_rot=q_rot, slots=slots, positions=pos, last_index=last, cu_seqlens=cu)
+
+
+def attention_prefill(q, k_pool, v_pool, tables, start_pos, lane_len, *, q_heads, kv_heads, head_dim, block_tokens, layers, layer, scale, softcap=0.0, window=0,
+                      chunk=0, value_dim=0, exact_weights=False, sink=None, cos_table=None, sin_table=None, rot_from=0):
+    """Attention of lanes of several tokens over f16 pools that hold every key.  Returns (f32 rows, f16 rows); what is not written is NaN."""
+    q = _f32(q)
+    lens = np.asarray([len(t) for t in tables], dtype=np.int32)
+    arrays = dict(start_pos=np.asarray(start_pos, dtype=np.int32), lane_len=np.asarray(lane_len, dtype=np.int32), table_len=lens,
+                  table_off=np.asarray(np.cumsum(lens) - lens, dtype=np.int32), tables=np.asarray([b for t in tables for b in t], dtype=np.uint32),
+                  q=q, k_pool=k_pool, v_pool=v_pool, out=np.full_like(q, np.nan))
+    if cos_table is not None:
+        arrays.update(cos_table=_f32(cos_table), sin_table=_f32(sin_table))
+    assert k_pool.dtype == v_pool.dtype == np.float16
+    c, f = capi.AttnCase(), capi.AttnForms()
+    c.lanes, c.total_tokens, c.q_heads, c.kv_heads, c.head_dim = len(lens), q.shape[0], q_heads, kv_heads, head_dim
+    c.block_tokens, c.layers, c.layer, c.pool_blocks, c.kv_f16 = block_tokens, layers, layer, k_pool.shape[0], 1
+    c.scale, c.softcap, c.window = scale, softcap, window
+    if cos_table is not None:
+        c.rope_capacity, c.rotary_dim = arrays["cos_table"].shape[0], 2 * arrays["cos_table"].shape[1]
+    for name, arr in arrays.items():
+        setattr(c, name, arr.ctypes.data)
+    half = np.full(q.shape, np.nan, dtype=np.float16)
+    sink = None if sink is None else _f32(sink)
+    f.value_dim, f.exact_weights, f.chunk, f.rot_from = value_dim, 1 if exact_weights else 0, chunk, rot_from
+    f.sink, f.out_half = None if sink is None else sink.ctypes.data, half.ctypes.data
+    capi.check(capi.lib().mk_k_attention_prefill(C.byref(c), C.byref(f)))
+    return arrays["out"], half
