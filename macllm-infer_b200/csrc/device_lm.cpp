@@ -46,8 +46,8 @@ void DeviceLm::alloc_tick(size_t extra_stage_bytes) {
     logits_.alloc((size_t)B * spec_.vocab * 4);
     argmax_scratch_.alloc(argmax_scratch_bytes(B));
     argmax_scratch_.zero(stream_);
-    const size_t bytes = (size_t)B * sizeof(LaneHeader) + (size_t)(pool_->max_blocks() + B) * 4 + (size_t)T * 8 + 128 +
-                         (size_t)B * (sizeof(LaneSampling) + sizeof(CowCopy)) + 16 + extra_stage_bytes;
+    stage_rest_ = (size_t)B * sizeof(LaneHeader) + (size_t)T * 8 + 128 + (size_t)B * (sizeof(LaneSampling) + sizeof(CowCopy)) + 16 + extra_stage_bytes;
+    const size_t bytes = stage_rest_ + (size_t)(pool_->max_blocks() + B) * 4;
     stage_host_.ensure(bytes);
     stage_dev_.alloc(bytes);
     out_host_.ensure((size_t)B * spec_.vocab * 4 + (size_t)B * 4 + 16);
@@ -66,6 +66,14 @@ DeviceLm::Tick DeviceLm::stage_tick(const std::vector<LmLane>& lanes, KvReservat
     }
     if (t.B > cfg_.max_batch_lanes) throw std::runtime_error("batch has more lanes than max_batch_lanes");
     if (t.T > cfg_.max_batch_tokens) throw std::runtime_error("batch has more tokens than max_batch_tokens");
+    // lanes that share pages name them once each, so their tables can be longer than the pool (the last tick was read: nobody uses the buffers)
+    size_t table_entries = 0;
+    for (int i = 0; i < t.B; ++i) table_entries += r.lane_blocks((size_t)i).size();
+    if (const size_t need = stage_rest_ + table_entries * 4; need > stage_host_.size() || need > stage_dev_.size()) {
+        const size_t bytes = need + need / 2;  // histories grow
+        stage_host_.ensure(bytes);
+        stage_dev_.ensure(bytes);
+    }
     t.hp = stage_host_.as<uint8_t>();
     t.dp = stage_dev_.as<uint8_t>();
     // the per-lane headers, block tables and token ids

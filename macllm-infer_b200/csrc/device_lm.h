@@ -84,6 +84,7 @@ private:
     std::vector<const char*> prof_names_;
     std::vector<KernelProfile> prof_;
     PinnedBuf stage_host_, out_host_;
+    size_t stage_rest_ = 0;  // bytes of a tick's staging besides the block tables, at most
     DevBuf stage_dev_, argmax_scratch_;
     int out_lanes_ = 0, out_rows_ = 0;
     uint32_t out_flags_ = 0;

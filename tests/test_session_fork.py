@@ -112,3 +112,30 @@ def test_copy_on_write_page_copy_matches_the_oracle(mk, eng, tmp_path_factory, k
     model.synchronize()
     ps, os_ = model.pool_stats(), om.pool.stats()
     assert ps["live_blocks"] == os_["live_blocks"] and ps["reserved_blocks"] == os_["reserved_blocks"] == 0
+
+
+@pytest.mark.gpu
+def test_lanes_that_share_more_pages_than_the_pool_has(mk, eng, tmp_path_factory):
+    """64 lanes over one prefix name its pages 64 times: 7808 table entries with a pool of 256 pages.  The results are those of a pool that could
+    hold every lane's pages."""
+    seed = importlib.import_module("macllm_infer_b200.seed_gguf")
+    spec = seed.scaled("tinyllama-1.1b", layers=1, vocab=512)
+    path = tmp_path_factory.mktemp("fork") / "llama.gguf"
+    seed.write_seed_gguf(path, spec, seed=0)
+    prefix = 1936
+    got = []
+    for capacity in (4096, 64 * (prefix + 32)):
+        model = eng.Model.load_gguf(path, kv_dtype="f16", max_batch_tokens=64, max_batch_lanes=64, kv_capacity_tokens=capacity)
+        rng = np.random.default_rng(0)
+        prompt = rng.integers(3, spec.vocab, prefix)
+        first = model.new_session()
+        for at in range(0, prefix, 64):
+            model.forward_batch([(first, prompt[at:at + 64], at)])
+        sessions = [first] + [first.fork_prefix(prefix) for _ in range(63)]
+        rows = []
+        for step in range(3):
+            ids = rng.integers(3, spec.vocab, 64)
+            logits, _ = model.forward_batch([(s, [int(t)], prefix + step) for s, t in zip(sessions, ids)])
+            rows.append(logits)
+        got.append(np.stack(rows))
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
