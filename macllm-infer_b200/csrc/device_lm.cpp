@@ -33,7 +33,7 @@ void DeviceLm::open_device() {
     status_.zero(stream_);
 }
 
-void DeviceLm::alloc_tick(size_t extra_stage_bytes) {
+void DeviceLm::alloc_tick(size_t extra_stage_bytes, size_t block_tables) {
     const int T = cfg_.max_batch_tokens, B = cfg_.max_batch_lanes;
     cu_.alloc((size_t)(B + 1) * 4);
     pos_.alloc((size_t)T * 4);
@@ -47,7 +47,8 @@ void DeviceLm::alloc_tick(size_t extra_stage_bytes) {
     argmax_scratch_.alloc(argmax_scratch_bytes(B));
     argmax_scratch_.zero(stream_);
     stage_rest_ = (size_t)B * sizeof(LaneHeader) + (size_t)T * 8 + 128 + (size_t)B * (sizeof(LaneSampling) + sizeof(CowCopy)) + 16 + extra_stage_bytes;
-    const size_t bytes = stage_rest_ + (size_t)(pool_->max_blocks() + B) * 4;
+    stage_tables_ = block_tables;
+    const size_t bytes = stage_rest_ + stage_tables_ * (size_t)(pool_->max_blocks() + B) * 4;
     stage_host_.ensure(bytes);
     stage_dev_.alloc(bytes);
     out_host_.ensure((size_t)B * spec_.vocab * 4 + (size_t)B * 4 + 16);
@@ -69,7 +70,7 @@ DeviceLm::Tick DeviceLm::stage_tick(const std::vector<LmLane>& lanes, KvReservat
     // lanes that share pages name them once each, so their tables can be longer than the pool (the last tick was read: nobody uses the buffers)
     size_t table_entries = 0;
     for (int i = 0; i < t.B; ++i) table_entries += r.lane_blocks((size_t)i).size();
-    if (const size_t need = stage_rest_ + table_entries * 4; need > stage_host_.size() || need > stage_dev_.size()) {
+    if (const size_t need = stage_rest_ + stage_tables_ * table_entries * 4; need > stage_host_.size() || need > stage_dev_.size()) {
         const size_t bytes = need + need / 2;  // histories grow
         stage_host_.ensure(bytes);
         stage_dev_.ensure(bytes);

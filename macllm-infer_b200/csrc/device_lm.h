@@ -26,8 +26,8 @@ protected:
     DeviceLm(const ModelConfig& cfg, const std::vector<const char*>& profile_classes);
     // Selects the device (throws when there is none: no CPU fallback) and creates the stream and events.
     void open_device();
-    // Buffers of a tick: call once the pool exists.  `extra_stage_bytes` is what the model stages on top.
-    void alloc_tick(size_t extra_stage_bytes);
+    // Buffers of a tick: call once the pool exists.  `extra_stage_bytes` is what the model stages on top, `block_tables` how often it stages the lanes' block tables.
+    void alloc_tick(size_t extra_stage_bytes, size_t block_tables = 1);
 
     struct Tick {
         int B = 0, T = 0, R = 0;  // lanes, tokens, rows projected to logits
@@ -84,7 +84,8 @@ private:
     std::vector<const char*> prof_names_;
     std::vector<KernelProfile> prof_;
     PinnedBuf stage_host_, out_host_;
-    size_t stage_rest_ = 0;  // bytes of a tick's staging besides the block tables, at most
+    size_t stage_rest_ = 0;    // bytes of a tick's staging besides the block tables, at most
+    size_t stage_tables_ = 1;  // how often it holds the lanes' block tables, at most
     DevBuf stage_dev_, argmax_scratch_;
     int out_lanes_ = 0, out_rows_ = 0;
     uint32_t out_flags_ = 0;

@@ -500,12 +500,12 @@ void MixerLm::alloc_activations() {
         }
     }
     for (const LatentGeometry& g : latent_geo_) extra += (size_t)latent_max_entries((int)T, g.ctas) * 32 + (size_t)T * 4 + 32;
-    extra += wide_.size() * ((size_t)B * sizeof(LaneHeader) + (size_t)(T + B) * 8 + (size_t)T * 4 + (size_t)(pool_->max_blocks() + B) * 4 + 64);
+    extra += wide_.size() * ((size_t)B * sizeof(LaneHeader) + (size_t)(T + B) * 8 + (size_t)T * 4 + 64);
     attn_part_o_.alloc(part_o);
     attn_part_ml_.alloc(part_ml);
     attn_counters_.alloc(counters);
     attn_counters_.zero(stream_);
-    alloc_tick(extra);
+    alloc_tick(extra, 1 + wide_.size());
 }
 
 // ---------------------------------------------------------------------------- forward

@@ -167,6 +167,7 @@ private:
     void matmul_scatter(const Dense& W, const RowImage& x, int T, const MatmulScatter& to);
     void set_norm(RowUpdateArgs& a, const Norm& n) const;
     int latent_geometry(int ctas, bool tc, bool wide, int window);
+    void count_blocks(size_t n);
     void plan_latent(Tick& t, const std::vector<int32_t>& start, const std::vector<int32_t>& n_tokens, const std::vector<int32_t>& n_blocks, KvReservation& r);
 
     // Branch outputs not yet added to the residual stream.

@@ -134,12 +134,7 @@ void MixerLm::load_latent(const SafetensorsFile& f, int l) {
     w.geometry = latent_geometry(tc ? latent_tc_groups(H) : 1, tc, wide, a.window);
     if (a.rot_dim > 0) w.rope = rope_table(a.rot);
     if (a.sink) upload_f32(f.values(m + "sink", {H}), w.sink);
-    if (wide && iota_.size() == 0) {
-        std::vector<uint32_t> n((size_t)(pool_->max_blocks() + cfg_.max_batch_lanes));
-        for (size_t i = 0; i < n.size(); ++i) n[i] = (uint32_t)i;
-        iota_.upload(n.data(), n.size() * 4, stream_);
-        MK_CUDA(cudaStreamSynchronize(stream_));
-    }
+    if (wide) count_blocks((size_t)(pool_->max_blocks() + cfg_.max_batch_lanes));
 
     upload_dense(f, {{m + "uq", H * (a.dim + a.rot_dim), 0, 1, 0, 0, a.dim + a.rot_dim, w.q_width, a.dim, w.q_rot0, a.rot.dims}}, (int64_t)H * w.q_width, a.q_rank, w.uq);
     const int64_t uk_bytes = (int64_t)H * a.dim * a.kv_rank * esz_, uv_bytes = (int64_t)H * a.vdim * a.kv_rank * esz_;
@@ -176,6 +171,15 @@ void MixerLm::load_latent(const SafetensorsFile& f, int l) {
 
 // ---------------------------------------------------------------------------- a tick's work lists
 
+// iota_: 0, 1, 2, ... up to `n` at least, the block table of expanded latents.  No tick is in flight.
+void MixerLm::count_blocks(size_t n) {
+    if (n * 4 <= iota_.size()) return;
+    std::vector<uint32_t> v(n + n / 2);
+    for (size_t i = 0; i < v.size(); ++i) v[i] = (uint32_t)i;
+    iota_.upload(v.data(), v.size() * 4, stream_);
+    MK_CUDA(cudaStreamSynchronize(stream_));
+}
+
 void MixerLm::plan_latent(Tick& t, const std::vector<int32_t>& start, const std::vector<int32_t>& n_tokens, const std::vector<int32_t>& n_blocks, KvReservation& r) {
     for (LatentGeometry& g : latent_geo_) {
         plan_latent_attention(start.data(), n_tokens.data(), n_blocks.data(), t.B, g.ctas, g.wide ? kWideFrom : INT_MAX, g.tc, g.plan, g.window);
@@ -206,6 +210,7 @@ void MixerLm::plan_latent(Tick& t, const std::vector<int32_t>& start, const std:
             w.keys += s0 + n - first_key;
         }
         if (w.rows.empty()) continue;
+        count_blocks(w.blocks.size());  // lanes that share pages expand them once each: more blocks than the pool has
         w.off_hdr = stage_bytes(t, w.hdr.data(), w.hdr.size() * sizeof(LaneHeader));
         w.off_tiles = stage_bytes(t, w.tiles.data(), w.tiles.size() * 4);
         w.off_rows = stage_bytes(t, w.rows.data(), w.rows.size() * 4);

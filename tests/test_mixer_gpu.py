@@ -512,6 +512,27 @@ def test_a_fork_carries_pages_and_state(mk, built, name, compute):
     model.close()
 
 
+@pytest.mark.parametrize("name", ["looped", "convolved"])
+def test_prompts_of_forks_that_share_more_pages_than_the_pool_has(mk, built, name):
+    """Latents of long prompts are expanded lane by lane, shared pages once for each: 60 of them out of a pool of 27.  A pool that could hold
+    every lane's pages gives the same bits."""
+    folder, oracle, cfg = built(name)
+    toks = tokens_of(200, cfg["vocab"], seed=8)
+    tails = [tokens_of(40, cfg["vocab"], seed=30 + i) for i in range(4)]
+    got = []
+    for capacity in (432, 1024):
+        model = mc.load(folder, "bfloat16", capacity=capacity)
+        a = model.new_session()
+        model.forward_batch([(a, toks, 0)], want_tokens=False)
+        sessions = [a] + [a.fork_prefix(200) for _ in tails[1:]]
+        rows, _ = model.forward_batch([(s, t, 200) for s, t in zip(sessions, tails)], want_tokens=False, rows=[range(40)] * 4)
+        got.append(rows)
+        model.close()
+    assert np.array_equal(got[0], got[1])
+    for i, t in enumerate(tails):
+        mc.assert_rows(got[0][40 * i:40 * i + 40], oracle.logits(toks + t)[200:], "bfloat16")
+
+
 @pytest.mark.parametrize("name", ["second", "looped", "experts", "convolved"])
 def test_a_refused_forward_leaves_the_state_alone(mk, built, capi, name):
     folder, oracle, cfg = built(name)
