@@ -698,21 +698,24 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
-        // The commits that hand back the last stages are waited for by nobody else, and in a pair they come from the other CTA: none may find
-        // this one gone.  Where a wait gave up, copies in flight land first.
-        loaded = __shfl_sync(0xffffffffu, loaded, 0);
-        gave_up = __shfl_sync(0xffffffffu, (int)gave_up, 0) != 0;
-        if (lane < STAGES && (uint32_t)lane < loaded) {
-            const uint32_t ph = ((loaded - 1 - lane) / STAGES) & 1;
-            if (gave_up || !mbar_wait(&empty[lane], ph, HG_SPIN_LIMIT)) {
-                atomicExch(p.status, 11);
-                if (rank == 0) mbar_wait(&full[lane], ph, HG_SPIN_LIMIT);
+    if constexpr (PAIR) {
+        if (warp == 0) {
+            // The commits that hand back the last stages come from the leader, and nobody else waits for them: none may find this CTA gone.  (A
+            // CTA by itself sees its accumulator's commit, the last of a row of commits of one thread.)  Where a wait gave up, copies
+            // in flight land first.
+            loaded = __shfl_sync(0xffffffffu, loaded, 0);
+            gave_up = __shfl_sync(0xffffffffu, (int)gave_up, 0) != 0;
+            if (lane < STAGES && (uint32_t)lane < loaded) {
+                const uint32_t ph = ((loaded - 1 - lane) / STAGES) & 1;
+                if (gave_up || !mbar_wait(&empty[lane], ph, HG_SPIN_LIMIT)) {
+                    atomicExch(p.status, 11);
+                    if (rank == 0) mbar_wait(&full[lane], ph, HG_SPIN_LIMIT);
+                }
             }
+            __syncwarp();
         }
-        __syncwarp();
+        cluster_sync();  // the peer is done with this CTA's barriers and shared memory
     }
-    if constexpr (PAIR) cluster_sync();  // the peer is done with this CTA's barriers and shared memory
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
