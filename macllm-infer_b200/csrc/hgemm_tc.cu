@@ -917,22 +917,28 @@ HgemmPlan single_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t 
     return pl;
 }
 
-// Wide calls can go in 256 x 256 tiles of two CTAs instead.  Measured on a B200 with K = 2048 and 11008, microseconds: a pair's tile takes
-// 0.36 per block of K and 1.2 besides, a CTA's 128 x 128 tile 0.27 and 0.8, its 128 x 256 tile 0.41 and 1.2; K shares cost their partial
-// sums twice at about 5 TB/s.  Fewest rounds of CTAs times tile time wins (L2 flushed, 22016 x 2048 at 2048 tokens: 152 -> 138 us, 8192 x 2048: 89 -> 62).
+// Wide calls can go in 256 x 256 tiles of two CTAs instead.  Microseconds a round of CTAs takes on a B200 with kb blocks of K, from launches of one to
+// nineteen rounds at K = 256 ... 11008 with the L2 flushed: a pair's tiles 0.31 kb + 2.9, at least 4.75 (its stores); 128 x 256 tiles of one CTA
+// 0.33 kb + 3.2, and 0.41 kb where K is long; 128 x 128 tiles 0.25 kb + 1.35.  A launch of pairs takes 1.8 more.  K shares cost their partial sums
+// twice at about 5 TB/s.  The fewest microseconds win: pairs for several rounds or long K (22016 x 2048 at 2048 tokens: 152 -> 143 us, 8192 x 2048
+// at 2048: 88 -> 64), one CTA a tile for a single round of short K (2048 x 2048 at 1420: 25.4 in pairs, 23.6) and for K up to 512 (8192 x 256 at
+// 2048: 29.6 and 25.6).
 bool pair_plan(int64_t rows, int64_t cols, int T, int max_splits, size_t scratch_floats, const HgemmPlan& single, HgemmPlan& pairs) {
     if (T <= 128 || rows <= HG_BM) return false;
     const int64_t kb = cols / HG_BK, row_tiles = (rows + HG_BM - 1) / HG_BM, n_tiles = (T + 255) / 256, tiles = (row_tiles + 1) / 2 * n_tiles;
     auto shares_us = [&](int s) { return s > 1 ? 8.0 * s * T * (double)rows / 5e6 : 0.0; };
     auto rounds = [](int64_t items, int64_t at_once) { return (double)((items + at_once - 1) / at_once); };
-    double best = rounds((int64_t)single.row_tiles * single.n_tiles * single.splits, 148) *
-                      ((single.bn == 256 ? 0.41 : 0.27) * single.kb_per_split + (single.bn == 256 ? 1.2 : 0.8)) + shares_us(single.splits);
+    auto pair_us = [](double k) { return std::max({4.75, 0.31 * k + 2.9, 0.345 * k}); };
+    auto wide_us = [](double k) { return std::max(0.33 * k + 3.2, 0.405 * k); };
+    auto narrow_us = [](double k) { return std::max(0.25 * k + 1.35, 0.27 * k); };
+    double best = rounds((int64_t)single.row_tiles * single.n_tiles * single.splits, 148) * (single.bn == 256 ? wide_us(single.kb_per_split) : narrow_us(single.kb_per_split)) +
+                  shares_us(single.splits);
     bool better = false;
     for (int s = 1; s <= std::max(1, std::min(max_splits, 16)); ++s) {
         const int64_t per = (kb + s - 1) / s;
         if (s > 1 && (per < 4 || (size_t)s * T * rows * 4 > ((size_t)16 << 20) || (size_t)s * T * rows > scratch_floats)) break;
         if ((kb + per - 1) / per != s) continue;
-        const double us = rounds(tiles * s, 74) * (0.36 * (double)per + 1.2) + shares_us(s);
+        const double us = 1.8 + rounds(tiles * s, 74) * pair_us((double)per) + shares_us(s);
         if (us >= best) continue;
         best = us;
         better = true;
