@@ -8,6 +8,7 @@ scheduler ticks, read back generated tokens.  Everything runs in libmacllm_b200.
 from __future__ import annotations
 
 import ctypes as C
+from array import array
 from dataclasses import dataclass
 
 import numpy as np
@@ -229,7 +230,11 @@ class Model:
         arr["session"] = [s._h.value or 0 if s._h else 0 for s, _, _ in lanes]
         arr["n_tokens"] = counts
         arr["input_ids"] = flat.ctypes.data + 4 * (np.cumsum(counts, dtype=np.int64) - counts).astype(np.uint64) if counts else 0
-        arr["start_pos"] = (C.c_int32 * len(lanes))(*[p for _, _, p in lanes])   # ctypes takes whole numbers only
+        starts = [p for _, _, p in lanes]
+        try:
+            arr["start_pos"] = array("i", starts)   # whole numbers only, like a ctypes field, which takes three times as long
+        except OverflowError:
+            arr["start_pos"] = (C.c_int32 * len(starts))(*starts)   # a field wraps
         return C.cast(arr.ctypes.data, C.POINTER(capi.Lane)), (arr, flat)
 
     def forward_batch(self, lanes, want_logits=True, want_tokens=True, rows=None):
