@@ -17,6 +17,8 @@ WEIGHTS = {
     "qgemv_q4k_kernel": {"W"},
     "qgemv_q6k_kernel": {"ql_p", "qh_p", "sc_p", "d_p"},
     "qgemv_q80_kernel": {"qs_p", "d_p"},
+    "qgemv_q6k_row_kernel": {"ql_p", "qh_p", "sc_p", "d_p"},
+    "qgemv_q80_row_kernel": {"qs_p", "d_p"},
     "f32_gemv_kernel": {"W"},
     "f32_gemv_tile_kernel": {"W"},
     "f32_matmul_kernel": {"w"},
