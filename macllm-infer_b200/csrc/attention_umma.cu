@@ -99,12 +99,11 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     fence_after();
     const uint32_t tmem = tmem_slot;
     pdl_trigger();
-    pdl_wait();
-
+    // the work list, the lanes' headers and their block tables were staged ahead of the tick's first launch; everything else waits
     const int g = a.q_heads / a.kv_heads;
     const int work = blockIdx.x / a.kv_heads, kvh = blockIdx.x - work * a.kv_heads;
     const int lane_id = a.tiles[2 * work], row0 = a.tiles[2 * work + 1];
-    const int rows_per_head = AU_ITEMS / g;
+    const int rows_shift = __ffs(AU_ITEMS / g) - 1, rows_per_head = 1 << rows_shift;  // groups are powers of two
     const LaneHeader hdr = a.hdr[lane_id];
     const int n_rows = min(rows_per_head, hdr.n_tokens - row0);
     const int p_first = hdr.start_pos + row0, p_last = p_first + n_rows - 1;
@@ -117,9 +116,15 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         bool ok = true;
         uint32_t page = 0;
         int t = 0;
+        if (lane == 0) {
+            prefetch_tensormap(&tm_k);
+            prefetch_tensormap(&tm_v);
+        }
+        if (k_begin + lane * AU_PAGE < k_hi) page = a.tables[hdr.table_off + ((k_begin + lane * AU_PAGE) >> a.bt_shift)];
+        pdl_wait();
         for (; t < n_tiles && ok; ++t) {
             const int pos0 = k_begin + t * AU_KEYS, pages = min(AU_KEYS / AU_PAGE, (k_hi - pos0 + AU_PAGE - 1) / AU_PAGE);
-            if ((t & 7) == 0) {  // the page ids of the next eight tiles sit in the lanes
+            if ((t & 7) == 0 && t > 0) {  // the page ids of the next eight tiles sit in the lanes
                 const int pos = pos0 + lane * AU_PAGE;
                 page = pos < k_hi ? a.tables[hdr.table_off + (pos >> a.bt_shift)] : 0u;
             }
@@ -152,6 +157,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         }
     } else if (warp == 5) {
         // ---- MMA issuer
+        pdl_wait();
         if (lane == 0) {
             constexpr uint32_t i_scores = f16_idesc(AU_ITEMS, AU_KEYS, false), i_out = f16_idesc(AU_ITEMS, DV, true);
             const uint32_t q_addr = smem_u32(qs), k_addr = smem_u32(ks), v_addr = smem_u32(vs);
@@ -193,37 +199,48 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     } else {
         // ---- one item per thread
         const int ldq = a.ldq > 0 ? a.ldq : a.q_heads * D, ldo = a.q_heads * D;
-        constexpr int CHUNKS = D / 8;
-#pragma unroll 4
-        for (int i = tid; i < AU_ITEMS * CHUNKS; i += AU_ITEMS) {
-            const int item = i / CHUNKS, c = (i - item * CHUNKS) * 8;
-            const int hq = item / rows_per_head, r = item - hq * rows_per_head;
-            uint32_t h[4] = {0u, 0u, 0u, 0u};
-            if (r < n_rows) {
-                const float* src = a.q + (int64_t)(a.cu_seqlens[lane_id] + row0 + r) * ldq + (kvh * g + hq) * D + c;
-                float4 x0 = *reinterpret_cast<const float4*>(src), x1 = *reinterpret_cast<const float4*>(src + 4);
-                if (c >= a.rot_from && c < a.rot_from + a.rot_dims) {
+        constexpr int CHUNKS = D / 8, BATCH = 8;
+        pdl_wait();
+        const int64_t first_row = a.cu_seqlens[lane_id] + row0;
+        // the queries, eight pieces of a thread on their way together: a short prompt's CTA waits for little else (a launch of 64 rows, 16 heads of 128
+        // over 4, took 14.5 us with four at a time and the work list read behind the wait, this 10.0; 16 heads of 256 over 8: 21.3 and 14.4; 64 lanes
+        // of 32 rows, 32 heads of 128 over 8: 36.4 and 27.1)
+#pragma unroll 1
+        for (int i0 = tid; i0 < AU_ITEMS * CHUNKS; i0 += BATCH * AU_ITEMS) {
+            float4 x[BATCH][2];
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                const int i = i0 + k * AU_ITEMS, item = i / CHUNKS, c = (i - item * CHUNKS) * 8, hq = item >> rows_shift, r = item & (rows_per_head - 1);
+                x[k][0] = x[k][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < n_rows) {
+                    const float* src = a.q + (first_row + r) * ldq + (kvh * g + hq) * D + c;
+                    x[k][0] = *reinterpret_cast<const float4*>(src);
+                    x[k][1] = *reinterpret_cast<const float4*>(src + 4);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                const int i = i0 + k * AU_ITEMS, item = i / CHUNKS, c = (i - item * CHUNKS) * 8, r = item & (rows_per_head - 1);
+                float4 &x0 = x[k][0], &x1 = x[k][1];
+                if (r < n_rows && c >= a.rot_from && c < a.rot_from + a.rot_dims) {
                     const int64_t pair0 = (int64_t)(p_first + r) * (a.rot_dims / 2) + (c - a.rot_from) / 2;
                     float* p[4][2] = {{&x0.x, &x0.y}, {&x0.z, &x0.w}, {&x1.x, &x1.y}, {&x1.z, &x1.w}};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (c - a.rot_from + 2 * k >= a.rot_dims) break;
-                        const float cs = a.cos_t[pair0 + k], sn = a.sin_t[pair0 + k], u = *p[k][0], v = *p[k][1];
-                        *p[k][0] = u * cs - v * sn;
-                        *p[k][1] = v * cs + u * sn;
+                    for (int j = 0; j < 4; ++j) {
+                        if (c - a.rot_from + 2 * j >= a.rot_dims) break;
+                        const float cs = a.cos_t[pair0 + j], sn = a.sin_t[pair0 + j], u = *p[j][0], v = *p[j][1];
+                        *p[j][0] = u * cs - v * sn;
+                        *p[j][1] = v * cs + u * sn;
                     }
                 }
-                h[0] = half2_bits(x0.x, x0.y);
-                h[1] = half2_bits(x0.z, x0.w);
-                h[2] = half2_bits(x1.x, x1.y);
-                h[3] = half2_bits(x1.z, x1.w);
+                *reinterpret_cast<uint4*>(qs + (c >> 6) * AU_QPANEL + item * 128 + (((c & 63) * 2) ^ ((item & 7) << 4))) =
+                    make_uint4(half2_bits(x0.x, x0.y), half2_bits(x0.z, x0.w), half2_bits(x1.x, x1.y), half2_bits(x1.z, x1.w));
             }
-            *reinterpret_cast<uint4*>(qs + (c >> 6) * AU_QPANEL + item * 128 + (((c & 63) * 2) ^ ((item & 7) << 4))) = make_uint4(h[0], h[1], h[2], h[3]);
         }
         fence_async_smem();
         bar_arrive(q_full);
 
-        const int hq = tid / rows_per_head, r = tid - hq * rows_per_head;
+        const int hq = tid >> rows_shift, r = tid & (rows_per_head - 1);
         const int pos = p_first + r, lo = attention_first_key(pos, a.window, a.chunk), lo_last = attention_first_key(p_last, a.window, a.chunk);
         const uint32_t my = tmem + ((uint32_t)(warp * 32) << 16);
         const float two_over_cap = a.softcap != 0.f ? 2.0f / a.softcap : 0.f;
@@ -314,7 +331,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 const float m = m_run * 0.6931471805599453f, sink = a.sink[kvh * g + hq], top = fmaxf(m, sink), f = __expf(m - top);
                 inv = f / (sum * f + __expf(sink - top));
             }
-            const int64_t at = (int64_t)(a.cu_seqlens[lane_id] + row0 + r) * ldo + (kvh * g + hq) * D;
+            const int64_t at = (first_row + r) * ldo + (kvh * g + hq) * D;
 #pragma unroll 1
             for (int c = 0; c < DV; c += 32) {
                 uint32_t o[32];

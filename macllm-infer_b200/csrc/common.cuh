@@ -95,7 +95,7 @@ inline bool pdl_enabled() {
 // Launch `kernel` with programmatic stream serialisation, in clusters of `cluster` CTAs.  Ahead of its pdl_wait() such a kernel may touch only what
 // no launch since the last ordinary one writes or (where it writes itself) reads, because every launch in between may still be running: weights,
 // and what was there before the tick.  That last ordinary launch is the batch descriptor's, at the start of every tick, and these rely on it:
-// attn_decode_kernel reads its work list, block tables and older pages early, embed_kernel reads the ids and writes its rows, and the kernels of
+// attn_decode_kernel reads its work list, block tables and older pages early, attn_umma_kernel its work list and block tables, embed_kernel reads the ids and writes its rows, and the kernels of
 // recurrent layers read their lane lists and the lanes' states.
 template <typename... Params, typename... Args>
 inline void launch_pdl_cluster(void (*kernel)(Params...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {

@@ -41,6 +41,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int 
         ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void prefetch_tensormap(const void* tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Operand in shared memory.  Reduction along the rows' bytes (K-major): `lead` is not used.  Reduction from row to row (MN-major):
