@@ -7,7 +7,8 @@
 // thread: a row of scores comes in one piece, so maximum and sum need no exchange; P goes back as f16 (EXACT: as the f16 number
 // and the f16 rounding of what it left, two products).  The scores of the next tile are made while this tile's softmax runs.
 // The running maximum follows only when a tile exceeds it by more than kSlack (weights stay below 2^kSlack, well inside f16), so
-// the accumulators in tensor memory are hardly ever rescaled.  Every wait is bounded.
+// the accumulators in tensor memory are hardly ever rescaled (conditional rescaling, as the authors of FlashAttention-4 describe it).  Every wait
+// is bounded.
 //
 // What bounds it: exponentials (16 per clock and SM; a soft cap takes two more per score) and the tensor pipe are about level at head size
 // 128.  Heads of up to 128 run two CTAs per SM (96 KB of shared memory, 256 columns of tensor memory each), so that one's softmax runs under

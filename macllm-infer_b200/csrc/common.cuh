@@ -74,9 +74,9 @@ __host__ __device__ __forceinline__ int64_t kv_page_index(int64_t blk, int layer
 // Programmatic dependent launch: a kernel launched through launch_pdl may start (be scheduled, run its
 // prologue) while the previous kernel of the stream is still running; pdl_wait() blocks until that kernel has
 // completed and its writes are visible, so it must precede the first access to anything the predecessor wrote
-// or still reads.  Such data never comes in through a `const T* __restrict__` parameter: that promises that nobody writes it while the kernel
-// runs, and lets the compiler load it ahead of the wait.  pdl_trigger() lets the next kernel of the stream begin its own launch early.  Both are no-ops
-// for kernels launched the ordinary way.
+// or still reads.  Such data never comes in through a `const T* __restrict__` parameter: that promises that nobody writes it
+// while the kernel runs, and lets the compiler load it ahead of the wait.  pdl_trigger() lets the next kernel of the stream begin its own
+// launch early.  Both are no-ops for kernels launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -95,8 +95,8 @@ inline bool pdl_enabled() {
 // Launch `kernel` with programmatic stream serialisation, in clusters of `cluster` CTAs.  Ahead of its pdl_wait() such a kernel may touch only what
 // no launch since the last ordinary one writes or (where it writes itself) reads, because every launch in between may still be running: weights,
 // and what was there before the tick.  That last ordinary launch is the batch descriptor's, at the start of every tick, and these rely on it:
-// attn_decode_kernel reads its work list, block tables and older pages early, attn_umma_kernel its work list and block tables, embed_kernel reads the ids and writes its rows, and the kernels of
-// recurrent layers read their lane lists and the lanes' states.
+// attn_decode_kernel reads its work list, block tables and older pages early, attn_umma_kernel its work list and block tables, embed_kernel
+// reads the ids and writes its rows, and the kernels of recurrent layers read their lane lists and the lanes' states.
 template <typename... Params, typename... Args>
 inline void launch_pdl_cluster(void (*kernel)(Params...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg{};

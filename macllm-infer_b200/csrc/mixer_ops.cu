@@ -169,7 +169,8 @@ __device__ __forceinline__ Pack<VEC> norm_pack(const RowUpdateArgs& a, const Row
 
 // Shared memory: the row, its neighbour (n_mix > 0), and a staging row for a second normed branch.
 // THREADS: twice as many where the rows leave SMs idle - a row's latency counts then, and with 2048 columns every thread has one pack
-// (16 rows: 6.3 -> 5.0 us from launch to launch).
+// (16 rows: 6.3 -> 5.0 us from launch to launch).  The squares of a row are then added in another order: its last bits depend on whether the tick
+// has up to 148 rows or more, as those of the matmuls around it do.
 template <int VEC, int THREADS>
 __global__ void __launch_bounds__(THREADS) row_update_kernel(RowUpdateArgs a) {
     extern __shared__ __align__(16) float ru_smem[];

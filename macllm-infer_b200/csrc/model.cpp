@@ -276,7 +276,7 @@ void Model::ep_init(const uint8_t* id) {
 // The column width the expert-grouped matmuls are launched with: rows of one expert are processed in chunks of that many,
 // and a chunk costs the same whether it is full or not, so a tick whose experts see a handful of rows each runs narrow
 // chunks (an expert with more rows than one chunk takes a second pass over its weights), a wide tick runs full ones.
-// MACLLM_B200_MOE_CHUNK=16|32|64 pins it.
+// MACLLM_B200_MOE_CHUNK=16|32|64|128 pins it.
 static int moe_chunk_rows(int T, int k, int experts) {
     static const int pinned = [] { const char* e = std::getenv("MACLLM_B200_MOE_CHUNK"); return e ? atoi(e) : 0; }();
     if (pinned == 16 || pinned == 32 || pinned == 64 || pinned == 128) return pinned;
@@ -1009,8 +1009,8 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
                                    stream_);
             } else if (moe_stream) {
                 // the routed rows grouped by expert as f16, then the expert-grouped tensor-core matmuls: gate|up with the
-                // activation in its epilogue (f16 out), down on those rows.  Every expert's weights are read once per 64
-                // of its rows; the row ranges stay on the device.
+                // activation in its epilogue (f16 out), down on those rows.  Every expert's weights are read once per
+                // chunk of up to 128 of its rows; the row ranges stay on the device.
                 prof_begin(KC_MOE, 4.0 * P * H, 0);
                 launch_gather_rows_half(xf.xh, tok_of_pos_.as<int32_t>(), P, H, e_xh_.as<__half>(), stream_);
                 prof_end();

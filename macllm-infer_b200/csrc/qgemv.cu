@@ -8,13 +8,12 @@
 // Only the weights are promised to the compiler as constant (const __restrict__): a load of such memory may move in front of pdl_wait(), and
 // what a predecessor produces must not.
 //
-// Memory plan: one warp owns one output row and streams that row's blocks with 128-bit (Q4_K,
+// Memory plan: a warp streams the blocks of its output rows with 128-bit (Q4_K,
 // Q8_0) or 64-bit (Q6_K planes) loads, eight lanes per 256-weight block, so a warp consumes whole
 // 128-byte lines; activations (T*K bytes) are re-read from L1/L2.  Each weight byte leaves HBM once
-// per call when T <= NT; larger T re-walks the row from cache in passes.  A warp takes R output rows that follow one
-// another: their weights travel together, and an activation that was fetched meets all of them (with one row per warp and
-// eight sums whatever T, 32000 x 2048 in Q6_K took 26 us at one activation row,
-// this 15).
+// per call when T <= NT; larger T re-walks the row from cache in passes.  Where there are warps for every
+// scheduler all the same, a warp takes R output rows that follow one another: their weights travel together, and an activation that was
+// fetched meets all of them (with one row per warp and eight sums whatever T, 32000 x 2048 in Q6_K took 26 us at one activation row, this 15).
 #include "kernels.h"
 #include "mma_bf16.cuh"
 #include <algorithm>

@@ -1,5 +1,6 @@
-// Blackwell tensor-core and TMA primitives shared by kernels: bounded mbarrier waits, box loads, tcgen05 products and tensor-memory
-// moves.  Operands are tiles of 128-byte swizzled rows in shared memory (8-row groups 1024 bytes apart) or f16 rows in tensor memory.
+// Blackwell tensor-core and TMA primitives of the prefill attention (the matmul kernels keep forms of their own): bounded mbarrier waits, box
+// loads, tcgen05 products and tensor-memory moves.  Operands are tiles of 128-byte swizzled rows in shared memory (8-row groups 1024 bytes apart)
+// or f16 rows in tensor memory.
 #pragma once
 #include "common.cuh"
 
