@@ -60,7 +60,7 @@ WORKLOAD_NAMES = ["tinyllama-1.1b-batch4", "smollm3-3b-ragged64", "qwen3-8b-pref
 # benchmark's shapes (dram__bytes_read.sum + dram__bytes_write.sum over the bytes counted here; profiles/).  The
 # roofline block scales the live per-launch algorithmic bytes by these ratios.
 NCU_TRAFFIC_RATIO = {
-    "hgemm_tc": (98.8 + 21.4) / (90.2 + 8.4 + 45.1),      # gate|up with the activation in the epilogue: every operand once; part of the f16 output is still in L2 at kernel end
+    "hgemm_tc": (98.7 + 25.3) / (90.2 + 8.4 + 45.1),      # gate|up with the activation in the epilogue: every operand once; part of the f16 output is still in L2 at kernel end
     "paged_attention": (77.0 + 1.9) / (72.4 + 4.2),
     "qstream_tc": (25.70 + 0.004) / (25.36 + 0.26),         # streamed gate|up of a decode tick: every weight block once, the partial sums stay in L2
 }
