@@ -7,15 +7,15 @@
 // once at load time: w = f16(dequant(block)), one rounding per weight.  The GEMM is then the plain
 // y[t][n] = sum_k xh[t][k] * wh[n][k] with f32 accumulation in tensor memory.
 //
-// One persistent CTA per SM, 320 threads in three roles:
+// One persistent CTA per SM, 320 threads (576 in pairs) in three roles:
 //   warp 0   - one lane issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of 128 x 64 weight
 //              and BN x 64 activation boxes into a ring of shared-memory stages;
 //   warp 1   - one lane issues the MMAs (tcgen05.mma kind::f16, M = 128 weight rows, N = BN tokens,
 //              four K = 16 steps per block of 64), commits each stage back to the loader, and commits the tile
 //              to the epilogue; two accumulators in tensor memory alternate so the next tile's main
 //              loop runs under the previous tile's epilogue;
-//   warps 2-9 - read the accumulator (tcgen05.ld, one lane per weight row, two warps per lane quadrant that take
-//              every other 32 columns), apply scale / soft cap and store f32 results (32 consecutive rows of one
+//   warps 2-9 - (2-17 in pairs) read the accumulator (tcgen05.ld, one lane per weight row, two or four warps per lane quadrant that take
+//              32 columns in turn), apply scale / soft cap and store f32 results (32 consecutive rows of one
 //              token per store instruction).  A tile's main loop is as long as K, its epilogue is not: with short K
 //              it is the epilogue's instructions that count, hence eight warps and whole 32-column groups without
 //              a test per column.
@@ -36,8 +36,10 @@ namespace {
 
 constexpr int HG_BM = 128;
 constexpr int HG_BK = 64;  // 64 halves = 128 bytes = one swizzle row
-constexpr int HG_EPI_THREADS = 256;
-constexpr int HG_THREADS = 64 + HG_EPI_THREADS;
+// Pairs run 16 epilogue warps: their gated epilogue is a chain of exponentials and divisions per feature, which eight warps (two per scheduler) could
+// not finish under the next tile's products (22016 x 2048 at 2048 tokens, gated: 161 -> 147 us; plain 143.8 and 144.6).
+constexpr int hg_epi_threads(bool pair) { return pair ? 512 : 256; }
+constexpr int hg_threads(bool pair) { return 64 + hg_epi_threads(pair); }
 constexpr uint32_t HG_SPIN_LIMIT = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -285,6 +287,7 @@ struct HgSmem {
     static constexpr int B_ROWS = PAIR ? BN / 2 : BN;   // activation rows that this CTA loads
     static constexpr int B_BYTES = B_ROWS * HG_BK * 2;
     static constexpr int KB = hg_stage_blocks(BN);
+    static constexpr int EPI_THREADS = hg_epi_threads(PAIR);
     static constexpr int STAGE_BYTES = KB * (A_BYTES + B_BYTES);
     static constexpr size_t TOTAL = (size_t)STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
@@ -332,10 +335,11 @@ __device__ __forceinline__ void gated_columns(const uint32_t (&r)[32], int n, bo
 // PAIR: two CTAs of a cluster make one 256 x BN tile; each holds half of the weight rows and their accumulators, and half of the
 // activation rows.
 template <int BN, int STAGES, bool GATED, bool PAIR>
-__global__ void __launch_bounds__(HG_THREADS, 1)
+__global__ void __launch_bounds__(hg_threads(PAIR), 1)
 hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1,
                 const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ HgParams p) {
     using L = HgSmem<BN, STAGES, PAIR>;
+    constexpr int EPI_THREADS = L::EPI_THREADS, COL_GROUPS = EPI_THREADS / 128;
     constexpr int LD_COLS = BN >= 32 ? 32 : BN, HG_KB = L::KB;
     extern __shared__ uint8_t hg_smem_raw[];
     __shared__ int32_t first_item[HG_MAX_EXPERTS + 1];  // grouped by expert: items of the experts before
@@ -363,7 +367,7 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], (PAIR ? 2 : 1) * HG_EPI_THREADS);
+            mbar_init(&acc_empty[i], (PAIR ? 2 : 1) * EPI_THREADS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -568,8 +572,8 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             }
         }
     } else {
-        // ---- epilogue: warps 2..9 own TMEM lane quadrants (warp % 4), two each
-        const int quad = warp & 3, odd_group = (warp - 2) >> 2;
+        // ---- epilogue: warps 2 and up own TMEM lane quadrants (warp % 4), two each, or four in pairs
+        const int quad = warp & 3, col_group = (warp - 2) >> 2;
         const int etid = (int)threadIdx.x - 64;  // among the epilogue threads
         const bool plain = p.out_scale == 1.0f && p.softcap == 0.f;
         if (GATED || p.part[0].act_post != nullptr) pdl_wait();   // the factors of the rows, or the gates, come from a predecessor
@@ -590,7 +594,7 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 "bar.red.and.pred p, 1, %2, q;\n\t"
                 "selp.u32 %0, 1, 0, p;\n\t}"
                 : "=r"(all_got)
-                : "r"(got), "n"(HG_EPI_THREADS)
+                : "r"(got), "n"(EPI_THREADS)
                 : "memory");
             if (!all_got) {
                 if (etid == 0) atomicExch(p.status, 14);
@@ -603,7 +607,7 @@ hgemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             float* dst = p.splits > 1 ? p.partial + (int64_t)split * p.T * p.rows : part.y;
             const int ld = p.splits > 1 ? p.rows : part.ldy;
 #pragma unroll 1
-            for (int cb = odd_group * LD_COLS; cb < BN; cb += 2 * LD_COLS) {
+            for (int cb = col_group * LD_COLS; cb < BN; cb += COL_GROUPS * LD_COLS) {
                 if (tok0 + cb >= tile.tok_end) break;  // uniform over the warp: nothing but padding from here on
                 // the factors of the chunk's tokens, one per lane, on their way with the accumulators
                 float pre = 1.0f, post = 1.0f;
@@ -760,8 +764,8 @@ void launch_hg(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& 
     constexpr size_t smem = HgSmem<BN, STAGES, PAIR>::TOTAL;
     auto* kernel = p.scattered != 0 && p.scatter.gate != nullptr ? hgemm_tc_kernel<BN, STAGES, true, PAIR> : hgemm_tc_kernel<BN, STAGES, false, PAIR>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (PAIR) launch_pdl_cluster(kernel, 2, dim3(grid), dim3(HG_THREADS), smem, s, tw, tx, tw1, tx1, p);
-    else launch_pdl(kernel, dim3(grid), dim3(HG_THREADS), smem, s, tw, tx, tw1, tx1, p);
+    if (PAIR) launch_pdl_cluster(kernel, 2, dim3(grid), dim3(hg_threads(PAIR)), smem, s, tw, tx, tw1, tx1, p);
+    else launch_pdl(kernel, dim3(grid), dim3(hg_threads(PAIR)), smem, s, tw, tx, tw1, tx1, p);
     MK_LAUNCH_CHECK();
 }
 
