@@ -707,7 +707,8 @@ int32_t mk_k_grouped_qmatmul(int32_t type, const void* w, const void* up_w, int3
  * tiles, K shares, K blocks (of 64) per share, floats of partial sums, 1 when two CTAs share a tile of 256 rows, 0}, for a matrix of one
  * input and scratch for any number of shares (mk_k_half_matmul_plan: otherwise); path MK_PATH_STREAM (T <= 64): out =
  * {token-tile width, row tiles, (group of row tiles, 256-column block) items, persistent CTAs, partial-sum slots, floats
- * of partial sums, row tiles per group, groups}.  Needs no GPU. */
+ * of partial sums, row tiles per group, groups}.  Needs no GPU.  Calls of so few rows that warps stream
+ * their own weights (csrc/narrow_mma.h: up to 16 on MK_PATH_HALF, up to 8 on MK_PATH_STREAM) are cut otherwise, into at most as many shares. */
 int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t* out8);
 /* Host-only: the same for MK_PATH_HALF with scratch_floats floats for partial sums (negative: any number); may_pair 0: stacked projections whose
  * borders lie inside pairs of row tiles, so that every tile stays on one CTA. */

@@ -39,6 +39,8 @@
 #include "qstream_tc.h"
 #include "hgemm_tc.h"
 #include "kernels.h"
+#include "kquant_half.cuh"
+#include "narrow_mma.h"
 #include <cuda.h>
 #include <algorithm>
 
@@ -52,8 +54,7 @@ constexpr int QS_EPI_WARPS = 8;
 constexpr int QS_THREADS = (3 + QS_CONV_WARPS + QS_EPI_WARPS) * 32;  // 864
 constexpr int QS_MAX_STAGES = 8;
 constexpr int qs_x_stages(int bn) { return bn <= 64 ? 3 : 2; }    // activation blocks in flight (L2 latency)
-constexpr int QS_Q4K_UNIT = QS_BM * 144;                         // 18432
-constexpr int QS_Q6K_UNIT = QS_BM * (128 + 64 + 16) + 256;       // 26880: ql, qh, scales planes + d (f16, padded)
+constexpr int QS_Q4K_UNIT = kQ4Unit, QS_Q6K_UNIT = kQ6Unit;
 constexpr int QS_ACC = 4;                                        // most accumulators in tensor memory
 constexpr int qs_accumulators(int bn) { return bn <= 64 ? QS_ACC : 2; }
 constexpr int QS_SMEM_LIMIT = 212 * 1024;                        // rings of the widest form, beside 8 KB of job table
@@ -165,80 +166,22 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
         : "memory");
 }
 
-// ---- Q4_K ------------------------------------------------------------------------------------------------------
-// Half a row's 256-wide block: groups 4h .. 4h + 3 of 32 weights, whose scales and minima come out of `hdr` (d, dmin, the twelve scale bytes)
-// four at a time.  `blk` is the row's 144-byte block; groups 2J and 2J + 1 share the 32 bytes at 16 + 32 J, low nibbles / high nibbles.
-// Four nibbles become (1024 + q) or, where they are, (1024 + 16 q) as f16 by byte permutation; a fma with the scale (a sixteenth of it) and -1024
-// (-64) of it gives sc * q exactly (below 1024); then fma(sc * q, d, -dmin * m): the dequantised weight, rounded once.  The scales too stay
-// in f16, where whole numbers below 64 and one product's rounding are what they are in f32.
-// The converters' integer instructions bound a narrow matmul: a group at a time, with its scales by way of f32 and its bytes
-// read twice, a block took half as many of them again (75776 x 2048 at one row: 35.3 us, this 34.1; at 64 rows 38.9 and 37.1).
-struct Q4Half {
-    uint32_t sc4, m4;
-    __half2 d, nd;
-    __device__ __forceinline__ Q4Half(const uint4& hdr, int h) {
-        if (h == 0) {
-            sc4 = hdr.y & 0x3F3F3F3Fu;
-            m4 = hdr.z & 0x3F3F3F3Fu;
-        } else {
-            sc4 = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
-            m4 = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
-        }
-        const uint32_t dd = __byte_perm(hdr.x, 0, 0x1010), nn = __byte_perm(hdr.x, 0, 0x3232) ^ 0x80008000u;
-        d = *reinterpret_cast<const __half2*>(&dd);
-        nd = *reinterpret_cast<const __half2*>(&nn);
-    }
-    // byte i of four as an f16 pair
-    static __device__ __forceinline__ __half2 pair(uint32_t four, int i) {
-        const uint32_t p = __byte_perm(four, 0x64646464u, 0x4040 + 0x0101 * i);
-        return __hadd2(*reinterpret_cast<const __half2*>(&p), __float2half2_rn(-1024.f));
-    }
-    // group g (0 .. 3 of this half) out of its eight words
-    template <int g>
-    __device__ __forceinline__ void convert(const uint32_t (&words)[8], uint32_t (&out)[16]) const {
-        constexpr bool HIGH = (g & 1) != 0;
-        const __half2 sc = pair(sc4, g), nm = __hmul2(nd, pair(m4, g));
-        const __half2 s = HIGH ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc, nb = __hmul2(sc, __float2half2_rn(HIGH ? -64.f : -1024.f));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t bytes = words[i] & (HIGH ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
-            const uint32_t p01 = __byte_perm(bytes, 0x64646464u, 0x4140), p23 = __byte_perm(bytes, 0x64646464u, 0x4342);
-            const __half2 h01 = __hfma2(__hfma2(*reinterpret_cast<const __half2*>(&p01), s, nb), d, nm);
-            const __half2 h23 = __hfma2(__hfma2(*reinterpret_cast<const __half2*>(&p23), s, nb), d, nm);
-            out[2 * i] = *reinterpret_cast<const uint32_t*>(&h01);
-            out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h23);
-        }
-    }
-};
+// The converters' integer instructions bound a narrow matmul: a group at a time, with its scales by way of f32 and its bytes read twice, a
+// block took half as many of them again (75776 x 2048 at one row: 35.3 us, this 34.1; at 64 rows 38.9 and 37.1).
 __device__ __forceinline__ void load_words(const uint8_t* p, uint32_t (&words)[8]) {
     const uint4 a = *reinterpret_cast<const uint4*>(p), b = *reinterpret_cast<const uint4*>(p + 16);
     words[0] = a.x; words[1] = a.y; words[2] = a.z; words[3] = a.w;
     words[4] = b.x; words[5] = b.y; words[6] = b.z; words[7] = b.w;
 }
 
-// ---- Q6_K ------------------------------------------------------------------------------------------------------
-// Unit layout: ql plane [128 rows][128 B], qh plane [128][64 B], scales plane [128][16 B], d [128] f16.  The 16-byte
-// chunks of a row of the ql and qh planes are stored at chunk ^ (row & 7) / chunk ^ (row & 3) so that the 32 rows a
-// warp reads at once fall into different banks.
-constexpr int Q6_QL = 0, Q6_QH = QS_BM * 128, Q6_SC = Q6_QH + QS_BM * 64, Q6_D = Q6_SC + QS_BM * 16;
-// Four 6-bit values, a byte each, -> (q - 32) * s.
-__device__ __forceinline__ void q6_to_weights(uint32_t q, __half2 s, uint32_t& o01, uint32_t& o23) {
-    uint32_t p01 = __byte_perm(q, 0x64646464u, 0x4140);
-    uint32_t p23 = __byte_perm(q, 0x64646464u, 0x4342);
-    const __half2 bias = __float2half2_rn(-1056.f);  // 1024 + q - 1056 = q - 32, exact
-    __half2 h01 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&p01), bias), s);
-    __half2 h23 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&p23), bias), s);
-    o01 = *reinterpret_cast<uint32_t*>(&h01);
-    o23 = *reinterpret_cast<uint32_t*>(&h23);
-}
 // Quarter qq (32 weights) of half n of the block: weight l of the group comes from ql[64 n + 32 (qq & 1) + l] (low nibbles for qq < 2, high nibbles otherwise) with
 // its two high bits in qh[32 n + l] at bit 2 qq; scales sc[8 n + 2 qq] for l < 16 and sc[8 n + 2 qq + 1] for l >= 16.
 __device__ __forceinline__ void convert_q6k_group(const uint8_t* raw, int row, int G, uint32_t (&out)[16]) {
     const int n = G >> 2, qq = G & 3;
-    const uint8_t* ql_row = raw + Q6_QL + row * 128;
-    const uint8_t* qh_row = raw + Q6_QH + row * 64;
-    const int8_t* sc = reinterpret_cast<const int8_t*>(raw + Q6_SC + row * 16) + 8 * n + 2 * qq;
-    const float d = __half2float(*reinterpret_cast<const __half*>(raw + Q6_D + row * 2));
+    const uint8_t* ql_row = raw + row * 128;
+    const uint8_t* qh_row = raw + kQ6Qh + row * 64;
+    const int8_t* sc = reinterpret_cast<const int8_t*>(raw + kQ6Sc + row * 16) + 8 * n + 2 * qq;
+    const float d = __half2float(*reinterpret_cast<const __half*>(raw + kQ6D + row * 2));
     const __half2 s0 = __float2half2_rn(d * (float)sc[0]), s1 = __float2half2_rn(d * (float)sc[1]);
     const int sh_lo = (qq >> 1) * 4, sh_hi = 2 * qq;
 #pragma unroll
@@ -744,17 +687,17 @@ __global__ void retile_q6k_kernel(const uint8_t* ql, const uint8_t* qh, const ui
         const int r = in_unit >> 3, ch = in_unit & 7;
         const int64_t row = tile * QS_BM + r;
         if (row < rows) v = *reinterpret_cast<const uint4*>(ql + ((row * nb + blk) * 128 + ch * 16));
-        *reinterpret_cast<uint4*>(out + Q6_QL + r * 128 + ((ch ^ (r & 7)) << 4)) = v;
+        *reinterpret_cast<uint4*>(out + r * 128 + ((ch ^ (r & 7)) << 4)) = v;
     } else if (in_unit < QS_BM * 12) {  // qh: 4 chunks per row
         const int k = in_unit - QS_BM * 8, r = k >> 2, ch = k & 3;
         const int64_t row = tile * QS_BM + r;
         if (row < rows) v = *reinterpret_cast<const uint4*>(qh + ((row * nb + blk) * 64 + ch * 16));
-        *reinterpret_cast<uint4*>(out + Q6_QH + r * 64 + ((ch ^ (r & 3)) << 4)) = v;
+        *reinterpret_cast<uint4*>(out + kQ6Qh + r * 64 + ((ch ^ (r & 3)) << 4)) = v;
     } else if (in_unit < QS_BM * 13) {  // scales: 1 chunk per row
         const int r = in_unit - QS_BM * 12;
         const int64_t row = tile * QS_BM + r;
         if (row < rows) v = *reinterpret_cast<const uint4*>(sc + (row * nb + blk) * 16);
-        *reinterpret_cast<uint4*>(out + Q6_SC + r * 16) = v;
+        *reinterpret_cast<uint4*>(out + kQ6Sc + r * 16) = v;
     } else {  // d: 8 rows per chunk
         const int k = in_unit - QS_BM * 13;
         __half h[8];
@@ -762,7 +705,7 @@ __global__ void retile_q6k_kernel(const uint8_t* ql, const uint8_t* qh, const ui
             const int64_t row = tile * QS_BM + k * 8 + i;
             h[i] = row < rows ? d[row * nb + blk] : __float2half(0.f);
         }
-        *reinterpret_cast<uint4*>(out + Q6_D + k * 16) = *reinterpret_cast<uint4*>(h);
+        *reinterpret_cast<uint4*>(out + kQ6D + k * 16) = *reinterpret_cast<uint4*>(h);
     }
 }
 
@@ -908,6 +851,33 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
     const int64_t rows = W.rows + (W2 ? W2->rows : 0);
     const int row_tiles = W.row_tiles + (W2 ? W2->row_tiles : 0);
     const int sms = device_sm_count();
+    if (narrow_preferred(NarrowFormat::Blocks, rows, W.cols, T, gated)) {
+        const bool any_q6 = W.fmt != 0 || (W2 != nullptr && W2->fmt != 0);
+        const NarrowPlan np = narrow_plan(NarrowFormat::Blocks, any_q6, rows, W.cols, T, gated ? 1 : max_splits, partial_floats, 1, sms);
+        if (np.ok) {
+            NarrowCall c;
+            c.format = NarrowFormat::Blocks;
+            c.w = W.tiled.ptr();
+            c.w2 = W2 != nullptr ? W2->tiled.ptr() : nullptr;
+            c.rows = rows;
+            c.rows_first = W.rows;
+            c.cols = W.cols;
+            c.q6 = W.fmt != 0;
+            c.q6_2 = W2 != nullptr && W2->fmt != 0;
+            c.x = xh;
+            c.T = T;
+            c.y = y;
+            c.ldy = ldy;
+            c.partial = partial;
+            c.status = status;
+            const GatedAct act{gated_act == 0 ? GatedAct::Silu : GatedAct::GeluTanh};
+            if (gated) c.act = &act;
+            c.yh = yh;
+            c.ldyh = ldyh;
+            launch_narrow_mma(c, np, s);
+            return np.shares;
+        }
+    }
     QStreamPlan pl = qstream_plan(row_tiles, nb, rows, T, gated ? 1 : max_splits, gated, sms);
     if (pl.slots > 1 && pl.partial_floats > partial_floats) pl = qstream_plan(row_tiles, nb, rows, T, 1, true, sms);
     alignas(64) CUtensorMap tx;
