@@ -76,6 +76,10 @@ protected:
 private:
     void prof_resolve();
     cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr;
+    static constexpr int kOutParts = 4;
+    cudaEvent_t ev_part_[kOutParts - 1] = {};   // behind all but the last part of the logits
+    int out_parts_ = 1;
+    size_t out_part(size_t bytes, int i) const { return i == out_parts_ ? bytes : bytes / (size_t)out_parts_ / 256 * 256 * (size_t)i; }
     bool timed_ = false;
     // profiling: one event pair per launch group, resolved after the tick's barrier
     struct ProfSpan { int cls; double bytes, flops; cudaEvent_t a, b; };

@@ -315,7 +315,7 @@ namespace {
 // Appends a row of logits to each result, which has room for it.
 void record_rows(const std::vector<std::pair<EngineResult*, const float*>>& rows, int vocab) {
     const int n = (int)rows.size();
-#pragma omp parallel for schedule(static) num_threads(std::min(8, n)) if ((size_t)n * (size_t)vocab >= (size_t)1 << 18)
+#pragma omp parallel for schedule(static) num_threads(std::min(8, n)) if ((size_t)n * (size_t)vocab >= (size_t)1 << 16)
     for (int i = 0; i < n; ++i) rows[(size_t)i].first->logits.insert(rows[(size_t)i].first->logits.end(), rows[(size_t)i].second, rows[(size_t)i].second + vocab);
 }
 }  // namespace

@@ -39,7 +39,7 @@ inline PrefixDigest prefix_hash_block(const PrefixDigest& previous, uint32_t blo
     h.update_u32le(block_index);
     h.update_u32le(n);
     h.update(previous.data(), 32);
-    for (uint32_t i = 0; i < n; ++i) h.update_u32le(tokens[i]);
+    h.update(tokens, (size_t)n * 4);  // the host is little-endian
     return h.finish();
 }
 
