@@ -48,6 +48,13 @@ __device__ __forceinline__ uint32_t pack_half2(float x, float y) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// The 8 x 8 tile of f16 numbers that a warp holds as (row lane / 4, columns 2 (lane % 4), + 1), transposed.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+    uint32_t r;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+
 // What f16 rounding left of two attention weights, as f16 numbers themselves.
 __device__ __forceinline__ uint32_t pack_half2_rest(float x, float y, uint32_t rounded) {
     const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&rounded));
@@ -70,21 +77,22 @@ __device__ __forceinline__ float sink_scale(float m, float l, float sink) {
 // block-wide barrier inside the loop), keep their own running max / sum / output, and merge through shared
 // memory at the end.  n_shares == 1: the CTA writes the normalised output.  Otherwise it writes its unnormalised
 // partial, and the CTA that arrives last at the lane's counter merges the shares.
-// LOW8: at most eight query heads per KV head, so rows 8-15 of the A operand are zero and everything that concerns
-// them (half of the softmax and of the accumulator rescaling) is skipped.
+// A KV head has at most eight query heads, so the heads are the N of the products and keys (scores) or dimensions (outputs) the M: S^T = K Q^T, O^T = V^T P^T.
+// With the heads as M half of every product and accumulator was zeros.  A lane then holds two heads of its tile's keys g and g + 8; the weights turn
+// into the operand of the second product by two 8 x 8 transposes.
 // History does not wait for the predecessor: every key but the newest was written before this tick's first kernel, so the first tiles are
 // requested ahead of pdl_wait.  THREADS: while the CTAs have an SM each, four more warps help with what is not a walk - a CTA has up to ten
 // head vectors to prepare, whose shares come from the L2 one after the other (4 lanes of 300 keys, 32 heads of 64 over 4: 17 -> 11 us a launch, one
 // lane of 200, 16 heads of 128 over 4: 13 -> 9); with two CTAs on an SM the registers are worth more (64 lanes: 27 us, 37 with the help).
-template <int D, int STAGES, bool LOW8, bool EXACT, int THREADS>
+template <int D, int STAGES, bool EXACT, int THREADS, int WALKERS>
 __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
-    constexpr int NH = LOW8 ? 1 : 2;  // accumulator row halves that can hold live rows
     constexpr int DP = D + 8;
     constexpr int KT = 16;
-    constexpr int NT_O = D / 8;
+    constexpr int NT_O = D / 16;      // tiles of 16 dimensions
+    constexpr int OP = D + 4;         // floats between heads of a warp's partial result: a fragment's lanes hit all banks
     constexpr int CHUNKS = D / 8;
     constexpr int RING_HALVES = STAGES * 2 * KT * DP;  // per warp: STAGES x (K tile + V tile)
-    static_assert(RING_HALVES * 2 >= 16 * D * 4 + 16 * 2 * 4, "a warp's ring must hold its partial result");
+    static_assert(RING_HALVES * 2 >= 8 * OP * 4 + 8 * 2 * 4, "a warp's ring must hold its partial result");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* Qs = reinterpret_cast<__half*>(smem_raw);  // [16][DP]
     __half* rings = Qs + 16 * DP;
@@ -94,30 +102,65 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
     const int kvh = blockIdx.y;
     const int g = a.q_heads / a.kv_heads;
     const float two_over_cap = a.softcap != 0.f ? 2.0f / a.softcap : 0.f;
-    pdl_trigger();
     // one 32-byte record per work item, so that nothing but the block table and the queries is a dependent load
     const int4 e0 = reinterpret_cast<const int4*>(a.entries)[2 * blockIdx.x];
     const int4 e1 = reinterpret_cast<const int4*>(a.entries)[2 * blockIdx.x + 1];
     const int lane_id = e0.x, split = e0.y, n_splits = e0.z, start_pos = e0.w, table_off = e1.x, q_off = e1.y, first_entry = e1.z;
     const int ldq = a.ldq > 0 ? a.ldq : a.q_heads * D;
 
-    // Rows straight from the projection's output (see AttnTcArgs::fused_rope): one warp per head, the head vector staged
+    // Rows straight from the projection's output (see AttnTcArgs::fused_rope): whole heads per warp, the head vectors staged
     // in f32; the group's query heads, and in the CTA that walks the lane's newest keys also the new K and V rows, which
     // reach the pool before any tile is requested (block-wide barrier below).
-    __shared__ __align__(16) float head_stage[THREADS / 32][D];
-    auto prepare_head = [&](int kind, int item) {  // kind 0: query head `item` of the group; 1 / 2: the new K / V row
-        float* xs = head_stage[warp];
-        rope_head_prepare(a.rk, kind, kind == 0 ? kvh * g + item : kvh, q_off, start_pos, xs, lane);
-        if (kind == 0) {
-            for (int i = lane; i < D; i += 32) Qs[item * DP + i] = __float2half_rn(xs[i]);
+    constexpr int WARPS = THREADS / 32, MAX_HEADS = (10 + WARPS - 1) / WARPS;   // of a warp
+    __shared__ __align__(16) float head_stage[WARPS * MAX_HEADS][D];
+    RopeAngles angles = {};
+    if (a.fused_rope) angles = rope_angles(a.rk, start_pos, lane);
+    auto put_head = [&](int h, const float* xs) {  // head h of the group's query heads, then the new K and V row
+        if (h < g) {
+            for (int i = lane; i < D; i += 32) Qs[h * DP + i] = __float2half_rn(xs[i]);
         } else {
             const int64_t blk = a.tables[table_off + (start_pos >> a.bt_shift)];
             const int64_t base = ((kv_page_index(blk, a.layer, a.layers, a.pool_blocks) * a.kv_heads + kvh) * a.block_tokens +
                                   (start_pos & (a.block_tokens - 1))) * (int64_t)D;
-            __half* pool = reinterpret_cast<__half*>(kind == 1 ? a.rk.k_pool : a.rk.v_pool);
+            __half* pool = reinterpret_cast<__half*>(h == g ? a.rk.k_pool : a.rk.v_pool);
             for (int i = lane; i < D; i += 32) pool[base + i] = __float2half_rn(xs[i]);
         }
-        __syncwarp();
+    };
+    auto prepare_heads = [&](int n_heads) {
+        const float* src[MAX_HEADS];
+        float* xs[MAX_HEADS];
+        int parts[MAX_HEADS];
+        int64_t stride[MAX_HEADS];
+        uintptr_t place = 0;
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < MAX_HEADS; ++k) {
+            const int h = warp + k * WARPS, kind = h < g ? 0 : (h == g ? 1 : 2);
+            xs[k] = head_stage[warp + k * WARPS];
+            src[k] = nullptr;
+            parts[k] = kind == 2 ? a.rk.v_splits : a.rk.qk_splits;
+            stride[k] = kind == 2 ? a.rk.v_split_stride : a.rk.qk_split_stride;
+            if (h < n_heads) {
+                src[k] = rope_head_source(a.rk, kind, kind == 0 ? kvh * g + h : kvh, q_off);
+                place |= reinterpret_cast<uintptr_t>(src[k]) | (uintptr_t)(stride[k] * 4);
+                n = k + 1;
+            }
+        }
+        const bool whole = a.rk.d == D && rope_head_width(a.rk, 2) == D;
+        if (whole && D % 128 == 0 && (place & 15) == 0) rope_sum_heads<float4>(src, parts, stride, n, D, xs, lane);
+        else if (whole && (place & 7) == 0) rope_sum_heads<float2>(src, parts, stride, n, D, xs, lane);
+        else
+            for (int k = 0; k < n; ++k) {
+                const int kind = warp + k * WARPS < g ? 0 : (warp + k * WARPS == g ? 1 : 2);
+                rope_sum_shares<float>(src[k], parts[k], stride[k], rope_head_width(a.rk, kind), xs[k], lane);
+            }
+#pragma unroll
+        for (int k = 0; k < MAX_HEADS; ++k) {
+            if (k >= n) break;
+            const int h = warp + k * WARPS, kind = h < g ? 0 : (h == g ? 1 : 2);
+            rope_head_finish(a.rk, kind, kind == 0 ? kvh * g + h : kvh, angles, xs[k], lane);
+            put_head(h, xs[k]);
+        }
     };
     const int p = start_pos;  // the query's position
     int k_lo = attention_first_key(p, a.window, a.chunk);
@@ -130,22 +173,22 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
     }
     const int k_begin = k_lo / 16 * 16;
     const int n_tiles = k_hi > k_begin ? (k_hi - k_begin + KT - 1) / KT : 0;
-    const int my_tiles = warp < 4 && n_tiles > warp ? (n_tiles - warp + 3) / 4 : 0;  // tiles warp, warp + 4, ...
+    const int my_tiles = warp < WALKERS && n_tiles > warp ? (n_tiles - warp + WALKERS - 1) / WALKERS : 0;  // tiles warp, warp + WALKERS, ...
 
     const __half* kp = reinterpret_cast<const __half*>(a.k_pool);
     const __half* vp = reinterpret_cast<const __half*>(a.v_pool);
-    __half* ring = rings + (warp & 3) * RING_HALVES;
+    __half* ring = rings + (warp % WALKERS) * RING_HALVES;
     uint32_t tile_blk = 0;
     auto load_tile = [&](int i) {  // the warp's i-th tile into stage i % STAGES (called with i = 0, 1, 2, ... in order)
         __half* kd = ring + (i % STAGES) * 2 * KT * DP;
         __half* vd = kd + KT * DP;
         // 16 keys starting at a multiple of 16 lie in one page (block_tokens is a multiple of 16): one table
         // lookup, then the tile is one contiguous run of 16 * D halves in each pool
-        const int pos0 = k_begin + (warp + 4 * i) * KT;
+        const int pos0 = k_begin + (warp + WALKERS * i) * KT;
         // the page ids of the warp's next 32 tiles sit in the lanes (fetched together, off the critical path)
         if ((i & 31) == 0) {
             const int t = i + lane;
-            tile_blk = t < my_tiles ? a.tables[table_off + ((k_begin + (warp + 4 * t) * KT) >> a.bt_shift)] : 0u;
+            tile_blk = t < my_tiles ? a.tables[table_off + ((k_begin + (warp + WALKERS * t) * KT) >> a.bt_shift)] : 0u;
         }
         const int64_t blk = __shfl_sync(0xffffffffu, tile_blk, i & 31);
         const int64_t src0 = ((kv_page_index(blk, a.layer, a.layers, a.pool_blocks) * a.kv_heads + kvh) * a.block_tokens +
@@ -162,7 +205,7 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
     };
 
     // tiles that may travel before the predecessor is done: all but the one with the newest key
-    const int old_tiles = my_tiles - (my_tiles > 0 && k_begin + (warp + 4 * (my_tiles - 1)) * KT + KT > p ? 1 : 0);
+    const int old_tiles = my_tiles - (my_tiles > 0 && k_begin + (warp + WALKERS * (my_tiles - 1)) * KT + KT > p ? 1 : 0);
     const int early = min(old_tiles, STAGES - 1);
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i)
@@ -170,14 +213,13 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
             load_tile(i);
             cp_async_commit();
         }
-    // rows of the A operand without a query head
-    for (int i = tid; i < (16 - g) * CHUNKS; i += THREADS) *reinterpret_cast<uint4*>(Qs + (g + i / CHUNKS) * DP + (i % CHUNKS) * 8) = make_uint4(0u, 0u, 0u, 0u);
+    // rows of the operand without a query head
+    for (int i = tid; i < (8 - g) * CHUNKS; i += THREADS) *reinterpret_cast<uint4*>(Qs + (g + i / CHUNKS) * DP + (i % CHUNKS) * 8) = make_uint4(0u, 0u, 0u, 0u);
     pdl_wait();
     if (a.fused_rope) {
-        const int n_heads = g + (split == n_splits - 1 ? 2 : 0);
-        for (int h = warp; h < n_heads; h += THREADS / 32) prepare_head(h < g ? 0 : (h == g ? 1 : 2), h);
+        prepare_heads(g + (split == n_splits - 1 ? 2 : 0));
     } else {
-        // the group's query heads -> rows 0..g-1 of the A operand
+        // the group's query heads -> rows 0..g-1 of the operand
         for (int i = tid; i < g * CHUNKS; i += THREADS) {
             const int item = i / CHUNKS, c = (i - item * CHUNKS) * 8;
             const float* src = a.q + (int64_t)q_off * ldq + (kvh * g + item) * D + c;
@@ -193,17 +235,18 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
             if (i < my_tiles) load_tile(i);
             cp_async_commit();
         }
+    pdl_trigger();
 
-    float o_acc[NT_O][4];
+    float o_acc[NT_O][4];   // (dimension gid, heads 2 tq, 2 tq + 1), (dimension gid + 8, the same)
 #pragma unroll
     for (int j = 0; j < NT_O; ++j) o_acc[j][0] = o_acc[j][1] = o_acc[j][2] = o_acc[j][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    const bool live_r[2] = {gid < g, gid + 8 < g};
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // of the two heads; the sum counts this lane's keys only
     constexpr bool Q_IN_REGS = D <= 128;
-    uint32_t qf[Q_IN_REGS ? D / 16 : 1][4];
+    uint32_t qf[Q_IN_REGS ? D / 32 : 1][4];
+    const __half* q_at = Qs + (lane & 7) * DP + (lane >> 3) * 8;
     if (Q_IN_REGS) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) ldmatrix_x4(qf[Q_IN_REGS ? kk : 0], Qs + (lane & 15) * DP + kk * 16 + (lane >> 4) * 8);
+        for (int kk = 0; kk < D / 32; ++kk) ldmatrix_x4(qf[Q_IN_REGS ? kk : 0], q_at + kk * 32);
     }
 
     for (int i = 0; i < my_tiles; ++i) {
@@ -214,175 +257,155 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
         const __half* kt = ring + (i % STAGES) * 2 * KT * DP;
         const __half* vt = kt + KT * DP;
 
-        float sc[2][4];
+        float sc[4], even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 2; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-            uint32_t af[4], bf[4];
-            if (!Q_IN_REGS) ldmatrix_x4(af, Qs + (lane & 15) * DP + kk * 16 + (lane >> 4) * 8);
-            ldmatrix_x4(bf, kt + ((lane & 7) + (lane >> 4) * 8) * DP + kk * 16 + ((lane >> 3) & 1) * 8);
-            mma16816(sc[0], Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0] : af, bf[0], bf[1]);
-            mma16816(sc[1], Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0] : af, bf[2], bf[3]);
+        for (int kk = 0; kk < D / 32; ++kk) {
+            uint32_t a0[4], a1[4], bf[4];
+            if (!Q_IN_REGS) ldmatrix_x4(bf, q_at + kk * 32);
+            ldmatrix_x4(a0, kt + (lane & 15) * DP + kk * 32 + (lane >> 4) * 8);
+            ldmatrix_x4(a1, kt + (lane & 15) * DP + kk * 32 + 16 + (lane >> 4) * 8);
+            mma16816(even, a0, Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0][0] : bf[0], Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0][1] : bf[1]);
+            mma16816(odd, a1, Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0][2] : bf[2], Q_IN_REGS ? qf[Q_IN_REGS ? kk : 0][3] : bf[3]);
         }
-        const int tile_pos = k_begin + (warp + 4 * i) * KT;
-        // a tile that lies wholly inside the share needs no masking (rows without a query head hold zeros and are
-        // never stored)
+        const int tile_pos = k_begin + (warp + WALKERS * i) * KT;
+        // a tile that lies wholly inside the share needs no masking (heads that do not exist hold zeros and are never stored)
         const bool full_tile = tile_pos >= k_lo && tile_pos + KT <= k_hi;
-        float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-            for (int e = 0; e < 2 * NH; ++e) {
-                int h = e >> 1;
-                int pos = tile_pos + j * 8 + 2 * tq + (e & 1);
-                float v = sc[j][e] * a.scale;
-                if (a.softcap != 0.f) v = capped(v, a.softcap, two_over_cap);
-                bool vis = full_tile || (live_r[h] && pos >= k_lo && pos < k_hi);  // k_lo / k_hi carry causality and the window
-                v = vis ? v : -INFINITY;
-                sc[j][e] = v;
-                tmax[h] = fmaxf(tmax[h], v);
-            }
+        for (int e = 0; e < 4; ++e) {
+            const int pos = tile_pos + gid + 8 * (e >> 1);
+            float v = (even[e] + odd[e]) * a.scale;
+            if (a.softcap != 0.f) v = capped(v, a.softcap, two_over_cap);
+            sc[e] = full_tile || (pos >= k_lo && pos < k_hi) ? v : -INFINITY;  // k_lo / k_hi carry causality and the window
         }
-        float alpha[2] = {1.f, 1.f}, m_use[2] = {0.f, 0.f};
+        float alpha[2], m_use[2];
 #pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
-            tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
-            float m_new = fmaxf(m_run[h], tmax[h]);
+        for (int h = 0; h < 2; ++h) {
+            float top = fmaxf(sc[h], sc[2 + h]);
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+            const float m_new = fmaxf(m_run[h], top);
             m_use[h] = m_new == -INFINITY ? 0.f : m_new;
             alpha[h] = m_run[h] == -INFINITY ? 0.f : __expf(m_run[h] - m_use[h]);
             m_run[h] = m_new;
         }
-        float psum[2] = {0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-            for (int e = 0; e < 2 * NH; ++e) {
-                int h = e >> 1;
-                float pe = sc[j][e] == -INFINITY ? 0.f : __expf(sc[j][e] - m_use[h]);
-                sc[j][e] = pe;
-                psum[h] += pe;
-            }
-            if (LOW8) sc[j][2] = sc[j][3] = 0.f;
-        }
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 1);
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 2);
-            l_run[h] = l_run[h] * alpha[h] + psum[h];
-        }
+        for (int e = 0; e < 4; ++e) sc[e] = sc[e] == -INFINITY ? 0.f : __expf(sc[e] - m_use[e & 1]);
+        l_run[0] = l_run[0] * alpha[0] + (sc[0] + sc[2]);
+        l_run[1] = l_run[1] * alpha[1] + (sc[1] + sc[3]);
 #pragma unroll
         for (int j = 0; j < NT_O; ++j) {
             o_acc[j][0] *= alpha[0];
-            o_acc[j][1] *= alpha[0];
-            if (!LOW8) {
-                o_acc[j][2] *= alpha[1];
-                o_acc[j][3] *= alpha[1];
-            }
+            o_acc[j][1] *= alpha[1];
+            o_acc[j][2] *= alpha[0];
+            o_acc[j][3] *= alpha[1];
         }
-        uint32_t pf[4] = {pack_half2(sc[0][0], sc[0][1]), LOW8 ? 0u : pack_half2(sc[0][2], sc[0][3]), pack_half2(sc[1][0], sc[1][1]),
-                          LOW8 ? 0u : pack_half2(sc[1][2], sc[1][3])};
-        uint32_t pr[4] = {0u, 0u, 0u, 0u};
-        if constexpr (EXACT)
+        const uint32_t p0 = pack_half2(sc[0], sc[1]), p1 = pack_half2(sc[2], sc[3]);
+        const uint32_t b0 = transpose_8x8(p0), b1 = transpose_8x8(p1);
+        uint32_t r0 = 0u, r1 = 0u;
+        if constexpr (EXACT) {
+            r0 = transpose_8x8(pack_half2_rest(sc[0], sc[1], p0));
+            r1 = transpose_8x8(pack_half2_rest(sc[2], sc[3], p1));
+        }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (!LOW8 || (i & 1) == 0) pr[i] = pack_half2_rest(sc[i >> 1][(i & 1) * 2], sc[i >> 1][(i & 1) * 2 + 1], pf[i]);
-#pragma unroll
-        for (int j = 0; j < NT_O; j += 2) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(bf, vt + ((lane & 7) + ((lane >> 3) & 1) * 8) * DP + j * 8 + (lane >> 4) * 8);
-            mma16816(o_acc[j], pf, bf[0], bf[1]);
-            mma16816(o_acc[j + 1], pf, bf[2], bf[3]);
-            if constexpr (EXACT) {
-                mma16816(o_acc[j], pr, bf[0], bf[1]);
-                mma16816(o_acc[j + 1], pr, bf[2], bf[3]);
-            }
+        for (int j = 0; j < NT_O; ++j) {
+            uint32_t af[4];
+            ldmatrix_x4_trans(af, vt + ((lane >> 4) * 8 + (lane & 7)) * DP + j * 16 + ((lane >> 3) & 1) * 8);
+            mma16816(o_acc[j], af, b0, b1);
+            if constexpr (EXACT) mma16816(o_acc[j], af, r0, r1);
         }
         __syncwarp();  // the stage is refilled by the next iteration's load
     }
     cp_async_wait<0>();
     __syncwarp();
 
-    // each warp leaves (max, sum, output) of its live rows in its own ring, then everyone merges
-    float* w_o = reinterpret_cast<float*>(ring);            // [16][D]
-    float* w_ml = w_o + 16 * D;                              // [16][2]
+    // each warp leaves (max, sum, output) of its live heads in its own ring, then everyone merges
+    float* w_o = reinterpret_cast<float*>(ring);            // [8][OP]
+    float* w_ml = w_o + 8 * OP;                              // [8][2]
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        int item = gid + 8 * h;
-        if (item >= g || warp >= 4) continue;
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 4);
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 8);
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 16);
+        const int item = 2 * tq + h;
+        if (item >= g || warp >= WALKERS) continue;
 #pragma unroll
-        for (int j = 0; j < NT_O; ++j)
-            *reinterpret_cast<float2*>(w_o + item * D + j * 8 + 2 * tq) = make_float2(o_acc[j][2 * h], o_acc[j][2 * h + 1]);
-        if (tq == 0) {
+        for (int j = 0; j < NT_O; ++j) {
+            w_o[item * OP + j * 16 + gid] = o_acc[j][h];
+            w_o[item * OP + j * 16 + gid + 8] = o_acc[j][2 + h];
+        }
+        if (gid == 0) {
             w_ml[item * 2] = m_run[h];
             w_ml[item * 2 + 1] = l_run[h];
         }
     }
     __syncthreads();
     const int64_t slot = ((int64_t)blockIdx.x * a.kv_heads + kvh) * 16;
-    // merged, normalised outputs of this (lane, KV head): g * D consecutive values of the lane's output row
-    // (all threads of the CTA call this together; the query tile is dead by now and lends its shared memory: g * D
-    // floats fit in it for up to eight query heads per KV head)
-    float* stage = reinterpret_cast<float*>(Qs);
-    auto finish = [&](auto&& value_of) {
+    // merged, normalised outputs of this (lane, KV head): g * D consecutive values of the lane's output row, eight per thread (one head's)
+    auto finish = [&](auto&& values_of) {
         const int64_t row = q_off;
         const int col0 = kvh * g * D;
-        const bool fuse_quant = a.qout.qs != nullptr;  // uniform
-        if (!fuse_quant) {
-            for (int idx = tid; idx < g * D; idx += THREADS) {
-                float v = value_of(idx);
-                if (a.out != nullptr) a.out[row * a.q_heads * D + col0 + idx] = v;
-                if (a.out_h != nullptr) a.out_h[row * a.q_heads * D + col0 + idx] = __float2half_rn(v);
-            }
-            return;
-        }
-        for (int idx = tid; idx < g * D; idx += THREADS) {
-            float v = value_of(idx);
-            stage[idx] = v;
-            if (a.out != nullptr) a.out[row * a.q_heads * D + col0 + idx] = v;
-        }
-        __syncthreads();
-        // one warp per 256-wide group, eight consecutive values per lane (g * D is a multiple of 256 here)
-        for (int grp = warp; grp < g * D / 256; grp += THREADS / 32) {
+        for (int i8 = tid; i8 < g * D / 8; i8 += THREADS) {
             float v[8];
+            values_of(i8 * 8, v);
+            if (a.out != nullptr) store8(a.out + row * a.q_heads * D + col0 + i8 * 8, v);
+            // one warp per 256-wide group (g * D is a multiple of 256 where the rows are quantised)
+            if (a.qout.qs != nullptr) quant_group(v, lane, a.qkind, a.qout, row, a.q_heads * D, col0 / 256 + (i8 >> 5));
+            else if (a.out_h != nullptr) {
+                __half2 h[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = stage[grp * 256 + lane * 8 + i];
-            quant_group(v, lane, a.qkind, a.qout, row, a.q_heads * D, col0 / 256 + grp);
+                for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+                *reinterpret_cast<uint4*>(a.out_h + row * a.q_heads * D + col0 + i8 * 8) = *reinterpret_cast<const uint4*>(h);
+            }
         }
     };
-    auto merged_local = [&](int idx, float& m_out, float& l_out) {
-        int item = idx / D, c = idx - item * D;
-        float m = -INFINITY;
+    // the walkers' sums of eight values of one head, as one walker's
+    auto merged_local = [&](int idx, float (&o)[8], float& m_out, float& l_out) {
+        const int item = idx / D, c = idx - item * D;
+        const float* first = reinterpret_cast<const float*>(rings);
+        constexpr int STEP = RING_HALVES / 2;   // floats between walkers
+        float mw[WALKERS], m = -INFINITY, l = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) m = fmaxf(m, reinterpret_cast<const float*>(rings + w * RING_HALVES)[16 * D + item * 2]);
-        float l = 0.f, o = 0.f;
+        for (int w = 0; w < WALKERS; ++w) {
+            mw[w] = first[w * STEP + 8 * OP + item * 2];
+            m = fmaxf(m, mw[w]);
+        }
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const float* ro = reinterpret_cast<const float*>(rings + w * RING_HALVES);
-            float mw = ro[16 * D + item * 2];
-            if (mw != -INFINITY) {
-                float f = __expf(mw - m);
-                l += ro[16 * D + item * 2 + 1] * f;
-                o += ro[item * D + c] * f;
-            }
+        for (int i = 0; i < 8; ++i) o[i] = 0.f;
+#pragma unroll
+        for (int w = 0; w < WALKERS; ++w) {
+            const float f = mw[w] == -INFINITY ? 0.f : __expf(mw[w] - m);   // a walker without keys left zeros
+            float x[8];
+            load8(first + w * STEP + item * OP + c, x);
+            l += first[w * STEP + 8 * OP + item * 2 + 1] * f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] += x[i] * f;
         }
         m_out = m;
         l_out = l;
-        return o;
+    };
+    auto normalise = [&](int idx, float (&o)[8], float m, float l) {
+        if (a.sink != nullptr) {
+            const float s = sink_scale(m, l, a.sink[kvh * g + idx / D]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] *= s;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = o[i] / l;
+        }
     };
     if (n_splits == 1) {
-        finish([&](int idx) {
+        finish([&](int idx, float (&o)[8]) {
             float m, l;
-            float o = merged_local(idx, m, l);
-            return a.sink != nullptr ? o * sink_scale(m, l, a.sink[kvh * g + idx / D]) : o / l;
+            merged_local(idx, o, m, l);
+            normalise(idx, o, m, l);
         });
     } else {
-        for (int idx = tid; idx < g * D; idx += THREADS) {
-            int item = idx / D, c = idx - item * D;
-            float m, l;
-            float o = merged_local(idx, m, l);
-            a.part_o[(slot + item) * D + c] = o;
+        for (int i8 = tid; i8 < g * D / 8; i8 += THREADS) {
+            const int idx = i8 * 8, item = idx / D, c = idx - item * D;
+            float o[8], m, l;
+            merged_local(idx, o, m, l);
+            store8(a.part_o + (slot + item) * D + c, o);
             if (c == 0) {
                 a.part_ml[(slot + item) * 2] = m;
                 a.part_ml[(slot + item) * 2 + 1] = l;
@@ -401,22 +424,23 @@ __global__ void __launch_bounds__(THREADS) attn_decode_kernel(AttnTcArgs a) {
         __syncthreads();
         if (s_last) {
             __threadfence();
-            finish([&](int idx) {
-                int item = idx / D, c = idx - item * D;
-                float m = -INFINITY;
-                for (int sp = 0; sp < n_splits; ++sp)
-                    m = fmaxf(m, __ldcg(a.part_ml + (((int64_t)(first_entry + sp) * a.kv_heads + kvh) * 16 + item) * 2));
-                float l = 0.f, o = 0.f;
+            finish([&](int idx, float (&o)[8]) {
+                const int item = idx / D, c = idx - item * D;
+                const int64_t first = ((int64_t)first_entry * a.kv_heads + kvh) * 16 + item, step = (int64_t)a.kv_heads * 16;
+                float m = -INFINITY, l = 0.f;
+                for (int sp = 0; sp < n_splits; ++sp) m = fmaxf(m, __ldcg(a.part_ml + (first + sp * step) * 2));
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = 0.f;
+#pragma unroll 4
                 for (int sp = 0; sp < n_splits; ++sp) {
-                    const int64_t ps = ((int64_t)(first_entry + sp) * a.kv_heads + kvh) * 16 + item;
-                    float ms = __ldcg(a.part_ml + ps * 2);
-                    if (ms != -INFINITY) {
-                        float f = __expf(ms - m);
-                        l += __ldcg(a.part_ml + ps * 2 + 1) * f;
-                        o += __ldcg(a.part_o + ps * D + c) * f;
-                    }
+                    const int64_t ps = first + sp * step;
+                    const float ms = __ldcg(a.part_ml + ps * 2), f = ms == -INFINITY ? 0.f : __expf(ms - m);
+                    const float4 x = __ldcg(reinterpret_cast<const float4*>(a.part_o + ps * D + c)), y = __ldcg(reinterpret_cast<const float4*>(a.part_o + ps * D + c + 4));
+                    l += __ldcg(a.part_ml + ps * 2 + 1) * f;
+                    o[0] += x.x * f; o[1] += x.y * f; o[2] += x.z * f; o[3] += x.w * f;
+                    o[4] += y.x * f; o[5] += y.y * f; o[6] += y.z * f; o[7] += y.w * f;
                 }
-                return a.sink != nullptr ? o * sink_scale(m, l, a.sink[kvh * g + item]) : o / l;
+                normalise(idx, o, m, l);
             });
         }
     }
@@ -455,13 +479,14 @@ template <int D, bool EXACT>
 void launch_for_dim(const AttnTcArgs& a, cudaStream_t s) {
     if (a.n_entries > 0) {
         constexpr int STAGES = D >= 256 ? 2 : 3;
-        constexpr size_t smem = (size_t)(16 + 4 * STAGES * 2 * 16) * (D + 8) * sizeof(__half);
+        constexpr int ALONE_WALKERS = D >= 256 ? 4 : 8;
+        auto smem = [](int walkers) { return (size_t)(16 + walkers * STAGES * 2 * 16) * (D + 8) * sizeof(__half); };
         dim3 grid((unsigned)a.n_entries, (unsigned)a.kv_heads);
-        const bool low8 = a.q_heads / a.kv_heads <= 8, alone = a.n_entries * a.kv_heads <= kPlanSms;
-        auto* kernel = alone ? (low8 ? attn_decode_kernel<D, STAGES, true, EXACT, 256> : attn_decode_kernel<D, STAGES, false, EXACT, 256>)
-                             : (low8 ? attn_decode_kernel<D, STAGES, true, EXACT, 128> : attn_decode_kernel<D, STAGES, false, EXACT, 128>);
-        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-        launch_pdl(kernel, grid, dim3(alone ? 256 : 128), smem, s, a);
+        const bool alone = a.n_entries * a.kv_heads <= kPlanSms;
+        auto* kernel = alone ? attn_decode_kernel<D, STAGES, EXACT, 256, ALONE_WALKERS> : attn_decode_kernel<D, STAGES, EXACT, 128, 4>;
+        const size_t bytes = smem(alone ? ALONE_WALKERS : 4);
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
+        launch_pdl(kernel, grid, dim3(alone ? 256 : 128), bytes, s, a);
         MK_LAUNCH_CHECK();
     }
     if (a.n_dec_lanes > 0) {  // lanes whose keys were shared out over several CTAs

@@ -36,31 +36,67 @@ __device__ __forceinline__ void rope_sum_shares(const float* src, int n_parts, i
     }
 }
 
-// One warp.  kind: 0 = q, 1 = k, 2 = v; hh = head index within its kind; t = packed token row; x = the warp's row
-// of shared memory, holding the finished head (zero-filled to the row width) on return (after a __syncwarp).
-__device__ __forceinline__ void rope_head_prepare(const RopeKvArgs& a, int kind, int hh, int t, int position, float* x, int lane) {
-    const int d = kind == 2 && a.dv > 0 ? a.dv : a.d;
-    const float* src = kind == 0 ? a.q + (int64_t)t * a.ldq + hh * d : (kind == 1 ? a.k + (int64_t)t * a.ldk + hh * d : a.v + (int64_t)t * a.ldv + hh * d);
-    const int n_parts = kind == 2 ? a.v_splits : a.qk_splits;
-    const int64_t part_stride = kind == 2 ? a.v_split_stride : a.qk_split_stride;
-    // the rotation's angles do not wait for the shares
-    const bool turns = kind != 2 && a.cos_t != nullptr;
-    const int half = a.rotary_dim / 2;
-    float rc[RK_MAX_D / 64], rs[RK_MAX_D / 64];
-    if (turns) {
-        const float* c = a.cos_t + (int64_t)position * half;
-        const float* s = a.sin_t + (int64_t)position * half;
+// The same for up to N heads of one warp that lie d floats each: their first loads, and those of every share, are on their way together.
+template <typename V, int N>
+__device__ __forceinline__ void rope_sum_heads(const float* const (&src)[N], const int (&n_parts)[N], const int64_t (&stride)[N], int n, int d, float* const (&x)[N], int lane) {
+    constexpr int W = sizeof(V) / 4;
+    int most = 1;
 #pragma unroll
-        for (int j = 0; j < RK_MAX_D / 64; ++j) {
-            const int i = lane + 32 * j;
-            rc[j] = i < half ? c[i] : 0.f;
-            rs[j] = i < half ? s[i] : 0.f;
+    for (int k = 0; k < N; ++k)
+        if (k < n) most = max(most, n_parts[k]);
+    for (int i = lane * W; i < d; i += 32 * W) {
+        V v[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (k < n) v[k] = *reinterpret_cast<const V*>(src[k] + i);
+        constexpr int AHEAD = 3;
+        for (int sp = 1; sp < most; sp += AHEAD) {
+            V w[AHEAD][N];
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j)
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    if (k < n && sp + j < n_parts[k]) w[j][k] = *reinterpret_cast<const V*>(src[k] + (int64_t)(sp + j) * stride[k] + i);
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j)
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    if (k < n && sp + j < n_parts[k]) rope_add(v[k], w[j][k]);
         }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (k < n) *reinterpret_cast<V*>(x[k] + i) = v[k];
     }
-    const uintptr_t place = reinterpret_cast<uintptr_t>(src) | (uintptr_t)(part_stride * 4);
-    if ((d & 127) == 0 && (place & 15) == 0) rope_sum_shares<float4>(src, n_parts, part_stride, d, x, lane);
-    else if ((d & 63) == 0 && (place & 7) == 0) rope_sum_shares<float2>(src, n_parts, part_stride, d, x, lane);
-    else rope_sum_shares<float>(src, n_parts, part_stride, d, x, lane);
+}
+
+// What a lane turns its share of a head by: constant tables, so they can be fetched ahead of everything.
+struct RopeAngles {
+    float c[RK_MAX_D / 64], s[RK_MAX_D / 64];
+};
+__device__ __forceinline__ RopeAngles rope_angles(const RopeKvArgs& a, int position, int lane) {
+    RopeAngles r;
+    const int half = a.rotary_dim / 2;
+    const float* c = a.cos_t + (int64_t)position * half;
+    const float* s = a.sin_t + (int64_t)position * half;
+#pragma unroll
+    for (int j = 0; j < RK_MAX_D / 64; ++j) {
+        const int i = lane + 32 * j;
+        r.c[j] = a.cos_t != nullptr && i < half ? c[i] : 0.f;
+        r.s[j] = a.cos_t != nullptr && i < half ? s[i] : 0.f;
+    }
+    return r;
+}
+
+// Where a head's f32 vector begins.  kind: 0 = q, 1 = k, 2 = v; hh = head index within its kind; t = packed token row.
+__device__ __forceinline__ int rope_head_width(const RopeKvArgs& a, int kind) { return kind == 2 && a.dv > 0 ? a.dv : a.d; }
+__device__ __forceinline__ const float* rope_head_source(const RopeKvArgs& a, int kind, int hh, int t) {
+    const int d = rope_head_width(a, kind);
+    return kind == 0 ? a.q + (int64_t)t * a.ldq + hh * d : (kind == 1 ? a.k + (int64_t)t * a.ldk + hh * d : a.v + (int64_t)t * a.ldv + hh * d);
+}
+
+// One warp: bias, norm and rotation of the sums in x (the warp's row of shared memory), zeros up to the row width; a __syncwarp at the end.
+__device__ __forceinline__ void rope_head_finish(const RopeKvArgs& a, int kind, int hh, const RopeAngles& angles, float* x, int lane) {
+    const int d = rope_head_width(a, kind), half = a.rotary_dim / 2;
     const float* bias = kind == 0 ? a.q_bias : (kind == 1 ? a.k_bias : a.v_bias);
     if (bias != nullptr) {
         __syncwarp();
@@ -78,7 +114,7 @@ __device__ __forceinline__ void rope_head_prepare(const RopeKvArgs& a, int kind,
         for (int i = lane; i < d; i += 32) x[i] = x[i] / m * nw[i];
         __syncwarp();
     }
-    if (turns) {
+    if (kind != 2 && a.cos_t != nullptr) {
         float r1[RK_MAX_D / 64], r2[RK_MAX_D / 64];
         const int step = a.interleaved ? 2 : 1, off = a.interleaved ? 1 : half;
 #pragma unroll
@@ -86,8 +122,8 @@ __device__ __forceinline__ void rope_head_prepare(const RopeKvArgs& a, int kind,
             const int i = lane + 32 * j;
             if (i >= half) break;
             const float x1 = x[i * step], x2 = x[i * step + off];
-            r1[j] = __fsub_rn(__fmul_rn(x1, rc[j]), __fmul_rn(x2, rs[j]));
-            r2[j] = __fadd_rn(__fmul_rn(x1, rs[j]), __fmul_rn(x2, rc[j]));
+            r1[j] = __fsub_rn(__fmul_rn(x1, angles.c[j]), __fmul_rn(x2, angles.s[j]));
+            r2[j] = __fadd_rn(__fmul_rn(x1, angles.s[j]), __fmul_rn(x2, angles.c[j]));
         }
         __syncwarp();
 #pragma unroll
@@ -99,6 +135,21 @@ __device__ __forceinline__ void rope_head_prepare(const RopeKvArgs& a, int kind,
         }
         __syncwarp();
     }
+}
+
+// One warp, one head: x holds the finished head (zero-filled to the row width) on return.
+__device__ __forceinline__ void rope_head_prepare(const RopeKvArgs& a, int kind, int hh, int t, int position, float* x, int lane) {
+    const int d = rope_head_width(a, kind);
+    const float* src = rope_head_source(a, kind, hh, t);
+    const int n_parts = kind == 2 ? a.v_splits : a.qk_splits;
+    const int64_t part_stride = kind == 2 ? a.v_split_stride : a.qk_split_stride;
+    RopeAngles angles = {};
+    if (kind != 2) angles = rope_angles(a, position, lane);   // the rotation's angles do not wait for the shares
+    const uintptr_t place = reinterpret_cast<uintptr_t>(src) | (uintptr_t)(part_stride * 4);
+    if ((d & 127) == 0 && (place & 15) == 0) rope_sum_shares<float4>(src, n_parts, part_stride, d, x, lane);
+    else if ((d & 63) == 0 && (place & 7) == 0) rope_sum_shares<float2>(src, n_parts, part_stride, d, x, lane);
+    else rope_sum_shares<float>(src, n_parts, part_stride, d, x, lane);
+    rope_head_finish(a, kind, hh, angles, x, lane);
 }
 
 }  // namespace mk
