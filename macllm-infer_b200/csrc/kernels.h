@@ -29,6 +29,7 @@ struct NormQuantArgs {
     const int32_t* row_index = nullptr;
     int act_kind = ACT_Q8K;
     ActQ out;
+    bool half_only = false;  // out.xh alone is read: the 8-bit blocks are made but need not be written
 };
 void launch_add_norm_quant(const NormQuantArgs& a, cudaStream_t s);
 

@@ -688,6 +688,7 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
         na.dim = H;
         na.act_kind = kind;
         na.out = xa;
+        na.half_only = !stream_T && w.qkv_half.ready && T >= hgemm_min_rows_ && xa.xh != nullptr;  // the stacked f16 image reads nothing else
         prof_begin(KC_NORM_QUANT, 9.0 * T * H, 0);
         launch_add_norm_quant(na, stream_);
         prof_end();
@@ -905,6 +906,9 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
         int fkind = act_kind_of(w.gate.w);
         const bool ep_dp = cfg_.ep_size > 1 && cfg_.ep_mode == 1 && ls.moe;  // the exchange moves f16 rows at every width
         ActQ xf = act_view(a_qs_, a_d_, a_bs_, a_xh_, T, H, fkind, f16_T || ep_dp);
+        // wide ticks: one GEMM over the interleaved gate/up image writes act(gate) * up as f16, which is all the
+        // f16 GEMM of the down projection reads; no f32 gate|up round trip and no separate activation kernel
+        const bool gated_gemm = !ls.moe && !stream_gu && w.gu_half.ready && w.down.half.ready && T >= hgemm_min_rows_ && xf.xh != nullptr && f16_T;
         NormQuantArgs nf;
         nf.h = h_.as<float>();
         nf.a = wo_splits > 1 ? tc_ws_.partial.as<float>() : proj_.as<float>();
@@ -918,6 +922,7 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
         nf.act_kind = fkind;
         nf.out = xf;
         nf.normed_out = ls.moe ? normed_.as<float>() : nullptr;
+        nf.half_only = !ls.moe && gated_gemm;
         prof_begin(KC_NORM_QUANT, 13.0 * T * H, 0);
         launch_add_norm_quant(nf, stream_);
         prof_end();
@@ -927,9 +932,6 @@ void Model::run_forward(const std::vector<LmLane>& lanes, KvReservation& r, uint
             float* gp = gu_.as<float>();
             float* up = gp + ms_.ffn;
             int gu_splits = 1;
-            // wide ticks: one GEMM over the interleaved gate/up image writes act(gate) * up as f16, which is all the
-            // f16 GEMM of the down projection reads; no f32 gate|up round trip and no separate activation kernel
-            const bool gated_gemm = !stream_gu && w.gu_half.ready && w.down.half.ready && T >= hgemm_min_rows_ && xf.xh != nullptr && f16_T;
             // narrow ticks, gated form: act(gate) * up leaves the streamed matmul as f16, which is what the streamed down
             // projection reads (the activation is the f16 rounding of the f32 value, not an 8-bit block image)
             const bool gated_stream = stream_gu && qstream_gated_ && stream_down;

@@ -14,19 +14,15 @@ namespace mk {
 
 __device__ __forceinline__ void quant8_q8k(const float (&v)[8], int lane, int8_t* qs, float* d, int16_t* bsums, __half* xh) {
     float amax = 0.f, mx = 0.f;
-    int idx = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         float ax = fabsf(v[i]);
-        if (ax > amax) { amax = ax; idx = lane * 8 + i; mx = v[i]; }
+        if (ax > amax) { amax = ax; mx = v[i]; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-        int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        float om = __shfl_xor_sync(0xffffffffu, mx, o);
-        if (oa > amax || (oa == amax && oi < idx)) { amax = oa; idx = oi; mx = om; }
-    }
+    // the largest magnitude of the block, and its first holder's value (lanes hold the values in order); magnitudes compare like their bits
+    const uint32_t mine = __float_as_uint(amax), top = __reduce_max_sync(0xffffffffu, mine);
+    mx = __shfl_sync(0xffffffffu, mx, __ffs((int)__ballot_sync(0xffffffffu, mine == top)) - 1);
+    amax = __uint_as_float(top);
     int8_t q[8];
     int sum = 0;
     float dd = 0.f;
@@ -43,16 +39,17 @@ __device__ __forceinline__ void quant8_q8k(const float (&v)[8], int lane, int8_t
         }
         dd = 1.0f / iscale;
     }
-    int2 packed;
-    packed.x = (uint8_t)q[0] | ((uint8_t)q[1] << 8) | ((uint8_t)q[2] << 16) | ((uint32_t)(uint8_t)q[3] << 24);
-    packed.y = (uint8_t)q[4] | ((uint8_t)q[5] << 8) | ((uint8_t)q[6] << 16) | ((uint32_t)(uint8_t)q[7] << 24);
-    *reinterpret_cast<int2*>(qs + lane * 8) = packed;
     if (xh != nullptr) {
         __half2 hv[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) hv[i] = __floats2half2_rn(__fmul_rn(dd, (float)q[2 * i]), __fmul_rn(dd, (float)q[2 * i + 1]));
         *reinterpret_cast<uint4*>(xh + lane * 8) = *reinterpret_cast<uint4*>(hv);
     }
+    if (qs == nullptr) return;   // nothing but the f16 image is wanted
+    int2 packed;
+    packed.x = (uint8_t)q[0] | ((uint8_t)q[1] << 8) | ((uint8_t)q[2] << 16) | ((uint32_t)(uint8_t)q[3] << 24);
+    packed.y = (uint8_t)q[4] | ((uint8_t)q[5] << 8) | ((uint8_t)q[6] << 16) | ((uint32_t)(uint8_t)q[7] << 24);
+    *reinterpret_cast<int2*>(qs + lane * 8) = packed;
     int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
     if ((lane & 1) == 0) bsums[lane >> 1] = (int16_t)pair;
     if (lane == 0) *d = dd;
@@ -70,23 +67,24 @@ __device__ __forceinline__ void quant8_q80(const float (&v)[8], int lane, int8_t
     int8_t q[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = (int8_t)roundf(v[i] * id);
-    int2 packed;
-    packed.x = (uint8_t)q[0] | ((uint8_t)q[1] << 8) | ((uint8_t)q[2] << 16) | ((uint32_t)(uint8_t)q[3] << 24);
-    packed.y = (uint8_t)q[4] | ((uint8_t)q[5] << 8) | ((uint8_t)q[6] << 16) | ((uint32_t)(uint8_t)q[7] << 24);
-    *reinterpret_cast<int2*>(qs + lane * 8) = packed;
     if (xh != nullptr) {
         __half2 hv[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) hv[i] = __floats2half2_rn(__fmul_rn(ddh, (float)q[2 * i]), __fmul_rn(ddh, (float)q[2 * i + 1]));
         *reinterpret_cast<uint4*>(xh + lane * 8) = *reinterpret_cast<uint4*>(hv);
     }
+    if (qs == nullptr) return;
+    int2 packed;
+    packed.x = (uint8_t)q[0] | ((uint8_t)q[1] << 8) | ((uint8_t)q[2] << 16) | ((uint32_t)(uint8_t)q[3] << 24);
+    packed.y = (uint8_t)q[4] | ((uint8_t)q[5] << 8) | ((uint8_t)q[6] << 16) | ((uint32_t)(uint8_t)q[7] << 24);
+    *reinterpret_cast<int2*>(qs + lane * 8) = packed;
     if ((lane & 3) == 0) d[lane >> 2] = ddh;
 }
 
-// Quantise group `grp` (256 values, eight per lane) of output row r.
-__device__ __forceinline__ void quant_group(const float (&v)[8], int lane, int kind, const ActQ& out, int64_t r, int dim, int grp) {
+// Quantise group `grp` (256 values, eight per lane) of output row r.  half_only: the blocks themselves are not written, only their f16 image.
+__device__ __forceinline__ void quant_group(const float (&v)[8], int lane, int kind, const ActQ& out, int64_t r, int dim, int grp, bool half_only = false) {
     if (out.qs == nullptr) return;
-    int8_t* qs = out.qs + r * dim + grp * 256;
+    int8_t* qs = half_only ? nullptr : out.qs + r * dim + grp * 256;
     __half* xh = out.xh ? out.xh + r * dim + grp * 256 : nullptr;
     if (kind == ACT_Q8K) {
         quant8_q8k(v, lane, qs, out.d + r * (dim / 256) + grp, out.bsums + r * (dim / 16) + grp * 16, xh);
