@@ -196,23 +196,26 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
     auto stage_x = [&] {
         const int chunks = (s1 - s0) * (COLS / 8);   // 16-byte chunks per token
         const __half* x = p.x + (int64_t)input * p.T * p.cols + s0 * COLS;
-        for (int c = threadIdx.x; c < chunks; c += NM_THREADS) {
-            int at = c;
-            if constexpr (BLOCKS) {
+        if constexpr (!BLOCKS) {
+            // all on their way at once, behind the weights that are
+            for (int c = threadIdx.x; c < chunks; c += NM_THREADS)
+                for (int tok = 0; tok < p.T; ++tok) nm_copy16(nm_smem(xs + tok * pitch + c * 16), reinterpret_cast<const uint4*>(x + (int64_t)tok * p.cols) + c);
+            nm_commit();
+            nm_wait<0>();
+        } else {
+            for (int c = threadIdx.x; c < chunks; c += NM_THREADS) {
                 // bits of a chunk's number inside its block: half, 64-wide run, low / high nibbles (the last two the other way round in Q6_K), half of
                 // 32, eight columns; a lane's chunk t is (run, half of 32)
                 const int half = (c >> 4) & 1, b3 = (c >> 3) & 1, b2 = (c >> 2) & 1, sub = c & 1;
                 const int run = p.q6 ? b2 : b3, high = p.q6 ? b3 : b2;
-                at = (c & ~31) + ((half * 2 + high) * 2 + sub) * 4 + ((run << 1) | ((c >> 1) & 1));
-            }
+                const int at = (c & ~31) + ((half * 2 + high) * 2 + sub) * 4 + ((run << 1) | ((c >> 1) & 1));
 #pragma unroll 4
-            for (int tok = 0; tok < p.T; ++tok) {
-                uint4 v = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)tok * p.cols) + c);
-                if constexpr (BLOCKS) {
+                for (int tok = 0; tok < p.T; ++tok) {   // no more at a time: the instructions are fetched anew by every launch
                     // columns (0, 2), (1, 3) of every four, as the nibbles of a word come apart
-                    v = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
+                    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)tok * p.cols) + c);
+                    *reinterpret_cast<uint4*>(xs + tok * pitch + at * 16) =
+                        make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
                 }
-                *reinterpret_cast<uint4*>(xs + tok * pitch + at * 16) = v;
             }
         }
     };
