@@ -672,7 +672,8 @@ __global__ void __launch_bounds__(256) gated_act_kernel(Shares gu, int ff, RowIm
 // ------------------------------------------------------------------------------------------------ embedding with positions
 
 // Shared memory: the row.
-__global__ void __launch_bounds__(RU_THREADS) embed_norm_kernel(EmbedNormArgs a) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) embed_norm_kernel(EmbedNormArgs a) {
     extern __shared__ __align__(16) float en_row[];
     __shared__ float red[32];
     pdl_trigger();
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(RU_THREADS) embed_norm_kernel(EmbedNormArgs a)
     const int64_t row = blockIdx.x, at = (int64_t)a.ids[row] * a.width;
     const double pos = (double)a.positions[row];
     constexpr double kTwoPi = 6.283185307179586476925;
-    for (int i = threadIdx.x; 2 * i < a.width; i += RU_THREADS) {
+    for (int i = threadIdx.x; 2 * i < a.width; i += THREADS) {
         double angle = pos * a.freq[i];
         angle -= rint(angle / kTwoPi) * kTwoPi;
         float sn, cs;
@@ -692,8 +693,8 @@ __global__ void __launch_bounds__(RU_THREADS) embed_norm_kernel(EmbedNormArgs a)
         }
     }
     __syncthreads();
-    const RowStats st = row_stats<1>(en_row, a.width, a.eps, red);
-    for (int c = threadIdx.x; c < a.width; c += RU_THREADS) {
+    const RowStats st = row_stats<1, THREADS>(en_row, a.width, a.eps, red);
+    for (int c = threadIdx.x; c < a.width; c += THREADS) {
         const float v = (en_row[c] - st.mean) / st.root * a.norm_w[c];
         a.x[row * a.width + c] = v;
         if (a.image.any()) a.image.put(row, c, v);
@@ -703,9 +704,10 @@ __global__ void __launch_bounds__(RU_THREADS) embed_norm_kernel(EmbedNormArgs a)
 
 // ------------------------------------------------------------------------------------------------ latents, polynomial activation
 
-constexpr int LP_THREADS = 256;
+constexpr int LP_THREADS = 256, LP_FEW_THREADS = 1024;
 
 // Three block sums behind one barrier.
+template <int THREADS>
 __device__ __forceinline__ float3 block_sum3(float3 v, float (*red)[3]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     v.x = warp_sum(v.x);
@@ -719,7 +721,7 @@ __device__ __forceinline__ float3 block_sum3(float3 v, float (*red)[3]) {
     __syncthreads();
     float3 r = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < LP_THREADS / 32; ++i) {
+    for (int i = 0; i < THREADS / 32; ++i) {
         r.x += red[i][0];
         r.y += red[i][1];
         r.z += red[i][2];
@@ -727,9 +729,9 @@ __device__ __forceinline__ float3 block_sum3(float3 v, float (*red)[3]) {
     return r;
 }
 
-template <int VEC>
+template <int VEC, int THREADS>
 __device__ __forceinline__ void poly_row(const LatentPrepArgs& a, int64_t row, float* z, float (*red)[3]) {
-    const int step = LP_THREADS * VEC;
+    const int step = THREADS * VEC;
     float3 ss = make_float3(0.f, 0.f, 0.f);
     for (int c = threadIdx.x * VEC; c < a.ff; c += step) {
         Pack<VEC> v = share_pack<VEC>(a.y, row, a.ff_col + c);
@@ -744,7 +746,7 @@ __device__ __forceinline__ void poly_row(const LatentPrepArgs& a, int64_t row, f
         }
         store_pack<VEC>(z + c, v);
     }
-    ss = block_sum3(ss, red);
+    ss = block_sum3<THREADS>(ss, red);
     const float n = (float)a.ff;
     const float k1 = a.poly[0] / sqrtf(ss.x / n + a.eps), k2 = a.poly[1] / sqrtf(ss.y / n + a.eps), k3 = a.poly[2] / sqrtf(ss.z / n + a.eps), k0 = a.poly[3];
     for (int c = threadIdx.x * VEC; c < a.ff; c += step) {
@@ -756,16 +758,17 @@ __device__ __forceinline__ void poly_row(const LatentPrepArgs& a, int64_t row, f
     zero_tail(a.ff_image, row, a.ff);
 }
 
-// Shared memory: max(ff, q_rank + kv_rank + rot_width) floats.
-template <int VEC>
-__global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(LatentPrepArgs a) {
+// Shared memory: max(ff, q_rank + kv_rank + rot_width) floats.  THREADS: a narrow tick's rows leave SMs idle, and a row of 8192 values is eight loads
+// after one another for 256 threads (16 rows: 8.3 us a launch) or two for 1024 (LP_FEW_THREADS).
+template <int VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS) latent_prep_kernel(LatentPrepArgs a) {
     extern __shared__ __align__(16) float lp_row[];
-    __shared__ float red[LP_THREADS / 32][3];
+    __shared__ float red[THREADS / 32][3];
     pdl_trigger();
     pdl_wait();
     const int64_t row = blockIdx.x;
     if (a.q_rank == 0 || blockIdx.y == 1) {
-        poly_row<VEC>(a, row, lp_row, red);
+        poly_row<VEC, THREADS>(a, row, lp_row, red);
         return;
     }
     float *kv = lp_row + a.q_rank, *rot = kv + a.kv_rank;
@@ -775,13 +778,13 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(LatentPrepArgs 
     auto stage = [&](float* dst, int n, int col) {
         float s = 0.f;
         if (a.lat_vec) {
-            for (int c = threadIdx.x * 4; c < n; c += LP_THREADS * 4) {
+            for (int c = threadIdx.x * 4; c < n; c += THREADS * 4) {
                 const float4 v = a.y.at4(row, col + c);
                 *reinterpret_cast<float4*>(dst + c) = v;
                 s = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, s))));
             }
         } else {
-            for (int c = threadIdx.x; c < n; c += LP_THREADS) {
+            for (int c = threadIdx.x; c < n; c += THREADS) {
                 const float v = a.y.at(row, col + c);
                 dst[c] = v;
                 s = fmaf(v, v, s);
@@ -791,16 +794,16 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(LatentPrepArgs 
     };
     ss.x = stage(lp_row, a.q_rank, a.q_col);
     ss.y = stage(kv, a.kv_rank, a.kv_col);
-    for (int c = threadIdx.x; c < a.rot_width; c += LP_THREADS) rot[c] = a.y.at(row, a.rot_col + c);
-    ss = block_sum3(ss, red);
+    for (int c = threadIdx.x; c < a.rot_width; c += THREADS) rot[c] = a.y.at(row, a.rot_col + c);
+    ss = block_sum3<THREADS>(ss, red);
     const float rq = sqrtf(ss.x / (float)a.q_rank + a.eps), rk = sqrtf(ss.y / (float)a.kv_rank + a.eps);
     if (a.lat_vec) {
-        for (int c = threadIdx.x * 4; c < a.q_rank; c += LP_THREADS * 4) {
+        for (int c = threadIdx.x * 4; c < a.q_rank; c += THREADS * 4) {
             const float4 v = *reinterpret_cast<const float4*>(lp_row + c), w = *reinterpret_cast<const float4*>(a.q_norm + c);
             a.q_image.put4(row, c, make_float4(v.x / rq * w.x, v.y / rq * w.y, v.z / rq * w.z, v.w / rq * w.w));
         }
     } else {
-        for (int c = threadIdx.x; c < a.q_rank; c += LP_THREADS) a.q_image.put(row, c, lp_row[c] / rq * a.q_norm[c]);
+        for (int c = threadIdx.x; c < a.q_rank; c += THREADS) a.q_image.put(row, c, lp_row[c] / rq * a.q_norm[c]);
     }
     zero_tail(a.q_image, row, a.q_rank);
     auto value = [&](int c) {  // column c of the page row
@@ -811,7 +814,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(LatentPrepArgs 
         const float cs = a.cos_t[turn0 + (i >> 1)], sn = a.sin_t[turn0 + (i >> 1)];
         return (i & 1) == 0 ? rot[i] * cs - rot[i ^ 1] * sn : rot[i] * cs + rot[i ^ 1] * sn;
     };
-    for (int c = threadIdx.x * 2; c < a.kv_width; c += LP_THREADS * 2) {  // a row is a multiple of 64 wide
+    for (int c = threadIdx.x * 2; c < a.kv_width; c += THREADS * 2) {  // a row is a multiple of 64 wide
         const float x = value(c), y = value(c + 1);
         if (a.pool_f16) *reinterpret_cast<__half2*>(static_cast<__half*>(a.pool) + at + c) = __floats2half2_rn(x, y);
         else *reinterpret_cast<float2*>(static_cast<float*>(a.pool) + at + c) = make_float2(x, y);
@@ -1028,8 +1031,10 @@ void launch_embed_norm(const EmbedNormArgs& a, cudaStream_t s) {
     if (a.rows <= 0) return;
     const size_t smem = (size_t)a.width * 4;
     if (smem > (size_t)200 * 1024) throw std::runtime_error("launch_embed_norm: the model is too wide");
-    ensure_dynamic_smem(reinterpret_cast<const void*>(&embed_norm_kernel), smem);
-    launch_pdl(embed_norm_kernel, dim3((unsigned)a.rows), dim3(RU_THREADS), smem, s, a);
+    const bool few = a.rows <= device_sm_count();   // an angle in 64 bits per pair of columns: as many threads as there are (16 rows of 2048: 10 us with 256)
+    auto* kernel = few ? embed_norm_kernel<4 * RU_THREADS> : embed_norm_kernel<RU_THREADS>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    launch_pdl(kernel, dim3((unsigned)a.rows), dim3(few ? 4 * RU_THREADS : RU_THREADS), smem, s, a);
     MK_LAUNCH_CHECK();
 }
 
@@ -1047,9 +1052,10 @@ void launch_latent_prep(const LatentPrepArgs& in, cudaStream_t s) {
     if (smem > (size_t)220 * 1024) throw std::runtime_error("launch_latent_prep: the feed-forward or the latents are too wide");
     const bool vec = a.ff % 4 == 0 && a.ff_col % 4 == 0 && a.y.ld % 4 == 0 && a.y.stride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.y.p) & 15) == 0;
     const dim3 grid((unsigned)a.rows, a.q_rank > 0 && a.ff > 0 ? 2u : 1u);
-    auto* kernel = vec ? latent_prep_kernel<4> : latent_prep_kernel<1>;
+    const bool few = (int64_t)grid.x * grid.y <= device_sm_count();
+    auto* kernel = few ? (vec ? latent_prep_kernel<4, LP_FEW_THREADS> : latent_prep_kernel<1, LP_FEW_THREADS>) : (vec ? latent_prep_kernel<4, LP_THREADS> : latent_prep_kernel<1, LP_THREADS>);
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    launch_pdl(kernel, grid, dim3(LP_THREADS), smem, s, a);
+    launch_pdl(kernel, grid, dim3(few ? LP_FEW_THREADS : LP_THREADS), smem, s, a);
     MK_LAUNCH_CHECK();
 }
 
