@@ -41,10 +41,17 @@ __device__ __forceinline__ void ls_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void ls_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// `n` rows of `width` floats, row i from src(i), into dst rows `pitch` floats apart; `vec`: everything is 16-byte aligned.
-template <typename Src>
+// `n` rows of `width` floats, row i from src(i), into dst rows `pitch` floats apart; `vec`: everything is 16-byte aligned.  USUAL: the width
+// there mostly is, for which a thread's place in the rows takes no division (a quarter of a scan's instructions otherwise).
+template <int USUAL, typename Src>
 __device__ __forceinline__ void fetch_rows(float* dst, int pitch, int n, int width, bool vec, Src src) {
-    if (vec) {
+    if (vec && width == USUAL) {
+        constexpr int PER = USUAL / 4;
+        for (int i = threadIdx.x; i < n * PER; i += blockDim.x) {
+            const int r = i / PER, c = i % PER * 4;
+            ls_cp_async16(dst + r * pitch + c, src(r) + c);
+        }
+    } else if (vec) {
         const int per = width >> 2;
         for (int i = threadIdx.x; i < n * per; i += blockDim.x) {
             const int r = i / per, c = (i - r * per) * 4;
@@ -191,9 +198,9 @@ linear_state_kernel(const __grid_constant__ typename LsArgs<RULE>::type ra) {
         auto fetch_heads = [&](const Shares& y, int x_col, int k_col, int v_col) {
             if (y.n == 1) {
                 const bool yv = vec && (y.ld & 3) == 0;
-                fetch_rows(s, KD, m, a.dim, yv, [&](int r) { return y.p + (r0 + r) * y.ld + x_col; });
-                fetch_rows(s + TT * KD, KD, m, a.dim, yv, [&](int r) { return y.p + (r0 + r) * y.ld + k_col; });
-                fetch_rows(s_v, cols, m, my_cols, yv && (my_cols & 3) == 0, [&](int r) { return y.p + (r0 + r) * y.ld + v_col; });
+                fetch_rows<KD>(s, KD, m, a.dim, yv, [&](int r) { return y.p + (r0 + r) * y.ld + x_col; });
+                fetch_rows<KD>(s + TT * KD, KD, m, a.dim, yv, [&](int r) { return y.p + (r0 + r) * y.ld + k_col; });
+                fetch_rows<L::COLS * LS_WIDE_WARPS>(s_v, cols, m, my_cols, yv && (my_cols & 3) == 0, [&](int r) { return y.p + (r0 + r) * y.ld + v_col; });
             } else {
                 sum_rows(s, KD, m, a.dim, y, r0, x_col);
                 sum_rows(s + TT * KD, KD, m, a.dim, y, r0, k_col);
@@ -203,12 +210,12 @@ linear_state_kernel(const __grid_constant__ typename LsArgs<RULE>::type ra) {
         if constexpr (RULE == LS_WKV) {
             const int h0 = head * a.dim;
             fetch_heads(ra.rkv, ra.r_col + h0, ra.k_col + h0, ra.v_col + h0 + col0);
-            fetch_rows(s + 2 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.decay + (r0 + r) * a.heads * a.dim + h0; });
+            fetch_rows<KD>(s + 2 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.decay + (r0 + r) * a.heads * a.dim + h0; });
         } else if constexpr (CHANNEL) {
             const int h0 = head * a.dim;
             fetch_heads(ra.y, ra.r_col + h0, ra.k_col + h0, ra.v_col + head * a.vdim + col0);
-            fetch_rows(s + 2 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.decay + (r0 + r) * a.heads * a.dim + h0; });
-            fetch_rows(s + 3 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.removal + (r0 + r) * a.heads * a.dim + h0; });
+            fetch_rows<KD>(s + 2 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.decay + (r0 + r) * a.heads * a.dim + h0; });
+            fetch_rows<KD>(s + 3 * TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.removal + (r0 + r) * a.heads * a.dim + h0; });
         } else if constexpr (RULE == LS_MLSTM) {
             const int h0 = head * a.dim;
             fetch_heads(ra.y, ra.q_col + h0, ra.k_col + h0, ra.v_col + head * a.vdim + col0);
@@ -241,9 +248,9 @@ linear_state_kernel(const __grid_constant__ typename LsArgs<RULE>::type ra) {
         } else {
             const int kv_head = head / (a.heads / ra.kv_heads);
             const int64_t kw = (int64_t)ra.kv_heads * a.dim, vw = (int64_t)a.heads * a.vdim;
-            fetch_rows(s, KD, m, a.dim, vec, [&](int r) { return ra.q + (r0 + r) * kw + kv_head * a.dim; });
-            fetch_rows(s + TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.k + (r0 + r) * kw + kv_head * a.dim; });
-            fetch_rows(s_v, cols, m, my_cols, vec && (my_cols & 3) == 0, [&](int r) { return ra.v + (r0 + r) * vw + head * a.vdim + col0; });
+            fetch_rows<KD>(s, KD, m, a.dim, vec, [&](int r) { return ra.q + (r0 + r) * kw + kv_head * a.dim; });
+            fetch_rows<KD>(s + TT * KD, KD, m, a.dim, vec, [&](int r) { return ra.k + (r0 + r) * kw + kv_head * a.dim; });
+            fetch_rows<L::COLS * LS_WIDE_WARPS>(s_v, cols, m, my_cols, vec && (my_cols & 3) == 0, [&](int r) { return ra.v + (r0 + r) * vw + head * a.vdim + col0; });
             for (int r = threadIdx.x; r < m; r += blockDim.x) {
                 ls_cp_async4(s_c + 4 * r, ra.decay + (r0 + r) * a.heads + head);
                 ls_cp_async4(s_c + 4 * r + 1, ra.beta + (r0 + r) * a.heads + head);
