@@ -14,6 +14,7 @@
 // per call when T <= NT; larger T re-walks the row from cache in passes.  Where there are warps for every
 // scheduler all the same, a warp takes R output rows that follow one another: their weights travel together, and an activation that was
 // fetched meets all of them (with one row per warp and eight sums whatever T, 32000 x 2048 in Q6_K took 26 us at one activation row, this 15).
+// Two to eight activation rows of a tall Q6_K matrix go to tensor cores instead (q6k_rows.cu).
 #include "kernels.h"
 #include "mma_bf16.cuh"
 #include <algorithm>
@@ -580,6 +581,9 @@ static void launch_qgemv_impl(const QWeight& W, const ActQ& x, int T, float* y, 
 void launch_qgemv(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap,
                   cudaStream_t s) {
     if (T <= 0 || W.rows <= 0) return;
+    // a tile of sixteen rows for every SM: 2368 x 2048 10.2 us against 10.2 at two activation rows, 10.1 / 12.3 at four, 10.2 / 16.4 at
+    // eight; 8192 x 2048 12.6 / 16.4, 12.5 / 20.7, 14.2 / 30.7; 32000 x 2048 21.4 / 30.7, 21.1 / 38.7, 22.5 / 69.7 (caches flushed)
+    if (W.rows >= (int64_t)16 * device_sm_count() && q6k_rows_cover(W, x, T)) return launch_q6k_rows(W, x, T, y, ldy, out_scale, softcap, s);
     launch_qgemv_impl(W, x, T, y, ldy, out_scale, softcap, 1, Group{}, s);
 }
 
