@@ -222,7 +222,6 @@ struct QsParams {
     float* partial;
     int32_t* status;
     long long* prof;              // optional [5][8]: cycles per role of CTA 0 (measuring aid)
-    int dbg;                      // with prof only: 1 skip the conversion arithmetic, 2 skip the TMEM stores, 4 skip the MMAs
 };
 
 template <int BN>
@@ -456,12 +455,10 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
                 const uint32_t d_acc = tmem_base + (uint32_t)slot * BN;
                 const uint32_t a_addr = tmem_base + QS_A_COL0 + buf * 128;
                 if (elect_one()) {
-                    if (!(PROF && (p.dbg & 4))) {
 #pragma unroll
-                        for (int k = 0; k < 16; ++k)
-                            umma_f16_ts(d_acc, a_addr + 8 * k, b_stage + (uint64_t)(((k >> 2) * BN * 128) >> 4) + (uint64_t)(2 * (k & 3)), idesc,
-                                        (first && k == 0) ? 0u : 1u);
-                    }
+                    for (int k = 0; k < 16; ++k)
+                        umma_f16_ts(d_acc, a_addr + 8 * k, b_stage + (uint64_t)(((k >> 2) * BN * 128) >> 4) + (uint64_t)(2 * (k & 3)), idesc,
+                                    (first && k == 0) ? 0u : 1u);
                     umma_commit(&a_empty[buf]);
                     if (last) umma_commit(&acc_full[slot]);
                 }
@@ -512,12 +509,7 @@ qstream_tc_kernel(const __grid_constant__ CUtensorMap tm_x, QsParams p) {
                     const uint32_t t_dst = tmem_base + ((uint32_t)(quad * 32) << 16) + QS_A_COL0 + buf * 128 + 64 * h;
                     const bool q6 = ((!GROUPED && tile >= p.tiles_a) ? p.fmt_b : p.fmt_a) != 0;
                     uint32_t w[16];
-                    if (PROF && (p.dbg & 1)) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) w[i] = n + i;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) tmem_st16(t_dst + 16 * q, w);
-                    } else if (!q6) {
+                    if (!q6) {
                         const uint8_t* blk = raw + row * 144;
                         uint32_t q0[8], q1[8], w2[16];
                         const Q4Half half(*reinterpret_cast<const uint4*>(blk), h);
@@ -909,7 +901,6 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
     p.partial = partial;
     p.status = status;
     p.prof = g_qs_prof;
-    { const char* e = getenv("MACLLM_B200_QS_DBG"); p.dbg = (g_qs_prof != nullptr && e != nullptr) ? atoi(e) : 0; }
     if (pl.bn == 16) launch_qs<16>(tx, p, pl.ctas, s);
     else if (pl.bn == 32) launch_qs<32>(tx, p, pl.ctas, s);
     else launch_qs<64>(tx, p, pl.ctas, s);
