@@ -17,6 +17,7 @@
 #include "narrow_mma.h"
 #include "kernels.h"
 #include "kquant_half.cuh"
+#include "narrow_ring.h"
 #include <cuda_bf16.h>
 
 namespace mk {
@@ -121,7 +122,9 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
     const int i0 = (int)((int64_t)cta * p.groups / p.per_share_ctas), i1 = (int)((int64_t)(cta + 1) * p.groups / p.per_share_ctas);
     const int s0 = (int)((int64_t)share * p.n_steps / p.shares), s1 = (int)((int64_t)(share + 1) * p.n_steps / p.shares);
     const int a0 = s0 + kw * (s1 - s0) / KW, a1 = s0 + (kw + 1) * (s1 - s0) / KW;   // this warp's steps
-    int to_load = (i1 - i0) * (a1 - a0);
+    // a row group may reach past the matrix: an image's last row is copied again, a block format's 128-row tile is filled up with zeros that stay where they are
+    const int live_groups = BLOCKS ? narrow_live_groups(i0, i1, rg_shift, sub_tile, (p.rows + 15) / 16) : i1 - i0;
+    NarrowRing copies(n_stages, live_groups * (a1 - a0));
     pdl_trigger();
 
     if constexpr (BLOCKS) {
@@ -132,22 +135,20 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
         __syncwarp();
     }
 
-    // ---- the warp's copies, in the order in which it uses them: step load_st of row group load_i into ring stage load_stage
-    int load_i = i0, load_st = a0, load_stage = 0;
+    // ---- the warp's copies, in the order in which it uses them: step load_st of row group load_i
+    int load_i = i0, load_st = a0;
     const uint8_t *src0 = nullptr, *src1 = nullptr;   // image: this lane's 16 bytes of rows r and r + 8
     auto copy_step = [&] {
-        if (to_load == 0) return;
-        --to_load;
-        const uint32_t dst = nm_smem(ring + load_stage * stage_bytes);
+        if (!copies.more()) return;
+        const uint32_t dst = nm_smem(ring + copies.load_stage * stage_bytes);
         if constexpr (BLOCKS) {
-            const int tile = (load_i << rg_shift) + sub_tile;
-            // a row group may reach past the matrix, whose last 128-row tile is filled up with zeros
-            if (lane == 0 && tile * 16 < p.rows) {
+            if (lane == 0) {
+                const int tile = (load_i << rg_shift) + sub_tile;
                 const bool second = tile >= p.tiles_first;
                 const int rt = second ? tile - p.tiles_first : tile, r0 = (rt & 7) * 16;
                 const bool q6 = (second ? p.q6_2 : p.q6) != 0;
                 const uint8_t* unit = (second ? p.w2 : p.w) + ((int64_t)(rt >> 3) * p.n_steps + load_st) * (q6 ? kQ6Unit : kQ4Unit);
-                const uint32_t bar = nm_smem(&full[warp][load_stage]);
+                const uint32_t bar = nm_smem(&full[warp][copies.load_stage]);
                 nm_expect(bar, q6 ? NM_Q6_STEP : NM_Q4_STEP);
                 if (!q6) {
                     nm_bulk(dst, unit + r0 * 144, NM_Q4_STEP, bar);
@@ -176,7 +177,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
             load_st = a0;
             ++load_i;
         }
-        load_stage = load_stage + 1 == n_stages ? 0 : load_stage + 1;
+        copies.loaded();
     };
     for (int i = 0; i < n_stages - 1; ++i) {
         copy_step();
@@ -223,8 +224,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
 #pragma unroll
     for (int j = 0; j < NT; ++j) x_tok[j] = xs + min(8 * j + g, p.T - 1) * pitch;
 
-    int stage = 0, buffer = 0;
-    uint32_t phase = 0;
+    int buffer = 0;
     bool ok = true;
     for (int i = i0; i < i1; ++i) {
         if (const int next = p.n_inputs > 1 ? input_of(i) : 0; next != input) {
@@ -245,7 +245,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
         int x_off = (a0 - s0) * COLS * 2;
         for (int st = a0; st < a1; ++st, x_off += COLS * 2) {
             copy_step();
-            const uint8_t* src = ring + stage * stage_bytes;
+            const uint8_t* src = ring + copies.stage * stage_bytes;
             if constexpr (!BLOCKS) {
                 nm_commit();
                 nm_wait<NM_IMAGE_STAGES - 1>();   // each lane reads what it copied itself
@@ -263,9 +263,13 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
                     nm_mma<BF16>(acc[3 % CHAINS][j], v01.z, v11.z, v01.w, v11.w, b.z, b.w);
                 }
             } else if (live) {
-                if (ok && !nm_wait_full(nm_smem(&full[warp][stage]), phase)) {
+                if (ok && !nm_wait_full(nm_smem(&full[warp][copies.stage]), copies.phase)) {
                     ok = false;
-                    atomicExch(p.status, 31);
+                    atomicExch(p.status, 34);
+                    // what this lane has under way lands before the CTA is gone (lane 0 asks for all of it)
+                    copies.give_up((i0 + live_groups - i) * (a1 - a0) - (st - a0), [&](int at, uint32_t parity) {
+                        if (lane == 0) nm_wait_full(nm_smem(&full[warp][at]), parity);
+                    });
                 }
                 // where the lanes' chunks lie for this matrix's format: 16 bytes apart in its own order, else in two runs
                 const bool own = q6 == (p.q6 != 0);
@@ -337,12 +341,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
                 }
                 __syncwarp();   // the stage is refilled next
             }
-            if (stage + 1 == n_stages) {
-                stage = 0;
-                phase ^= 1;
-            } else {
-                ++stage;
-            }
+            copies.used();
         }
 
         // ---- the warps' slices of K meet
@@ -408,10 +407,6 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
             }
         }
     }
-    if constexpr (BLOCKS)
-        if (!ok) {  // a wait gave up: what is under way lands before the CTA is gone
-            for (int i = 0; i < n_stages; ++i) nm_wait_full(nm_smem(&full[warp][i]), phase);
-        }
 }
 
 size_t nm_smem_bytes(NarrowFormat format, bool q6, int T, int64_t share_cols) {
