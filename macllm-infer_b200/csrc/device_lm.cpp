@@ -195,6 +195,8 @@ void DeviceLm::finish_tick(const Tick& t, int prof_class) {
     // results travel to pinned host memory on the same stream; the barrier is in fetch_output
     uint8_t* oh = out_host_.as<uint8_t>();
     const size_t tok_off = (size_t)((t.flags & FWD_WANT_LOGITS) ? t.R : 0) * spec_.vocab * 4;
+    // the status word, the descriptor's error word and the tokens in one copy, ahead of the logits: they are there with the first part of these
+    MK_CUDA(cudaMemcpyAsync(oh + tok_off, status_.ptr(), 8 + ((t.flags & FWD_WANT_TOKENS) ? (size_t)B * 4 : 0), cudaMemcpyDeviceToHost, stream_));
     // many rows in parts, so that the host copies one on while the next is on its way
     out_parts_ = tok_off >= ((size_t)2 << 20) ? kOutParts : 1;
     for (int i = 0; tok_off != 0 && i < out_parts_; ++i) {
@@ -202,8 +204,6 @@ void DeviceLm::finish_tick(const Tick& t, int prof_class) {
         MK_CUDA(cudaMemcpyAsync(oh + a, logits_.as<uint8_t>() + a, b - a, cudaMemcpyDeviceToHost, stream_));
         if (i + 1 < out_parts_) MK_CUDA(cudaEventRecord(ev_part_[i], stream_));
     }
-    // the status word, the descriptor's error word and the tokens in one copy
-    MK_CUDA(cudaMemcpyAsync(oh + tok_off, status_.ptr(), 8 + ((t.flags & FWD_WANT_TOKENS) ? (size_t)B * 4 : 0), cudaMemcpyDeviceToHost, stream_));
     d2h_bytes_ += 8 + (int64_t)tok_off + ((t.flags & FWD_WANT_TOKENS) ? (int64_t)B * 4 : 0);
     MK_CUDA(cudaEventRecord(ev_stop_, stream_));
     timed_ = true;
@@ -224,16 +224,18 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     // Two threads per part: with eight, whose cores go to sleep between ticks with the lines in their caches, the next transfer into the buffer took up to
     // 1000 us for 8 MB where it takes 160 (64 lanes, the last of eight ticks wants logits: 1950 us with its read-back before, 1200 so).
     size_t copied = 0;
+    int32_t flags[2];
     if (logits != nullptr && tok_off != 0)
         for (int i = 0; i + 1 < out_parts_; ++i) {
             MK_CUDA(cudaEventSynchronize(ev_part_[i]));
+            memcpy(flags, oh + tok_off, 8);
+            if ((flags[0] | flags[1]) != 0) break;   // a failed forward leaves the caller's buffer as it is
             copied = out_part(tok_off, i + 1);
             const size_t a = out_part(tok_off, i);
             copy_wide(reinterpret_cast<uint8_t*>(logits) + a, oh + a, copied - a, 2);
         }
     MK_CUDA(cudaStreamSynchronize(stream_));
     if (profiling_) prof_resolve();
-    int32_t flags[2];
     memcpy(flags, oh + tok_off, 8);
     if (flags[1] != 0) throw std::runtime_error("batch descriptor index out of range on the device (flag " + std::to_string(flags[1]) + ")");
     if (flags[0] != 0) {
