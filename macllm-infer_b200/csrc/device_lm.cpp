@@ -221,8 +221,9 @@ std::string DeviceLm::status_message(int32_t status) const {
 void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     const uint8_t* oh = out_host_.as<uint8_t>();
     const size_t tok_off = (size_t)((out_flags_ & FWD_WANT_LOGITS) ? out_rows_ : 0) * spec_.vocab * 4;
-    // Two threads per part: with eight, whose cores go to sleep between ticks with the lines in their caches, the next transfer into the buffer took up to
-    // 1000 us for 8 MB where it takes 160 (64 lanes, the last of eight ticks wants logits: 1950 us with its read-back before, 1200 so).
+    // Eight threads per part: a fresh destination is page faults above all, and two threads fall behind the transfer.  A forward of a two-layer model with its
+    // logits, us in one part with eight threads / four parts with two / four parts with eight: 37 rows of 32000 389 / 444 / 373, 64 rows 507 / 606 / 459, 128 rows
+    // 824 / 1116 / 684, 64 rows of 128000 1268 / 1845 / 1049, 64 rows of 256000 3098 / 6764 / 3009; after 20 ms of sleep the parts win as well.
     size_t copied = 0;
     int32_t flags[2];
     if (logits != nullptr && tok_off != 0)
@@ -232,7 +233,7 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
             if ((flags[0] | flags[1]) != 0) break;   // a failed forward leaves the caller's buffer as it is
             copied = out_part(tok_off, i + 1);
             const size_t a = out_part(tok_off, i);
-            copy_wide(reinterpret_cast<uint8_t*>(logits) + a, oh + a, copied - a, 2);
+            copy_wide(reinterpret_cast<uint8_t*>(logits) + a, oh + a, copied - a);
         }
     MK_CUDA(cudaStreamSynchronize(stream_));
     if (profiling_) prof_resolve();
@@ -245,7 +246,7 @@ void DeviceLm::fetch_output(float* logits, uint32_t* tokens) {
     }
     if (logits) {
         if (!(out_flags_ & FWD_WANT_LOGITS)) throw std::runtime_error("logits were not requested for this forward");
-        copy_wide(reinterpret_cast<uint8_t*>(logits) + copied, oh + copied, tok_off - copied, 2);
+        copy_wide(reinterpret_cast<uint8_t*>(logits) + copied, oh + copied, tok_off - copied);
     }
     if (tokens) {
         if (!(out_flags_ & FWD_WANT_TOKENS)) throw std::runtime_error("tokens were not requested for this forward");

@@ -45,14 +45,14 @@ private:
 };
 
 // memcpy on several host threads where one would spend milliseconds, most of them in first touches of the destination.
-inline void copy_wide(void* dst, const void* src, size_t bytes, int threads = 8) {
+inline void copy_wide(void* dst, const void* src, size_t bytes) {
     constexpr size_t kPiece = (size_t)128 << 10;
     const int pieces = (int)((bytes + kPiece - 1) / kPiece);
     if (pieces < 4) {
         if (bytes) memcpy(dst, src, bytes);
         return;
     }
-#pragma omp parallel for schedule(static) num_threads(std::min(threads, pieces))
+#pragma omp parallel for schedule(static) num_threads(std::min(8, pieces))
     for (int i = 0; i < pieces; ++i)
         memcpy(static_cast<char*>(dst) + (size_t)i * kPiece, static_cast<const char*>(src) + (size_t)i * kPiece, std::min(kPiece, bytes - (size_t)i * kPiece));
 }

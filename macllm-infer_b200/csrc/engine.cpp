@@ -312,7 +312,8 @@ static inline uint64_t next_u64(uint64_t& state) {
 static inline float next_uniform(uint64_t& state) { return (float)(next_u64(state) >> 40) * (1.0f / 16777216.0f); }
 
 namespace {
-// Appends a row of logits to each result, which has room for it.
+// Appends a row of logits to each result, which has room for it: mostly first touches, so several threads from 64 K values on (twelve ticks of 64 recorded
+// rows of 32000: 24.7 ms with two threads, 16.3 with four, 10.9 with eight; of four rows 2.5 ms on one thread, 2.0 with four).
 void record_rows(const std::vector<std::pair<EngineResult*, const float*>>& rows, int vocab) {
     const int n = (int)rows.size();
 #pragma omp parallel for schedule(static) num_threads(std::min(8, n)) if ((size_t)n * (size_t)vocab >= (size_t)1 << 16)
