@@ -44,12 +44,12 @@ void launch_actmul_quant(const float* gate, const float* up, int ld, int T, int 
 // against 8-bit activation blocks (CUDA-core path, any T; best for T <= 8).
 void launch_qgemv(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap,
                   cudaStream_t s);
-// Expert-grouped form: W holds `experts` matrices of W.rows x W.cols back to back; output rows
-// [offsets[e], offsets[e+1]) are computed with expert e's matrix.  Output row p reads activation row
-// src_row[p] (identity when src_row is null).
 // Two to eight activation rows of a Q6_K matrix of many rows, on tensor cores (launch_qgemv picks it).
 bool q6k_rows_cover(const QWeight& W, const ActQ& x, int T);
 void launch_q6k_rows(const QWeight& W, const ActQ& x, int T, float* y, int ldy, float out_scale, float softcap, cudaStream_t s);
+// Expert-grouped form: W holds `experts` matrices of W.rows x W.cols back to back; output rows
+// [offsets[e], offsets[e+1]) are computed with expert e's matrix.  Output row p reads activation row
+// src_row[p] (identity when src_row is null).
 void launch_qgemv_grouped(const QWeight& W, int experts, const int32_t* offsets, const int32_t* src_row, const ActQ& x,
                           float* y, int ldy, cudaStream_t s);
 // F32 weight matrix (MoE router): y[t][n] = sum_k x[t][k] W[n][k], f32 activations.

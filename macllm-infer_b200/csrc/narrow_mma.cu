@@ -1,9 +1,9 @@
-// Matmul of the narrowest ticks, y[t][n] = sum_k x[t][k] W[n][k] for up to 32 rows: a few lanes decoding.
+// Matmul of the narrowest ticks, y[t][n] = sum_k x[t][k] W[n][k] for up to 16 rows (8 of Q4_K / Q6_K weights): a few lanes decoding.
 //
 // At this width a matmul is bound by what stands around its weight stream: the tcgen05 kernels hand every tile from a loader to (converters to) an
 // issuer to an epilogue, and a 2048 x 2048 matrix at one row spends more on those hand-overs than on its 2 - 8 MB.  Here nothing is handed over.  A
 // warp copies its own weights into a ring, turns them into A fragments of mma.sync.m16n8k16 in registers and adds up; warps meet once per row tile, to
-// add their K slices.  The tensor rate of mma.sync does not count: 16 rows x 16 columns of weights take 1 to 4 instructions, against some 20 to
+// add their K slices.  The tensor rate of mma.sync does not count: 16 rows x 16 columns of weights take one or two instructions, against some 20 to
 // unpack Q4_K.
 //
 // K is permuted so that every operand is read in runs of 16 bytes: lane (g, t) of a warp supplies rows g and g + 8 of A and row g (token) of B, and
@@ -410,7 +410,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
 }
 
 size_t nm_smem_bytes(NarrowFormat format, bool q6, int T, int64_t share_cols) {
-    const int nt = T <= 8 ? 1 : (T <= 16 ? 2 : 4);
+    const int nt = T <= 8 ? 1 : 2;
     const int ring = format != NarrowFormat::Blocks ? NM_IMAGE_STAGES * NM_IMAGE_STEP : (q6 ? NM_Q6_STAGES * NM_Q6_STEP : NM_Q4_STAGES * NM_Q4_STEP);
     return (size_t)NM_WARPS * ring + 2 * (size_t)NM_WARPS * 8 * nt * NM_RED_PITCH * 4 +
            (size_t)T * (share_cols * 2 + 64);
@@ -418,7 +418,9 @@ size_t nm_smem_bytes(NarrowFormat format, bool q6, int T, int64_t share_cols) {
 
 template <NarrowFormat FORMAT>
 void launch_nm(const NmParams& p, const NarrowPlan& plan, cudaStream_t s) {
-    auto* kernel = p.T <= 8 ? narrow_mma_kernel<FORMAT, 1> : (p.T <= 16 ? narrow_mma_kernel<FORMAT, 2> : narrow_mma_kernel<FORMAT, 4>);
+    auto* kernel = narrow_mma_kernel<FORMAT, 1>;
+    if constexpr (FORMAT != NarrowFormat::Blocks)
+        if (p.T > 8) kernel = narrow_mma_kernel<FORMAT, 2>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), plan.smem);
     launch_pdl(kernel, dim3(plan.ctas), dim3(NM_THREADS), plan.smem, s, p);
     MK_LAUNCH_CHECK();
@@ -432,19 +434,18 @@ void launch_nm(const NmParams& p, const NarrowPlan& plan, cudaStream_t s) {
 // 22016 x 2048 20.5 / 22.2 gated, 20.5 / 18.5 otherwise, 75776 x 2048 38 / 34.5; 16 tokens of 22016 x 2048 gated 26.6 / 22.2.  In a tick it counts besides that
 // these CTAs are small enough to start under the kernel before: q|k|v of one lane 8.0 -> 3.8 us after its norm, and the norm that adds no shares 4 -> 2.9.
 bool narrow_preferred(NarrowFormat format, int64_t rows, int64_t cols, int T, bool gated) {
-    if (format != NarrowFormat::Blocks) return T <= 16;
-    return T <= 8 && (gated || rows * cols <= (int64_t)32 << 20);
+    if (format != NarrowFormat::Blocks) return T <= kNarrowImageRows;
+    return T <= kNarrowBlockRows && (gated || rows * cols <= (int64_t)32 << 20);
 }
 
 NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, int max_shares, size_t scratch_floats, int n_inputs, int sms) {
     NarrowPlan best;
     const bool blocks = format == NarrowFormat::Blocks;
-    if (T <= 0 || T > kNarrowMaxRows || cols % nm_step_cols(blocks) != 0) return best;
+    if (T <= 0 || T > (blocks ? kNarrowBlockRows : kNarrowImageRows) || cols % nm_step_cols(blocks) != 0) return best;
     const int64_t steps = cols / nm_step_cols(blocks), tiles = (rows + 15) / 16;
-    const int nt = T <= 8 ? 1 : (T <= 16 ? 2 : 4);
     // Microseconds of a step on one CTA of an SM (half as long again with two), of a meeting of the warps, of staging the activations and of adding
     // shares: fitted to launches of 2048 ... 75776 rows at K = 2048 and 11008, 1 to 16 tokens.
-    const double step_us = blocks ? (q6 ? 0.55 : 0.42) + 0.05 * (nt - 1) : 0.38 + 0.03 * (nt - 1);
+    const double step_us = blocks ? (q6 ? 0.55 : 0.42) : (T <= 8 ? 0.38 : 0.41);
     for (int shift = 0; shift <= 3; ++shift) {
         const int RG = 1 << shift, KW = NM_WARPS >> shift;
         const int64_t groups = (tiles + RG - 1) / RG;

@@ -6,7 +6,7 @@
 
 namespace mk {
 
-constexpr int kNarrowMaxRows = 32;      // activation rows of a call
+constexpr int kNarrowImageRows = 16, kNarrowBlockRows = 8;   // most activation rows of a call: on a 16-bit image, on Q4_K / Q6_K units
 
 // RG row tiles of 16 are a CTA's work at a time, 8 / RG of its warps share the K of each; `shares` CTAs share K besides and leave partial sums.
 struct NarrowPlan {
