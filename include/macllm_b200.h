@@ -707,12 +707,17 @@ int32_t mk_k_grouped_qmatmul(int32_t type, const void* w, const void* up_w, int3
  * tiles, K shares, K blocks (of 64) per share, floats of partial sums, 1 when two CTAs share a tile of 256 rows, 0}, for a matrix of one
  * input and scratch for any number of shares (mk_k_half_matmul_plan: otherwise); path MK_PATH_STREAM (T <= 64): out =
  * {token-tile width, row tiles, (group of row tiles, 256-column block) items, persistent CTAs, partial-sum slots, floats
- * of partial sums, row tiles per group, groups}.  Needs no GPU.  Calls of so few rows that warps stream
- * their own weights (csrc/narrow_mma.h: up to 16 on MK_PATH_HALF, up to 8 on MK_PATH_STREAM) are cut otherwise, into at most as many shares. */
+ * of partial sums, row tiles per group, groups}.  Needs no GPU.  This is the cut of the kernels that add up in tensor memory; which calls of a few rows
+ * another kernel takes, and how it cuts them, mk_k_narrow_matmul_plan says. */
 int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t* out8);
 /* Host-only: the same for MK_PATH_HALF with scratch_floats floats for partial sums (negative: any number); may_pair 0: stacked projections whose
  * borders lie inside pairs of row tiles, so that every tile stays on one CTA. */
 int32_t mk_k_half_matmul_plan(int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t scratch_floats, int32_t may_pair, int64_t* out8);
+/* Host-only: the cut of calls of so few rows that warps stream their own weights.  path MK_PATH_HALF (16-bit images; type is not read) or MK_PATH_STREAM
+ * (Q4_K / Q6_K); gated: rows interleaved gate / up, finished in the launch (no shares); scratch_floats: room for partial sums (negative: any).  out = {1 when the
+ * call is taken, else 0 and nothing else holds, 16-row tiles that a CTA takes at a time, K shares, CTAs, bytes of shared memory of a CTA, floats of partial sums}. */
+int32_t mk_k_narrow_matmul_plan(int32_t path, int32_t type, int64_t rows, int64_t cols, int32_t T, int32_t gated, int32_t max_splits, int64_t scratch_floats,
+                                int64_t* out6);
 
 /* Host-only: how mk_k_grouped_qmatmul cuts a call on MK_PATH_STREAM.  rows_per_expert: rows of an expert's matrix (gate and up together when
  * gated), a multiple of 128; rows_total: routed rows; max_rows_per_expert: the most any expert is expected to have.  out = {rows of a chunk, row

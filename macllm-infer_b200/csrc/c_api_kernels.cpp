@@ -5,6 +5,7 @@
 #include "device_util.h"
 #include "kernels.h"
 #include "hgemm_tc.h"
+#include "narrow_mma.h"
 #include "qstream_tc.h"
 #include "host_sampler.h"
 #include "attention_tc.h"
@@ -172,7 +173,10 @@ void qmatmul_case(int32_t type, const void* w, int64_t rows, int64_t cols, const
         *avg_ms = (float)(total / iters);
     }
     MK_CUDA(cudaDeviceSynchronize());
-    if (stream && getenv("MACLLM_B200_QS_PROF") != nullptr) {
+    const bool narrow = stream && narrow_plan(NarrowFormat::Blocks, type == MK_TYPE_Q6_K, rows, cols, T, false, stream_splits, qs_partial.size() / 4, 1, device_sm_count()).ok;
+    if (narrow && getenv("MACLLM_B200_QS_PROF") != nullptr) {
+        fprintf(stderr, "[qstream prof] %d rows: taken by the kernel whose warps stream their own weights, which has no such roles\n", T);
+    } else if (stream && getenv("MACLLM_B200_QS_PROF") != nullptr) {
         // one more launch with CTA 0 recording where each of its roles waited (printed to stderr)
         DevBuf prof((41 + 2000) * sizeof(long long));
         prof.zero(nullptr);
@@ -1002,6 +1006,20 @@ int32_t mk_k_half_matmul_plan(int64_t rows, int64_t cols, int32_t T, int32_t max
         const HgemmPlan p = hgemm_tc_plan(rows, cols, T, max_splits, scratch_floats < 0 ? SIZE_MAX : (size_t)scratch_floats, may_pair != 0);
         const int64_t v[8] = {p.bn, p.row_tiles, p.n_tiles, p.splits, p.kb_per_split, (int64_t)p.partial_floats, p.pairs ? 1 : 0, 0};
         memcpy(out8, v, sizeof v);
+    });
+}
+
+int32_t mk_k_narrow_matmul_plan(int32_t path, int32_t type, int64_t rows, int64_t cols, int32_t T, int32_t gated, int32_t max_splits, int64_t scratch_floats,
+                                int64_t* out6) {
+    return guarded([&] {
+        if (rows <= 0 || cols <= 0 || T <= 0 || out6 == nullptr) throw std::runtime_error("mk_k_narrow_matmul_plan: arguments out of range");
+        if (path != MK_PATH_HALF && path != MK_PATH_STREAM) throw std::runtime_error("mk_k_narrow_matmul_plan: only the f16-image and the streamed path are planned on the host");
+        const bool blocks = path == MK_PATH_STREAM;
+        if (blocks && type != MK_TYPE_Q4_K && type != MK_TYPE_Q6_K) throw std::runtime_error("mk_k_narrow_matmul_plan: the streamed matmul covers Q4_K and Q6_K matrices");
+        const NarrowPlan p = narrow_plan(blocks ? NarrowFormat::Blocks : NarrowFormat::F16, blocks && type == MK_TYPE_Q6_K, rows, cols, T, gated != 0, max_splits,
+                                         scratch_floats < 0 ? SIZE_MAX : (size_t)scratch_floats, 1, kPlanSms);
+        const int64_t v[6] = {p.ok ? 1 : 0, p.RG, p.shares, p.ctas, (int64_t)p.smem, (int64_t)p.partial_floats};
+        memcpy(out6, v, sizeof v);
     });
 }
 

@@ -1057,33 +1057,30 @@ int launch_hgemm_any(const HalfWeight& W, const __half* xh, int T, float* y, int
     if (xh == nullptr) throw std::runtime_error("launch_hgemm_tc: f16 activations missing");
     if (out_scale != 1.0f || softcap != 0.f || ws.partial == nullptr) max_splits = 1;
     const NarrowFormat format = W.bf16 ? NarrowFormat::BF16 : NarrowFormat::F16;
-    if (narrow_preferred(format, W.rows, W.cols, T, act != nullptr)) {
-        const NarrowPlan np = narrow_plan(format, false, W.rows, W.cols, T, act != nullptr || scatter != nullptr ? 1 : max_splits,
-                                          ws.partial != nullptr ? ws.partial_floats : 0, W.n_groups, device_sm_count());
-        if (np.ok) {
-            NarrowCall c;
-            c.format = format;
-            c.w = W.values.ptr();
-            c.rows = W.rows;
-            c.cols = W.cols;
-            c.n_inputs = W.n_groups;
-            for (int g = 0; g < kMaxRowGroups; ++g) c.input_end[g] = W.group_end[g];
-            c.input_tiles = W.group_tiles;
-            c.x = xh;
-            c.T = T;
-            c.y = y;
-            c.ldy = ldy;
-            c.out_scale = out_scale;
-            c.softcap = softcap;
-            c.partial = ws.partial;
-            c.status = ws.status;
-            c.act = act;
-            c.yh = yh;
-            c.ldyh = ldyh;
-            c.scatter = scatter;
-            launch_narrow_mma(c, np, s);
-            return np.shares;
-        }
+    if (const NarrowPlan np = narrow_plan(format, false, W.rows, W.cols, T, act != nullptr, scatter != nullptr ? 1 : max_splits,
+                                          ws.partial != nullptr ? ws.partial_floats : 0, W.n_groups, device_sm_count()); np.ok) {
+        NarrowCall c;
+        c.format = format;
+        c.w = W.values.ptr();
+        c.rows = W.rows;
+        c.cols = W.cols;
+        c.n_inputs = W.n_groups;
+        for (int g = 0; g < kMaxRowGroups; ++g) c.input_end[g] = W.group_end[g];
+        c.input_tiles = W.group_tiles;
+        c.x = xh;
+        c.T = T;
+        c.y = y;
+        c.ldy = ldy;
+        c.out_scale = out_scale;
+        c.softcap = softcap;
+        c.partial = ws.partial;
+        c.status = ws.status;
+        c.act = act;
+        c.yh = yh;
+        c.ldyh = ldyh;
+        c.scatter = scatter;
+        launch_narrow_mma(c, np, s);
+        return np.shares;
     }
     const HgemmPlan pl = hgemm_tc_plan(W.rows, W.cols, T, max_splits, ws.partial != nullptr ? ws.partial_floats : 0, whole_pairs(W));
     alignas(64) CUtensorMap tx;

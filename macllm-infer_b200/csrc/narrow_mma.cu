@@ -433,15 +433,16 @@ void launch_nm(const NmParams& p, const NarrowPlan& plan, cudaStream_t s) {
 // streams, while a gated matrix leaves SMs idle there (its row tiles are not cut): 2048 x 2048 8.8 / 10.3, 3072 x 2048 10.2 / 12.3, 2048 x 11008 14.9 / 14.4,
 // 22016 x 2048 20.5 / 22.2 gated, 20.5 / 18.5 otherwise, 75776 x 2048 38 / 34.5; 16 tokens of 22016 x 2048 gated 26.6 / 22.2.  In a tick it counts besides that
 // these CTAs are small enough to start under the kernel before: q|k|v of one lane 8.0 -> 3.8 us after its norm, and the norm that adds no shares 4 -> 2.9.
-bool narrow_preferred(NarrowFormat format, int64_t rows, int64_t cols, int T, bool gated) {
+static bool narrow_preferred(NarrowFormat format, int64_t rows, int64_t cols, int T, bool gated) {
     if (format != NarrowFormat::Blocks) return T <= kNarrowImageRows;
     return T <= kNarrowBlockRows && (gated || rows * cols <= (int64_t)32 << 20);
 }
 
-NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, int max_shares, size_t scratch_floats, int n_inputs, int sms) {
+NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, bool gated, int max_shares, size_t scratch_floats, int n_inputs, int sms) {
     NarrowPlan best;
     const bool blocks = format == NarrowFormat::Blocks;
-    if (T <= 0 || T > (blocks ? kNarrowBlockRows : kNarrowImageRows) || cols % nm_step_cols(blocks) != 0) return best;
+    if (T <= 0 || cols % nm_step_cols(blocks) != 0 || !narrow_preferred(format, rows, cols, T, gated)) return best;
+    if (gated) max_shares = 1;   // its pairs of rows are finished by the CTA that has their sums
     const int64_t steps = cols / nm_step_cols(blocks), tiles = (rows + 15) / 16;
     // Microseconds of a step on one CTA of an SM (half as long again with two), of a meeting of the warps, of staging the activations and of adding
     // shares: fitted to launches of 2048 ... 75776 rows at K = 2048 and 11008, 1 to 16 tokens.

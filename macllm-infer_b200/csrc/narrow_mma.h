@@ -16,9 +16,9 @@ struct NarrowPlan {
     bool ok = false;                    // there is a plan within the scratch and the shared memory
 };
 enum class NarrowFormat : int { F16 = 0, BF16 = 1, Blocks = 2 };  // Blocks: Q4_K / Q6_K units
-// Whether a call is better off here than on the tcgen05 kernels.
-bool narrow_preferred(NarrowFormat format, int64_t rows, int64_t cols, int T, bool gated);
-NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, int max_shares, size_t scratch_floats, int n_inputs, int sms);
+// The cut of a call that is better off here than on the tcgen05 kernels; not ok: it is theirs.  Launches and the host's query go by it alike.  q6: a
+// matrix of the call is in Q6_K.
+NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, bool gated, int max_shares, size_t scratch_floats, int n_inputs, int sms);
 
 struct NarrowCall {
     NarrowFormat format = NarrowFormat::F16;

@@ -843,32 +843,29 @@ int launch_qstream_tc(const QStreamWeight& W, const __half* xh, int T, float* y,
     const int64_t rows = W.rows + (W2 ? W2->rows : 0);
     const int row_tiles = W.row_tiles + (W2 ? W2->row_tiles : 0);
     const int sms = device_sm_count();
-    if (narrow_preferred(NarrowFormat::Blocks, rows, W.cols, T, gated)) {
-        const bool any_q6 = W.fmt != 0 || (W2 != nullptr && W2->fmt != 0);
-        const NarrowPlan np = narrow_plan(NarrowFormat::Blocks, any_q6, rows, W.cols, T, gated ? 1 : max_splits, partial_floats, 1, sms);
-        if (np.ok) {
-            NarrowCall c;
-            c.format = NarrowFormat::Blocks;
-            c.w = W.tiled.ptr();
-            c.w2 = W2 != nullptr ? W2->tiled.ptr() : nullptr;
-            c.rows = rows;
-            c.rows_first = W.rows;
-            c.cols = W.cols;
-            c.q6 = W.fmt != 0;
-            c.q6_2 = W2 != nullptr && W2->fmt != 0;
-            c.x = xh;
-            c.T = T;
-            c.y = y;
-            c.ldy = ldy;
-            c.partial = partial;
-            c.status = status;
-            const GatedAct act{gated_act == 0 ? GatedAct::Silu : GatedAct::GeluTanh};
-            if (gated) c.act = &act;
-            c.yh = yh;
-            c.ldyh = ldyh;
-            launch_narrow_mma(c, np, s);
-            return np.shares;
-        }
+    const bool any_q6 = W.fmt != 0 || (W2 != nullptr && W2->fmt != 0);
+    if (const NarrowPlan np = narrow_plan(NarrowFormat::Blocks, any_q6, rows, W.cols, T, gated, max_splits, partial_floats, 1, sms); np.ok) {
+        NarrowCall c;
+        c.format = NarrowFormat::Blocks;
+        c.w = W.tiled.ptr();
+        c.w2 = W2 != nullptr ? W2->tiled.ptr() : nullptr;
+        c.rows = rows;
+        c.rows_first = W.rows;
+        c.cols = W.cols;
+        c.q6 = W.fmt != 0;
+        c.q6_2 = W2 != nullptr && W2->fmt != 0;
+        c.x = xh;
+        c.T = T;
+        c.y = y;
+        c.ldy = ldy;
+        c.partial = partial;
+        c.status = status;
+        const GatedAct act{gated_act == 0 ? GatedAct::Silu : GatedAct::GeluTanh};
+        if (gated) c.act = &act;
+        c.yh = yh;
+        c.ldyh = ldyh;
+        launch_narrow_mma(c, np, s);
+        return np.shares;
     }
     QStreamPlan pl = qstream_plan(row_tiles, nb, rows, T, gated ? 1 : max_splits, gated, sms);
     if (pl.slots > 1 && pl.partial_floats > partial_floats) pl = qstream_plan(row_tiles, nb, rows, T, 1, true, sms);

@@ -286,6 +286,13 @@ def half_matmul_plan(rows: int, cols: int, T: int, max_splits: int = 16, scratch
     return dict(zip(_HALF_PLAN, map(int, out)))
 
 
+def narrow_matmul_plan(path: int, qtype: int, rows: int, cols: int, T: int, gated: bool = False, max_splits: int = 16, scratch_floats: int = -1) -> dict | None:
+    """Host-only: the cut of a call of so few rows that warps stream their own weights; None: matmul_plan's holds."""
+    out = np.zeros(6, dtype=np.int64)
+    capi.check(capi.lib().mk_k_narrow_matmul_plan(path, qtype, rows, cols, T, 1 if gated else 0, max_splits, scratch_floats, _p(out)))
+    return dict(zip(("tiles", "shares", "ctas", "smem", "partial_floats"), map(int, out[1:]))) if out[0] else None
+
+
 def grouped_matmul_plan(experts: int, rows_per_expert: int, rows_total: int, max_rows_per_expert: int) -> dict:
     """Host-only: how the expert-grouped streamed matmul cuts a call."""
     out = np.zeros(4, dtype=np.int64)
