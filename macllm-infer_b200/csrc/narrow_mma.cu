@@ -225,7 +225,7 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
     for (int j = 0; j < NT; ++j) x_tok[j] = xs + min(8 * j + g, p.T - 1) * pitch;
 
     int buffer = 0;
-    bool ok = true;
+    uint32_t given_up = 0;
     for (int i = i0; i < i1; ++i) {
         if (const int next = p.n_inputs > 1 ? input_of(i) : 0; next != input) {
             input = next;   // the old input's readers met at the sums of the group before
@@ -263,13 +263,9 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
                     nm_mma<BF16>(acc[3 % CHAINS][j], v01.z, v11.z, v01.w, v11.w, b.z, b.w);
                 }
             } else if (live) {
-                if (ok && !nm_wait_full(nm_smem(&full[warp][copies.stage]), copies.phase)) {
-                    ok = false;
+                if (given_up == 0 && !nm_wait_full(nm_smem(&full[warp][copies.stage]), copies.phase)) {
+                    given_up = copies.give_up((i0 + live_groups - i) * (a1 - a0) - (st - a0));
                     atomicExch(p.status, 34);
-                    // what this lane has under way lands before the CTA is gone (lane 0 asks for all of it)
-                    copies.give_up((i0 + live_groups - i) * (a1 - a0) - (st - a0), [&](int at, uint32_t parity) {
-                        if (lane == 0) nm_wait_full(nm_smem(&full[warp][at]), parity);
-                    });
                 }
                 // where the lanes' chunks lie for this matrix's format: 16 bytes apart in its own order, else in two runs
                 const bool own = q6 == (p.q6 != 0);
@@ -407,6 +403,9 @@ narrow_mma_kernel(const __grid_constant__ NmParams p) {
             }
         }
     }
+    if constexpr (BLOCKS)
+        if (given_up != 0 && lane == 0)   // what is under way lands before the CTA is gone (lane 0 asks for all copies)
+            NarrowRing::drain(n_stages, given_up, [&](int at, uint32_t parity) { nm_wait_full(nm_smem(&full[warp][at]), parity); });
 }
 
 size_t nm_smem_bytes(NarrowFormat format, bool q6, int T, int64_t share_cols) {

@@ -31,16 +31,20 @@ struct NarrowRing {
             ++stage;
         }
     }
-    // The wait for the present stage was in vain, `left` copies (that one included, the later ones asked for or not) before the end: nothing more is asked
-    // for, and wait(stage, parity) is called for every copy that is under way.  Only those: a stage that was not asked for again has a phase
-    // that never completes.
-    template <typename Wait>
-    MK_RING void give_up(int left, Wait wait) {
+    // The wait for the present stage was in vain, `left` copies (that one included, the later ones asked for or not) before the last: nothing more is asked
+    // for.  Returns what drain() is to be given, never 0.
+    MK_RING uint32_t give_up(int left) {
         to_load = 0;
-        for (int j = 0; j < (left < stages ? left : stages); ++j) {
-            const int at = stage + j;
-            if (at < stages) wait(at, phase);
-            else wait(at - stages, phase ^ 1);
+        return (uint32_t)(left < stages ? left : stages) | (uint32_t)stage << 8 | phase << 16;
+    }
+    // wait(stage, parity) for every copy that was under way when the ring was given up.  Only those: a stage that was not asked for again has a phase that
+    // never completes.
+    template <typename Wait>
+    static MK_RING void drain(int stages, uint32_t given_up, Wait wait) {
+#pragma unroll 1
+        for (int j = 0; j < (int)(given_up & 255); ++j) {
+            const int at = (int)(given_up >> 8 & 255) + j;
+            wait(at < stages ? at : at - stages, given_up >> 16 ^ (at < stages ? 0u : 1u));
         }
     }
 };

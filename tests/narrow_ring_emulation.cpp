@@ -41,21 +41,18 @@ extern "C" int emu_narrow_ring(int stages, int i0, int i1, int rg_shift, int sub
         ring.loaded();
     };
     for (int i = 0; i < stages - 1; ++i) copy_step();
-    bool ok = true;
+    uint32_t given_up = 0;
     int n = 0;
     for (int i = i0; i < i1; ++i)
         for (int st = a0; st < a1; ++st, ++n) {
             copy_step();
-            if (i < i0 + groups && ok) {
-                if (n != fails) {
-                    w.wait(ring.stage, ring.phase);
-                } else {
-                    ok = false;
-                    ring.give_up((i0 + groups - i) * (a1 - a0) - (st - a0), [&](int at, uint32_t parity) { w.wait(at, parity); });
-                }
+            if (i < i0 + groups && given_up == 0) {
+                if (n != fails) w.wait(ring.stage, ring.phase);
+                else given_up = ring.give_up((i0 + groups - i) * (a1 - a0) - (st - a0));
             }
             ring.used();
         }
+    if (given_up != 0) mk::NarrowRing::drain(stages, given_up, [&](int at, uint32_t parity) { w.wait(at, parity); });
     for (const Barrier& b : w.bars) wrong += b.armed;
     return wrong + w.wrong;
 }
