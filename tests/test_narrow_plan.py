@@ -20,6 +20,11 @@ def test_calls_that_are_taken(env):
     assert image(2048, 2080, 4) is None and blocks(2048, 2112, 4) is None        # no whole steps of K
     assert blocks(2048, 11008, 8) and blocks(2048, 11008, 9) is None
     assert blocks(16384, 2048, 1) and blocks(16512, 2048, 1) is None             # 32 M weights
+    # gated: by how many SMs the other kernel's whole row tiles keep busy, as measured: 59, 58, 65, 76 and 100 %
+    shapes = ((11264, 2048), (22016, 2048), (24576, 4096), (28672, 3584), (75776, 2048))
+    for kind, T, taken in ((capi.TYPE_Q4_K, 1, 3), (capi.TYPE_Q4_K, 2, 3), (capi.TYPE_Q4_K, 3, 2), (capi.TYPE_Q4_K, 8, 2), (capi.TYPE_Q6_K, 4, 5), (capi.TYPE_Q6_K, 5, 3),
+                           (capi.TYPE_Q6_K, 8, 3), (capi.TYPE_Q4_K, 9, 0), (capi.TYPE_Q6_K, 9, 0)):
+        assert [ops.narrow_matmul_plan(capi.PATH_STREAM, kind, *s, T, gated=True) is not None for s in shapes] == [i < taken for i in range(5)], (kind, T)
     with pytest.raises(capi.MkError, match="Q4_K and Q6_K"):
         ops.narrow_matmul_plan(capi.PATH_STREAM, capi.TYPE_Q8_0, 2048, 2048, 1)
     with pytest.raises(capi.MkError, match="planned on the host"):
