@@ -485,6 +485,15 @@ __global__ void __launch_bounds__(128) head_norm_gate_vec_kernel(LinearStateArgs
         for (int c = a.heads * a.vdim + (int)(threadIdx.x % G); c < a.image.end(); c += G) a.image.put(row, c, 0.f);
 }
 
+// The most shared memory that leaves room for n such CTAs on an SM, and not for one more: it is given out in pieces of 128 bytes, and each CTA takes another
+// 1024 of the SM's 228 KB.
+constexpr size_t shared_of_one_in(int n) { return (size_t)(228 * 1024 / n / 128 * 128 - 1024); }
+constexpr bool shared_fits(int n) {
+    const size_t taken = (shared_of_one_in(n) + 127) / 128 * 128 + 1024;
+    return n * taken <= 228 * 1024 && (n + 1) * taken > 228 * 1024;
+}
+static_assert(shared_fits(1) && shared_fits(2) && shared_fits(3) && shared_fits(4) && shared_fits(5) && shared_fits(6));
+
 template <int KD, LsRule RULE, bool FINISH>
 void launch_variant(const typename LsArgs<RULE>::type& ra, cudaStream_t s) {
     const LinearStateArgs& a = ra.common;
@@ -499,8 +508,10 @@ void launch_variant(const typename LsArgs<RULE>::type& ra, cudaStream_t s) {
         // As much shared memory as leaves no SM more CTAs than an even share: they start under the kernel before, wherever it leaves room, and a
         // launch takes as long as its fullest SM.  Rows of 128 x 128 heads, one lane: 16 heads 0.29 -> 0.20 us each, 32 heads 0.37 -> 0.26, 64 heads
         // level at 0.38; a prompt tick of three to five lanes 324 -> 303 us.  The other rules, with half as many steps in a row's chain, gain nothing.
+        // More than four CTAs do not fit an SM's registers (98 to 123 a thread; 183 with 256 columns, which is two).
+        constexpr int RESIDENT = KD == 256 ? 2 : 4;
         const int64_t sms = device_sm_count(), share = ((int64_t)grid.x * grid.y * grid.z + sms - 1) / sms;
-        if (share <= 6) smem = std::max(smem, (size_t)(228 * 1024 / share - 1024));
+        if (share <= RESIDENT) smem = std::max(smem, shared_of_one_in((int)share));
     }
     ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     launch_pdl(kernel, grid, dim3((unsigned)warps * 32), smem, s, ra);
