@@ -596,6 +596,11 @@ int32_t mk_k_quantize(int32_t act_kind, const float* x, int32_t T, int32_t K, in
 int32_t mk_k_add_norm(float* h, const float* a, float a_scale, const float* post_w, const float* norm_w, float eps, int32_t rows,
                       int32_t dim, float* normed_out);
 
+/* The same with what the next matmul reads: the quantised rows (as mk_k_quantize) and xh [rows][dim], their values as f16; dim a multiple of 256.
+ * half_only: the blocks need not be written, and where they are not, qs, d and bsums come back as they were. */
+int32_t mk_k_add_norm_quant(float* h, const float* a, float a_scale, const float* post_w, const float* norm_w, float eps, int32_t rows, int32_t dim,
+                            int32_t act_kind, int32_t half_only, int8_t* qs, float* d, int16_t* bsums, uint16_t* xh);
+
 /* LinearOp::forward for a quantised matrix (src/model_weights.rs:346-377): y [T][rows] = x [T][cols] . W^T,
  * W given as GGUF block bytes of `type`. */
 int32_t mk_k_qmatmul(int32_t type, const void* w, int64_t rows, int64_t cols, const float* x, int32_t T, float* y, int32_t path);

@@ -245,6 +245,7 @@ SIGNATURES = {
     "mk_unpermute_qk_rows": (_i32, [C.c_void_p, _i64, _i64, _i32, C.c_void_p]),
     "mk_k_quantize": (_i32, [_i32, P, _i32, _i32, P, P, P]),
     "mk_k_add_norm": (_i32, [P, P, _f32, P, P, _f32, _i32, _i32, P]),
+    "mk_k_add_norm_quant": (_i32, [P, P, _f32, P, P, _f32, _i32, _i32, _i32, _i32, P, P, P, P]),
     "mk_k_qmatmul": (_i32, [_i32, P, _i64, _i64, P, _i32, P, _i32]),
     "mk_k_qmatmul_time": (_i32, [_i32, P, _i64, _i64, P, _i32, _i32, _i32, C.POINTER(_f32)]),
     "mk_k_q4k_matmul_tc_noalloc_dev": (_i32, [P, _i64, _i64, P, _i32, P, P]),

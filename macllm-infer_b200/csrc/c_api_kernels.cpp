@@ -91,6 +91,43 @@ int32_t mk_k_add_norm(float* h, const float* a, float a_scale, const float* post
     });
 }
 
+int32_t mk_k_add_norm_quant(float* h, const float* a, float a_scale, const float* post_w, const float* norm_w, float eps, int32_t rows, int32_t dim,
+                            int32_t act_kind, int32_t half_only, int8_t* qs, float* d, int16_t* bsums, uint16_t* xh) {
+    return guarded([&] {
+        require_device();
+        if (rows <= 0 || dim <= 0 || dim % 256 != 0 || h == nullptr || qs == nullptr || d == nullptr || bsums == nullptr || xh == nullptr)
+            throw std::runtime_error("mk_k_add_norm_quant: rows of a multiple of 256 values, and buffers for all that is made of them");
+        const size_t n = (size_t)rows * dim, nd = n / (act_kind == ACT_Q8K ? 256 : 32);
+        DevBuf dh(n * 4), da, dpw, dnw;
+        dh.upload(h, n * 4);
+        NormQuantArgs na;
+        na.h = dh.as<float>();
+        if (a) { da.alloc(n * 4); da.upload(a, n * 4); na.a = da.as<float>(); }
+        if (post_w) { dpw.alloc((size_t)dim * 4); dpw.upload(post_w, (size_t)dim * 4); na.post_w = dpw.as<float>(); }
+        if (norm_w) { dnw.alloc((size_t)dim * 4); dnw.upload(norm_w, (size_t)dim * 4); na.norm_w = dnw.as<float>(); }
+        na.a_scale = a_scale;
+        na.eps = eps;
+        na.rows = rows;
+        na.dim = dim;
+        na.act_kind = act_kind;
+        na.half_only = half_only != 0;
+        ActBufs ab;
+        na.out = ab.view(rows, dim, act_kind, true);
+        // what is not written keeps what the caller had there
+        ab.qs.upload(qs, n);
+        ab.d.upload(d, nd * 4);
+        ab.bs.upload(bsums, n / 16 * 2);
+        launch_add_norm_quant(na, nullptr);
+        MK_CUDA(cudaDeviceSynchronize());
+        dh.download(h, n * 4);
+        ab.qs.download(qs, n);
+        ab.d.download(d, nd * 4);
+        ab.bs.download(bsums, n / 16 * 2);
+        ab.xh.download(xh, n * 2);
+        MK_CUDA(cudaDeviceSynchronize());
+    });
+}
+
 namespace {
 
 // Shared body of mk_k_qmatmul and mk_k_qmatmul_time: upload, quantise the activations once, then run the

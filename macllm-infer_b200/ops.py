@@ -72,6 +72,21 @@ def add_norm(h, a=None, a_scale=1.0, post_w=None, norm_w=None, eps=1e-5):
     return h, out
 
 
+def add_norm_quant(h, a=None, a_scale=1.0, post_w=None, norm_w=None, eps=1e-5, act_kind: int = 0, half_only: bool = False, fill: int = 0):
+    """Returns (updated residual, quantised rows, block factors, sums of sixteen, f16 image); what is not written is left at `fill`."""
+    h = _f32(h).copy()
+    rows, dim = h.shape
+    a = None if a is None else _f32(a)
+    post_w = None if post_w is None else _f32(post_w)
+    norm_w = None if norm_w is None else _f32(norm_w)
+    qs = np.full((rows, dim), fill, dtype=np.int8)
+    d = np.full((rows, dim // (256 if act_kind == 0 else 32)), fill, dtype=np.float32)
+    bs = np.full((rows, dim // 16), fill, dtype=np.int16)
+    xh = np.empty((rows, dim), dtype=np.float16)
+    capi.check(capi.lib().mk_k_add_norm_quant(_p(h), _p(a), a_scale, _p(post_w), _p(norm_w), eps, rows, dim, act_kind, 1 if half_only else 0, _p(qs), _p(d), _p(bs), _p(xh)))
+    return h, qs, d, bs, xh
+
+
 def qmatmul(qtype: int, w_bytes: np.ndarray, rows: int, cols: int, x: np.ndarray, path: int = capi.PATH_AUTO) -> np.ndarray:
     x = _f32(x)
     T = x.shape[0]
