@@ -611,6 +611,19 @@ int32_t mk_k_qmatmul(int32_t type, const void* w, int64_t rows, int64_t cols, co
 int32_t mk_k_qmatmul_time(int32_t type, const void* w, int64_t rows, int64_t cols, const float* x, int32_t T, int32_t path,
                           int32_t iters, float* avg_ms);
 
+/* Two matrices in one launch of the streamed matmul, as the decode ticks have them, T <= 64 rows.  act < 0: the stacked product y [T][rows + rows2], Q4_K and
+ * Q6_K in any order, rows a multiple of 128 (q | k beside v).  act 0 SiLU / 1 tanh GELU: w the gate and w2 the up matrix, both Q4_K of `rows` rows,
+ * y [T][rows] = act(gate . x) * (up . x), rounded through f16. */
+int32_t mk_k_stacked_qmatmul(int32_t type, const void* w, int64_t rows, int32_t type2, const void* w2, int64_t rows2, int64_t cols, const float* x, int32_t T,
+                             int32_t act, float* y);
+/* The matmul of mixer-built decoders: w [rows][cols] and x are rounded to bf16, cols a multiple of 64.  groups > 1: stacked projections of group_rows[g]
+ * rows (multiples of 128), each with an input of its own, x [groups][T][cols].  part_rows 0: y [T][rows].  part_rows > 0: the result scattered - of
+ * every part_rows rows the first part_valid are kept, value (t, part p, i) goes to y [row_map ? row_map[t] : t][p * part_valid + i], times
+ * sigmoid(the sum over gate_n of gate [gate_n][rows of y][columns of y]) where gate is given; rows from rest_from on (a multiple of 32) go to rest [T][rows - rest_from]
+ * instead where rest is given. */
+int32_t mk_k_bf16_matmul(const float* w, int64_t rows, int64_t cols, const int64_t* group_rows, int32_t groups, const float* x, int32_t T, int32_t part_rows,
+                         int32_t part_valid, const int32_t* row_map, int64_t rest_from, const float* gate, int32_t gate_n, float* y, float* rest);
+
 /* Allocation-free tensor-core matmul for Q4_K weights.  This entry point has no counterpart in the
  * reference; it exists for hosts that may not allocate GPU memory on the request path - a serving
  * process that owns the whole device arena and forbids cudaMalloc there, or a sandboxed plugin whose

@@ -248,6 +248,8 @@ SIGNATURES = {
     "mk_k_add_norm_quant": (_i32, [P, P, _f32, P, P, _f32, _i32, _i32, _i32, _i32, P, P, P, P]),
     "mk_k_qmatmul": (_i32, [_i32, P, _i64, _i64, P, _i32, P, _i32]),
     "mk_k_qmatmul_time": (_i32, [_i32, P, _i64, _i64, P, _i32, _i32, _i32, C.POINTER(_f32)]),
+    "mk_k_stacked_qmatmul": (_i32, [_i32, P, _i64, _i32, P, _i64, _i64, P, _i32, _i32, P]),
+    "mk_k_bf16_matmul": (_i32, [P, _i64, _i64, P, _i32, P, _i32, _i32, _i32, P, _i64, P, _i32, P, P]),
     "mk_k_q4k_matmul_tc_noalloc_dev": (_i32, [P, _i64, _i64, P, _i32, P, P]),
     "mk_k_embed": (_i32, [_i32, P, _i64, _i64, P, _i32, _f32, P]),
     "mk_k_actmul": (_i32, [P, P, _i32, _i32, _i32, P]),

@@ -271,6 +271,150 @@ int32_t mk_k_qmatmul_time(int32_t type, const void* w, int64_t rows, int64_t col
     });
 }
 
+namespace {
+
+// The rows y of a matmul, or where it left K shares, those added in share order.
+void read_matmul(float* out, int shares, const DevBuf& partial, const DevBuf& y, size_t n) {
+    std::vector<float> parts((size_t)shares * n);
+    (shares > 1 ? partial : y).download(parts.data(), parts.size() * 4);
+    MK_CUDA(cudaDeviceSynchronize());
+    for (size_t i = 0; i < n; ++i) {
+        float v = parts[i];
+        for (int s = 1; s < shares; ++s) v += parts[(size_t)s * n + i];
+        out[i] = v;
+    }
+}
+
+void require_no_status(const DevBuf& status) {
+    int32_t st = 0;
+    status.download(&st, 4);
+    MK_CUDA(cudaDeviceSynchronize());
+    if (st != 0) throw std::runtime_error("tensor-core matmul: a bounded wait inside the kernel gave up (status " + std::to_string(st) + ")");
+}
+
+}  // namespace
+
+int32_t mk_k_stacked_qmatmul(int32_t type, const void* w, int64_t rows, int32_t type2, const void* w2, int64_t rows2, int64_t cols, const float* x, int32_t T,
+                             int32_t act, float* y) {
+    return guarded([&] {
+        require_device();
+        const bool gated = act >= 0;
+        auto block_format = [](int32_t t) { return t == MK_TYPE_Q4_K || t == MK_TYPE_Q6_K; };
+        if (!block_format(type) || !block_format(type2) || T < 1 || T > kQStreamMaxRows || rows < 1 || rows2 < 1 || act > 1)
+            throw std::runtime_error("mk_k_stacked_qmatmul: Q4_K and Q6_K matrices and 1 to 64 rows");
+        if (gated && (type != MK_TYPE_Q4_K || type2 != MK_TYPE_Q4_K || rows != rows2)) throw std::runtime_error("mk_k_stacked_qmatmul: gate and up are Q4_K matrices of as many rows");
+        DeviceWeight a, b;
+        QStreamWeight qa, qb;
+        auto retile = [&](int32_t t, const void* src, int64_t n, DeviceWeight& d, QStreamWeight& q) {
+            upload_weight(t, src, n, cols, d);
+            if (t == MK_TYPE_Q4_K) build_qstream_weight(d.w.p0, n, cols, q, nullptr);
+            else build_qstream_weight_q6k(d.w, q, nullptr);
+        };
+        if (gated) {
+            const size_t bytes = (size_t)rows * (size_t)(cols / 256) * 144;
+            std::vector<uint8_t> both(2 * bytes);
+            memcpy(both.data(), w, bytes);
+            memcpy(both.data() + bytes, w2, bytes);
+            upload_weight(type, both.data(), 2 * rows, cols, a);
+            build_qstream_weight(a.w.p0, 2 * rows, cols, qa, nullptr, rows);
+        } else {
+            retile(type, w, rows, a, qa);
+            retile(type2, w2, rows2, b, qb);
+        }
+        const size_t n = (size_t)T * (size_t)(gated ? rows : rows + rows2);
+        DevBuf dx((size_t)T * cols * 4), dy(n * 4), partial(kSplitScratchBytes), status(4);
+        dx.upload(x, (size_t)T * cols * 4);
+        status.zero(nullptr);
+        ActBufs ab;
+        const ActQ xa = ab.view(T, (int)cols, ACT_Q8K, true);
+        NormQuantArgs na;
+        na.h = dx.as<float>();
+        na.rows = T;
+        na.dim = (int)cols;
+        na.act_kind = ACT_Q8K;
+        na.out = xa;
+        launch_add_norm_quant(na, nullptr);
+        if (!gated) {
+            const int shares = launch_qstream_tc(qa, xa.xh, T, dy.as<float>(), (int)(rows + rows2), partial.as<float>(), partial.size() / 4, status.as<int32_t>(), nullptr, 16, &qb);
+            require_no_status(status);
+            read_matmul(y, shares, partial, dy, n);
+            return;
+        }
+        launch_qstream_tc(qa, xa.xh, T, nullptr, 0, nullptr, 0, status.as<int32_t>(), nullptr, 1, nullptr, act, dy.as<__half>(), (int)rows);
+        require_no_status(status);
+        std::vector<uint16_t> h(n);
+        dy.download(h.data(), n * 2);
+        MK_CUDA(cudaDeviceSynchronize());
+        for (size_t i = 0; i < n; ++i) y[i] = __half2float(__ushort_as_half(h[i]));
+    });
+}
+
+int32_t mk_k_bf16_matmul(const float* w, int64_t rows, int64_t cols, const int64_t* group_rows, int32_t groups, const float* x, int32_t T, int32_t part_rows,
+                         int32_t part_valid, const int32_t* row_map, int64_t rest_from, const float* gate, int32_t gate_n, float* y, float* rest) {
+    return guarded([&] {
+        require_device();
+        if (rows < 1 || cols < 64 || cols % 64 != 0 || T < 1 || groups < 1 || (groups > 1 && group_rows == nullptr)) throw std::runtime_error("mk_k_bf16_matmul: rows of a multiple of 64 values");
+        const bool scattered = part_rows > 0;
+        const int64_t kept = rest != nullptr ? rest_from : rows;
+        if (scattered && (part_valid < 1 || part_valid > part_rows || kept % part_rows != 0 || kept > rows || (rest != nullptr && (rest_from % 32 != 0 || rest_from == rows)) ||
+                          (gate != nullptr && gate_n < 1)))
+            throw std::runtime_error("mk_k_bf16_matmul: whole parts, and the rest from a multiple of 32 on");
+        if (scattered && row_map != nullptr)
+            for (int32_t t = 0; t < T; ++t)
+                if (row_map[t] < 0 || row_map[t] >= T) throw std::runtime_error("mk_k_bf16_matmul: row map out of range");
+        HalfWeight W;
+        build_bf16_weight(w, rows, cols, W, nullptr, groups > 1 ? std::vector<int64_t>(group_rows, group_rows + groups) : std::vector<int64_t>());
+        const size_t nx = (size_t)groups * T * cols, ld = scattered ? (size_t)(kept / part_rows * part_valid) : (size_t)rows, n = (size_t)T * ld;
+        std::vector<__nv_bfloat16> xb(nx);
+        for (size_t i = 0; i < nx; ++i) xb[i] = __float2bfloat16_rn(x[i]);
+        DevBuf dx(nx * 2), dy(n * 4), partial(kSplitScratchBytes), status(4), map, dg, dr;
+        dx.upload(xb.data(), nx * 2);
+        dy.zero(nullptr);
+        status.zero(nullptr);
+        HgemmScratch hs;
+        hs.status = status.as<int32_t>();
+        hs.partial = partial.as<float>();
+        hs.partial_floats = partial.size() / 4;
+        if (!scattered) {
+            const int shares = launch_hgemm_tc(W, dx.as<__half>(), T, dy.as<float>(), (int)rows, 1.f, 0.f, hs, nullptr, 16);
+            require_no_status(status);
+            read_matmul(y, shares, partial, dy, n);
+            return;
+        }
+        MatmulScatter to;
+        to.out = dy.ptr();
+        to.part_rows = part_rows;
+        to.part_valid = part_valid;
+        to.ld_part = part_valid;
+        to.ld_row = (int64_t)ld;
+        if (row_map != nullptr) {
+            map.alloc((size_t)T * 4);
+            map.upload(row_map, (size_t)T * 4);
+            to.row_map = map.as<int32_t>();
+        }
+        if (gate != nullptr) {
+            dg.alloc((size_t)gate_n * n * 4);
+            dg.upload(gate, (size_t)gate_n * n * 4);
+            to.gate = dg.as<float>();
+            to.gate_n = gate_n;
+            to.gate_ld = (int)ld;
+            to.gate_stride = (int64_t)n;
+        }
+        const size_t nr = (size_t)T * (size_t)(rows - kept);
+        if (rest != nullptr) {
+            dr.alloc(nr * 4);
+            to.rest = dr.as<float>();
+            to.rest_from = (int)rest_from;
+            to.ld_rest = rows - kept;
+        }
+        launch_hgemm_tc_scatter(W, dx.as<__half>(), T, to, hs, nullptr);
+        require_no_status(status);
+        read_matmul(y, 1, partial, dy, n);
+        if (rest != nullptr) dr.download(rest, nr * 4);
+        MK_CUDA(cudaDeviceSynchronize());
+    });
+}
+
 int32_t mk_k_embed(int32_t type, const void* w, int64_t rows, int64_t cols, const uint32_t* ids, int32_t T, float scale,
                    float* out) {
     return guarded([&] {

@@ -105,6 +105,39 @@ def qmatmul_time(qtype: int, w_bytes: np.ndarray, rows: int, cols: int, x: np.nd
     return float(ms.value)
 
 
+def stacked_qmatmul(qtype: int, w_bytes, rows: int, qtype2: int, w2_bytes, rows2: int, cols: int, x, act: int = -1) -> np.ndarray:
+    """Two block matrices in one launch: x @ [w; w2].T, or with act 0 / 1 f16(act(x @ w.T) * (x @ w2.T)) as f32."""
+    x = _f32(x)
+    w_bytes, w2_bytes = np.ascontiguousarray(w_bytes), np.ascontiguousarray(w2_bytes)
+    y = np.empty((x.shape[0], rows if act >= 0 else rows + rows2), dtype=np.float32)
+    capi.check(capi.lib().mk_k_stacked_qmatmul(qtype, _p(w_bytes), rows, qtype2, _p(w2_bytes), rows2, cols, _p(x), x.shape[0], act, _p(y)))
+    return y
+
+
+def bf16_matmul(w, x, group_rows=None) -> np.ndarray:
+    """x @ w.T of bf16 operands; group_rows: stacked projections, x [groups, T, cols] has an input for each."""
+    w, x = _f32(w), _f32(x)
+    groups = 1 if group_rows is None else len(group_rows)
+    sizes = None if group_rows is None else np.ascontiguousarray(group_rows, dtype=np.int64)
+    T = x.shape[-2]
+    y = np.empty((T, w.shape[0]), dtype=np.float32)
+    capi.check(capi.lib().mk_k_bf16_matmul(_p(w), w.shape[0], w.shape[1], _p(sizes), groups, _p(x), T, 0, 0, None, 0, None, 0, _p(y), None))
+    return y
+
+
+def bf16_matmul_scattered(w, x, part_rows: int, part_valid: int, row_map=None, rest_from: int | None = None, gate=None):
+    """The same scattered: (kept columns of every part by destination row, rows from rest_from on or None)."""
+    w, x = _f32(w), _f32(x)
+    T, kept = x.shape[0], w.shape[0] if rest_from is None else rest_from
+    row_map = None if row_map is None else np.ascontiguousarray(row_map, dtype=np.int32)
+    gate = None if gate is None else _f32(gate)
+    y = np.empty((T, kept // part_rows * part_valid), dtype=np.float32)
+    rest = None if rest_from is None else np.empty((T, w.shape[0] - rest_from), dtype=np.float32)
+    capi.check(capi.lib().mk_k_bf16_matmul(_p(w), w.shape[0], w.shape[1], None, 1, _p(x), T, part_rows, part_valid, _p(row_map), 0 if rest_from is None else rest_from,
+                                           _p(gate), 0 if gate is None else gate.shape[0], _p(y), _p(rest)))
+    return y, rest
+
+
 def embed(qtype: int, w_bytes: np.ndarray, rows: int, cols: int, ids, scale: float = 1.0) -> np.ndarray:
     ids = np.ascontiguousarray(ids, dtype=np.uint32)
     out = np.empty((len(ids), cols), dtype=np.float32)
