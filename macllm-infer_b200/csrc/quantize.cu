@@ -193,6 +193,8 @@ __global__ void add_inplace_kernel(float* h, const float* a, float scale, int64_
 
 // One CTA per row, NG groups of 256 per warp held in registers (dim <= 8 warps * NG * 256).
 // SHARED: the branch output comes in shares; the registers that several of them take on their way are spared otherwise.
+// A CTA per row at any number of rows: eight (four) of them on an SM hide each other's loads and barriers.  Half as many CTAs that walk several rows, the
+// next one's values on their way, took 13.9 us against 13.0 for 2048 rows of 2048 and 23.9 each of 3584; prompt ticks of 1200 and 4096 rows of 2048 were 1.5 % longer.
 template <int NG, bool SHARED>
 __global__ void __launch_bounds__(NQ_THREADS) add_norm_quant_fast_kernel(NormQuantArgs a) {
     __shared__ float red[32];
@@ -293,86 +295,6 @@ __global__ void __launch_bounds__(NQ_THREADS) add_norm_quant_fast_kernel(NormQua
     }
 }
 
-// The same on wide ticks: as many CTAs as fit, each with rows of its own one after the other, the next one's values on their way while this
-// one is summed, normed and quantised.  With a CTA per row an SM waited for loads, two barriers and a launch in turn (2048 rows of 2048: 18 us, 63 MB
-// through the L2).  The sums are added in the order of the kernel above.
-template <int NG>
-__global__ void __launch_bounds__(NQ_THREADS, NG == 1 ? 4 : 2) add_norm_quant_rows_kernel(NormQuantArgs a) {
-    __shared__ float red[2][NQ_THREADS / 32];
-    pdl_trigger();
-    const int dim = a.dim, groups = dim / 256;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float nw[NG][8], pw[NG][8], x[NG][8], y[NG][8];
-    bool live[NG];
-#pragma unroll
-    for (int g = 0; g < NG; ++g) {
-        const int grp = warp + g * 8;
-        live[g] = grp < groups;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) nw[g][i] = pw[g][i] = x[g][i] = y[g][i] = 0.f;
-        if (live[g]) load8(a.norm_w + grp * 256 + lane * 8, nw[g]);
-        if (live[g] && a.post_w != nullptr) load8(a.post_w + grp * 256 + lane * 8, pw[g]);
-    }
-    int buffer = 0;
-    auto row_sum = [&](float v) {
-        v = warp_sum(v);
-        if (lane == 0) red[buffer][warp] = v;
-        __syncthreads();
-        v = warp_sum(lane < NQ_THREADS / 32 ? red[buffer][lane] : 0.f);
-        buffer ^= 1;
-        return v;
-    };
-    pdl_wait();
-    auto fetch = [&](int r) {
-#pragma unroll
-        for (int g = 0; g < NG; ++g)
-            if (live[g]) {
-                const int64_t at = (int64_t)r * dim + (warp + g * 8) * 256 + lane * 8;
-                load8(a.h + at, x[g]);
-                load8(a.a + at, y[g]);
-            }
-    };
-    int r = blockIdx.x;
-    if (r < a.rows) fetch(r);
-    for (; r < a.rows; r += gridDim.x) {
-        float v[NG][8];
-        float post_m = 1.f;
-        if (a.post_w != nullptr) {
-            float ss = 0.f;
-#pragma unroll
-            for (int g = 0; g < NG; ++g)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) ss += y[g][i] * y[g][i];
-            post_m = sqrtf(row_sum(ss) / (float)dim + a.eps);
-        }
-        float ss = 0.f;
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-            if (a.post_w != nullptr) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) y[g][i] = y[g][i] / post_m * pw[g][i];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[g][i] = x[g][i] + y[g][i] * a.a_scale;
-                ss += v[g][i] * v[g][i];
-            }
-            if (live[g]) store8(a.h + (int64_t)r * dim + (warp + g * 8) * 256 + lane * 8, v[g]);
-        }
-        if (r + (int)gridDim.x < a.rows) fetch(r + gridDim.x);
-        const float m = sqrtf(row_sum(ss) / (float)dim + a.eps);
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-            if (!live[g]) continue;  // uniform per warp
-            const int grp = warp + g * 8;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[g][i] = v[g][i] / m * nw[g][i];
-            if (a.normed_out != nullptr) store8(a.normed_out + (int64_t)r * dim + grp * 256 + lane * 8, v[g]);
-            quant_group(v[g], lane, a.act_kind, a.out, r, dim, grp, a.half_only);
-        }
-    }
-}
-
 // Rows that need no row-wide statistic: one warp per (row, 256-value group), any number of rows.
 __global__ void __launch_bounds__(NQ_THREADS) quant_groups_kernel(const float* x, int ld, int rows, int dim, int kind, ActQ out) {
     const int groups = dim / 256;
@@ -426,15 +348,6 @@ void launch_add_norm_quant(const NormQuantArgs& a, cudaStream_t s) {
         launch_pdl(quant_groups_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(NQ_THREADS), 0, s, (const float*)a.h, a.dim, a.rows, a.dim, a.act_kind, a.out);
         MK_LAUNCH_CHECK();
         return;
-    }
-    if (vec_ok && a.dim <= 8 * 2 * 256 && a.a != nullptr && a.a_splits == 1 && a.norm_w != nullptr && a.row_index == nullptr) {
-        // several rows per CTA: from two rounds of CTAs on
-        const int ng = (a.dim / 256 + 7) / 8, ctas = device_sm_count() * (ng == 1 ? 4 : 2);
-        if (a.rows >= 2 * ctas) {
-            launch_pdl(ng == 1 ? add_norm_quant_rows_kernel<1> : add_norm_quant_rows_kernel<2>, dim3(ctas), dim3(NQ_THREADS), 0, s, a);
-            MK_LAUNCH_CHECK();
-            return;
-        }
     }
     if (vec_ok && a.dim <= 8 * 4 * 256) {
         int ng = (a.dim / 256 + 7) / 8;

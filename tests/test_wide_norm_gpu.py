@@ -1,5 +1,5 @@
-"""Residual add and norm of wide ticks, several rows per CTA: the bits of the kernel that gives every row a CTA, for rows that do not share out evenly over the
-CTAs and widths that leave some warps without a group."""
+"""Residual add and norm of wide ticks: the bits of narrow calls, for rows that do not share out evenly over the SMs and widths that leave some
+warps without a group."""
 import importlib
 
 import numpy as np
@@ -40,7 +40,7 @@ def test_quantised_rows_equal_those_of_narrow_calls(mk, rows, dim, kind):
     assert np.array_equal(whole[1], qs) and np.array_equal(whole[2], d) and (kind == 1 or np.array_equal(whole[3], bs))
     f16 = (d.repeat(256 if kind == 0 else 32, axis=1) * qs).astype(np.float16)
     assert np.array_equal(whole[4], f16)
-    for lo, hi in ((0, rows), (0, 500)):   # several rows per CTA, and a CTA per row
+    for lo, hi in ((0, rows), (0, 500)):
         h1, qs, d, bs, xh = ops.add_norm_quant(h[lo:hi], a[lo:hi], 1.0, None, w, 1e-6, kind, half_only=True, fill=77)
         assert np.array_equal(xh, whole[4][lo:hi]) and np.array_equal(h1, whole[0][lo:hi])
         assert (qs == 77).all() and (d == 77).all() and (bs == 77).all()
