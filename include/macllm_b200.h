@@ -732,7 +732,7 @@ int32_t mk_k_matmul_plan(int32_t path, int64_t rows, int64_t cols, int32_t T, in
  * borders lie inside pairs of row tiles, so that every tile stays on one CTA. */
 int32_t mk_k_half_matmul_plan(int64_t rows, int64_t cols, int32_t T, int32_t max_splits, int64_t scratch_floats, int32_t may_pair, int64_t* out8);
 /* Host-only: the cut of calls of so few rows that warps stream their own weights.  path MK_PATH_HALF (16-bit images; type is not read) or MK_PATH_STREAM
- * (Q4_K / Q6_K); gated: rows interleaved gate / up, finished in the launch (no shares); scratch_floats: room for partial sums (negative: any).  out = {1 when the
+ * (Q4_K / Q6_K); gated: rows interleaved gate / up (blocks: Q4_K), finished in the launch (no shares); scratch_floats: room for partial sums (negative: any).  out = {1 when the
  * call is taken, else 0 and nothing else holds, 16-row tiles that a CTA takes at a time, K shares, CTAs, bytes of shared memory of a CTA, floats of partial sums}. */
 int32_t mk_k_narrow_matmul_plan(int32_t path, int32_t type, int64_t rows, int64_t cols, int32_t T, int32_t gated, int32_t max_splits, int64_t scratch_floats,
                                 int64_t* out6);

@@ -1197,6 +1197,7 @@ int32_t mk_k_narrow_matmul_plan(int32_t path, int32_t type, int64_t rows, int64_
         if (path != MK_PATH_HALF && path != MK_PATH_STREAM) throw std::runtime_error("mk_k_narrow_matmul_plan: only the f16-image and the streamed path are planned on the host");
         const bool blocks = path == MK_PATH_STREAM;
         if (blocks && type != MK_TYPE_Q4_K && type != MK_TYPE_Q6_K) throw std::runtime_error("mk_k_narrow_matmul_plan: the streamed matmul covers Q4_K and Q6_K matrices");
+        if (blocks && gated != 0 && type != MK_TYPE_Q4_K) throw std::runtime_error("mk_k_narrow_matmul_plan: gate and up rows are interleaved in Q4_K only");
         const NarrowPlan p = narrow_plan(blocks ? NarrowFormat::Blocks : NarrowFormat::F16, blocks && type == MK_TYPE_Q6_K, rows, cols, T, gated != 0, max_splits,
                                          scratch_floats < 0 ? SIZE_MAX : (size_t)scratch_floats, 1, kPlanSms);
         const int64_t v[6] = {p.ok ? 1 : 0, p.RG, p.shares, p.ctas, (int64_t)p.smem, (int64_t)p.partial_floats};

@@ -433,22 +433,21 @@ void launch_nm(const NmParams& p, const NarrowPlan& plan, cudaStream_t s) {
 // 16 628 / 764, 481 / 533, 599 / 622, 749 / 857, and with a head of 131072 rows at 16 still 693 / 703, 549 / 557, 670 / 680, 809 / 819.  32 tokens: 43 / 31.
 // Blocks: unpacking is a warp's own work here and sets the pace of long streams.  In ticks with the line at 20 M, 32 M and 64 M weights, one lane: 2048 wide
 // 403, 386 and 386, 4096 wide 690, 659 and 691, 3584 wide 678, 649 and 685; four lanes level.
-// Gated blocks: the kernel there leaves whole row tiles to its CTAs, so how much of the chip it uses follows from their number: 88 and 172 tiles keep
+// Gated blocks (Q4_K: no other format is interleaved): the kernel there leaves whole row tiles to its CTAs, so how much of the chip it uses follows from their number: 88 and 172 tiles keep
 // 59 % of the SMs busy on average, 192 keep 65, 224 keep 76.  Ticks of Q4_K models with these: 339 / 351, 386 / 402, 650 / 659, 685 / 653 at one
-// lane; 337 / 347, 395 / 410, 712 / 703, 715 / 694 at four; 364 / 362, 416 / 424, 744 / 716, 795 / 711 at eight.  Q6_K takes longer to unpack there too:
-// by itself at 65, 76 and 100 % 35 / 46, 38 / 42 and 43 / 47 at one token, 42 / 46, 47 / 42 and 53 / 47 at eight.
-static bool narrow_preferred(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, bool gated, int sms) {
+// lane; 337 / 347, 395 / 410, 712 / 703, 715 / 694 at four; 364 / 362, 416 / 424, 744 / 716, 795 / 711 at eight.
+static bool narrow_preferred(NarrowFormat format, int64_t rows, int64_t cols, int T, bool gated, int sms) {
     if (format != NarrowFormat::Blocks) return T <= kNarrowImageRows;
     if (T > kNarrowBlockRows) return false;
     if (!gated) return rows * cols <= (int64_t)32 << 20;
     const int64_t tiles = (rows + 127) / 128, most = (tiles + sms - 1) / sms, busy = 100 * tiles / (most * sms);
-    return q6 ? T <= 4 || busy <= 70 : busy <= (T <= 2 ? 70 : 62);
+    return busy <= (T <= 2 ? 70 : 62);
 }
 
 NarrowPlan narrow_plan(NarrowFormat format, bool q6, int64_t rows, int64_t cols, int T, bool gated, int max_shares, size_t scratch_floats, int n_inputs, int sms) {
     NarrowPlan best;
     const bool blocks = format == NarrowFormat::Blocks;
-    if (T <= 0 || cols % nm_step_cols(blocks) != 0 || !narrow_preferred(format, q6, rows, cols, T, gated, sms)) return best;
+    if (T <= 0 || cols % nm_step_cols(blocks) != 0 || !narrow_preferred(format, rows, cols, T, gated, sms)) return best;
     if (gated) max_shares = 1;   // its pairs of rows are finished by the CTA that has their sums
     const int64_t steps = cols / nm_step_cols(blocks), tiles = (rows + 15) / 16;
     // Microseconds of a step on one CTA of an SM (half as long again with two), of a meeting of the warps, of staging the activations and of adding
