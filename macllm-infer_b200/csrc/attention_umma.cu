@@ -18,6 +18,7 @@
 // 236 -> 53 us; 16 heads of 128 over 4, prompts of 32 - 1024 tokens: 70 -> 27 us.
 #include "attention_tc.h"
 #include "hgemm_tc.h"
+#include "tile_phases.h"
 #include "umma.cuh"
 #include <cuda.h>
 
@@ -70,7 +71,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     using L = Au<D, DV>;
     constexpr int ST = L::STAGES;
     extern __shared__ uint8_t au_smem[];
-    __shared__ uint64_t bars[4 * ST + 6];
+    __shared__ uint64_t bars[4 * ST + 7];
     __shared__ uint32_t tmem_slot;
     uint64_t *k_full = bars, *k_empty = bars + ST, *v_full = bars + 2 * ST, *v_empty = bars + 3 * ST, *s_full = bars + 4 * ST, *p_full = s_full + 2, *q_full = s_full + 4,
              *o_done = s_full + 5;
@@ -89,9 +90,9 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         for (int i = 0; i < 2; ++i) {
             bar_init(&s_full[i], 1);
             bar_init(&p_full[i], AU_ITEMS);
+            bar_init(&o_done[i], 1);
         }
         bar_init(q_full, AU_ITEMS);
-        bar_init(o_done, 1);
         bar_init_fence();
     }
     if (warp == 5) tmem_alloc(&tmem_slot, L::TMEM);
@@ -163,15 +164,15 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             constexpr uint32_t i_scores = f16_idesc(AU_ITEMS, AU_KEYS, false), i_out = f16_idesc(AU_ITEMS, DV, true);
             const uint32_t q_addr = smem_u32(qs), k_addr = smem_u32(ks), v_addr = smem_u32(vs);
             auto scores = [&](int t) {
-                const int st = t % ST;
+                const int st = t % ST, area = tile_phase(t).at;
                 if (!bar_wait(&k_full[st], t / ST & 1)) return false;
                 fence_after();
                 const uint64_t q = sw128_desc(q_addr), k = sw128_desc(k_addr + st * L::K_BYTES);
 #pragma unroll
                 for (int i = 0; i < D / 16; ++i)
-                    mma(tmem + DV + (t & 1) * AU_KEYS, q + (i >> 2) * (AU_QPANEL / 16) + (i & 3) * 2, k + (i >> 2) * (AU_PANEL / 16) + (i & 3) * 2, i_scores, i > 0);
+                    mma(tmem + DV + area * AU_KEYS, q + (i >> 2) * (AU_QPANEL / 16) + (i & 3) * 2, k + (i >> 2) * (AU_PANEL / 16) + (i & 3) * 2, i_scores, i > 0);
                 commit(&k_empty[st]);
-                commit(&s_full[t & 1]);
+                commit(&s_full[area]);
                 return true;
             };
             bool ok = bar_wait(q_full, 0);
@@ -182,10 +183,11 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 // thread run in the order of their issue
                 if (t + 1 < n_tiles) ok = scores(t + 1);
                 const int st = t % ST;
-                ok = ok && bar_wait(&v_full[st], t / ST & 1) && bar_wait(&p_full[t & 1], t >> 1 & 1);
+                const TilePhase ph = tile_phase(t);
+                ok = ok && bar_wait(&v_full[st], t / ST & 1) && bar_wait(&p_full[ph.at], ph.parity);
                 if (!ok) break;
                 fence_after();
-                const uint32_t p = tmem + DV + (t & 1) * AU_KEYS;
+                const uint32_t p = tmem + DV + ph.at * AU_KEYS;
                 const uint64_t v = sw128_desc(v_addr + st * L::V_BYTES, AU_PANEL);
 #pragma unroll
                 for (int i = 0; i < AU_KEYS / 16; ++i) {
@@ -193,7 +195,7 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     if constexpr (EXACT) mma_tmem_a(tmem, p + AU_KEYS / 2 + i * 8, v + i * 128, i_out, true);
                 }
                 commit(&v_empty[st]);
-                commit(o_done);
+                commit(&o_done[ph.at]);
             }
             if (!ok) atomicExch(a.status, 32);
         }
@@ -249,10 +251,11 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         float m_run = -INFINITY, sum = 0.f;
         bool ok = true;
         for (int t = 0; t < n_tiles; ++t) {
-            ok = __all_sync(0xffffffffu, bar_wait(&s_full[t & 1], t >> 1 & 1));
+            const TilePhase ph = tile_phase(t);
+            ok = __all_sync(0xffffffffu, bar_wait(&s_full[ph.at], ph.parity));
             if (!ok) break;
             fence_after();
-            const uint32_t s_at = my + DV + (t & 1) * AU_KEYS;
+            const uint32_t s_at = my + DV + ph.at * AU_KEYS;
             float s[AU_KEYS];
             tmem_ld32(s_at, reinterpret_cast<uint32_t*>(s));
             tmem_ld32(s_at + 32, reinterpret_cast<uint32_t*>(s) + 32);
@@ -278,7 +281,8 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 const float m_new = grow ? m_tile : m_run;
                 const float alpha = m_run == -INFINITY ? 1.0f : ex2(m_run - m_new);
                 if (t > 0) {
-                    ok = __all_sync(0xffffffffu, bar_wait(o_done, (t - 1) & 1));
+                    const TilePhase before = tile_phase(t - 1);
+                    ok = __all_sync(0xffffffffu, bar_wait(&o_done[before.at], before.parity));
                     if (!ok) break;
                     fence_after();
 #pragma unroll 1
@@ -322,9 +326,12 @@ attn_umma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             }
             tmem_wait_st();
             fence_before();
-            bar_arrive(&p_full[t & 1]);
+            bar_arrive(&p_full[ph.at]);
         }
-        if (ok) ok = __all_sync(0xffffffffu, bar_wait(o_done, (n_tiles - 1) & 1));
+        if (ok) {
+            const TilePhase last = tile_phase(n_tiles - 1);
+            ok = __all_sync(0xffffffffu, bar_wait(&o_done[last.at], last.parity));
+        }
         if (ok) {
             fence_after();
             float inv = 1.0f / sum;
